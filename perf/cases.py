@@ -218,3 +218,78 @@ def tolerance(case):
     if case["kind"] == "gemv" and case["x"] == "f32":
         return {"rel": 1e-6}
     return {"rel": 1e-3, "max": 0.04}
+
+
+# ---- the same results in 64 bits ---------------------------------------------------------------------------------
+
+E2M1_LEVELS = [0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0]
+UE4M3_LEVELS = [(b & 7) * 2.0 ** -9 if b < 8 else (8 + (b & 7)) * 2.0 ** ((b >> 3) - 10) for b in range(0x7f)]
+
+
+def _nearest(v, levels):
+    """The nearest of the ascending levels, the lower one of a tie."""
+    table = torch.tensor(levels, dtype=torch.float64, device=v.device)
+    return table[torch.bucketize(v.double(), (table[1:] + table[:-1]) / 2)]
+
+
+def _nvfp4(x, g=None):
+    """What NVFP4 codes of x stand for, in 64 bits; the quantiser's own steps are 32-bit by contract (scale of the tensor
+    amax / 2688, scale of a block amax / 6 over that as unsigned E4M3, ties down).  Divisors are tensors: a division by a
+    Python number would become a multiplication by its reciprocal."""
+    word = lambda v: torch.tensor(v, dtype=torch.float32, device=x.device)  # noqa: E731
+    x = x.float()
+    g = x.abs().max() / word(2688.0) if g is None else word(g)
+    out = torch.empty(x.shape, dtype=torch.float64, device=x.device)
+    for at in range(0, x.shape[0], 2048):
+        b = x[at: at + 2048].view(-1, x.shape[1] // 16, 16)
+        t = b.abs().amax(dim=2, keepdim=True) / word(6.0)
+        scale = _nearest((t / g).clamp_min(1e-8), UE4M3_LEVELS).float()
+        q = b / (scale.clamp_min(1e-8) * g)
+        out[at: at + 2048] = (_nearest(q.abs(), E2M1_LEVELS).copysign(q.double()) * (scale.double() * g.double())).view(-1, x.shape[1])
+    return out
+
+
+def _exact_weight(gen, n, k, outlier_rows=False):
+    w = torch.empty((n, k), device="cuda").normal_(0.0, 0.02, generator=gen)
+    if outlier_rows:
+        w[int(torch.randint(0, 128, (1,), generator=gen, device="cuda")):: 128] *= 8.0
+    return _nvfp4(w)
+
+
+def _silu_product(x, gate, up):
+    a = x @ gate.T
+    return a / (1.0 + torch.exp(-a)) * (x @ up.T)
+
+
+def exact(case, seed):
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    kind, m = case["kind"], case["m"]
+    if kind == "step":
+        parts = []
+        for n, k in _layer(case) * case["layers"]:
+            w = _exact_weight(gen, n, k)
+            parts.append((_activations(gen, m, k).double() @ w.T).reshape(-1))
+        return torch.cat(parts)
+    if kind == "gemv":
+        dtype = torch.float32 if case["x"] == "f32" else torch.bfloat16
+        x = _activations(gen, m, case["k"], dtype).double()
+        y = x @ _exact_weight(gen, case["n"], case["k"], True).T
+        return y[0] if case["x"] == "f32" else y
+    hidden, inter = case.get("hidden"), case.get("inter")
+    if kind == "decode_mlp":
+        gate, up, down = (_exact_weight(gen, *shape) for shape in ((inter, hidden), (inter, hidden), (hidden, inter)))
+        x, residual = _activations(gen, m, hidden).double(), _activations(gen, m, hidden).double()
+        h = _silu_product(x, gate, up)
+        # the intermediate activation is handed out, and read by the second projection, as BF16
+        return {"h": h, "y": h.to(torch.bfloat16).double() @ down.T + residual}
+    if kind == "prefill":
+        n, k = case["n"], case["k"]
+        x = _activations(gen, m, k, torch.float32 if case["x"] == "f32" else torch.bfloat16)
+        y = _nvfp4(x, 90.0 / 2688.0 if case["given_scale"] else None) @ _exact_weight(gen, n, k, True).T
+        return y + torch.randn((m, n), generator=gen, device="cuda").to(torch.bfloat16).double() if case["residual"] else y
+    x = _activations(gen, m, hidden)
+    gate, up, down = (_exact_weight(gen, *shape) for shape in ((inter, hidden), (inter, hidden), (hidden, inter)))
+    residual = torch.randn((m, hidden), generator=gen, device="cuda").to(torch.bfloat16).double()
+    h = _silu_product(_nvfp4(x), gate, up)
+    # the epilogue rounds the intermediate activation to BF16 before it quantises it
+    return _nvfp4(h.to(torch.bfloat16), 20.0 * (0.02 ** 2 * hidden * 1.4) / 2688.0) @ down.T + residual
