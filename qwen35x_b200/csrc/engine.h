@@ -76,11 +76,10 @@ struct q35b_weight {
   // batch_mutex (the only state of a weight that changes after q35b_weight_create*).
   struct q35b_gemv_batch * stream_batch[9] = {nullptr};
   std::mutex batch_mutex;
-  // Tensor maps of the GEMMs, encoded once at creation (build_weight_maps): B tiles of the 1-CTA kernel in its two
-  // widths, and the 2-CTA kernel's 96-row code boxes and 4-chunk scale boxes.
+  // Tensor maps of the GEMMs, encoded once at creation (build_weight_maps): 128-row code boxes of the
+  // one-CTA kernels, and the 2-CTA kernel's code boxes and 4-chunk scale boxes.
   bool has_maps = false;
   alignas(64) CUtensorMap tmap_codes_128;
-  alignas(64) CUtensorMap tmap_codes_256;
   alignas(64) CUtensorMap tmap2_codes;
   alignas(64) CUtensorMap tmap2_sf;
 };
@@ -146,12 +145,7 @@ int launch_gemm_w4a4(const q35b_weight * w, const uint8_t * a_codes, const uint8
                      cudaStream_t s, const GemmQuantOut * qout = nullptr, const GemmGather * gather = nullptr);
 
 
-// gemm_wstream.cu: weight-streaming projection for 1..128 operand rows (small-M prefill, tensor-core decode)
-bool gemm_wstream_eligible(const q35b_weight * w, int m);
-int launch_gemm_wstream(const q35b_weight * w, const uint8_t * a_codes, const uint8_t * a_scales_tiled, const float * g_dev,
-                        int m, void * c_bf16, int ldc, const void * residual_bf16, int ldr, unsigned int * status_dev,
-                        cudaStream_t s);
-
+// gemm_wstream.cu: decode work lists on the tensor cores
 struct WBatch;  // decode work list on the tensor path (digit-expanded activations)
 int wbatch_build(const q35b_gemv_item * items, int count, int m, int digits, WBatch ** out);
 int wbatch_launch(const WBatch * b, cudaStream_t s);

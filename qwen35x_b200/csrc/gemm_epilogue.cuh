@@ -137,6 +137,25 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
   return *reinterpret_cast<const uint32_t *>(&h);
 }
 
+// gate/up -> NVFP4: 32 accumulator columns (8 gate, 8 up, 8 gate, 8 up) of row `row` -> one block of 16 outputs.
+__device__ __forceinline__ void store_nvfp4_chunk32(const uint32_t (&r)[32], int row, int col0, float alpha, float alpha_up,
+                                                    const GemmEpilogue & ep, float q_g) {
+  float v[16];
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float gv = __uint_as_float(r[16 * j + i]) * alpha;
+      const float uv = __uint_as_float(r[16 * j + 8 + i]) * alpha_up;
+      v[8 * j + i] = __bfloat162float(__float2bfloat16_rn(silu_mul(gv, uv)));
+    }
+  }
+  uint2 packed;
+  const uint32_t sb = quantize_block<kEngine>(v, q_g, false, packed);
+  *reinterpret_cast<uint2 *>(ep.q_codes + static_cast<size_t>(row) * ep.q_ld + (col0 >> 2)) = packed;
+  ep.q_scales[tiled_scale_offset(row, ep.q_slot0 + (col0 >> 5), ep.q_slots)] = static_cast<uint8_t>(sb);
+}
+
 // r: 32 accumulator columns starting at global column col0 (a multiple of 32) of row `row`; n = accumulator columns
 // of the whole problem (weight rows); g = the activation tensor's scale.
 // to_peers: also repeat every store on the other ranks (one 32-byte piece per lane); a caller that forwards whole
@@ -152,21 +171,7 @@ __device__ __forceinline__ void gemm_store_chunk32(const uint32_t (&r)[32], int 
   if (ep.gate_up) {
     const float alpha_up = g * ep.s2_up;
     if (ep.q_codes != nullptr) {
-      // n % 32 == 0 is checked on the host, so the chunk is whole
-      float v[16];
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const float gv = __uint_as_float(r[16 * j + i]) * alpha;
-          const float uv = __uint_as_float(r[16 * j + 8 + i]) * alpha_up;
-          v[8 * j + i] = __bfloat162float(__float2bfloat16_rn(silu_mul(gv, uv)));
-        }
-      }
-      uint2 packed;
-      const uint32_t sb = quantize_block<kEngine>(v, q_g, false, packed);
-      *reinterpret_cast<uint2 *>(ep.q_codes + static_cast<size_t>(row) * ep.q_ld + (col0 >> 2)) = packed;
-      ep.q_scales[tiled_scale_offset(row, ep.q_slot0 + (col0 >> 5), ep.q_slots)] = static_cast<uint8_t>(sb);
+      store_nvfp4_chunk32(r, row, col0, alpha, alpha_up, ep, q_g);  // n % 32 == 0 is checked on the host: the chunk is whole
       return;
     }
     __nv_bfloat16 * dst = c + static_cast<size_t>(row) * ldc + (col0 >> 1);

@@ -430,7 +430,6 @@ int make_sf_map(CUtensorMap * map, const void * base, long long chunks) {
 int build_weight_maps(q35b_weight * w) {
   if (w->rows <= 0 || (w->k % 64) != 0) return Q35B_OK;  // such a weight never reaches a GEMM
   if (const int st = make_code_map(&w->tmap_codes_128, w->codes, w->rows, w->k / 2, 128)) return st;
-  if (const int st = make_code_map(&w->tmap_codes_256, w->codes, w->rows, w->k / 2, 256)) return st;
   if (const int st = make_code_map(&w->tmap2_codes, w->codes, w->rows, w->k / 2, kCtaBRows)) return st;
   const long long chunks = static_cast<long long>((w->rows + 127) / 128) * (w->k / 64);
   if (const int st = make_sf_map(&w->tmap2_sf, w->scales_tiled, chunks)) return st;

@@ -1,29 +1,34 @@
-// W4A4 prefill GEMM for sm_100a: C[M, N] (bf16) = (Aq . Wq^T) * g * s2 with
-// tcgen05.mma kind::mxf4nvf4 (block16, UE4M3 scale factors), TMEM accumulators,
-// TMA-fed shared-memory ring.
+// W4A4 prefill GEMM for sm_100a, weight rows on the 128-row side of the tensor-core tile, K split over a cluster:
+// C[M, N] (bf16) = (Aq . Wq^T) * g * s2 with tcgen05.mma kind::mxf4nvf4 (block16, UE4M3 scale factors), TMEM
+// accumulators, TMA-fed shared-memory ring.
 //
 // Replaces the reference's cuBLASLt FP4 call and the passes around it
 // (src/runtime/cuda_bench.cu:1056-1167 run_nvfp4_cublaslt_prefill_projection_device,
 // the fp32->bf16 pass at src/kernels/cuda/prefill.cu:639) and the SM120
-// mma.sync projection (src/runtime/cuda_bench.cu:431-484).
+// mma.sync projection (src/runtime/cuda_bench.cu:431-484) for problems too small to fill the chip with the
+// 256 x 256 tiles of gemm_w4a4_2cta.cu.
 //
 // Operands in HBM
-//   A codes  [M, K/2]  E2M1 pairs, K-major (activation quantiser output)
-//   B codes  [N, K/2]  E2M1 pairs, K-major (checkpoint order, untouched)
-//   SFA/SFB  128x4 tiles of 512 bytes (row-block major), one tile = the scale
+//   W codes  [N, K/2]  E2M1 pairs, K-major (checkpoint order, untouched)      -> UMMA A, 128 rows
+//   X codes  [M, K/2]  E2M1 pairs, K-major (activation quantiser output)      -> UMMA B, 16..128 tokens
+//   scales   128x4 tiles of 512 bytes (row-block major), one tile = the scale
 //            factors of a 128-row x 64-column operand slab = exactly the
 //            shared-memory image tcgen05.cp 32x128b.warpx4 copies to TMEM.
 //
-// One CTA computes a 128 x BLOCK_N output tile.  Per 256-element K step the
-// producer warp lands A (128 rows x 128 B, 128B-swizzled) and B (BLOCK_N rows)
-// by TMA and the two scale slabs by bulk copies; the MMA warp copies the scale
-// factors to TMEM and issues four K=64 MMAs; four epilogue warps read the fp32
-// accumulator from TMEM, scale by g*s2, convert to bf16 and store.
+// What bounds it: such a problem is a few megabytes of weights, about a microsecond of HBM, so what counts is how many
+// SMs pull them and how long the serial chain of K steps is.  One CTA per 128 x 128 tile leaves [2560, 9216] on 20 SMs
+// with 36 steps each.  Here `split` CTAs (1, 2, 4 or 8, a cluster) share a tile, each taking a contiguous part of its
+// K steps; they leave their fp32 accumulators in shared memory, meet at a cluster barrier, and every CTA adds up and
+// stores its share of the tokens, reading the others' partial sums over distributed shared memory in rank order (the
+// result does not depend on timing, and no workspace in HBM is needed).  The sums come back from shared memory with
+// lanes along the weight rows, so output rows are stored in whole 256-byte pieces, and rows that start at an odd
+// address still in 64-byte ones.
 //
 // Every mbarrier wait is bounded: on expiry the kernel writes a code to
-// *status, abandons the tile, still frees its TMEM and returns.
+// *status, abandons the tile, still meets its cluster, frees its TMEM and returns.
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "engine.h"
@@ -33,30 +38,26 @@
 namespace q35b {
 namespace {
 
-constexpr int kBlockM = 128;
-constexpr int kBlockKBytes = 128;        // one 128B swizzle row = 256 FP4 elements
+constexpr int kRows = 128;               // weight rows per tile (UMMA M)
+constexpr int kMaxCols = 128;            // tokens per tile (UMMA N, a multiple of 16)
+constexpr int kStepBytes = 128;          // one 128B swizzle row = 256 FP4 elements of K
 constexpr int kMmaPerStage = 4;          // four K=64 MMAs per stage
 constexpr int kSfChunk = 512;            // scale factors of 128 rows x 64 columns
-constexpr int kThreads = 192;            // warp 0 TMA, warp 1 MMA, warps 2..5 epilogue
+constexpr int kABytes = kRows * kStepBytes;
+constexpr int kSfBytes = kMmaPerStage * kSfChunk;
+constexpr int kThreads = 512;            // warps 0-2 weight loads, MMA, activation loads; all sixteen the epilogue
+constexpr int kMaxStages = 8;
+constexpr int kMaxSplit = 8;
+constexpr int kPitch = kRows + 4;        // floats per token of the partial sums in shared memory
+constexpr int kAccCols = 128;            // accumulators: up to four partial ones of few tokens side by side
+constexpr int kSfSetCols = 32;           // two sets of scale-factor columns, used by stages in turn
+constexpr int kTmemCols = 256;
+constexpr int kFixedBytes = 1024 /*alignment slack*/ + 256 /*barriers*/;
+// Two CTAs per SM where the grid has that many: one's prologue and epilogue run under the other's loads.
+constexpr int kSmemHalf = 112 * 1024, kSmemFull = 224 * 1024;
 constexpr uint32_t kWaitLimit = 1u << 20;  // try_wait polls before giving up (well under a second)
 
-enum StatusCode : unsigned { kStatusProducerWait = 1, kStatusMmaWait = 2, kStatusEpilogueWait = 3 };
-
-template <int BLOCK_N>
-struct Cfg {
-  static constexpr int kStages = (BLOCK_N == 256) ? 4 : 6;
-  static constexpr int kABytes = kBlockM * kBlockKBytes;
-  static constexpr int kBBytes = BLOCK_N * kBlockKBytes;
-  static constexpr int kSfaBytes = kMmaPerStage * kSfChunk;
-  static constexpr int kSfbChunks = (BLOCK_N + 127) / 128;
-  static constexpr int kSfbBytes = kSfbChunks * kMmaPerStage * kSfChunk;
-  static constexpr int kStageBytes = kABytes + kBBytes + kSfaBytes + kSfbBytes;
-  static constexpr int kSmemBytes = kStages * kStageBytes + 1024 /*alignment slack*/ + 256 /*barriers*/;
-  static constexpr int kAccCols = BLOCK_N;
-  static constexpr int kSfaCols = kMmaPerStage * 4;
-  static constexpr int kSfbCols = kMmaPerStage * 4 * kSfbChunks;
-  static constexpr int kTmemCols = (kAccCols + kSfaCols + kSfbCols) <= 128 ? 128 : ((kAccCols + kSfaCols + kSfbCols) <= 256 ? 256 : 512);
-};
+enum StatusCode : unsigned { kStatusProducerWait = 1, kStatusMmaWait = 2, kStatusEpilogueWait = 3, kStatusActWait = 4 };
 
 // ---- PTX wrappers -----------------------------------------------------------
 
@@ -136,15 +137,14 @@ __device__ __forceinline__ uint64_t desc_sf(uint32_t saddr) {
 }
 
 // Instruction descriptor, kind::mxf4nvf4: A,B = E2M1 (1), K-major, UE4M3
-// scale factors (0), M = 128, N = BLOCK_N, dense K = 64.
-template <int BLOCK_N>
-__device__ __forceinline__ uint32_t instr_desc() {
+// scale factors (0), M = 128, N = n_cols, dense K = 64.
+__device__ __forceinline__ uint32_t instr_desc(int n_cols) {
   uint32_t d = 0;
   d |= 1u << 7;                                  // a_format = E2M1
   d |= 1u << 10;                                 // b_format = E2M1
-  d |= static_cast<uint32_t>(BLOCK_N >> 3) << 17;  // n_dim
+  d |= static_cast<uint32_t>(n_cols >> 3) << 17;   // n_dim
   d |= 0u << 23;                                 // scale format UE4M3
-  d |= static_cast<uint32_t>(kBlockM >> 4) << 24;  // m_dim
+  d |= static_cast<uint32_t>(kRows >> 4) << 24;    // m_dim
   return d;
 }
 
@@ -166,67 +166,125 @@ __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
-    "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-    "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-    "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+    "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+    "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-      "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-      "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-      "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
     : "r"(taddr)
     : "memory");
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t map_to_rank(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+// Sum over the cluster's partial sums at byte offset `off` of every rank's `src`, in rank order.
+template <int SPLIT>
+__device__ __forceinline__ float4 sum4(const uint32_t (&src)[SPLIT], uint32_t off) {
+  float4 v[SPLIT];
+#pragma unroll
+  for (int q = 0; q < SPLIT; ++q) {
+    if constexpr (SPLIT == 1) {
+      asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[q].x), "=f"(v[q].y), "=f"(v[q].z), "=f"(v[q].w) : "r"(src[q] + off));
+    } else {
+      asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[q].x), "=f"(v[q].y), "=f"(v[q].z), "=f"(v[q].w) : "r"(src[q] + off));
+    }
+  }
+#pragma unroll
+  for (int q = 1; q < SPLIT; ++q) {
+    v[0].x += v[q].x; v[0].y += v[q].y; v[0].z += v[q].z; v[0].w += v[q].w;
+  }
+  return v[0];
+}
+
+// With few tokens an MMA is far shorter than the tensor pipe's latency, and the four MMAs of a stage, if they all
+// accumulate into the same columns, run one after the other at that latency.  They go to different partial
+// accumulators then (as many as fit), which the epilogue adds.
+__device__ __forceinline__ int partial_accumulators(int n_cols) { return 4 * n_cols <= kAccCols ? 4 : (2 * n_cols <= kAccCols ? 2 : 1); }
+
+enum Epi : int { kEpiPlain = 0, kEpiGateUp = 1, kEpiNvfp4 = 2 };
+
+// The first `count` of four BF16 values, element by element.
+__device__ __forceinline__ void store4_narrow(__nv_bfloat16 * dst, uint2 p, int count) {
+  uint16_t * d = reinterpret_cast<uint16_t *>(dst);
+  if (count > 0) d[0] = static_cast<uint16_t>(p.x);
+  if (count > 1) d[1] = static_cast<uint16_t>(p.x >> 16);
+  if (count > 2) d[2] = static_cast<uint16_t>(p.y);
+  if (count > 3) d[3] = static_cast<uint16_t>(p.y >> 16);
+}
+
+// The same store on every other rank of a gathering launch; out of line, so that launches without peers do not fetch it.
+__device__ __noinline__ void store4_to_peers(const GemmEpilogue & ep, size_t at, uint2 p, int count, bool whole) {
+#pragma unroll 1
+  for (int i = 0; i < ep.n_peers; ++i) {
+    if (whole) {
+      *reinterpret_cast<uint2 *>(ep.peer_c[i] + at) = p;
+    } else {
+      store4_narrow(ep.peer_c[i] + at, p, count);
+    }
+  }
 }
 
 // ---- kernel -------------------------------------------------------------------
 
-template <int BLOCK_N>
-__global__ void __launch_bounds__(kThreads, 1)
-gemm_w4a4_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                         const uint8_t * __restrict__ sfa, const uint8_t * __restrict__ sfb,
-                         const float * __restrict__ g_dev, const GemmEpilogue ep, int m, int n, int k_bytes,
-                         int sfb_row_blocks, __nv_bfloat16 * __restrict__ c, int ldc, unsigned int * status) {
-  using C = Cfg<BLOCK_N>;
+// grid (weight row blocks, token tiles, SPLIT), cluster (1, 1, SPLIT).
+template <int SPLIT, int EPI>
+__global__ void __launch_bounds__(kThreads, 2)
+gemm_w4a4_ksplit_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
+                        const uint8_t * __restrict__ sfw, const uint8_t * __restrict__ sfx,
+                        const float * __restrict__ g_dev, const __grid_constant__ GemmEpilogue ep, int m, int n, int k_bytes, int stages,
+                        int ring_bytes, int box_cols, int tile_cols, int vec, __nv_bfloat16 * __restrict__ c, int ldc, unsigned int * status) {
   extern __shared__ uint8_t smem_raw[];
   // 1024-byte alignment for the 128B-swizzled operand tiles.
   uint8_t * smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  const int b_bytes = box_cols * kStepBytes;
   uint8_t * smem_a = smem;
-  uint8_t * smem_b = smem_a + C::kStages * C::kABytes;
-  uint8_t * smem_sfa = smem_b + C::kStages * C::kBBytes;
-  uint8_t * smem_sfb = smem_sfa + C::kStages * C::kSfaBytes;
-  uint64_t * bars = reinterpret_cast<uint64_t *>(smem_sfb + C::kStages * C::kSfbBytes);
-  // bars[0..S) full, bars[S..2S) empty, bars[2S] accumulator ready; then the TMEM base word.
-  uint32_t * tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * C::kStages + 1);
+  uint8_t * smem_b = smem_a + stages * kABytes;
+  uint8_t * smem_sfa = smem_b + stages * b_bytes;
+  uint8_t * smem_sfb = smem_sfa + stages * kSfBytes;
+  uint64_t * bars = reinterpret_cast<uint64_t *>(smem + ring_bytes);
+  uint64_t * full = bars;                  // [stages]: both producers' bytes have landed
+  uint64_t * empty = bars + kMaxStages;    // [stages]: the MMAs that read the stage have retired
+  uint64_t * acc_full = bars + 2 * kMaxStages;
+  uint32_t * tmem_slot = reinterpret_cast<uint32_t *>(acc_full + 1);
+  float * part = reinterpret_cast<float *>(smem);  // [tokens][kPitch] partial sums, over the ring once it is done with
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int tile_n = blockIdx.x;
-  const int tile_m = blockIdx.y;
+  const int rb = blockIdx.x;
+  const int token0 = static_cast<int>(blockIdx.y) * tile_cols;
+  const int rank = SPLIT > 1 ? static_cast<int>(cluster_rank()) : 0;
+  const int tokens = min(tile_cols, m - token0);
+  const int n_cols = (tokens + 15) & ~15;
   const int sf_col_blocks = k_bytes >> 5;                        // K/64: 512-byte scale tiles per row block
   const int k_steps = (sf_col_blocks + kMmaPerStage - 1) / kMmaPerStage;
+  const int ks0 = rank * k_steps / SPLIT, ks1 = (rank + 1) * k_steps / SPLIT;
+  const int parts = partial_accumulators(n_cols);
 
-  // Launched with programmatic stream serialisation: the grid may be scheduled under the tail of the previous kernel,
-  // but reads and writes nothing before that kernel is complete.
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  // A tile that finds an error already recorded does nothing: after one expired wait the rest of the grid drains.
+  // An error recorded by an earlier tile: load and compute nothing, but meet the cluster and free the TMEM.
   __shared__ unsigned int s_abort;
-  if (threadIdx.x == 0) s_abort = *reinterpret_cast<volatile unsigned int *>(status);
-  __syncthreads();
-  if (s_abort != 0u) return;
-
   if (threadIdx.x == 0) {
-    for (int i = 0; i < C::kStages; ++i) {
-      mbar_init(smem_u32(bars + i), 1);
-      mbar_init(smem_u32(bars + C::kStages + i), 1);
+    s_abort = *reinterpret_cast<volatile unsigned int *>(status);
+    for (int i = 0; i < stages; ++i) {
+      mbar_init(smem_u32(full + i), 2);
+      mbar_init(smem_u32(empty + i), 1);
     }
-    mbar_init(smem_u32(bars + 2 * C::kStages), 1);
+    mbar_init(smem_u32(acc_full), 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(static_cast<uint32_t>(C::kTmemCols))
+                 "r"(static_cast<uint32_t>(kTmemCols))
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -234,109 +292,222 @@ gemm_w4a4_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tmem_acc = tmem_base;
-  const uint32_t tmem_sfa = tmem_base + C::kAccCols;
-  const uint32_t tmem_sfb = tmem_sfa + C::kSfaCols;
+  const bool aborted = s_abort != 0u;
+  // Launched with programmatic stream serialisation: weights are constant and start loading at once; activations,
+  // residuals and every store come after griddepcontrol.wait, when all earlier work of the stream is complete.
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   if (warp == 0) {
-    // ---------------- TMA producer ----------------
-    if (elect_one()) {
-      const uint8_t * sfa_rb = sfa + static_cast<size_t>(tile_m) * sf_col_blocks * kSfChunk;
-      for (int ks = 0; ks < k_steps; ++ks) {
-        const int stage = ks % C::kStages;
-        const uint32_t phase = (ks / C::kStages) & 1;
-        if (!mbar_wait(smem_u32(bars + C::kStages + stage), phase ^ 1)) {
+    // ---------------- weight loads ----------------
+    if (elect_one() && !aborted) {
+      const uint8_t * sf = sfw + static_cast<size_t>(rb) * sf_col_blocks * kSfChunk;
+      int stage = 0;
+      uint32_t phase = 0;
+      for (int ks = ks0; ks < ks1; ++ks) {
+        if (!mbar_wait(smem_u32(empty + stage), phase ^ 1)) {
           atomicExch(status, kStatusProducerWait);
           break;
         }
-        const int valid = min(kMmaPerStage, sf_col_blocks - ks * kMmaPerStage);
-        int sfb_valid_chunks = 0;
-#pragma unroll
-        for (int i = 0; i < C::kSfbChunks; ++i) {
-          if (tile_n * C::kSfbChunks + i < sfb_row_blocks) ++sfb_valid_chunks;
+        const uint32_t sf_bytes = min(kMmaPerStage, sf_col_blocks - ks * kMmaPerStage) * kSfChunk;
+        const uint32_t bar = smem_u32(full + stage);
+        mbar_expect_tx(bar, kABytes + sf_bytes);
+        tma_load_2d(smem_u32(smem_a + stage * kABytes), &tmap_w, bar, ks * kStepBytes, rb * kRows);
+        bulk_load(smem_u32(smem_sfa + stage * kSfBytes), sf + static_cast<size_t>(ks) * kSfBytes, sf_bytes, bar);
+        if (++stage == stages) {
+          stage = 0;
+          phase ^= 1;
         }
-        const uint32_t full = smem_u32(bars + stage);
-        const uint32_t tx = C::kABytes + C::kBBytes + valid * kSfChunk * (1 + sfb_valid_chunks);
-        mbar_expect_tx(full, tx);
-        tma_load_2d(smem_u32(smem_a + stage * C::kABytes), &tmap_a, full, ks * kBlockKBytes, tile_m * kBlockM);
-        tma_load_2d(smem_u32(smem_b + stage * C::kBBytes), &tmap_b, full, ks * kBlockKBytes, tile_n * BLOCK_N);
-        bulk_load(smem_u32(smem_sfa + stage * C::kSfaBytes), sfa_rb + static_cast<size_t>(ks) * kMmaPerStage * kSfChunk,
-                  valid * kSfChunk, full);
-#pragma unroll
-        for (int i = 0; i < C::kSfbChunks; ++i) {
-          const int rb = tile_n * C::kSfbChunks + i;
-          if (rb < sfb_row_blocks) {
-            bulk_load(smem_u32(smem_sfb + stage * C::kSfbBytes + i * kMmaPerStage * kSfChunk),
-                      sfb + (static_cast<size_t>(rb) * sf_col_blocks + static_cast<size_t>(ks) * kMmaPerStage) * kSfChunk,
-                      valid * kSfChunk, full);
-          }
+      }
+    }
+  } else if (warp == 2) {
+    // ---------------- activation loads ----------------
+    if (elect_one() && !aborted) {
+      asm volatile("griddepcontrol.wait;" ::: "memory");
+      const uint8_t * sf = sfx + static_cast<size_t>(token0 >> 7) * sf_col_blocks * kSfChunk;
+      int stage = 0;
+      uint32_t phase = 0;
+      for (int ks = ks0; ks < ks1; ++ks) {
+        if (!mbar_wait(smem_u32(empty + stage), phase ^ 1)) {
+          atomicExch(status, kStatusActWait);
+          break;
+        }
+        const uint32_t sf_bytes = min(kMmaPerStage, sf_col_blocks - ks * kMmaPerStage) * kSfChunk;
+        const uint32_t bar = smem_u32(full + stage);
+        mbar_expect_tx(bar, b_bytes + sf_bytes);
+        tma_load_2d(smem_u32(smem_b + stage * b_bytes), &tmap_x, bar, ks * kStepBytes, token0);
+        bulk_load(smem_u32(smem_sfb + stage * kSfBytes), sf + static_cast<size_t>(ks) * kSfBytes, sf_bytes, bar);
+        if (++stage == stages) {
+          stage = 0;
+          phase ^= 1;
         }
       }
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (elect_one()) {
-      const uint32_t idesc = instr_desc<BLOCK_N>();
+    if (elect_one() && !aborted) {
+      const uint32_t idesc = instr_desc(n_cols);
+      const uint32_t sfb_off = static_cast<uint32_t>(token0 & 127) >> 5;  // a 64-token tile may start in the middle of a scale tile
       bool ok = true;
-      for (int ks = 0; ks < k_steps && ok; ++ks) {
-        const int stage = ks % C::kStages;
-        const uint32_t phase = (ks / C::kStages) & 1;
-        if (!mbar_wait(smem_u32(bars + stage), phase)) {
+      int stage = 0;
+      uint32_t phase = 0;
+      for (int ks = ks0; ks < ks1; ++ks) {
+        const int it = ks - ks0;
+        if (!mbar_wait(smem_u32(full + stage), phase)) {
           atomicExch(status, kStatusMmaWait);
           ok = false;
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const int valid = min(kMmaPerStage, sf_col_blocks - ks * kMmaPerStage);
-        const uint32_t a_base = smem_u32(smem_a + stage * C::kABytes);
-        const uint32_t b_base = smem_u32(smem_b + stage * C::kBBytes);
-        const uint32_t sfa_base = smem_u32(smem_sfa + stage * C::kSfaBytes);
-        const uint32_t sfb_base = smem_u32(smem_sfb + stage * C::kSfbBytes);
-        for (int j = 0; j < valid; ++j) {
-          utccp_sf(tmem_sfa + j * 4, desc_sf(sfa_base + j * kSfChunk));
+        // the address field of a descriptor counts 16-byte units, so stepping one is an add
+        const uint64_t a_desc = desc_k_sw128(smem_u32(smem_a + stage * kABytes));
+        const uint64_t b_desc = desc_k_sw128(smem_u32(smem_b + stage * b_bytes));
+        const uint64_t sfa_desc = desc_sf(smem_u32(smem_sfa + stage * kSfBytes));
+        const uint64_t sfb_desc = desc_sf(smem_u32(smem_sfb + stage * kSfBytes));
+        const uint32_t sf_set = tmem_base + kAccCols + (it & 1) * kSfSetCols;
 #pragma unroll
-          for (int i = 0; i < C::kSfbChunks; ++i) {
-            utccp_sf(tmem_sfb + (j * C::kSfbChunks + i) * 4, desc_sf(sfb_base + (i * kMmaPerStage + j) * kSfChunk));
+        for (int j = 0; j < kMmaPerStage; ++j) {
+          if (j < valid) {
+            utccp_sf(sf_set + j * 4, sfa_desc + j * (kSfChunk >> 4));
+            utccp_sf(sf_set + 16 + j * 4, sfb_desc + j * (kSfChunk >> 4));
           }
         }
-        for (int j = 0; j < valid; ++j) {
-          umma_mxf4nvf4(tmem_acc, desc_k_sw128(a_base + j * 32), desc_k_sw128(b_base + j * 32), idesc,
-                        tmem_sfa + j * 4, tmem_sfb + j * C::kSfbChunks * 4, (ks | j) != 0 ? 1u : 0u);
+#pragma unroll
+        for (int j = 0; j < kMmaPerStage; ++j) {
+          if (j < valid) {
+            umma_mxf4nvf4(tmem_base + (j & (parts - 1)) * n_cols, a_desc + j * 2, b_desc + j * 2, idesc, sf_set + j * 4,
+                          sf_set + 16 + j * 4 + sfb_off, (it * kMmaPerStage + j) >= parts ? 1u : 0u);
+          }
         }
-        umma_commit(smem_u32(bars + C::kStages + stage));  // frees the stage when these MMAs and copies retire
+        umma_commit(smem_u32(empty + stage));  // frees the stage when these MMAs and copies retire
+        if (++stage == stages) {
+          stage = 0;
+          phase ^= 1;
+        }
       }
-      if (ok) umma_commit(smem_u32(bars + 2 * C::kStages));  // accumulator complete
+      if (ok) umma_commit(smem_u32(acc_full));  // accumulator complete, and with it every load of the ring consumed
     }
-  } else {
-    // ---------------- epilogue: TMEM -> registers -> bf16 -> global ----------------
+  }
+  __syncwarp();
+
+  // ---------------- epilogue: TMEM -> shared memory -> sum over the cluster -> global ----------------
+  bool ran = !aborted;
+  if (ran && !mbar_wait(smem_u32(acc_full), 0)) {
+    if (lane == 0) atomicExch(status, kStatusEpilogueWait);
+    ran = false;
+  }
+  if (ran) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const int quarter = warp & 3;                 // TMEM lanes this warp may touch
-    const int row = tile_m * kBlockM + quarter * 32 + lane;
-    const bool ready = mbar_wait(smem_u32(bars + 2 * C::kStages), 0);
-    if (!ready) {
-      if (lane == 0) atomicExch(status, kStatusEpilogueWait);
-    } else {
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const float g = __ldg(g_dev);
-      const float q_g = ep.q_g != nullptr ? __ldg(ep.q_g) : 1.0f;
-      const uint32_t taddr = tmem_acc + (static_cast<uint32_t>(quarter * 32) << 16);
+    const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+    // partial accumulators that were written: a slice of one short step has fewer MMAs than there are of them
+    const int mmas = min((ks1 - ks0) * kMmaPerStage, sf_col_blocks - ks0 * kMmaPerStage);
+    const int used = min(parts, mmas);
+    float * dst = part + quarter * 32 + lane;
 #pragma unroll 1
-      for (int c0 = 0; c0 < BLOCK_N; c0 += 32) {
-        uint32_t r[32];
-        tmem_ld32(taddr + c0, r);
+    for (int c0 = 16 * (warp >> 2); c0 < n_cols; c0 += 4 * (kThreads / 32)) {
+      uint32_t r[16];
+      tmem_ld16(taddr + c0, r);
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll 1
+      for (int p = 1; p < used; ++p) {
+        uint32_t r2[16];
+        tmem_ld16(taddr + p * n_cols + c0, r2);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (row < m) gemm_store_chunk32(r, row, tile_n * BLOCK_N + c0, n, g, ep, c, ldc, true, q_g);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) + __uint_as_float(r2[i]));
+      }
+#pragma unroll
+      for (int i = 0; i < 16; ++i) dst[(c0 + i) * kPitch] = __uint_as_float(r[i]);
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  if constexpr (SPLIT > 1) cluster_sync(); else __syncthreads();
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (warp == 1) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
+                 "r"(static_cast<uint32_t>(kTmemCols))
+                 : "memory");
+  }
+
+  if (ran) {
+    // this CTA's share of the tokens
+    const int t_begin = rank * n_cols / SPLIT, t_end = min((rank + 1) * n_cols / SPLIT, tokens);
+    const float g = __ldg(g_dev);
+    const float alpha = g * ep.s2, alpha_up = g * ep.s2_up;
+    uint32_t src[SPLIT];
+#pragma unroll
+    for (int q = 0; q < SPLIT; ++q) src[q] = SPLIT > 1 ? map_to_rank(smem_u32(part), q) : smem_u32(part);
+    const int row0 = rb * kRows;
+    // Compact loops: this code runs once per CTA, so what it costs is mostly the fetching of its instructions
+    // (unrolled four times and with the peers' stores inline it took 4.5 us at 128 tokens).
+    if constexpr (EPI == kEpiNvfp4) {
+      // one thread per token and 32 weight rows = one block of 16 outputs (n % 128 == 0 is checked on the host);
+      // lanes along the tokens, whose pitch spreads them over the banks
+      const float q_g = __ldg(ep.q_g);
+      const int live = t_end - t_begin;
+      for (int u = threadIdx.x; u < live * (kRows / 32); u += kThreads) {
+        const int t = t_begin + u % live, blk = u / live;
+        uint32_t r[32];
+#pragma unroll
+        for (int i = 0; i < 32; i += 4) {
+          const float4 a = sum4<SPLIT>(src, static_cast<uint32_t>(t * kPitch + 32 * blk + i) * 4u);
+          r[i] = __float_as_uint(a.x); r[i + 1] = __float_as_uint(a.y); r[i + 2] = __float_as_uint(a.z); r[i + 3] = __float_as_uint(a.w);
+        }
+        store_nvfp4_chunk32(r, token0 + t, row0 + 32 * blk, alpha, alpha_up, ep, q_g);
+      }
+    } else {
+      // one warp per token, four consecutive weight rows per lane
+      const int row = row0 + 4 * lane;
+      // output column of the lane's first value; a gate/up weight's rows alternate 8 gate / 8 up, so lanes l and l ^ 2
+      // hold matching gate and up rows and the first of them stores
+      const int col = EPI == kEpiGateUp ? (row >> 4) * 8 + (row & 7) : row;
+      const int count = EPI == kEpiGateUp ? ((lane & 2) == 0 ? n - (row + 8) : 0) : n - row;
+      const bool whole = vec != 0 && count >= 4;
+      const __nv_bfloat16 * res = ep.residual + static_cast<size_t>(token0 + t_begin + warp) * ep.ldr + row;
+      size_t at = static_cast<size_t>(token0 + t_begin + warp) * ldc + col;
+#pragma unroll 1
+      for (int t = t_begin + warp; t < t_end; t += kThreads / 32) {
+        const float4 a = sum4<SPLIT>(src, static_cast<uint32_t>(t * kPitch + 4 * lane) * 4u);
+        float v[4] = {a.x, a.y, a.z, a.w};
+        if constexpr (EPI == kEpiGateUp) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float up = __shfl_xor_sync(0xffffffffu, v[e], 2);
+            v[e] = silu_mul(v[e] * alpha, up * alpha_up);
+          }
+        } else {
+          float rv[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+          if (ep.residual != nullptr) {
+            if (whole) {
+              const uint2 p = __ldg(reinterpret_cast<const uint2 *>(res));
+              rv[0] = __uint_as_float(p.x << 16); rv[1] = __uint_as_float(p.x & 0xffff0000u);
+              rv[2] = __uint_as_float(p.y << 16); rv[3] = __uint_as_float(p.y & 0xffff0000u);
+            } else {
+#pragma unroll
+              for (int e = 0; e < 4; ++e) if (e < count) rv[e] = __bfloat162float(res[e]);
+            }
+            res += static_cast<size_t>(ep.ldr) * (kThreads / 32);
+          }
+#pragma unroll
+          for (int e = 0; e < 4; ++e) v[e] = fmaf(v[e], alpha, rv[e]);
+        }
+        const uint2 p = make_uint2(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]));
+        if (whole) {
+          *reinterpret_cast<uint2 *>(c + at) = p;
+        } else {
+          store4_narrow(c + at, p, count);
+        }
+        if (ep.n_peers > 0) store4_to_peers(ep, at, p, count, whole);
+        at += static_cast<size_t>(ldc) * (kThreads / 32);
       }
     }
   }
 
-  gemm_signal_peers(ep, true);
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  if (warp == 1) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
-                 "r"(static_cast<uint32_t>(C::kTmemCols))
-                 : "memory");
-  }
+  gemm_signal_peers(ep, ran);
+  __syncwarp();
+  if constexpr (SPLIT > 1) cluster_sync();  // no CTA may leave while another still reads its partial sums
 }
 
 // ---- host side ---------------------------------------------------------------
@@ -368,7 +539,7 @@ int make_code_map(CUtensorMap * map, const void * base, int rows, int k_bytes, i
   if (fn == nullptr) return fail(Q35B_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the CUDA driver.");
   const cuuint64_t dims[2] = {static_cast<cuuint64_t>(k_bytes), static_cast<cuuint64_t>(rows)};
   const cuuint64_t strides[1] = {static_cast<cuuint64_t>(k_bytes)};
-  const cuuint32_t box[2] = {static_cast<cuuint32_t>(kBlockKBytes), static_cast<cuuint32_t>(box_rows)};
+  const cuuint32_t box[2] = {static_cast<cuuint32_t>(kStepBytes), static_cast<cuuint32_t>(box_rows)};
   const cuuint32_t elem[2] = {1, 1};
   const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void *>(base), dims, strides, box, elem,
                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -381,24 +552,90 @@ int make_code_map(CUtensorMap * map, const void * base, int rows, int k_bytes, i
 
 namespace {
 
-template <int BLOCK_N>
-int launch_tile(const q35b_weight * w, const CUtensorMap & tmap_a, const uint8_t * a_scales, const float * g_dev, int m,
-                void * c, int ldc, const GemmEpilogue & ep, unsigned int * status, cudaStream_t s) {
-  using C = Cfg<BLOCK_N>;
+// Tokens per tile and CTAs per tile.
+//
+// Estimates in nanoseconds, fitted to CUDA-graph timings on B200: a K step takes 250, tokens cost 6.6 each in loads and
+// epilogue, and the exchange of a split costs 400 + 3.3 per token + 7 per token and doubling ([64, 2560] x [1024, 2560]:
+// 5.1 us unsplit, 4.9 split in two or four, 5.0 in eight; [9, 5760] x [108, 5760]: 7.9, 5.5, 4.0, 3.4 us;
+// [128, 9216] x [512, 9216]: 12.2, 8.9, 7.1, 6.9 us with 128 tokens per tile, 11.9, 8.3, 6.3, 5.8 us with 64).
+// Halving the tiles or splitting K pays only while all CTAs run at once ([128, 2560] x [18432, 2560], 144 tiles:
+// 7.3 us, 9.3 split in two, 9.0 with 64 tokens per tile), and a split has to gain 0.3 us to be worth it.
+struct Shape {
+  int tile_cols, split;
+};
+Shape choose_shape(int m, int row_blocks, int k_steps, int sms) {
+  Shape best = {kMaxCols, 1};
+  int best_ns = 0;
+  for (int cols = kMaxCols; cols >= 64; cols /= 2) {
+    const int tiles = row_blocks * ((m + cols - 1) / cols), live = std::min(cols, round_up_int(m, 16));
+    if (cols < kMaxCols && (m <= cols || tiles > sms)) break;
+    for (int split = 1, log2 = 0; split <= kMaxSplit; split *= 2, ++log2) {
+      if (split > 1 && (tiles * split > sms || k_steps < 2 * split)) break;
+      const int ns = (k_steps + split - 1) / split * 250 + live * 66 / 10 +
+                     (split > 1 ? 400 + live * 33 / 10 + live * 7 * log2 : 0);
+      if (best_ns == 0 || ns + (split > best.split ? 300 : 0) < best_ns) {
+        best = {cols, split};
+        best_ns = ns;
+      }
+    }
+  }
+  return best;
+}
+
+int launch_gemm_ksplit(const q35b_weight * w, const uint8_t * a_codes, const uint8_t * a_scales, const float * g_dev, int m,
+                       void * c, int ldc, const GemmEpilogue & ep, unsigned int * status, cudaStream_t s) {
+  const int row_blocks = (w->rows + kRows - 1) / kRows, k_steps = (w->k + 255) / 256;
+  const Shape shape = choose_shape(m, row_blocks, k_steps, sm_count());
+  const int tile_cols = shape.tile_cols, split = shape.split;
+  const int box_cols = std::min(tile_cols, round_up_int(m, 16));
+  CUtensorMap tmap_x;
+  if (const int st = make_code_map(&tmap_x, a_codes, m, w->k / 2, box_cols)) return st;
+  const int token_tiles = (m + tile_cols - 1) / tile_cols;
+  const int ctas = row_blocks * token_tiles * split;
+  const int stage_bytes = kABytes + box_cols * kStepBytes + 2 * kSfBytes;
+  const int budget = ctas > sm_count() ? kSmemHalf : kSmemFull;
+  const int stages = std::min({kMaxStages, (budget - kFixedBytes) / stage_bytes, std::max(2, (k_steps + split - 1) / split)});
+  // the partial sums reuse the ring, and want at least their own size
+  const int ring = round_up_int(std::max(stages * stage_bytes, box_cols * kPitch * 4), 128);
+  // 8-byte pieces of every row of the output (and of the residual and the peers' copies) are aligned
+  bool vec = (ldc % 4) == 0 && (reinterpret_cast<uintptr_t>(c) & 7u) == 0;
+  if (ep.residual != nullptr) vec = vec && (ep.ldr % 4) == 0 && (reinterpret_cast<uintptr_t>(ep.residual) & 7u) == 0;
+  for (int i = 0; i < ep.n_peers; ++i) vec = vec && (reinterpret_cast<uintptr_t>(ep.peer_c[i]) & 7u) == 0;
+  using Kernel = decltype(&gemm_w4a4_ksplit_kernel<1, kEpiPlain>);
+  static constexpr Kernel kernels[3][4] = {
+    {gemm_w4a4_ksplit_kernel<1, kEpiPlain>, gemm_w4a4_ksplit_kernel<2, kEpiPlain>, gemm_w4a4_ksplit_kernel<4, kEpiPlain>, gemm_w4a4_ksplit_kernel<8, kEpiPlain>},
+    {gemm_w4a4_ksplit_kernel<1, kEpiGateUp>, gemm_w4a4_ksplit_kernel<2, kEpiGateUp>, gemm_w4a4_ksplit_kernel<4, kEpiGateUp>, gemm_w4a4_ksplit_kernel<8, kEpiGateUp>},
+    {gemm_w4a4_ksplit_kernel<1, kEpiNvfp4>, gemm_w4a4_ksplit_kernel<2, kEpiNvfp4>, gemm_w4a4_ksplit_kernel<4, kEpiNvfp4>, gemm_w4a4_ksplit_kernel<8, kEpiNvfp4>}};
   static std::atomic<bool> attr_set[64];
-  auto kernel = gemm_w4a4_tcgen05_kernel<BLOCK_N>;
   if (!attr_set[w->device & 63].load(std::memory_order_acquire)) {
     // idempotent, so two threads getting here together is harmless
-    Q35B_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes),
-                  "cudaFuncSetAttribute(gemm smem)");
+    for (const auto & row : kernels) {
+      for (const Kernel f : row) {
+        Q35B_CUDA_TRY(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemFull), "cudaFuncSetAttribute(gemm smem)");
+      }
+    }
     attr_set[w->device & 63].store(true, std::memory_order_release);
   }
-  const dim3 grid((w->rows + BLOCK_N - 1) / BLOCK_N, (m + kBlockM - 1) / kBlockM);
-  const cudaError_t le = launch_pdl(kernel, grid, dim3(kThreads), C::kSmemBytes, s, tmap_a,
-                                    BLOCK_N == 256 ? w->tmap_codes_256 : w->tmap_codes_128, a_scales, w->scales_tiled, g_dev, ep, m,
-                                    w->rows, w->k / 2, (w->rows + 127) / 128, static_cast<__nv_bfloat16 *>(c), ldc, status);
+  const Kernel kernel = kernels[ep.q_codes != nullptr ? kEpiNvfp4 : (ep.gate_up ? kEpiGateUp : kEpiPlain)][split == 8 ? 3 : split >> 1];
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(row_blocks), static_cast<unsigned>(token_tiles), static_cast<unsigned>(split));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = static_cast<size_t>(ring + kFixedBytes);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = 1;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = static_cast<unsigned>(split);
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  const cudaError_t le = cudaLaunchKernelEx(&cfg, kernel, w->tmap_codes_128, tmap_x, static_cast<const uint8_t *>(w->scales_tiled),
+                                            a_scales, g_dev, ep, m, w->rows, w->k / 2, stages, ring, box_cols, tile_cols, vec ? 1 : 0,
+                                            static_cast<__nv_bfloat16 *>(c), ldc, status);
   count_launch();
-  Q35B_CUDA_TRY(le, "gemm_w4a4_tcgen05_kernel launch");
+  Q35B_CUDA_TRY(le, "gemm_w4a4_ksplit_kernel launch");
   return Q35B_OK;
 }
 
@@ -506,23 +743,21 @@ int launch_gemm_w4a4(const q35b_weight * w, const uint8_t * a_codes, const uint8
     // clears it (no memset in front of the launch: it would sit between this kernel and the one it overlaps with)
     if (const int st = default_status_word(&status_dev)) return st;
   }
-  // Large problems: pairs of CTAs on 256 x 256 tiles, persistent (gemm_w4a4_2cta.cu).
-  if (gemm_2cta_eligible(w, m)) {
+  // Large problems: pairs of CTAs on 256 x 256 tiles, persistent (gemm_w4a4_2cta.cu).  They need many tiles to win: up
+  // to two 128 x 128 tiles per SM the kernel above is faster (us, this kernel / pairs: [512, 2560] x [9216, 2560]
+  // 8.9 / 10.5, [768, ..] 15.6 / 14.4; [1024, 4096] x [4096, 4096] 10.8 / 12.2, [1536, ..] 19.4 / 17.7), up to three
+  // where K is short ([2048, 1024] x [3584, 1024] 10.7 / 11.0, [3072, ..] 15.3 / 13.9), only one where K is long
+  // ([768, 9216] x [2560, 9216] 13.6 / 17.3, [1536, ..] 19.8 / 18.3).  The pairs also store rows that are not 32-byte
+  // aligned element by element ([4096, 640] x [5000, 640] 24 / 133).
+  const long tiles = static_cast<long>((w->rows + kRows - 1) / kRows) * ((m + kMaxCols - 1) / kMaxCols);
+  const int k_steps = (w->k + 255) / 256;
+  const long few = static_cast<long>(sm_count()) * (k_steps <= 4 ? 3 : (k_steps <= 20 ? 2 : 1));
+  const bool rows_aligned = qout != nullptr || ((ldc % 16) == 0 && (reinterpret_cast<uintptr_t>(c_bf16) & 31u) == 0 &&
+                            (residual_bf16 == nullptr || ((ldr % 8) == 0 && (reinterpret_cast<uintptr_t>(residual_bf16) & 15u) == 0)));
+  if (gemm_2cta_eligible(w, m) && (gather != nullptr || (tiles > few && rows_aligned))) {
     return launch_gemm_w4a4_2cta(w, a_codes, a_scales_tiled, g_dev, m, c_bf16, ldc, ep, status_dev, s);
   }
-  // Up to 128 tokens: the weight streams through the 128-row side of the tile, every SM takes row blocks
-  // (gemm_wstream.cu); bound by HBM, not by the tensor pipe.
-  if (qout == nullptr && gather == nullptr && gemm_wstream_eligible(w, m)) {
-    return launch_gemm_wstream(w, a_codes, a_scales_tiled, g_dev, m, c_bf16, ldc, residual_bf16, ldr, status_dev, s);
-  }
-  CUtensorMap tmap_a;
-  if (const int st = make_code_map(&tmap_a, a_codes, m, w->k / 2, kBlockM)) return st;
-  // Small problems get narrower tiles so that more SMs have work.
-  const long tiles256 = static_cast<long>((w->rows + 255) / 256) * ((m + 127) / 128);
-  if (tiles256 >= sm_count() || w->rows <= 128) {
-    if (w->rows > 128) return launch_tile<256>(w, tmap_a, a_scales_tiled, g_dev, m, c_bf16, ldc, ep, status_dev, s);
-  }
-  return launch_tile<128>(w, tmap_a, a_scales_tiled, g_dev, m, c_bf16, ldc, ep, status_dev, s);
+  return launch_gemm_ksplit(w, a_codes, a_scales_tiled, g_dev, m, c_bf16, ldc, ep, status_dev, s);
 }
 
 }  // namespace q35b

@@ -15,16 +15,12 @@
 // a tile runs under the MMAs of the next, and four epilogue warps that turn accumulator lanes into BF16 outputs
 // y[token, row].
 //
-// Two uses:
-//   * small-M prefill (W4A4, 1..128 tokens): the operand rows are the tokens of q35b_quantize_nvfp4_bf16;
-//     replaces run_nvfp4_cublaslt_prefill_projection_device (src/runtime/cuda_bench.cu:1056-1167) for short
-//     sequences, where it is bound by the weight stream (HBM), not by the tensor pipe;
-//   * decode (W4A16, 1..8 tokens): every token is expanded into `digits` operand rows, an NVFP4 digit expansion of
-//     its BF16 activations (expand_digits_kernel below): digit j quantises what digits 0..j-1 left over, so the sum
-//     of the rows reproduces the activation to 6^-digits of its block's amax (digits = 5: 1.3e-4, far below BF16's
-//     own 2^-9), and the epilogue adds the digits' accumulator columns.  Replaces nvfp4_row_dot / matvec_nvfp4_bf16
-//     (src/kernels/cuda/decode_layers.cuh:200-284) with the FP4 decode done by the tensor core instead of by
-//     conversion instructions.
+// Decode (W4A16, 1..8 tokens): every token is expanded into `digits` operand rows, an NVFP4 digit expansion of
+// its BF16 activations (expand_digits_kernel below): digit j quantises what digits 0..j-1 left over, so the sum
+// of the rows reproduces the activation to 6^-digits of its block's amax (digits = 5: 1.3e-4, far below BF16's
+// own 2^-9), and the epilogue adds the digits' accumulator columns.  Replaces nvfp4_row_dot / matvec_nvfp4_bf16
+// (src/kernels/cuda/decode_layers.cuh:200-284) with the FP4 decode done by the tensor core instead of by
+// conversion instructions.
 //
 // Every wait is bounded; an expired wait records a code in *status and the role stops; the CTA still frees TMEM.
 #include <cuda_bf16.h>
@@ -58,25 +54,23 @@ constexpr int kSmemBudget = 220 * 1024;   // dynamic part; the staged tile descr
 enum StatusCode : unsigned { kWeightWait = 41, kActWait = 42, kMmaWait = 43, kMmaDrainWait = 44, kEpilogueWait = 45 };
 enum Epilogue : int { kEpiPlain = 0, kEpiGateUp = 1 };
 
-// One projection of the list.  Lives in device memory (work lists) or in the kernel's parameter space (single
-// projection); the tensor maps are read by the TMA unit from wherever the item is.
+// One projection of the list, in device memory; the tensor maps are read by the TMA unit from there.
 struct alignas(128) WItem {
   CUtensorMap tmap_w;            // weight codes [rows, K/2], box 128 rows x 128 bytes, 128B swizzle
   CUtensorMap tmap_x;            // operand codes [operand rows, K/2], box n_cols rows x 128 bytes, 128B swizzle
   const uint8_t * w_scales;      // weight scale tiles
   const uint8_t * x_scales;      // operand scale tiles (one 128-row block)
-  const float * x_g;             // the operand's scale: one device scalar, or one per token (g_stride = 1)
+  const float * x_g;             // the operand's scale, one per token
   __nv_bfloat16 * y;             // [tokens, ldy]
   const __nv_bfloat16 * residual;  // NULL or [tokens, ldr]
   int rows;                      // weight rows
   int k_steps;                   // K / 256
   int n_cols;                    // operand rows padded to a multiple of 16 (UMMA N)
   int tokens;
-  int digits;                    // operand rows per token (1: plain W4A4)
+  int digits;                    // operand rows per token
   int ldy, ldr;
   float s2, s2_up;
   int epilogue;
-  int g_stride;
 };
 
 struct alignas(8) WTile {
@@ -96,7 +90,6 @@ struct alignas(16) STile {
   const __nv_bfloat16 * residual;
   int row_block, rows, k_steps, n_cols, tokens, digits, ldy, ldr, epilogue;
   float s2, s2_up;
-  int g_stride;
 };
 constexpr int kMaxTilesInSmem = 40;
 
@@ -195,11 +188,10 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
 
 __device__ __forceinline__ float silu_mul(float g, float u) { return __fdividef(g, 1.0f + __expf(-g)) * u; }
 
-// items == nullptr: the one projection in `single`, tiles dealt round-robin (tile = row block);
-// otherwise CTA b walks tiles[cta_begin[b] .. cta_begin[b + 1]).
+// CTA b walks tiles[cta_begin[b] .. cta_begin[b + 1]).
 __global__ void __launch_bounds__(kThreads, 1)
-gemm_wstream_kernel(const __grid_constant__ WItem single, const WItem * __restrict__ items, const WTile * __restrict__ tiles,
-                    const int * __restrict__ cta_begin, int single_tiles, int stages, int b_slot_bytes, unsigned int * status) {
+gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__ tiles, const int * __restrict__ cta_begin,
+                    int stages, int b_slot_bytes, unsigned int * status) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t * smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint8_t * smem_a = smem;
@@ -216,24 +208,11 @@ gemm_wstream_kernel(const __grid_constant__ WItem single, const WItem * __restri
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  int tile_begin, n_tiles, tile_stride;
-  if (items == nullptr) {
-    tile_begin = blockIdx.x;
-    tile_stride = gridDim.x;
-    n_tiles = single_tiles > static_cast<int>(blockIdx.x) ? (single_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
-  } else {
-    tile_begin = cta_begin[blockIdx.x];
-    tile_stride = 1;
-    n_tiles = cta_begin[blockIdx.x + 1] - tile_begin;
-  }
+  const int tile_begin = cta_begin[blockIdx.x], n_tiles = cta_begin[blockIdx.x + 1] - tile_begin;
   auto describe = [&](int ti, STile & d) {
-    const WItem * it = &single;
-    int rb = tile_begin + ti * tile_stride;
-    if (items != nullptr) {
-      const WTile t = tiles[tile_begin + ti];
-      rb = t.row_block;
-      it = items + t.item;
-    }
+    const WTile t = tiles[tile_begin + ti];
+    const int rb = t.row_block;
+    const WItem * it = items + t.item;
     d.tmap_w = &it->tmap_w;
     d.tmap_x = &it->tmap_x;
     d.k_steps = it->k_steps;
@@ -252,7 +231,6 @@ gemm_wstream_kernel(const __grid_constant__ WItem single, const WItem * __restri
     d.epilogue = it->epilogue;
     d.s2 = it->s2;
     d.s2_up = it->s2_up;
-    d.g_stride = it->g_stride;
   };
   // tile descriptors are constant for the life of a work list (and of a launch): read them before anything else
   for (int ti = threadIdx.x; ti < min(n_tiles, kMaxTilesInSmem); ti += kThreads) describe(ti, stile[ti]);
@@ -417,7 +395,6 @@ gemm_wstream_kernel(const __grid_constant__ WItem single, const WItem * __restri
       const int rows = it->rows, tokens = it->tokens, digits = it->digits, n_cols = it->n_cols;
       const int row = rb * kRows + row_in_tile;
       const float * x_g = it->x_g;
-      const int g_stride = it->g_stride;
       const bool gate_up = it->epilogue == kEpiGateUp;
       const float s2 = it->s2, s2_up = it->s2_up;
       __nv_bfloat16 * y = it->y;
@@ -449,7 +426,7 @@ gemm_wstream_kernel(const __grid_constant__ WItem single, const WItem * __restri
           sum += __uint_as_float(r[i]);
           if (++jc == digits) {
             // one output value per (token, weight row); all lanes take the same path
-            const float gval = token < tokens ? __ldg(x_g + token * g_stride) : 0.0f;
+            const float gval = token < tokens ? __ldg(x_g + token) : 0.0f;
             const float alpha = gval * s2, alpha_up = gval * s2_up;
             if (gate_up) {
               // rows alternate 8 gate / 8 up: lane l holds gate row j, lane l ^ 8 the matching up row
@@ -609,54 +586,6 @@ int ensure_attr() {
 
 }  // namespace
 
-// ---- small-M prefill: one projection, item in the kernel's parameter space, nothing allocated -------------------
-
-// Prefill takes this kernel for up to 32 tokens (measured against the token-major 1-CTA kernel: 6.0 / 9.6 / 17.0 us
-// against 8.5 / 12.3 / 22.8 us at 16 tokens on [3584,1024] / [9216,2560] / [32768,2560]; slower from about 64 tokens
-// on, where its epilogue and the copy-to-MMA turnaround per stage outweigh the better spread over the SMs), unless
-// the weight has so few row blocks and so long a K that most SMs would idle ([2560, 9216]: 20 tiles).
-bool gemm_wstream_eligible(const q35b_weight * w, int m) {
-  if (w == nullptr || !w->has_maps || m < 1 || m > 32 || (w->k % 256) != 0 || w->rows <= 0) return false;
-  const int tiles = (w->rows + kRows - 1) / kRows, k_steps = w->k / 256;
-  return !(tiles < 24 && k_steps > 16);
-}
-
-int launch_gemm_wstream(const q35b_weight * w, const uint8_t * a_codes, const uint8_t * a_scales_tiled, const float * g_dev,
-                        int m, void * c_bf16, int ldc, const void * residual_bf16, int ldr, unsigned int * status_dev,
-                        cudaStream_t s) {
-  if (const int st = ensure_attr()) return st;
-  WItem item = {};
-  item.tmap_w = w->tmap_codes_128;
-  item.n_cols = round_up_int(m, 16);
-  if (const int st = make_code_map(&item.tmap_x, a_codes, m, w->k / 2, item.n_cols)) return st;
-  item.w_scales = w->scales_tiled;
-  item.x_scales = a_scales_tiled;
-  item.x_g = g_dev;
-  item.y = static_cast<__nv_bfloat16 *>(c_bf16);
-  item.residual = static_cast<const __nv_bfloat16 *>(residual_bf16);
-  item.rows = w->rows;
-  item.k_steps = w->k / 256;
-  item.tokens = m;
-  item.digits = 1;
-  item.ldy = ldc;
-  item.ldr = ldr;
-  item.s2 = w->s2;
-  item.s2_up = w->s2_up;
-  item.epilogue = w->gate_up ? kEpiGateUp : kEpiPlain;
-  item.g_stride = 0;
-  const int tiles = (w->rows + kRows - 1) / kRows;
-  const int b_slot = item.n_cols * kStepBytes;
-  const int stages = plan_stages(b_slot);
-  const int grid = std::max(1, std::min(tiles, sm_count()));
-  const cudaError_t le = launch_pdl(gemm_wstream_kernel, dim3(grid), dim3(kThreads), static_cast<size_t>(smem_for(stages, b_slot)), s,
-                                    item, static_cast<const WItem *>(nullptr), static_cast<const WTile *>(nullptr),
-                                    static_cast<const int *>(nullptr), tiles, stages, b_slot, status_dev);
-  count_launch();
-  Q35B_CUDA_TRY(le, "gemm_wstream_kernel launch");
-  return Q35B_OK;
-}
-
-
 // ---- decode work list on the tensor path ------------------------------------------------------------------------
 
 struct WBatch {
@@ -788,7 +717,6 @@ int wbatch_build(const q35b_gemv_item * items, int count, int m, int digits, WBa
     it.s2 = w->s2;
     it.s2_up = w->s2_up;
     it.epilogue = w->gate_up ? kEpiGateUp : kEpiPlain;
-    it.g_stride = 1;
     h_expand[i] = ExpandItem{static_cast<const __nv_bfloat16 *>(items[i].x_bf16), base + o_codes[i], base + o_scales[i],
                              reinterpret_cast<float *>(base + o_g[i]), w->k};
   }
@@ -813,9 +741,8 @@ int wbatch_launch(const WBatch * b, cudaStream_t s) {
                               b->digits);
   count_launch();
   Q35B_CUDA_TRY(le, "expand_digits_kernel launch");
-  WItem unused = {};
-  le = launch_pdl(gemm_wstream_kernel, dim3(b->grid), dim3(kThreads), static_cast<size_t>(b->smem), s, unused,
-                  static_cast<const WItem *>(b->items), static_cast<const WTile *>(b->tiles), static_cast<const int *>(b->cta_begin), 0,
+  le = launch_pdl(gemm_wstream_kernel, dim3(b->grid), dim3(kThreads), static_cast<size_t>(b->smem), s,
+                  static_cast<const WItem *>(b->items), static_cast<const WTile *>(b->tiles), static_cast<const int *>(b->cta_begin),
                   b->stages, b->b_slot, b->status);
   count_launch();
   Q35B_CUDA_TRY(le, "gemm_wstream_kernel launch");

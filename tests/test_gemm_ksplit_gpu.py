@@ -1,0 +1,62 @@
+"""The K-split prefill GEMM (weight rows on the 128-row side, a cluster of CTAs sharing a tile's K steps) where it can go
+wrong: token counts around the tile widths, weight rows that are no multiple of 4, 16 or 128 (narrow stores), a K of one
+short step, and row blocks few enough for every split.  Against the CPU oracle on the GPU quantiser's bytes; the result
+is one BF16 rounding of an fp32 sum, so it may differ from the oracle's by flipped roundings only: the relative L2 error
+of outputs that all flipped would be 2^-8 / sqrt(12) = 1.1e-3."""
+import numpy as np
+import pytest
+
+from helpers import from_torch_bf16, make_activations, make_weight, to_torch_bf16
+
+pytestmark = pytest.mark.gpu
+
+REL_L2_TOL = 1e-3
+
+SHAPES = [
+    # m, n, k
+    (1, 1, 64), (1, 3, 4096), (15, 127, 192), (16, 129, 512), (17, 108, 5760),  # split 1 .. 8, one short K step
+    (63, 512, 2304), (64, 512, 2304), (65, 512, 4672), (127, 250, 9216), (128, 256, 9216),  # 64- and 128-token tiles
+    (129, 2560, 320), (255, 1022, 1024), (300, 1001, 704),  # several token tiles, the last one partial
+    (1000, 3584, 256),  # more tiles than SMs
+]
+
+
+@pytest.mark.parametrize("residual", [False, True])
+@pytest.mark.parametrize("m,n,k", SHAPES)
+def test_against_oracle(engine, oracle, m, n, k, residual):
+    import torch
+
+    _, codes, scales, s2 = make_weight(n, k, seed=m + n + k)
+    xb = make_activations(m, k, m + 1, outlier_frac=0.001)
+    w = engine.Nvfp4Weight.from_host(codes, scales, s2)
+    a_codes, a_scales, g = engine.quantize_activations(to_torch_bf16(xb))
+    # a residual whose rows start at an odd address: the narrow path on an output that is aligned
+    wide = torch.randn((m, n + 1), generator=torch.Generator(device="cuda").manual_seed(m), device="cuda").to(torch.bfloat16)
+    res = wide[:, 1:] if residual else None
+    c = engine.gemm_w4a4(w, a_codes, a_scales, g, m, residual=res)
+    assert engine.gemm_default_status() == 0
+    e_codes, e_scales, e_g = oracle.quantize_nvfp4(xb)
+    eb, ef = oracle.gemm_w4a4(codes, scales, s2, e_codes, e_scales, e_g, threads=8)
+    want = oracle.bf16_to_f32(eb)
+    if residual:
+        want = torch.from_numpy(np.asarray(ef) + res.float().cpu().numpy()).to(torch.bfloat16).float().numpy()
+    err = oracle.rel_l2(oracle.bf16_to_f32(from_torch_bf16(c)), want)
+    assert err <= REL_L2_TOL, (m, n, k, err)
+
+
+@pytest.mark.parametrize("m", [1, 33, 100, 200, 513])
+@pytest.mark.parametrize("inter,k", [(64, 64), (192, 4096), (1000, 512)])
+def test_gate_up_matches_its_halves(engine, oracle, m, inter, k):
+    """silu(gate) * up of the fused epilogue against the two halves projected on their own (BF16 outputs): two roundings of
+    2^-9 on its inputs and one on the result, and silu's slope is at most 1.1."""
+    import torch
+
+    _, gc, gs, g2 = make_weight(inter, k, seed=inter + k)
+    _, uc, us, u2 = make_weight(inter, k, seed=inter + k + 1)
+    a = engine.quantize_activations(to_torch_bf16(make_activations(m, k, m)))
+    fused = engine.gemm_w4a4(engine.Nvfp4Weight.gate_up_from_host(gc, gs, g2, uc, us, u2), *a, m)
+    gate = engine.gemm_w4a4(engine.Nvfp4Weight.from_host(gc, gs, g2), *a, m).double()
+    up = engine.gemm_w4a4(engine.Nvfp4Weight.from_host(uc, us, u2), *a, m).double()
+    want = gate / (1 + torch.exp(-gate)) * up
+    assert engine.gemm_default_status() == 0
+    assert float((fused.double() - want).norm() / want.norm()) <= 3 * 2.0 ** -9
