@@ -321,7 +321,8 @@ int q35b_gemv_w4a16_bf16(const q35b_weight * w, const void * x_bf16, int m, void
       if (wm->stream_batch[m] == nullptr) {
         // first use with this token count: build (and upload) the single-projection work list
         q35b_gemv_item item{w, nullptr, nullptr, nullptr, 0};
-        if (const int st = gemv_batch_build(&item, 1, m, &wm->stream_batch[m])) return st;
+        // whole tiles only: calls from several threads and streams run this list at the same time
+        if (const int st = gemv_batch_build(&item, 1, m, false, &wm->stream_batch[m])) return st;
       }
       batch = wm->stream_batch[m];
     }
@@ -333,7 +334,7 @@ int q35b_gemv_w4a16_bf16(const q35b_weight * w, const void * x_bf16, int m, void
 size_t q35b_gemv_item_bytes(void) { return sizeof(q35b_gemv_item); }
 
 int q35b_gemv_batch_create(const q35b_gemv_item * items, int count, int m, q35b_gemv_batch ** out) {
-  return gemv_batch_build(items, count, m, out);
+  return gemv_batch_build(items, count, m, true, out);
 }
 
 int q35b_gemv_batch_create_tensor(const q35b_gemv_item * items, int count, int m, int digits, q35b_gemv_batch ** out) {

@@ -105,7 +105,9 @@ int launch_tile_scales(const uint8_t * scales_rowmajor, int rows, int scale_cols
 
 // gemv_stream.cu
 bool gemv_stream_eligible(const q35b_weight * w, int m);
-int gemv_batch_build(const q35b_gemv_item * items, int count, int m, struct q35b_gemv_batch ** out);
+// share_tiles: let several CTAs share a tile's K steps through counters and sums that belong to the list, whose runs then
+// must not overlap
+int gemv_batch_build(const q35b_gemv_item * items, int count, int m, bool share_tiles, struct q35b_gemv_batch ** out);
 int gemv_batch_build_tensor(const q35b_gemv_item * items, int count, int m, int digits, struct q35b_gemv_batch ** out);
 int gemv_batch_launch(const struct q35b_gemv_batch * b, const void * x_override, void * y_override, cudaStream_t s);
 void gemv_batch_free(struct q35b_gemv_batch * b);

@@ -71,8 +71,6 @@ constexpr int kDenseFrom = 5;  // token count from which the dense MMA mapping (
                                // two to four tokens the (block, token) mapping is 4-7 % faster
 __host__ __device__ constexpr int x_pad(int m_tokens) { return m_tokens >= kDenseFrom ? 32 : 16; }
 
-enum Epilogue : int { kEpiPlain = 0, kEpiGateUp = 1 };
-
 enum StatusCode : unsigned { kProducerWait = 11, kPrepWait = 12, kConsumerWait = 13, kConsumerXWait = 14, kDependencyWait = 15 };
 
 struct alignas(128) GemvItem {
@@ -86,26 +84,34 @@ struct alignas(128) GemvItem {
   float s2;
 };
 
-// Everything a CTA needs to know about one tile, staged in shared memory at kernel start so that no role chases
-// pointers through global memory at a tile boundary.
+// Everything a CTA needs to know about one tile, or about its part of a tile whose K steps are shared by several CTAs,
+// staged in shared memory at kernel start so that no role chases pointers through global memory at a tile boundary.
+// The order matters: with the fields that only shared tiles need in front of those every tile reads, a 4B-class step of
+// four tokens took 345 us instead of 341.
 struct alignas(16) GemvTile {
   int item;
   int row_block;
-  int k;
-  int k_steps;
+  int k;                           // columns of the projection
+  int k_steps;                     // K steps of this part, from k_step0 on
   int rows;
   float s2;
-  const uint8_t * scales;        // tiled scales of this row block
-  const uint8_t * codes;         // first code byte of this row block
+  const uint8_t * scales;          // tiled scales of this row block, from its first K step on
   const __nv_bfloat16 * x;
   __nv_bfloat16 * y;
   const __nv_bfloat16 * residual;  // NULL or [m, rows]: added before the BF16 rounding
   float s2_up;                     // gate/up weight: weight_scale_2 of the up rows
-  int epilogue;                    // kEpiPlain | kEpiGateUp
+  int flags;                       // kFlagGateUp | kFlagSignal
+  int k_step0;
+  int x0, x_len;                   // columns of the activations this CTA needs for this item (all its parts of it)
   int wait_item;                   // -1, or the item whose output this item's activations are
   unsigned int wait_count;         // completions that item reports per run (its tiles x 8 storing warps)
-  int signal;                      // nonzero: another item waits for this one, count every stored tile part
+  int split;                       // arrival counters of a shared tile
+  int slot0;                       // first of its slots of partial sums
+  unsigned short part, parts;      // this part, and how many the tile has (1: not shared)
 };
+static_assert(sizeof(GemvTile) == 96, "tile descriptors are copied as 16-byte words and planned for in shared memory");
+constexpr int kFlagGateUp = 1;   // rows alternate 8 gate / 8 up
+constexpr int kFlagSignal = 2;   // another item waits for this one: count every stored tile part
 
 __device__ __forceinline__ uint32_t smem_u32(const void * p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 
@@ -191,14 +197,42 @@ __device__ __forceinline__ float ue4m3_to_f32(uint32_t byte) {
   return __uint_as_float(byte * 0x100000u) * 0x1p120f;
 }
 
-// MT = number of 4-token groups (1 for M <= 4, 2 for M <= 8).
-template <int MT, int KS>
+// A tile whose K steps several CTAs share: every storing warp leaves its scaled sums (each part has its own fp16 scales;
+// `slots` is the first part's 512 bytes of this warp's row group, the next part's follow eight row groups on) and the
+// last one of its row group to arrive adds them all in part order and gets true.  Nobody waits.  Out of line: it runs
+// a few times per CTA, and inline it made every other tile slower (2-3 % of a step at four and eight tokens).
+__device__ __noinline__ bool meet_parts(float4 & sum, float * slots, unsigned int * arrival, int part, int parts, int lane) {
+  float4 * mine = reinterpret_cast<float4 *>(slots) + lane;
+  constexpr int kNext = kRowGroups * 32;  // float4s between parts
+  mine[part * kNext] = sum;
+  __threadfence();
+  __syncwarp();
+  unsigned int before = 0;
+  if (lane == 0) before = atomicAdd(arrival, 1u);
+  if (__shfl_sync(0xffffffffu, before, 0) != static_cast<unsigned int>(parts - 1)) return false;
+  __threadfence();
+  if (lane == 0) *arrival = 0u;  // for the next run
+  sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 4
+  for (int p = 0; p < parts; ++p) {
+    const float4 o = __ldcg(mine + p * kNext);
+    sum.x += o.x;
+    sum.y += o.y;
+    sum.z += o.z;
+    sum.w += o.w;
+  }
+  return true;
+}
+
+// MT = number of 4-token groups (1 for M <= 4, 2 for M <= 8).  SHARED: some tiles of the list are shared by several CTAs
+// (compiled in everywhere, that part of the epilogue made a step whose tiles are whole 1-2 % slower).
+template <int MT, int KS, bool SHARED>
 __global__ void __launch_bounds__(cta_threads(KS), ctas_per_sm(KS))
 gemv_w4a16_stream_kernel(const GemvItem * __restrict__ items, const GemvTile * __restrict__ tiles,
                          const int * __restrict__ cta_begin, int m_tokens, const __nv_bfloat16 * x_override,
                          __nv_bfloat16 * y_override, int stages, int x_buf_halfs, int xs_buf_floats,
                          int x_bufs, unsigned long long * item_done,
-                         int counted_items, unsigned int * status, uint32_t wait_limit, unsigned int wait_extra) {
+                         int counted_items, float * partials, unsigned int * arrivals, unsigned int * status, uint32_t wait_limit, unsigned int wait_extra) {
   constexpr bool kDense = (MT == 2);  // five to eight tokens: dense MMA mapping
   constexpr int kConsumerWarps = consumer_warps(KS);
   constexpr int kConsumerShift = KS == 2 ? 4 : 3;  // log2(kConsumerWarps)
@@ -273,7 +307,7 @@ gemv_w4a16_stream_kernel(const GemvItem * __restrict__ items, const GemvTile * _
         const CUtensorMap * tmap = &items[tile->item].tmap;
         const int k_steps = tile->k_steps;
         const uint8_t * sc = tile->scales;
-        const int row0 = tile->row_block * kTileRows;
+        const int row0 = tile->row_block * kTileRows, byte0 = SHARED ? tile->k_step0 * kStepBytes : 0;
         for (int ks = 0; ks < k_steps; ++ks) {
           if (!mbar_wait(smem_u32(empty + stage), phase ^ 1, wait_limit)) {
             atomicCAS(status, 0u, kProducerWait);
@@ -283,7 +317,7 @@ gemv_w4a16_stream_kernel(const GemvItem * __restrict__ items, const GemvTile * _
           const uint32_t bar = smem_u32(full + stage);
           uint8_t * dst = ring + stage * kStageBytes;
           mbar_expect_tx(bar, kStageBytes);
-          tma_load_2d(smem_u32(dst), tmap, bar, ks * kStepBytes, row0);
+          tma_load_2d(smem_u32(dst), tmap, bar, byte0 + ks * kStepBytes, row0);
           bulk_load(smem_u32(dst + kCodesBytes), sc + static_cast<size_t>(ks) * kScaleBytes, kScaleBytes, bar);
           if (++stage == stages) {
             stage = 0;
@@ -345,14 +379,14 @@ gemv_w4a16_stream_kernel(const GemvItem * __restrict__ items, const GemvTile * _
         break;
       }
       if (lane == 0) {
-        const int k = tile->k;
+        const int k = tile->k, len = SHARED ? tile->x_len : k;
         const uint32_t bar = smem_u32(xfull + buf);
-        const __nv_bfloat16 * x = x_override != nullptr ? x_override : tile->x;
+        const __nv_bfloat16 * x = (x_override != nullptr ? x_override : tile->x) + (SHARED ? tile->x0 : 0);
         __half * xb = xbuf + buf * x_buf_halfs;
-        mbar_expect_tx(bar, static_cast<uint32_t>(m_tokens) * k * 2u);
+        mbar_expect_tx(bar, static_cast<uint32_t>(m_tokens) * len * 2u);
         for (int token = 0; token < m_tokens; ++token) {
-          bulk_load(smem_u32(xb + static_cast<size_t>(token) * (k + x_pad(m_tokens))), x + static_cast<size_t>(token) * k,
-                    static_cast<uint32_t>(k) * 2u, bar);
+          bulk_load(smem_u32(xb + static_cast<size_t>(token) * (len + x_pad(m_tokens))), x + static_cast<size_t>(token) * k,
+                    static_cast<uint32_t>(len) * 2u, bar);
         }
       }
       ++xi;
@@ -418,9 +452,10 @@ gemv_w4a16_stream_kernel(const GemvItem * __restrict__ items, const GemvTile * _
           // shared memory.  Both meeting points are bounded mbarrier waits.
           const int tshift = m_tokens > 4 ? 3 : (m_tokens > 2 ? 2 : (m_tokens > 1 ? 1 : 0));
           const int ctoken = cw & ((1 << tshift) - 1);
-          const int khalf = tile->k >> (kConsumerShift - tshift);  // columns per slice
+          const int x_len = SHARED ? tile->x_len : tile->k;
+          const int khalf = x_len >> (kConsumerShift - tshift);  // columns per slice
           const bool live = ctoken < m_tokens;
-          __half * crow = xbuf + buf * x_buf_halfs + static_cast<size_t>(ctoken) * (tile->k + x_pad(m_tokens)) + (cw >> tshift) * khalf;
+          __half * crow = xbuf + buf * x_buf_halfs + static_cast<size_t>(ctoken) * (x_len + x_pad(m_tokens)) + (cw >> tshift) * khalf;
           const uint32_t par = xi & 1;
           uint32_t amax_bits = 0;
           if (live) {
@@ -477,8 +512,8 @@ gemv_w4a16_stream_kernel(const GemvItem * __restrict__ items, const GemvTile * _
         ++xi;
       }
       const int k_steps = tile->k_steps;
-      const int xstride = tile->k + x_pad(m_tokens);
-      const __half * xb = xbuf + buf * x_buf_halfs;
+      const int xstride = (SHARED ? tile->x_len : tile->k) + x_pad(m_tokens);
+      const __half * xb = xbuf + buf * x_buf_halfs + (SHARED ? tile->k_step0 * 256 - tile->x0 : 0);
       const float * xs = xsbuf + buf * xs_buf_floats;
 
       float acc[MT][4];
@@ -590,6 +625,7 @@ gemv_w4a16_stream_kernel(const GemvItem * __restrict__ items, const GemvTile * _
         for (int i = 0; i < 4; ++i) acc[0][i] += acc[1][i];
       }
       constexpr int kGroups = kDense ? 1 : MT;  // float4 groups of sums a lane carries into the epilogue
+      static_assert(kGroups == 1, "the epilogue handles four sums per lane");
 
       // Meet the partner warp's half-K sums in shared memory (double-buffered by tile parity): the kh = 1 warp
       // writes, the kh = 0 warp adds, combines the two block halves (lanes t and t^2) and stores.
@@ -627,51 +663,59 @@ gemv_w4a16_stream_kernel(const GemvItem * __restrict__ items, const GemvTile * _
         }
         __nv_bfloat16 * y = y_override != nullptr ? y_override : tile->y;
         const int rows = tile->rows;
-        const float s2 = tile->s2;
+        const bool gate_up = (tile->flags & kFlagGateUp) != 0;
+        const float s2 = tile->s2, s2_up = gate_up ? tile->s2_up : s2;  // of rows r0 and r0 + 8
         const int row_a = tile->row_block * kTileRows + r0;
         const __nv_bfloat16 * residual = tile->residual;
-        const bool gate_up = tile->epilogue == kEpiGateUp;
-        const float s2_up = tile->s2_up;
+        const int parts = SHARED ? tile->parts : 1;
+        if constexpr (!kDense) {
+          // the two block halves of a chunk sit in lanes t and t ^ 2
 #pragma unroll
-        for (int ts = 0; ts < kGroups; ++ts) {
-          if constexpr (!kDense) {
-            // the two block halves of a chunk sit in lanes t and t ^ 2
+          for (int i = 0; i < 4; ++i) acc[0][i] += __shfl_xor_sync(0xffffffffu, acc[0][i], 2);
+        }
+        if (parts > 1) {
+          const int tok = 2 * (kDense ? t : t & 1);
+          const float u0 = xs[tok] * (kDense ? 256.0f : 1.0f), u1 = xs[tok + 1] * (kDense ? 256.0f : 1.0f);
+          float4 sum = make_float4(acc[0][0] * (u0 * s2), acc[0][1] * (u1 * s2), acc[0][2] * (u0 * s2_up), acc[0][3] * (u1 * s2_up));
+          if (!meet_parts(sum, partials + (static_cast<size_t>(tile->slot0) * kRowGroups + rg) * 128,
+                          arrivals + tile->split * kRowGroups + rg, tile->part, parts, lane)) continue;
+          acc[0][0] = sum.x;
+          acc[0][1] = sum.y;
+          acc[0][2] = sum.z;
+          acc[0][3] = sum.w;
+        }
+        // dense: this lane holds tokens 2t, 2t+1 of rows r0 and r0 + 8, with the block scales' 2^-8 still in
+        if (kDense || t < 2) {
+          const int tok0 = 2 * t;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) acc[ts][i] += __shfl_xor_sync(0xffffffffu, acc[ts][i], 2);
-          }
-          if (kDense || t < 2) {
-            // dense: this lane holds tokens 2t, 2t+1 of rows r0 and r0 + 8, with the block scales' 2^-8 still in
-            const int tok0 = kDense ? 2 * t : 4 * ts + 2 * t;
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-              if (tok0 + e < m_tokens) {
-                const float unscale = xs[tok0 + e] * (kDense ? 256.0f : 1.0f);  // undoes the token's fp16 scaling
-                if (gate_up) {
-                  // rows alternate 8 gate / 8 up: this lane's row r0 is gate row j, its row r0 + 8 the matching up row
-                  const int j = (row_a >> 4) * 8 + (row_a & 7);
-                  if (row_a + 8 < rows) {
-                    const float gate = acc[ts][e] * (unscale * s2);
-                    const float up = acc[ts][2 + e] * (unscale * s2_up);
-                    y[static_cast<size_t>(tok0 + e) * (rows >> 1) + j] = __float2bfloat16_rn(gate / (1.0f + expf(-gate)) * up);
-                  }
-                } else {
-                  const float f = unscale * s2;
-                  if (row_a < rows) {
-                    const size_t o = static_cast<size_t>(tok0 + e) * rows + row_a;
-                    const float r = residual != nullptr ? __bfloat162float(residual[o]) : 0.0f;
-                    y[o] = __float2bfloat16_rn(acc[ts][e] * f + r);
-                  }
-                  if (row_a + 8 < rows) {
-                    const size_t o = static_cast<size_t>(tok0 + e) * rows + row_a + 8;
-                    const float r = residual != nullptr ? __bfloat162float(residual[o]) : 0.0f;
-                    y[o] = __float2bfloat16_rn(acc[ts][2 + e] * f + r);
-                  }
+          for (int e = 0; e < 2; ++e) {
+            if (tok0 + e < m_tokens) {
+              const float unscale = xs[tok0 + e] * (kDense ? 256.0f : 1.0f);  // undoes the token's fp16 scaling
+              if (gate_up) {
+                // rows alternate 8 gate / 8 up: this lane's row r0 is gate row j, its row r0 + 8 the matching up row
+                const int j = (row_a >> 4) * 8 + (row_a & 7);
+                if (row_a + 8 < rows) {
+                  const float gate = acc[0][e] * (parts > 1 ? 1.0f : unscale * s2);
+                  const float up = acc[0][2 + e] * (parts > 1 ? 1.0f : unscale * s2_up);
+                  y[static_cast<size_t>(tok0 + e) * (rows >> 1) + j] = __float2bfloat16_rn(gate / (1.0f + expf(-gate)) * up);
+                }
+              } else {
+                const float f = parts > 1 ? 1.0f : unscale * s2;
+                if (row_a < rows) {
+                  const size_t o = static_cast<size_t>(tok0 + e) * rows + row_a;
+                  const float r = residual != nullptr ? __bfloat162float(residual[o]) : 0.0f;
+                  y[o] = __float2bfloat16_rn(acc[0][e] * f + r);
+                }
+                if (row_a + 8 < rows) {
+                  const size_t o = static_cast<size_t>(tok0 + e) * rows + row_a + 8;
+                  const float r = residual != nullptr ? __bfloat162float(residual[o]) : 0.0f;
+                  y[o] = __float2bfloat16_rn(acc[0][2 + e] * f + r);
                 }
               }
             }
           }
         }
-        if (tile->signal) {
+        if ((tile->flags & kFlagSignal) != 0) {
           // another item of this run reads these outputs: make the stores visible, then count this warp's part
           __threadfence();
           __syncwarp();
@@ -740,11 +784,15 @@ bool make_plan(int m, int max_k, Plan * p, int min_ks = 1) {
 }
 
 using StreamKernel = void (*)(const GemvItem *, const GemvTile *, const int *, int, const __nv_bfloat16 *, __nv_bfloat16 *,
-                              int, int, int, int, unsigned long long *, int, unsigned int *, uint32_t, unsigned int);
+                              int, int, int, int, unsigned long long *, int, float *, unsigned int *, unsigned int *, uint32_t, unsigned int);
 
-StreamKernel stream_kernel(int m, int ks) {
-  if (m < kDenseFrom) return ks == 1 ? gemv_w4a16_stream_kernel<1, 1> : gemv_w4a16_stream_kernel<1, 2>;
-  return ks == 1 ? gemv_w4a16_stream_kernel<2, 1> : gemv_w4a16_stream_kernel<2, 2>;
+StreamKernel stream_kernel(int m, int ks, bool shared) {
+  if (shared) {
+    if (m < kDenseFrom) return ks == 1 ? gemv_w4a16_stream_kernel<1, 1, true> : gemv_w4a16_stream_kernel<1, 2, true>;
+    return ks == 1 ? gemv_w4a16_stream_kernel<2, 1, true> : gemv_w4a16_stream_kernel<2, 2, true>;
+  }
+  if (m < kDenseFrom) return ks == 1 ? gemv_w4a16_stream_kernel<1, 1, false> : gemv_w4a16_stream_kernel<1, 2, false>;
+  return ks == 1 ? gemv_w4a16_stream_kernel<2, 1, false> : gemv_w4a16_stream_kernel<2, 2, false>;
 }
 
 // The plan for a list on the current device: the two-CTAs-per-SM shape only if two of its CTAs really fit on an SM
@@ -752,20 +800,26 @@ StreamKernel stream_kernel(int m, int ks) {
 cudaError_t plan_for_device(int m, int max_k, Plan * p, bool * fits) {
   *fits = make_plan(m, max_k, p);
   if (!*fits) return cudaSuccess;
-  cudaError_t e = cudaFuncSetAttribute(stream_kernel(m, p->ksplit), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       smem_budget(p->ksplit));
-  if (e != cudaSuccess) return e;
-  if (p->ksplit == 1) {
+  for (const bool shared : {false, true}) {
+    cudaError_t e = cudaFuncSetAttribute(stream_kernel(m, p->ksplit, shared), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         smem_budget(p->ksplit));
+    if (e != cudaSuccess) return e;
+    if (p->ksplit == 2) continue;
     int resident = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, stream_kernel(m, 1), cta_threads(1),
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, stream_kernel(m, 1, shared), cta_threads(1),
                                                       static_cast<size_t>(p->smem_bytes));
     if (e != cudaSuccess) return e;
     if (resident < 2) {
       *fits = make_plan(m, max_k, p, 2);
-      if (*fits) e = cudaFuncSetAttribute(stream_kernel(m, 2), cudaFuncAttributeMaxDynamicSharedMemorySize, smem_budget(2));
+      if (!*fits) return cudaSuccess;
+      for (const bool sh : {false, true}) {
+        e = cudaFuncSetAttribute(stream_kernel(m, 2, sh), cudaFuncAttributeMaxDynamicSharedMemorySize, smem_budget(2));
+        if (e != cudaSuccess) return e;
+      }
+      return cudaSuccess;
     }
   }
-  return e;
+  return cudaSuccess;
 }
 
 }  // namespace
@@ -785,7 +839,11 @@ struct q35b_gemv_batch {
   int * cta_begin = nullptr;
   unsigned int * status = nullptr;
   unsigned long long * item_done = nullptr;  // per item: storing warps that finished a tile in the current run
+  unsigned int * arrivals = nullptr;         // per shared tile and row group: parts that have left their sums
+  float * partials = nullptr;                // the parts' sums
+  size_t counter_bytes = 0;                  // status, item_done and arrivals, contiguous and zero between runs
   bool has_dependencies = false;
+  bool shared = false;                       // some tiles are shared by several CTAs
   size_t bytes_per_run = 0;
   uint32_t wait_limit = kWaitLimit;   // polls every device-side wait of a run may take
   unsigned int wait_extra = 0;        // test hook: completions demanded on top of what a dependency really delivers
@@ -811,7 +869,117 @@ int gemv_plan_debug(int m, int max_k, int * ctas, int * ring_stages, int * activ
   return Q35B_OK;
 }
 
-int gemv_batch_build(const q35b_gemv_item * items, int count, int m, q35b_gemv_batch ** out) {
+namespace {
+
+// What each CTA of a grid of `grid` does: contiguous runs of tiles (projection-major order) of about equal cost, level
+// by level (a CTA changes projection, and converts a new activation vector, as rarely as possible, and neighbouring
+// CTAs stream neighbouring rows; an item's level is one more than that of the item it runs after, and every level is
+// spread over all CTAs by itself, so that the whole grid works on the tiles something is waiting for).
+//
+// A tile goes to the CTA in whose share of the total its midpoint falls.  With whole tiles the down projection of one
+// layer, [2560, 9216], keeps 20 of 296 CTAs busy for 36 K steps each.  So where a level has fewer tiles than the grid has
+// CTAs, a CTA's share ends where it ends, inside a tile if need be, and the tile's parts meet in memory at the end (MLP
+// block [2560, 9216] at two tokens 40 -> 25 us, [512, 8192] 24 -> 15).  From five tokens on the conversion of the weights
+// bounds a CTA rather than the bandwidth all CTAs share, and an even split pays up to four tiles per CTA (a step of 41 us
+// at seven tokens 38); with fewer tokens the CTAs that finish early leave their bandwidth to the others, and meeting costs
+// more than it saves (steps of 19 us at one and two tokens: 20 and 22).
+// A part has at least kMinPart steps (parts of four or more: the blocks above 25 and 15 us, [3584, 3328] 24 instead of 20).
+// A level whose tiles are all short stays whole: meeting takes about as long as eight steps of a CTA that has an SM's
+// bandwidth to itself ([512, 1280] at four tokens 10.7 us whole, 12.5 shared; [768, 2048] 13.5 and 13.7).
+constexpr int kMinPart = 2;
+constexpr int kWholeSteps = 8;
+
+struct Assignment {
+  std::vector<std::vector<GemvTile>> per_cta;
+  int splits = 0, slots = 0;  // shared tiles, and parts of shared tiles
+  int max_x = 0;              // most activation columns any CTA needs of an item
+};
+
+Assignment assign_tiles(const std::vector<GemvTile> & all, const std::vector<int> & level, int max_level, int grid, int m, bool share_tiles) {
+  Assignment out;
+  out.per_cta.resize(grid);
+  for (int lv = 0; lv <= max_level; ++lv) {
+    long total = 0;
+    int tiles = 0, longest = 0;
+    for (const GemvTile & tl : all) {
+      if (level[tl.item] != lv) continue;
+      total += tl.k_steps + 1;
+      ++tiles;
+      longest = std::max(longest, tl.k_steps);
+    }
+    const bool share = share_tiles && longest > kWholeSteps && (tiles < grid || (m >= kDenseFrom && tiles < 4 * grid));
+    long done = 0;
+    int c = 0;
+    for (const GemvTile & tl : all) {
+      if (level[tl.item] != lv) continue;
+      const int cost = tl.k_steps + 1;
+      if (!share) {
+        while (c + 1 < grid && (done + cost / 2) * grid >= static_cast<long>(c + 1) * total) ++c;
+        out.per_cta[c].push_back(tl);
+        done += cost;
+        continue;
+      }
+      while (c + 1 < grid && (static_cast<long>(c + 1) * total + grid / 2) / grid <= done) ++c;  // shares that are full
+      std::vector<std::pair<int, int>> cuts;  // (CTA, end step) of the parts so far
+      int begin = 0;
+      while (begin < tl.k_steps) {
+        // where CTA c's share ends, in steps of this tile
+        const long end_cost = (static_cast<long>(c + 1) * total + grid / 2) / grid - done;
+        int end = c + 1 < grid ? static_cast<int>(std::min<long>(std::max<long>(end_cost, 0), tl.k_steps)) : tl.k_steps;
+        if (tl.k_steps - end < kMinPart) end = tl.k_steps;
+        if (end - begin >= kMinPart || (end == tl.k_steps && begin == 0)) {
+          cuts.emplace_back(c, end);
+          begin = end;
+        } else if (end == tl.k_steps && !cuts.empty()) {
+          cuts.back().second = end;  // too short a rest for the next CTA
+          begin = end;
+        }
+        if (begin < tl.k_steps || end_cost <= cost) c = std::min(c + 1, grid - 1);
+      }
+      done += cost;
+      if (cuts.size() > 1) ++out.splits;
+      int step = 0;
+      for (size_t i = 0; i < cuts.size(); ++i) {
+        GemvTile part = tl;
+        part.k_step0 = step;
+        part.k_steps = cuts[i].second - step;
+        part.scales = tl.scales + static_cast<size_t>(step) * kScaleBytes;
+        part.part = static_cast<unsigned short>(i);
+        part.parts = static_cast<unsigned short>(cuts.size());
+        part.split = out.splits - 1;
+        part.slot0 = out.slots;
+        step = cuts[i].second;
+        out.per_cta[cuts[i].first].push_back(part);
+      }
+      if (cuts.size() > 1) out.slots += static_cast<int>(cuts.size());
+    }
+  }
+  for (auto & tiles : out.per_cta) {
+    std::stable_sort(tiles.begin(), tiles.end(), [&](const GemvTile & a, const GemvTile & d) {
+      if (level[a.item] != level[d.item]) return level[a.item] < level[d.item];
+      return a.item != d.item ? a.item < d.item : a.row_block < d.row_block;
+    });
+    // the columns of an item's activations that any of the CTA's parts of it reads
+    for (size_t i = 0; i < tiles.size();) {
+      size_t j = i;
+      int lo = tiles[i].k_step0, hi = lo;
+      for (; j < tiles.size() && tiles[j].item == tiles[i].item; ++j) {
+        lo = std::min(lo, tiles[j].k_step0);
+        hi = std::max(hi, tiles[j].k_step0 + tiles[j].k_steps);
+      }
+      for (; i < j; ++i) {
+        tiles[i].x0 = lo * 256;
+        tiles[i].x_len = (hi - lo) * 256;
+      }
+      out.max_x = std::max(out.max_x, (hi - lo) * 256);
+    }
+  }
+  return out;
+}
+
+}  // namespace
+
+int gemv_batch_build(const q35b_gemv_item * items, int count, int m, bool share_tiles, q35b_gemv_batch ** out) {
   if (items == nullptr || out == nullptr || count <= 0) return fail(Q35B_ERR_ARGUMENT, "Invalid NVFP4 projection work list.");
   if (m < 1 || m > 8) return fail(Q35B_ERR_SHAPE, "NVFP4 decode projection supports 1..8 tokens.");
   *out = nullptr;
@@ -848,10 +1016,10 @@ int gemv_batch_build(const q35b_gemv_item * items, int count, int m, q35b_gemv_b
     delete b;
     return fail(Q35B_ERR_SHAPE, "Activations of the NVFP4 projection work list do not fit in shared memory.");
   }
-  const int grid_max = sm_count() * ctas_per_sm(b->plan.ksplit);
 
   std::vector<GemvTile> all;
   std::vector<GemvItem> h_items(count);
+  long total_steps = 0;
   for (int i = 0; i < count; ++i) {
     const q35b_weight * w = items[i].weight;
     GemvItem & it = h_items[i];
@@ -866,33 +1034,32 @@ int gemv_batch_build(const q35b_gemv_item * items, int count, int m, q35b_gemv_b
     it.k = w->k;
     it.k_steps = w->k / 256;
     it.s2 = w->s2;
+    bool signal = false;
+    for (int j = i + 1; j < count; ++j) signal = signal || items[j].after - 1 == i;
     for (int rb = 0; rb < (w->rows + kTileRows - 1) / kTileRows; ++rb) {
-      GemvTile tl;
+      GemvTile tl = {};
       tl.item = i;
       tl.row_block = rb;
       tl.k = w->k;
       tl.k_steps = it.k_steps;
+      tl.x_len = w->k;
       tl.rows = w->rows;
       tl.s2 = w->s2;
       tl.scales = w->scales_tiled + static_cast<size_t>(rb) * it.k_steps * kScaleBytes;
-      tl.codes = w->codes + static_cast<size_t>(rb) * kTileRows * (w->k / 2);
       tl.x = it.x;
       tl.y = it.y;
       tl.residual = static_cast<const __nv_bfloat16 *>(items[i].residual_bf16);
       tl.s2_up = w->s2_up;
-      tl.epilogue = w->gate_up ? kEpiGateUp : kEpiPlain;
+      tl.flags = (w->gate_up ? kFlagGateUp : 0) | (signal ? kFlagSignal : 0);
       tl.wait_item = items[i].after - 1;
-      tl.wait_count = 0;
-      tl.signal = 0;
+      tl.parts = 1;
       if (tl.wait_item >= 0) {
         const q35b_weight * dep = items[tl.wait_item].weight;
         tl.wait_count = static_cast<unsigned int>((dep->rows + kTileRows - 1) / kTileRows) * kRowGroups;
         b->has_dependencies = true;
       }
-      for (int j = i + 1; j < count; ++j) {
-        if (items[j].after - 1 == i) tl.signal = 1;
-      }
       all.push_back(tl);
+      total_steps += it.k_steps;
     }
     b->bytes_per_run += w->codes_bytes + w->scales_bytes;
   }
@@ -902,48 +1069,54 @@ int gemv_batch_build(const q35b_gemv_item * items, int count, int m, q35b_gemv_b
     if (items[i].after > 0) level[i] = level[items[i].after - 1] + 1;
     max_level = std::max(max_level, level[i]);
   }
-  const int grid = std::max(1, std::min<int>(grid_max, static_cast<int>(all.size())));
-  std::vector<std::vector<GemvTile>> per_cta(grid);
-  {
-    // Each CTA gets a contiguous run of tiles (projection-major order) of about equal cost: it changes projection,
-    // and therefore converts a new activation vector, as rarely as possible, and neighbouring CTAs stream
-    // neighbouring rows.  A tile goes to the CTA in whose share of the total cost its midpoint falls, so no CTA
-    // exceeds its share by more than half a tile.
-    // With dependencies the list is cut into levels (an item's level is one more than that of the item it runs
-    // after): every level is spread over all CTAs in this way by itself, and a CTA walks its levels in order, so the
-    // whole grid works on the tiles something is waiting for instead of a few CTAs owning them.
-    for (int lv = 0; lv <= max_level; ++lv) {
-      long total = 0;
-      for (const GemvTile & tl : all) total += level[tl.item] == lv ? tl.k_steps + 1 : 0;
-      long done = 0;
-      int c = 0;
-      for (const GemvTile & tl : all) {
-        if (level[tl.item] != lv) continue;
-        const long cost = tl.k_steps + 1;
-        while (c + 1 < grid && (done + cost / 2) * grid >= static_cast<long>(c + 1) * total) ++c;
-        per_cta[c].push_back(tl);
-        done += cost;
+  const int most = share_tiles ? static_cast<int>(std::min<long>(total_steps, 1 << 20)) : static_cast<int>(all.size());
+  auto grid_for = [&](int ksplit) { return std::max(1, std::min(sm_count() * ctas_per_sm(ksplit), most)); };
+  int grid = grid_for(b->plan.ksplit);
+  Assignment todo = assign_tiles(all, level, max_level, grid, m, share_tiles);
+  if (todo.splits == 0) {
+    // whole tiles only: no CTA without one
+    share_tiles = false;
+    grid = std::max(1, std::min(grid, static_cast<int>(all.size())));
+    todo = assign_tiles(all, level, max_level, grid, m, false);
+  }
+  if (share_tiles) {
+    // Parts of tiles need only their columns of the activations, so a list may fit the two-CTAs-per-SM shape, a second
+    // activation buffer or a deeper ring although its longest projection would not.
+    for (int ks = 1; ks <= b->plan.ksplit; ++ks) {
+      const int g = grid_for(ks);
+      Assignment a = ks == b->plan.ksplit ? todo : assign_tiles(all, level, max_level, g, m, true);
+      Plan p;
+      bool ok = false;
+      if (const cudaError_t pe = plan_for_device(m, std::max(a.max_x, 256), &p, &ok); pe != cudaSuccess) {
+        delete b;
+        return fail_cuda(pe, "planning the projection work list");
+      }
+      if (ok && p.ksplit == ks) {
+        b->plan = p;
+        grid = g;
+        todo = std::move(a);
+        break;
       }
     }
   }
   std::vector<GemvTile> h_tiles;
   std::vector<int> h_begin(grid + 1, 0);
   for (int c = 0; c < grid; ++c) {
-    std::stable_sort(per_cta[c].begin(), per_cta[c].end(), [&](const GemvTile & a, const GemvTile & d) {
-      if (level[a.item] != level[d.item]) return level[a.item] < level[d.item];
-      return a.item != d.item ? a.item < d.item : a.row_block < d.row_block;
-    });
     h_begin[c] = static_cast<int>(h_tiles.size());
-    for (const GemvTile & tl : per_cta[c]) h_tiles.push_back(tl);
+    for (const GemvTile & tl : todo.per_cta[c]) h_tiles.push_back(tl);
   }
   h_begin[grid] = static_cast<int>(h_tiles.size());
   b->grid = grid;
+  b->shared = todo.splits > 0;
 
   const size_t o_tiles = sizeof(GemvItem) * count;
   const size_t o_begin = (o_tiles + sizeof(GemvTile) * h_tiles.size() + 15) / 16 * 16;
   const size_t o_status = (o_begin + sizeof(int) * (grid + 1) + 15) / 16 * 16;
   const size_t o_done = o_status + 16;
-  const size_t total = o_done + sizeof(unsigned long long) * (count + 1);  // + the finished-CTA count
+  const size_t o_arrivals = o_done + sizeof(unsigned long long) * (count + 1);  // + the finished-CTA count
+  const size_t o_partials = (o_arrivals + sizeof(unsigned int) * kRowGroups * todo.splits + 127) / 128 * 128;
+  const size_t part_bytes = sizeof(float) * kRowGroups * 32 * 4;  // four sums per lane, in either MMA mapping
+  const size_t total = o_partials + part_bytes * todo.slots;
   cudaError_t e = cudaMalloc(&b->dev_base, total);
   if (e != cudaSuccess) {
     delete b;
@@ -955,10 +1128,13 @@ int gemv_batch_build(const q35b_gemv_item * items, int count, int m, q35b_gemv_b
   b->cta_begin = reinterpret_cast<int *>(base + o_begin);
   b->status = reinterpret_cast<unsigned int *>(base + o_status);
   b->item_done = reinterpret_cast<unsigned long long *>(base + o_done);
+  b->arrivals = reinterpret_cast<unsigned int *>(base + o_arrivals);
+  b->partials = reinterpret_cast<float *>(base + o_partials);
+  b->counter_bytes = o_partials - o_status;
   e = cudaMemcpy(b->items, h_items.data(), sizeof(GemvItem) * count, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(b->tiles, h_tiles.data(), sizeof(GemvTile) * h_tiles.size(), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(b->cta_begin, h_begin.data(), sizeof(int) * (grid + 1), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemset(b->status, 0, 16 + sizeof(unsigned long long) * (count + 1));
+  if (e == cudaSuccess) e = cudaMemset(b->status, 0, b->counter_bytes);
   if (e != cudaSuccess) {
     cudaFree(b->dev_base);
     delete b;
@@ -1002,9 +1178,9 @@ int gemv_batch_launch(const q35b_gemv_batch * b, const void * x_override, void *
   const GemvTile * d_tiles = b->tiles;
   const int * d_begin = b->cta_begin;
   const Plan & pl = b->plan;
-  const cudaError_t le = cudaLaunchKernelEx(&cfg, stream_kernel(b->m, pl.ksplit), d_items,
+  const cudaError_t le = cudaLaunchKernelEx(&cfg, stream_kernel(b->m, pl.ksplit, b->shared), d_items,
                                             d_tiles, d_begin, b->m, xo, yo, pl.stages, pl.x_buf_halfs, pl.xs_buf_floats,
-                                            pl.x_bufs, b->item_done, counted, b->status, b->wait_limit,
+                                            pl.x_bufs, b->item_done, counted, b->partials, b->arrivals, b->status, b->wait_limit,
                                             b->wait_extra);
   count_launch();
   Q35B_CUDA_TRY(le, "gemv_w4a16_stream_kernel launch");
@@ -1033,7 +1209,7 @@ int gemv_batch_debug_wait(q35b_gemv_batch * b, unsigned int wait_limit, unsigned
   b->wait_extra = extra_completions;
   // counts of a run that gave up stay behind: start the next run from zero
   if (b->item_done != nullptr) {
-    Q35B_CUDA_TRY(cudaMemset(b->status, 0, 16 + sizeof(unsigned long long) * (b->count + 1)), "cudaMemset(work list counters)");
+    Q35B_CUDA_TRY(cudaMemset(b->status, 0, b->counter_bytes), "cudaMemset(work list counters)");
   }
   return Q35B_OK;
 }
