@@ -7,11 +7,11 @@
 //
 // HBM layout read here: codes [rows, K/2] and scales [rows, K/16], both
 // row-major as in the checkpoint, so a warp that walks a row issues fully
-// coalesced 16-byte loads (32 codes per lane) and 2-byte scale loads.
+// coalesced loads (eight codes per lane).
 //
-// Dequantisation: an E2M1 nibble s|eem placed at fp16 bits 15|11:9 is the
-// value scaled by 2^-14 (exact, fp16 subnormals included); the 2^14 is folded
-// into the per-block scale, which is decoded once per 16 weights.
+// Dequantisation: the FP4 converter of sm_100a turns a byte into two exact
+// fp16 values, widened to fp32; the block scale multiplies the dot product of
+// a lane's eight weights.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -38,42 +38,6 @@ __device__ __forceinline__ float e4m3_to_f32(uint32_t b) {
   return (b & 0x80u) ? -mag : mag;
 }
 
-template <typename XT>
-struct XLoad;
-
-// 32 consecutive activations -> fp32 registers.
-template <>
-struct XLoad<__nv_bfloat16> {
-  static __device__ __forceinline__ void load32(const __nv_bfloat16 * p, float scale, float (&x)[32]) {
-    const uint4 * v = reinterpret_cast<const uint4 *>(p);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const uint4 q = __ldg(v + i);
-      const uint32_t r[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        x[i * 8 + j * 2 + 0] = __uint_as_float(r[j] << 16) * scale;
-        x[i * 8 + j * 2 + 1] = __uint_as_float(r[j] & 0xffff0000u) * scale;
-      }
-    }
-  }
-};
-
-template <>
-struct XLoad<float> {
-  static __device__ __forceinline__ void load32(const float * p, float scale, float (&x)[32]) {
-    const float4 * v = reinterpret_cast<const float4 *>(p);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const float4 q = __ldg(v + i);
-      x[i * 4 + 0] = q.x * scale;
-      x[i * 4 + 1] = q.y * scale;
-      x[i * 4 + 2] = q.z * scale;
-      x[i * 4 + 3] = q.w * scale;
-    }
-  }
-};
-
 __device__ __forceinline__ void store_out(__nv_bfloat16 * p, float v) { *p = __float2bfloat16_rn(v); }
 __device__ __forceinline__ void store_out(float * p, float v) { *p = v; }
 
@@ -96,71 +60,180 @@ __device__ __forceinline__ float block_dot(uint32_t w0, uint32_t w1, const float
   return acc;
 }
 
-// One warp owns RW consecutive rows; lanes stride over K in 32-code (16-byte)
-// pieces; a warp-shuffle tree finishes each (row, token) sum.
-// Requires K % 32 == 0.
-template <int M, int RW, typename XT, typename OT>
-__global__ void __launch_bounds__(kThreads)
-gemv_w4a16_simt_kernel(const uint8_t * __restrict__ codes, const uint8_t * __restrict__ scales,
-                       const XT * __restrict__ x, OT * __restrict__ y, int rows, int k, float s2_scaled,
-                       float x_scale) {
-  // Launched with programmatic stream serialisation: the grid may be scheduled while the previous kernel of the
-  // stream drains (a 2 MB projection is shorter than a launch), but reads and writes nothing before that kernel is
-  // complete and visible.
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  const int lane = threadIdx.x & 31;
-  const int warp = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
-  const int row0 = warp * RW;
-  if (row0 >= rows) return;
-  const int packed_cols = k >> 1;
-  const int scale_cols = k >> 4;
+// Eight E2M1 codes -> four exact fp32 pairs, with the FP4 converter of sm_100a.
+__device__ __forceinline__ void e2m1x8_to_f32(uint32_t w, float2 (&f)[4]) {
+  uint32_t h[4];
+  asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\t"
+      "mov.b32 {b0, b1, b2, b3}, %4;\n\t"
+      "cvt.rn.f16x2.e2m1x2 %0, b0;\n\t"
+      "cvt.rn.f16x2.e2m1x2 %1, b1;\n\t"
+      "cvt.rn.f16x2.e2m1x2 %2, b2;\n\t"
+      "cvt.rn.f16x2.e2m1x2 %3, b3;\n\t}"
+      : "=r"(h[0]), "=r"(h[1]), "=r"(h[2]), "=r"(h[3])
+      : "r"(w));
+#pragma unroll
+  for (int p = 0; p < 4; ++p) f[p] = __half22float2(*reinterpret_cast<const __half2 *>(&h[p]));
+}
 
-  float acc[RW][M];
+// Eight consecutive activations of a lane as four fp32 pairs.
+template <typename XT>
+struct XLoad;
+template <>
+struct XLoad<__nv_bfloat16> {
+  static __device__ __forceinline__ void load8(const __nv_bfloat16 * p, float, float2 (&x)[4]) {
+    const uint4 q = __ldg(reinterpret_cast<const uint4 *>(p));
+    x[0] = make_float2(__uint_as_float(q.x << 16), __uint_as_float(q.x & 0xffff0000u));
+    x[1] = make_float2(__uint_as_float(q.y << 16), __uint_as_float(q.y & 0xffff0000u));
+    x[2] = make_float2(__uint_as_float(q.z << 16), __uint_as_float(q.z & 0xffff0000u));
+    x[3] = make_float2(__uint_as_float(q.w << 16), __uint_as_float(q.w & 0xffff0000u));
+  }
+};
+template <>
+struct XLoad<float> {
+  static __device__ __forceinline__ void load8(const float * p, float scale, float2 (&x)[4]) {
+    const float4 a = __ldg(reinterpret_cast<const float4 *>(p)), b = __ldg(reinterpret_cast<const float4 *>(p) + 1);
+    x[0] = make_float2(a.x * scale, a.y * scale);
+    x[1] = make_float2(a.z * scale, a.w * scale);
+    x[2] = make_float2(b.x * scale, b.y * scale);
+    x[3] = make_float2(b.z * scale, b.w * scale);
+  }
+};
+
+// Two fp32 multiply-adds in one instruction, each rounded as fmaf is.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n\t.reg .b64 a, b, c, d;\n\t"
+      "mov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\t"
+      "fma.rn.f32x2 d, a, b, c;\n\t"
+      "mov.b64 {%0, %1}, d;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+
+// One warp owns RW consecutive rows and walks K in pieces of 256 columns, eight per lane, so that the activations of a
+// piece are one contiguous 16-byte load per lane and token (a lane that takes 32 columns at once, for a 16-byte code
+// load, makes every activation load touch 16 or, in fp32, 32 lines).  The codes and scales of the next two or four pieces
+// are in flight while the current ones are worked on; weights are constant, so the first ones are requested before the
+// previous kernel of the stream has finished.  With few rows KW = 4 warps share a row's pieces, and their sums meet in
+// shared memory in slice order.
+// Bound by the unpacking (half a conversion and a widening per weight) and, from about four tokens on, by the
+// multiply-adds.  Against the 32-columns-per-lane kernel before it, and where K was no multiple of 32 an element-wise
+// one: [3584, 1024] at one token 3.2 -> 2.6 us, [17286, 6720] at one fp32 token 61 -> 27, [9162, 8240] 141 -> 18,
+// [4540, 7536] at two tokens 66 -> 16, [8350, 1536] at eight 32 -> 12.5.
+constexpr int kPiece = 256;
+__host__ __device__ constexpr int pieces_ahead(int m) { return m <= 4 ? 4 : 2; }
+template <int M, int RW, int KW, typename XT, typename OT>
+__global__ void __launch_bounds__(kThreads)
+gemv_w4a16_rows_kernel(const uint8_t * __restrict__ codes, const uint8_t * __restrict__ scales,
+                       const XT * __restrict__ x, OT * __restrict__ y, int rows, int k, float s2,
+                       float x_scale) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int lane = threadIdx.x & 31;
+  constexpr int kAhead = pieces_ahead(M);
+  const int warp = threadIdx.x >> 5, slice = warp % KW;
+  const int row0 = (blockIdx.x * (kWarpsPerBlock / KW) + warp / KW) * RW;
+  const uint8_t * code_row[RW];
+  const uint8_t * scale_row[RW];
+#pragma unroll
+  for (int r = 0; r < RW; ++r) {
+    const int row = min(row0 + r, rows - 1);
+    code_row[r] = codes + static_cast<size_t>(row) * (k >> 1) + lane * 4;
+    scale_row[r] = scales + static_cast<size_t>(row) * (k >> 4) + (lane >> 1);
+  }
+  uint32_t cw[kAhead][RW], sc[kAhead][RW];
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const int c = k0 + u * kPiece;
+#pragma unroll
+      for (int r = 0; r < RW; ++r) {
+        cw[u][r] = 0u;
+        sc[u][r] = 0u;
+        if (c + lane * 8 < k) {
+          cw[u][r] = __ldcs(reinterpret_cast<const uint32_t *>(code_row[r] + (c >> 1)));
+          sc[u][r] = __ldcs(scale_row[r] + (c >> 4));
+        }
+      }
+    }
+  };
+  fetch(slice * kAhead * kPiece);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+
+  float2 acc[RW][M];
 #pragma unroll
   for (int r = 0; r < RW; ++r)
 #pragma unroll
-    for (int m = 0; m < M; ++m) acc[r][m] = 0.0f;
+    for (int m = 0; m < M; ++m) acc[r][m] = make_float2(0.0f, 0.0f);
 
-  for (int k0 = lane * 32; k0 < k; k0 += 32 * 32) {
-    uint4 cw[RW];
-    uint32_t sc[RW];
+  for (int k0 = slice * kAhead * kPiece; k0 < k; k0 += KW * kAhead * kPiece) {
+    uint32_t w[kAhead][RW], sb[kAhead][RW];
 #pragma unroll
-    for (int r = 0; r < RW; ++r) {
-      const int row = min(row0 + r, rows - 1);
-      cw[r] = __ldcs(reinterpret_cast<const uint4 *>(codes + static_cast<size_t>(row) * packed_cols + (k0 >> 1)));
-      sc[r] = __ldcs(reinterpret_cast<const unsigned short *>(scales + static_cast<size_t>(row) * scale_cols + (k0 >> 4)));
-    }
-#pragma unroll
-    for (int m = 0; m < M; ++m) {
-      float xv[32];
-      XLoad<XT>::load32(x + static_cast<size_t>(m) * k + k0, x_scale, xv);
+    for (int u = 0; u < kAhead; ++u)
 #pragma unroll
       for (int r = 0; r < RW; ++r) {
-        const float d0 = block_dot(cw[r].x, cw[r].y, xv);
-        const float d1 = block_dot(cw[r].z, cw[r].w, xv + 16);
-        acc[r][m] = fmaf(d0, e4m3_to_f32(sc[r] & 0xffu), acc[r][m]);
-        acc[r][m] = fmaf(d1, e4m3_to_f32(sc[r] >> 8), acc[r][m]);
+        w[u][r] = cw[u][r];
+        sb[u][r] = sc[u][r];
+      }
+    if (k0 + KW * kAhead * kPiece < k) fetch(k0 + KW * kAhead * kPiece);
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const int col = k0 + u * kPiece + lane * 8;
+      if (col < k) {
+        float2 wf[RW][4];
+        float s[RW];
+#pragma unroll
+        for (int r = 0; r < RW; ++r) {
+          e2m1x8_to_f32(w[u][r], wf[r]);
+          s[r] = e4m3_to_f32(sb[u][r]);
+        }
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+          float2 xv[4];
+          XLoad<XT>::load8(x + static_cast<size_t>(m) * k + col, x_scale, xv);
+#pragma unroll
+          for (int r = 0; r < RW; ++r) {
+            float2 d = make_float2(0.0f, 0.0f);
+#pragma unroll
+            for (int p = 0; p < 4; ++p) d = fma2(wf[r][p], xv[p], d);
+            acc[r][m] = fma2(d, make_float2(s[r], s[r]), acc[r][m]);
+          }
+        }
       }
     }
   }
 
+  __shared__ float part[KW > 1 ? kWarpsPerBlock : 1][M];
 #pragma unroll
   for (int r = 0; r < RW; ++r) {
 #pragma unroll
     for (int m = 0; m < M; ++m) {
-      float v = acc[r][m];
+      float v = acc[r][m].x + acc[r][m].y;
 #pragma unroll
       for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-      if (lane == 0 && row0 + r < rows) {
-        store_out(y + static_cast<size_t>(m) * rows + row0 + r, v * s2_scaled);
+      if (lane == 0) {
+        if constexpr (KW > 1) {
+          part[warp][m] = v;
+        } else if (row0 + r < rows) {
+          store_out(y + static_cast<size_t>(m) * rows + row0 + r, v * s2);
+        }
       }
+    }
+  }
+  if constexpr (KW > 1) {
+    static_assert(RW == 1, "slices of one row");
+    __syncthreads();
+    if (slice == 0 && lane < M && row0 < rows) {
+      float v = part[warp][lane];
+#pragma unroll
+      for (int q = 1; q < KW; ++q) v += part[warp + q][lane];
+      store_out(y + static_cast<size_t>(lane) * rows + row0, v * s2);
     }
   }
 }
 
-// Any K % 16 == 0: one warp per row, one 16-weight block per lane step, byte
-// loads.  Only shapes the vector kernel cannot take end up here.
+// Activations that are not 16-byte aligned (accepted where K is no multiple of 32): one warp per row, one 16-weight
+// block per lane step, element loads.
 template <typename XT, typename OT>
 __global__ void __launch_bounds__(kThreads)
 gemv_w4a16_generic_kernel(const uint8_t * __restrict__ codes, const uint8_t * __restrict__ scales,
@@ -214,27 +287,26 @@ dequant_bf16_kernel(const uint8_t * __restrict__ codes, const uint8_t * __restri
   dst[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
 }
 
+template <int M, int RW, int KW, typename XT, typename OT>
+int launch_rows(const q35b_weight * w, const XT * x, OT * y, float x_scale, cudaStream_t s) {
+  const int warps = (w->rows + RW - 1) / RW;
+  const int blocks = (warps * KW + kWarpsPerBlock - 1) / kWarpsPerBlock;
+  const cudaError_t le = launch_pdl(gemv_w4a16_rows_kernel<M, RW, KW, XT, OT>, dim3(static_cast<unsigned>(blocks)), dim3(kThreads), 0, s,
+                                    static_cast<const uint8_t *>(w->codes), static_cast<const uint8_t *>(w->scales), x, y, w->rows,
+                                    w->k, w->s2, x_scale);
+  count_launch();
+  Q35B_CUDA_TRY(le, "gemv_w4a16_rows_kernel launch");
+  return Q35B_OK;
+}
+
 template <int M, typename XT, typename OT>
 int launch_simt(const q35b_weight * w, const XT * x, OT * y, float x_scale, cudaStream_t s) {
-  constexpr int RW = (M <= 2) ? 2 : 1;
-  const int warps = (w->rows + RW - 1) / RW;
-  const int blocks = (warps + kWarpsPerBlock - 1) / kWarpsPerBlock;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(blocks));
-  cfg.blockDim = dim3(kThreads);
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  const uint8_t * codes = w->codes;
-  const uint8_t * scales = w->scales;
-  const cudaError_t le = cudaLaunchKernelEx(&cfg, gemv_w4a16_simt_kernel<M, RW, XT, OT>, codes, scales, x, y, w->rows, w->k,
-                                            w->s2 * 16384.0f, x_scale);
-  count_launch();
-  Q35B_CUDA_TRY(le, "gemv_w4a16_simt_kernel launch");
-  return Q35B_OK;
+  // Fewer rows than the chip holds blocks' worth of warps: four warps per row where K has pieces for them, else one.
+  // Two rows per warp share its activation loads ([5674, 7072] at four tokens: 22 us, with four rows 29).
+  const int sms = sm_count();
+  if (w->rows < kWarpsPerBlock * sms && w->k > pieces_ahead(M) * kPiece) return launch_rows<M, 1, 4>(w, x, y, x_scale, s);
+  if (w->rows < 2 * kWarpsPerBlock * sms) return launch_rows<M, 1, 1>(w, x, y, x_scale, s);
+  return launch_rows<M, 2, 1>(w, x, y, x_scale, s);
 }
 
 template <typename XT, typename OT>
@@ -248,10 +320,9 @@ int launch_any(const q35b_weight * w, const XT * x, int m, OT * y, float x_scale
   }
   if (const int st = check_weight_device(w)) return st;
   if ((w->k % 32) == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) != 0) {
-    // the vector kernel reads activations with 16-byte loads
     return fail(Q35B_ERR_ARGUMENT, "Activations of the NVFP4 projection must be 16-byte aligned.");
   }
-  if ((w->k % 32) != 0) {
+  if ((reinterpret_cast<uintptr_t>(x) & 15u) != 0) {
     const int blocks = (w->rows + kWarpsPerBlock - 1) / kWarpsPerBlock;
     gemv_w4a16_generic_kernel<XT, OT><<<blocks, kThreads, 0, s>>>(w->codes, w->scales, x, y, w->rows, w->k, m,
                                                                  w->s2 * 16384.0f, x_scale);
