@@ -107,7 +107,7 @@ def decode_entries(q, torch, device, peaks, shapes, layers, ms, label, row_outli
             batches = [q.GemvBatch(list(zip(ws, xs, ys)), m) for ws in weights]
         except q.Q35bError as e:
             # activations too large for the streaming kernel's shared memory: per-projection SIMT launches
-            kernel = f"gemv_w4a16_simt_kernel per projection ({e})"
+            kernel = f"gemv_w4a16_rows_kernel per projection ({e})"
             batches = []
 
             def run_set(ws):
@@ -142,7 +142,7 @@ def single_projection_entries(q, torch, device, peaks, n, k, ms, label, row_outl
     for m in ms:
         x = torch.randn((m, k), generator=gen, device=device).to(torch.bfloat16)
         y = torch.empty((m, n), dtype=torch.bfloat16, device=device)
-        for kernel, name in ((q.GEMV_SIMT, "gemv_w4a16_simt_kernel"), (q.GEMV_STREAM, "gemv_w4a16_stream_kernel")):
+        for kernel, name in ((q.GEMV_SIMT, "gemv_w4a16_rows_kernel"), (q.GEMV_STREAM, "gemv_w4a16_stream_kernel")):
             try:
                 graphs = [_capture(torch, stream, lambda w=w: q.gemv_w4a16(w, x, out=y, kernel=kernel)) for w in weights]
             except q.Q35bError:
