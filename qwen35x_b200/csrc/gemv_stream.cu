@@ -797,10 +797,11 @@ StreamKernel stream_kernel(int m, int ks, bool shared) {
 
 // The plan for a list on the current device: the two-CTAs-per-SM shape only if two of its CTAs really fit on an SM
 // (items that wait for other items rely on every CTA of the grid being resident).
-cudaError_t plan_for_device(int m, int max_k, Plan * p, bool * fits) {
+cudaError_t plan_for_device(int m, int max_k, bool share_tiles, Plan * p, bool * fits) {
   *fits = make_plan(m, max_k, p);
   if (!*fits) return cudaSuccess;
   for (const bool shared : {false, true}) {
+    if (shared && !share_tiles) break;  // a list of whole tiles never runs that kernel
     cudaError_t e = cudaFuncSetAttribute(stream_kernel(m, p->ksplit, shared), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          smem_budget(p->ksplit));
     if (e != cudaSuccess) return e;
@@ -1008,7 +1009,7 @@ int gemv_batch_build(const q35b_gemv_item * items, int count, int m, bool share_
     return fail_cuda(cudaGetLastError(), "cudaGetDevice");
   }
   bool fits = false;
-  if (const cudaError_t pe = plan_for_device(m, max_k, &b->plan, &fits); pe != cudaSuccess) {
+  if (const cudaError_t pe = plan_for_device(m, max_k, share_tiles, &b->plan, &fits); pe != cudaSuccess) {
     delete b;
     return fail_cuda(pe, "planning the projection work list");
   }
@@ -1073,7 +1074,7 @@ int gemv_batch_build(const q35b_gemv_item * items, int count, int m, bool share_
   auto grid_for = [&](int ksplit) { return std::max(1, std::min(sm_count() * ctas_per_sm(ksplit), most)); };
   int grid = grid_for(b->plan.ksplit);
   Assignment todo = assign_tiles(all, level, max_level, grid, m, share_tiles);
-  if (todo.splits == 0) {
+  if (share_tiles && todo.splits == 0) {
     // whole tiles only: no CTA without one
     share_tiles = false;
     grid = std::max(1, std::min(grid, static_cast<int>(all.size())));
@@ -1087,7 +1088,7 @@ int gemv_batch_build(const q35b_gemv_item * items, int count, int m, bool share_
       Assignment a = ks == b->plan.ksplit ? todo : assign_tiles(all, level, max_level, g, m, true);
       Plan p;
       bool ok = false;
-      if (const cudaError_t pe = plan_for_device(m, std::max(a.max_x, 256), &p, &ok); pe != cudaSuccess) {
+      if (const cudaError_t pe = plan_for_device(m, std::max(a.max_x, 256), true, &p, &ok); pe != cudaSuccess) {
         delete b;
         return fail_cuda(pe, "planning the projection work list");
       }
