@@ -26,6 +26,9 @@
 //
 // Every mbarrier wait is bounded: on expiry the kernel writes a code to
 // *status, abandons the tile, still meets its cluster, frees its TMEM and returns.
+// *status is read once per CTA, after griddepcontrol.wait: an earlier kernel of the stream may be what sets it to
+// zero.  By then the weight loads are under way, so a code found there stops the stores, not the loads, and the
+// CTAs of a cluster decide together.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -183,6 +186,11 @@ __device__ __forceinline__ uint32_t cluster_rank() {
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+__device__ __forceinline__ uint32_t ld_cluster_u32(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return v;
+}
 __device__ __forceinline__ uint32_t map_to_rank(uint32_t addr, uint32_t rank) {
   uint32_t r;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
@@ -271,10 +279,9 @@ gemm_w4a4_ksplit_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   const int ks0 = rank * k_steps / SPLIT, ks1 = (rank + 1) * k_steps / SPLIT;
   const int parts = partial_accumulators(n_cols);
 
-  // An error recorded by an earlier tile: load and compute nothing, but meet the cluster and free the TMEM.
-  __shared__ unsigned int s_abort;
+  __shared__ unsigned int s_stop;  // nonzero: an error is recorded, or a wait of this CTA expired
   if (threadIdx.x == 0) {
-    s_abort = *reinterpret_cast<volatile unsigned int *>(status);
+    s_stop = 0u;
     for (int i = 0; i < stages; ++i) {
       mbar_init(smem_u32(full + i), 2);
       mbar_init(smem_u32(empty + i), 1);
@@ -292,14 +299,13 @@ gemm_w4a4_ksplit_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
-  const bool aborted = s_abort != 0u;
   // Launched with programmatic stream serialisation: weights are constant and start loading at once; activations,
   // residuals and every store come after griddepcontrol.wait, when all earlier work of the stream is complete.
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   if (warp == 0) {
     // ---------------- weight loads ----------------
-    if (elect_one() && !aborted) {
+    if (elect_one()) {
       const uint8_t * sf = sfw + static_cast<size_t>(rb) * sf_col_blocks * kSfChunk;
       int stage = 0;
       uint32_t phase = 0;
@@ -321,7 +327,7 @@ gemm_w4a4_ksplit_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
     }
   } else if (warp == 2) {
     // ---------------- activation loads ----------------
-    if (elect_one() && !aborted) {
+    if (elect_one()) {
       asm volatile("griddepcontrol.wait;" ::: "memory");
       const uint8_t * sf = sfx + static_cast<size_t>(token0 >> 7) * sf_col_blocks * kSfChunk;
       int stage = 0;
@@ -344,7 +350,7 @@ gemm_w4a4_ksplit_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (elect_one() && !aborted) {
+    if (elect_one()) {
       const uint32_t idesc = instr_desc(n_cols);
       const uint32_t sfb_off = static_cast<uint32_t>(token0 & 127) >> 5;  // a 64-token tile may start in the middle of a scale tile
       bool ok = true;
@@ -387,16 +393,22 @@ gemm_w4a4_ksplit_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
       }
       if (ok) umma_commit(smem_u32(acc_full));  // accumulator complete, and with it every load of the ring consumed
     }
+  } else if (warp == 3) {
+    // ---------------- an error on record? ----------------
+    if (elect_one()) {
+      asm volatile("griddepcontrol.wait;" ::: "memory");
+      if (*reinterpret_cast<volatile unsigned int *>(status) != 0u) s_stop = 1u;
+    }
   }
   __syncwarp();
 
   // ---------------- epilogue: TMEM -> shared memory -> sum over the cluster -> global ----------------
-  bool ran = !aborted;
-  if (ran && !mbar_wait(smem_u32(acc_full), 0)) {
-    if (lane == 0) atomicExch(status, kStatusEpilogueWait);
-    ran = false;
-  }
-  if (ran) {
+  if (!mbar_wait(smem_u32(acc_full), 0)) {
+    if (lane == 0) {
+      atomicExch(status, kStatusEpilogueWait);
+      s_stop = 1u;
+    }
+  } else {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const int quarter = warp & 3;                 // TMEM lanes this warp may touch
     const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
@@ -430,8 +442,11 @@ gemm_w4a4_ksplit_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
                  "r"(static_cast<uint32_t>(kTmemCols))
                  : "memory");
   }
+  // One CTA's expired wait leaves no sums for the others to add: the whole cluster stores, or none of it does.
+  bool stop = s_stop != 0u;
+  if constexpr (SPLIT > 1) stop = __any_sync(0xffffffffu, ld_cluster_u32(map_to_rank(smem_u32(&s_stop), lane & (SPLIT - 1))) != 0u);
 
-  if (ran) {
+  if (!stop) {
     // this CTA's share of the tokens
     const int t_begin = rank * n_cols / SPLIT, t_end = min((rank + 1) * n_cols / SPLIT, tokens);
     const float g = __ldg(g_dev);
@@ -505,7 +520,7 @@ gemm_w4a4_ksplit_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
     }
   }
 
-  gemm_signal_peers(ep, ran);
+  gemm_signal_peers(ep, !stop);
   __syncwarp();
   if constexpr (SPLIT > 1) cluster_sync();  // no CTA may leave while another still reads its partial sums
 }

@@ -60,3 +60,33 @@ def test_gate_up_matches_its_halves(engine, oracle, m, inter, k):
     want = gate / (1 + torch.exp(-gate)) * up
     assert engine.gemm_default_status() == 0
     assert float((fused.double() - want).norm() / want.norm()) <= 3 * 2.0 ** -9
+
+
+@pytest.mark.parametrize("n,k", [(256, 256), (9216, 4096), (4608, 2560), (256, 4096)])  # split in 1, 2, 4 and 8
+def test_own_status_word_is_read_after_the_stream_has_set_it(engine, n, k):
+    """A status word that a kernel right in front of the GEMM sets to zero, one that lets its successor start early (the
+    single projection, whose outputs are zero for a zero input): the GEMM runs, every time.  With a code on record it
+    stores nothing and leaves the code."""
+    import torch
+
+    m, wide, iters = 8, 32768, 30
+    rnd = torch.Generator(device="cuda").manual_seed(1)
+    codes = torch.randint(0, 256, (wide, 3360), dtype=torch.uint8, device="cuda", generator=rnd)
+    scales = torch.randint(1, 0x7f, (wide, 420), dtype=torch.uint8, device="cuda", generator=rnd)
+    front = engine.Nvfp4Weight.from_device(codes, scales, 1e-3)
+    zero, words = torch.zeros(6720, device="cuda"), torch.empty(wide, device="cuda")
+    w = engine.Nvfp4Weight.from_device(codes[:n, :k // 2], scales[:n, :k // 16], 1e-3)
+    a = engine.quantize_activations(torch.randn((m, k), device="cuda", generator=rnd).to(torch.bfloat16))
+    want = engine.gemm_w4a4(w, *a, m)
+    status = words.view(torch.int32)[-1:]
+    c = torch.empty_like(want)
+    for i in range(iters):
+        c.fill_(float(i))
+        words.view(torch.int32).fill_(9)
+        engine.gemv_w4a16_f32(front, zero, out=words, kernel=engine.GEMV_SIMT)
+        engine.gemm_w4a4(w, *a, m, out=c, status=status)
+        assert int(status.item()) == 0 and torch.equal(c, want), i
+    c.fill_(3.0)
+    status.fill_(9)
+    engine.gemm_w4a4(w, *a, m, out=c, status=status)
+    assert int(status.item()) == 9 and bool((c == 3.0).all())
