@@ -26,9 +26,10 @@
 //
 // Every mbarrier wait is bounded: on expiry the kernel writes a code to
 // *status, abandons the tile, still meets its cluster, frees its TMEM and returns.
-// *status is read once per CTA, after griddepcontrol.wait: an earlier kernel of the stream may be what sets it to
-// zero.  By then the weight loads are under way, so a code found there stops the stores, not the loads, and the
-// CTAs of a cluster decide together.
+// *status counts only as read after griddepcontrol.wait: an earlier kernel of the stream may be what sets it to zero.
+// By then the weight loads are under way, so a code found there stops the stores, not the loads, and the CTAs of a
+// cluster decide together.  A CTA that reads a code at its start waits at once and reads again: after an expired wait
+// the rest of the grid drains instead of running into the same one tile by tile.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -58,7 +59,7 @@ constexpr int kTmemCols = 256;
 constexpr int kFixedBytes = 1024 /*alignment slack*/ + 256 /*barriers*/;
 // Two CTAs per SM where the grid has that many: one's prologue and epilogue run under the other's loads.
 constexpr int kSmemHalf = 112 * 1024, kSmemFull = 224 * 1024;
-constexpr uint32_t kWaitLimit = 1u << 20;  // try_wait polls before giving up (well under a second)
+constexpr uint32_t kWaitLimit = 1u << 20;  // try_wait polls before giving up (4 us each on B200, 4 s in all)
 
 enum StatusCode : unsigned { kStatusProducerWait = 1, kStatusMmaWait = 2, kStatusEpilogueWait = 3, kStatusActWait = 4 };
 
@@ -279,9 +280,15 @@ gemm_w4a4_ksplit_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   const int ks0 = rank * k_steps / SPLIT, ks1 = (rank + 1) * k_steps / SPLIT;
   const int parts = partial_accumulators(n_cols);
 
-  __shared__ unsigned int s_stop;  // nonzero: an error is recorded, or a wait of this CTA expired
+  __shared__ unsigned int s_abort;  // nonzero: an error was on record when this CTA started, it loads nothing
+  __shared__ unsigned int s_stop;   // nonzero: it stores nothing (that, an error found later, or an expired wait)
   if (threadIdx.x == 0) {
-    s_stop = 0u;
+    unsigned int code = *reinterpret_cast<volatile unsigned int *>(status);
+    if (code != 0u) {
+      asm volatile("griddepcontrol.wait;" ::: "memory");
+      code = *reinterpret_cast<volatile unsigned int *>(status);
+    }
+    s_abort = s_stop = code;
     for (int i = 0; i < stages; ++i) {
       mbar_init(smem_u32(full + i), 2);
       mbar_init(smem_u32(empty + i), 1);
@@ -299,13 +306,14 @@ gemm_w4a4_ksplit_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
+  const bool aborted = s_abort != 0u;
   // Launched with programmatic stream serialisation: weights are constant and start loading at once; activations,
   // residuals and every store come after griddepcontrol.wait, when all earlier work of the stream is complete.
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   if (warp == 0) {
     // ---------------- weight loads ----------------
-    if (elect_one()) {
+    if (elect_one() && !aborted) {
       const uint8_t * sf = sfw + static_cast<size_t>(rb) * sf_col_blocks * kSfChunk;
       int stage = 0;
       uint32_t phase = 0;
@@ -327,7 +335,7 @@ gemm_w4a4_ksplit_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
     }
   } else if (warp == 2) {
     // ---------------- activation loads ----------------
-    if (elect_one()) {
+    if (elect_one() && !aborted) {
       asm volatile("griddepcontrol.wait;" ::: "memory");
       const uint8_t * sf = sfx + static_cast<size_t>(token0 >> 7) * sf_col_blocks * kSfChunk;
       int stage = 0;
@@ -350,7 +358,7 @@ gemm_w4a4_ksplit_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (elect_one()) {
+    if (elect_one() && !aborted) {
       const uint32_t idesc = instr_desc(n_cols);
       const uint32_t sfb_off = static_cast<uint32_t>(token0 & 127) >> 5;  // a 64-token tile may start in the middle of a scale tile
       bool ok = true;
@@ -395,7 +403,7 @@ gemm_w4a4_ksplit_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
     }
   } else if (warp == 3) {
     // ---------------- an error on record? ----------------
-    if (elect_one()) {
+    if (elect_one() && !aborted) {
       asm volatile("griddepcontrol.wait;" ::: "memory");
       if (*reinterpret_cast<volatile unsigned int *>(status) != 0u) s_stop = 1u;
     }
@@ -403,12 +411,15 @@ gemm_w4a4_ksplit_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   __syncwarp();
 
   // ---------------- epilogue: TMEM -> shared memory -> sum over the cluster -> global ----------------
-  if (!mbar_wait(smem_u32(acc_full), 0)) {
+  bool ran = !aborted;
+  if (ran && !mbar_wait(smem_u32(acc_full), 0)) {
     if (lane == 0) {
       atomicExch(status, kStatusEpilogueWait);
       s_stop = 1u;
     }
-  } else {
+    ran = false;
+  }
+  if (ran) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const int quarter = warp & 3;                 // TMEM lanes this warp may touch
     const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
