@@ -307,8 +307,10 @@ gemm_w4a4_ksplit_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
   const bool aborted = s_abort != 0u;
-  // Launched with programmatic stream serialisation: weights are constant and start loading at once; activations,
-  // residuals and every store come after griddepcontrol.wait, when all earlier work of the stream is complete.
+  // Launched with programmatic stream serialisation: weights are constant and the first ring of them starts loading at
+  // once; activations, residuals and every store come after griddepcontrol.wait, when all earlier work of the stream is
+  // complete.  So does every mbarrier wait that can block: its bound is meant for this kernel's own loads and MMAs, not
+  // for however long the kernel before still runs.
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   if (warp == 0) {
@@ -318,6 +320,7 @@ gemm_w4a4_ksplit_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
       int stage = 0;
       uint32_t phase = 0;
       for (int ks = ks0; ks < ks1; ++ks) {
+        if (ks - ks0 == stages) asm volatile("griddepcontrol.wait;" ::: "memory");  // the stages so far were free
         if (!mbar_wait(smem_u32(empty + stage), phase ^ 1)) {
           atomicExch(status, kStatusProducerWait);
           break;
@@ -359,6 +362,7 @@ gemm_w4a4_ksplit_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
     if (elect_one() && !aborted) {
+      asm volatile("griddepcontrol.wait;" ::: "memory");
       const uint32_t idesc = instr_desc(n_cols);
       const uint32_t sfb_off = static_cast<uint32_t>(token0 & 127) >> 5;  // a 64-token tile may start in the middle of a scale tile
       bool ok = true;
@@ -409,6 +413,7 @@ gemm_w4a4_ksplit_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
     }
   }
   __syncwarp();
+  asm volatile("griddepcontrol.wait;" ::: "memory");
 
   // ---------------- epilogue: TMEM -> shared memory -> sum over the cluster -> global ----------------
   bool ran = !aborted;
@@ -446,7 +451,6 @@ gemm_w4a4_ksplit_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   if constexpr (SPLIT > 1) cluster_sync(); else __syncthreads();
-  asm volatile("griddepcontrol.wait;" ::: "memory");
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
