@@ -105,9 +105,10 @@ __device__ __forceinline__ void gemm_forward_rows_to_peers(const GemmEpilogue & 
 }
 
 // End of a gathering GEMM kernel; every thread of the CTA calls it after its last output store.
-// A CTA that ran no tiles because an earlier error is recorded (`ran` false) counts itself but the flags are not
-// written then: the other ranks' bounded waits expire and record the failure on their side too.
-__device__ __forceinline__ void gemm_signal_peers(const GemmEpilogue & ep, bool ran) {
+// Every CTA counts itself, also one that ran no tiles or gave one up, but with a code in *status (NULL: none kept) the
+// flags are not written: the other ranks' bounded waits expire and record the failure on their side too.  The last CTA
+// reads the word after all others have counted themselves, so a wait that expired in any of them is seen.
+__device__ __forceinline__ void gemm_signal_peers(const GemmEpilogue & ep, const unsigned int * status) {
   if (ep.done_counter == nullptr) return;
   __threadfence_system();  // this thread's stores, local and remote, before anything that follows
   __syncthreads();
@@ -121,7 +122,7 @@ __device__ __forceinline__ void gemm_signal_peers(const GemmEpilogue & ep, bool 
         epoch = *ep.send_seq + 1u;  // only this thread of the whole grid gets here
         *ep.send_seq = epoch;
       }
-      if (ran) {
+      if (status == nullptr || *reinterpret_cast<const volatile unsigned int *>(status) == 0u) {
         _Pragma("unroll") for (int i = 0; i < GemmEpilogue::kMaxPeers; ++i) if (i < ep.n_peers) *reinterpret_cast<volatile unsigned int *>(ep.peer_flag[i]) = epoch;
       }
     }

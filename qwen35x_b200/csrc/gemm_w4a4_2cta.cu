@@ -387,7 +387,7 @@ gemm_w4a4_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     }
   }
 
-  gemm_signal_peers(ep, !aborted);
+  gemm_signal_peers(ep, status);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   cluster_sync();  // neither CTA may leave while its partner can still signal its barriers or read its tiles

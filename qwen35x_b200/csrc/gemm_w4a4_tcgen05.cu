@@ -535,7 +535,7 @@ gemm_w4a4_ksplit_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
     }
   }
 
-  gemm_signal_peers(ep, !stop);
+  gemm_signal_peers(ep, status);
   __syncwarp();
   if constexpr (SPLIT > 1) cluster_sync();  // no CTA may leave while another still reads its partial sums
 }
