@@ -457,11 +457,10 @@ gemm_w4a4_ksplit_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
                  "r"(static_cast<uint32_t>(kTmemCols))
                  : "memory");
   }
-  // One CTA's expired wait leaves no sums for the others to add: the whole cluster stores, or none of it does.
-  bool stop = s_stop != 0u;
-  if constexpr (SPLIT > 1) stop = __any_sync(0xffffffffu, ld_cluster_u32(map_to_rank(smem_u32(&s_stop), lane & (SPLIT - 1))) != 0u);
-
-  if (!stop) {
+  // One CTA's expired wait leaves no sums for the others to add: the whole cluster stores, or none of it does.  Every
+  // lane asks one CTA, and the lanes are asked only when the first sums are there (0.2 us of a 7 us kernel).
+  const bool stop_lane = (SPLIT > 1 ? ld_cluster_u32(map_to_rank(smem_u32(&s_stop), lane & (SPLIT - 1))) : s_stop) != 0u;
+  {
     // this CTA's share of the tokens
     const int t_begin = rank * n_cols / SPLIT, t_end = min((rank + 1) * n_cols / SPLIT, tokens);
     const float g = __ldg(g_dev);
@@ -476,7 +475,7 @@ gemm_w4a4_ksplit_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
       // one thread per token and 32 weight rows = one block of 16 outputs (n % 128 == 0 is checked on the host);
       // lanes along the tokens, whose pitch spreads them over the banks
       const float q_g = __ldg(ep.q_g);
-      const int live = t_end - t_begin;
+      const int live = __any_sync(0xffffffffu, stop_lane) ? 0 : t_end - t_begin;
       for (int u = threadIdx.x; u < live * (kRows / 32); u += kThreads) {
         const int t = t_begin + u % live, blk = u / live;
         uint32_t r[32];
@@ -500,6 +499,7 @@ gemm_w4a4_ksplit_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
 #pragma unroll 1
       for (int t = t_begin + warp; t < t_end; t += kThreads / 32) {
         const float4 a = sum4<SPLIT>(src, static_cast<uint32_t>(t * kPitch + 4 * lane) * 4u);
+        if (__any_sync(0xffffffffu, stop_lane)) break;
         float v[4] = {a.x, a.y, a.z, a.w};
         if constexpr (EPI == kEpiGateUp) {
 #pragma unroll
