@@ -272,6 +272,17 @@ Q35B_API int q35b_gemm_w4a4_bf16(const q35b_weight * w, const uint8_t * a_codes,
                                  const float * input_scale_dev, int m, void * c_bf16, int ldc,
                                  unsigned int * status_dev, q35b_stream stream);
 
+/* Which kernel a prefill projection takes and in which order it sums K (host arithmetic only, no device needed), for a
+ * shard of `rows` rows of a tensor of n_total on a GPU of `sms` SMs; gather: q35b_gemm_w4a4_bf16_allgather;
+ * rows_aligned: output rows start on 32-byte and residual rows on 16-byte boundaries.  pairs: 1 for the kernel of CTA pairs on
+ * 256 x 256 tiles; else tile_cols tokens per tile, whose K steps `split` CTAs share, each with up to `accumulators`
+ * partial sums (fewer where a tile's tokens leave no room).
+ * What a caller may rely on: a row shard's columns are bit for bit those of the unsharded projection of the same
+ * tokens; and from 129 tokens on (split = accumulators = 1) a token's outputs do not depend on the other tokens of the
+ * call either, given the same activation scale. */
+Q35B_API int q35b_debug_gemm_plan(int m, int rows, int n_total, int k, int sms, int gather, int rows_aligned, int * pairs,
+                                  int * tile_cols, int * split, int * accumulators);
+
 /* Copies the library's status word of the current device to the host (synchronises the device) and clears it. */
 Q35B_API int q35b_gemm_default_status(unsigned int * status_out);
 

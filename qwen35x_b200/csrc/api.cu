@@ -420,6 +420,11 @@ int q35b_gemm_w4a4_bf16_residual(const q35b_weight * w, const uint8_t * a_codes,
                           residual_bf16, ldr, status_dev, static_cast<cudaStream_t>(stream));
 }
 
+int q35b_debug_gemm_plan(int m, int rows, int n_total, int k, int sms, int gather, int rows_aligned, int * pairs,
+                         int * tile_cols, int * split, int * accumulators) {
+  return gemm_plan_debug(m, rows, n_total, k, sms, gather != 0, rows_aligned != 0, pairs, tile_cols, split, accumulators);
+}
+
 /* Host-callable twins of the device encoders/decoders, so that their
  * equivalence with the reference's scan can be tested without a GPU. */
 uint8_t q35b_debug_encode_ue4m3(float v) { return encode_ue4m3(v); }

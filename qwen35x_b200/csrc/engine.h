@@ -117,6 +117,8 @@ int gemv_plan_debug(int m, int max_k, int * ctas_per_sm, int * ring_stages, int 
 int gemv_batch_debug_wait(struct q35b_gemv_batch * b, unsigned int wait_limit, unsigned int extra_completions);
 
 // gemm_w4a4_tcgen05.cu
+int gemm_plan_debug(int m, int rows, int n_total, int k, int sms, bool gather, bool rows_aligned, int * pairs, int * tile_cols,
+                    int * split, int * accumulators);
 int make_code_map(CUtensorMap * map, const void * base, int rows, int k_bytes, int box_rows);
 // Where a gate/up GEMM writes silu(gate) * up as an NVFP4 activation instead of BF16 (see gemm_epilogue.cuh).
 struct GemmQuantOut {
@@ -156,7 +158,7 @@ int wbatch_status(const WBatch * b, unsigned int * out);
 size_t wbatch_bytes(const WBatch * b);
 
 // gemm_w4a4_2cta.cu
-bool gemm_2cta_eligible(const q35b_weight * w, int m);
+bool gemm_2cta_eligible(int rows, int m, int k);
 struct GemmEpilogue;
 int make_sf_map(CUtensorMap * map, const void * base, long long chunks);
 int launch_gemm_w4a4_2cta(const q35b_weight * w, const uint8_t * a_codes, const uint8_t * a_scales_tiled, const float * g_dev,

@@ -437,9 +437,7 @@ int build_weight_maps(q35b_weight * w) {
   return Q35B_OK;
 }
 
-bool gemm_2cta_eligible(const q35b_weight * w, int m) {
-  return w->rows >= 192 && m >= 256 && (w->k % 64) == 0;
-}
+bool gemm_2cta_eligible(int rows, int m, int k) { return rows >= 192 && m >= 256 && (k % 64) == 0; }
 
 int launch_gemm_w4a4_2cta(const q35b_weight * w, const uint8_t * a_codes, const uint8_t * a_scales_tiled, const float * g_dev,
                           int m, void * c_bf16, int ldc, const GemmEpilogue & ep, unsigned int * status_dev,

@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 gemm_w4a4_ksplit_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                         const uint8_t * __restrict__ sfw, const uint8_t * __restrict__ sfx,
                         const float * __restrict__ g_dev, const __grid_constant__ GemmEpilogue ep, int m, int n, int k_bytes, int stages,
-                        int ring_bytes, int box_cols, int tile_cols, int vec, __nv_bfloat16 * __restrict__ c, int ldc, unsigned int * status) {
+                        int ring_bytes, int box_cols, int tile_cols, int accumulators, int vec, __nv_bfloat16 * __restrict__ c, int ldc, unsigned int * status) {
   extern __shared__ uint8_t smem_raw[];
   // 1024-byte alignment for the 128B-swizzled operand tiles.
   uint8_t * smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -278,7 +278,7 @@ gemm_w4a4_ksplit_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   const int sf_col_blocks = k_bytes >> 5;                        // K/64: 512-byte scale tiles per row block
   const int k_steps = (sf_col_blocks + kMmaPerStage - 1) / kMmaPerStage;
   const int ks0 = rank * k_steps / SPLIT, ks1 = (rank + 1) * k_steps / SPLIT;
-  const int parts = partial_accumulators(n_cols);
+  const int parts = min(partial_accumulators(n_cols), accumulators);
 
   __shared__ unsigned int s_abort;  // nonzero: an error was on record when this CTA started, it loads nothing
   __shared__ unsigned int s_stop;   // nonzero: it stores nothing (that, an error found later, or an expired wait)
@@ -593,13 +593,13 @@ namespace {
 struct Shape {
   int tile_cols, split;
 };
-Shape choose_shape(int m, int row_blocks, int k_steps, int sms) {
+Shape choose_shape(int m, int row_blocks, int k_steps, int sms, int max_split) {
   Shape best = {kMaxCols, 1};
   int best_ns = 0;
   for (int cols = kMaxCols; cols >= 64; cols /= 2) {
     const int tiles = row_blocks * ((m + cols - 1) / cols), live = std::min(cols, round_up_int(m, 16));
     if (cols < kMaxCols && (m <= cols || tiles > sms)) break;
-    for (int split = 1, log2 = 0; split <= kMaxSplit; split *= 2, ++log2) {
+    for (int split = 1, log2 = 0; split <= max_split; split *= 2, ++log2) {
       if (split > 1 && (tiles * split > sms || k_steps < 2 * split)) break;
       const int ns = (k_steps + split - 1) / split * 250 + live * 66 / 10 +
                      (split > 1 ? 400 + live * 33 / 10 + live * 7 * log2 : 0);
@@ -612,11 +612,44 @@ Shape choose_shape(int m, int row_blocks, int k_steps, int sms) {
   return best;
 }
 
+// The kernel and the shape for a projection of m tokens, and with them the order in which its K is summed.
+//
+// Up to kSplitTokens tokens a tile's K steps may be split over CTAs and the MMAs of a step over partial accumulators; how
+// depends on m, K and the rows of the whole tensor, not on those of the shard, so that the columns of a row shard are bit
+// for bit those of the unsharded projection.  Above, every kernel sums K in order into one accumulator, so that a token's
+// outputs depend neither on the shard nor on how many other tokens there are: ranks that share out the tokens, and groups
+// of tokens projected one after the other, get the bits of the whole.
+//
+// Large problems: pairs of CTAs on 256 x 256 tiles, persistent (gemm_w4a4_2cta.cu).  They need many tiles to win: up
+// to two 128 x 128 tiles per SM the kernel above is faster (us, this kernel / pairs: [512, 2560] x [9216, 2560]
+// 8.9 / 10.5, [768, ..] 15.6 / 14.4; [1024, 4096] x [4096, 4096] 10.8 / 12.2, [1536, ..] 19.4 / 17.7), up to three
+// where K is short ([2048, 1024] x [3584, 1024] 10.7 / 11.0, [3072, ..] 15.3 / 13.9), only one where K is long
+// ([768, 9216] x [2560, 9216] 13.6 / 17.3, [1536, ..] 19.8 / 18.3).  The pairs also store rows that are not 32-byte
+// aligned element by element ([4096, 640] x [5000, 640] 24 / 133).
+//
+// What the order costs, us in order / split ([m, 9216] x [2560, 9216]): 64 tokens 12.1 / 7.4, 128 12.3 / 8.4, 192
+// 12.4 / 9.6, 384 12.9 / 10.4, 512 13.8 / 13.6; [192, 8192] x [512, 8192] 11.0 / 6.2; with K up to 2560 nothing.
+constexpr int kSplitTokens = 128;
+struct GemmPlan {
+  bool pairs;
+  int tile_cols, split, accumulators;
+};
+GemmPlan plan_gemm(int m, int rows, int n_total, int k, int sms, bool gather, bool rows_aligned) {
+  const int k_steps = (k + 255) / 256, row_blocks = (rows + kRows - 1) / kRows;
+  if (m <= kSplitTokens) {
+    const Shape shape = choose_shape(m, (n_total + kRows - 1) / kRows, k_steps, sms, kMaxSplit);
+    return {false, shape.tile_cols, shape.split, kMmaPerStage};
+  }
+  const long tiles = static_cast<long>(row_blocks) * ((m + kMaxCols - 1) / kMaxCols);
+  const long few = static_cast<long>(sms) * (k_steps <= 4 ? 3 : (k_steps <= 20 ? 2 : 1));
+  if (gemm_2cta_eligible(rows, m, k) && (gather || (tiles > few && rows_aligned))) return {true, 0, 1, 1};
+  return {false, choose_shape(m, row_blocks, k_steps, sms, 1).tile_cols, 1, 1};
+}
+
 int launch_gemm_ksplit(const q35b_weight * w, const uint8_t * a_codes, const uint8_t * a_scales, const float * g_dev, int m,
-                       void * c, int ldc, const GemmEpilogue & ep, unsigned int * status, cudaStream_t s) {
+                       void * c, int ldc, const GemmEpilogue & ep, const GemmPlan & plan, unsigned int * status, cudaStream_t s) {
   const int row_blocks = (w->rows + kRows - 1) / kRows, k_steps = (w->k + 255) / 256;
-  const Shape shape = choose_shape(m, row_blocks, k_steps, sm_count());
-  const int tile_cols = shape.tile_cols, split = shape.split;
+  const int tile_cols = plan.tile_cols, split = plan.split;
   const int box_cols = std::min(tile_cols, round_up_int(m, 16));
   CUtensorMap tmap_x;
   if (const int st = make_code_map(&tmap_x, a_codes, m, w->k / 2, box_cols)) return st;
@@ -662,7 +695,7 @@ int launch_gemm_ksplit(const q35b_weight * w, const uint8_t * a_codes, const uin
   cfg.attrs = attr;
   cfg.numAttrs = 2;
   const cudaError_t le = cudaLaunchKernelEx(&cfg, kernel, w->tmap_codes_128, tmap_x, static_cast<const uint8_t *>(w->scales_tiled),
-                                            a_scales, g_dev, ep, m, w->rows, w->k / 2, stages, ring, box_cols, tile_cols, vec ? 1 : 0,
+                                            a_scales, g_dev, ep, m, w->rows, w->k / 2, stages, ring, box_cols, tile_cols, plan.accumulators, vec ? 1 : 0,
                                             static_cast<__nv_bfloat16 *>(c), ldc, status);
   count_launch();
   Q35B_CUDA_TRY(le, "gemm_w4a4_ksplit_kernel launch");
@@ -674,6 +707,20 @@ int launch_gemm_ksplit(const q35b_weight * w, const uint8_t * a_codes, const uin
 __device__ unsigned int g_default_status;
 
 }  // namespace
+
+int gemm_plan_debug(int m, int rows, int n_total, int k, int sms, bool gather, bool rows_aligned, int * pairs, int * tile_cols,
+                    int * split, int * accumulators) {
+  if (m < 1 || rows < 1 || n_total < rows || k < 64 || (k % 64) != 0 || sms < 1 || pairs == nullptr || tile_cols == nullptr ||
+      split == nullptr || accumulators == nullptr) {
+    return fail(Q35B_ERR_ARGUMENT, "Invalid arguments for the plan of an NVFP4 prefill projection.");
+  }
+  const GemmPlan p = plan_gemm(m, rows, n_total, k, sms, gather, rows_aligned);
+  *pairs = p.pairs ? 1 : 0;
+  *tile_cols = p.tile_cols;
+  *split = p.split;
+  *accumulators = p.accumulators;
+  return Q35B_OK;
+}
 
 int default_status_word(unsigned int ** out) {
   static std::mutex mutex;
@@ -773,21 +820,11 @@ int launch_gemm_w4a4(const q35b_weight * w, const uint8_t * a_codes, const uint8
     // clears it (no memset in front of the launch: it would sit between this kernel and the one it overlaps with)
     if (const int st = default_status_word(&status_dev)) return st;
   }
-  // Large problems: pairs of CTAs on 256 x 256 tiles, persistent (gemm_w4a4_2cta.cu).  They need many tiles to win: up
-  // to two 128 x 128 tiles per SM the kernel above is faster (us, this kernel / pairs: [512, 2560] x [9216, 2560]
-  // 8.9 / 10.5, [768, ..] 15.6 / 14.4; [1024, 4096] x [4096, 4096] 10.8 / 12.2, [1536, ..] 19.4 / 17.7), up to three
-  // where K is short ([2048, 1024] x [3584, 1024] 10.7 / 11.0, [3072, ..] 15.3 / 13.9), only one where K is long
-  // ([768, 9216] x [2560, 9216] 13.6 / 17.3, [1536, ..] 19.8 / 18.3).  The pairs also store rows that are not 32-byte
-  // aligned element by element ([4096, 640] x [5000, 640] 24 / 133).
-  const long tiles = static_cast<long>((w->rows + kRows - 1) / kRows) * ((m + kMaxCols - 1) / kMaxCols);
-  const int k_steps = (w->k + 255) / 256;
-  const long few = static_cast<long>(sm_count()) * (k_steps <= 4 ? 3 : (k_steps <= 20 ? 2 : 1));
   const bool rows_aligned = qout != nullptr || ((ldc % 16) == 0 && (reinterpret_cast<uintptr_t>(c_bf16) & 31u) == 0 &&
                             (residual_bf16 == nullptr || ((ldr % 8) == 0 && (reinterpret_cast<uintptr_t>(residual_bf16) & 15u) == 0)));
-  if (gemm_2cta_eligible(w, m) && (gather != nullptr || (tiles > few && rows_aligned))) {
-    return launch_gemm_w4a4_2cta(w, a_codes, a_scales_tiled, g_dev, m, c_bf16, ldc, ep, status_dev, s);
-  }
-  return launch_gemm_ksplit(w, a_codes, a_scales_tiled, g_dev, m, c_bf16, ldc, ep, status_dev, s);
+  const GemmPlan plan = plan_gemm(m, w->rows, w->n_total, w->k, sm_count(), gather != nullptr, rows_aligned);
+  if (plan.pairs) return launch_gemm_w4a4_2cta(w, a_codes, a_scales_tiled, g_dev, m, c_bf16, ldc, ep, status_dev, s);
+  return launch_gemm_ksplit(w, a_codes, a_scales_tiled, g_dev, m, c_bf16, ldc, ep, plan, status_dev, s);
 }
 
 }  // namespace q35b

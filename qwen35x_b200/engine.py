@@ -74,6 +74,8 @@ def lib() -> C.CDLL:
     L.q35b_gemv_batch_destroy.argtypes = [vp]
     L.q35b_gemv_batch_status.restype = i
     L.q35b_gemv_batch_status.argtypes = [vp, C.POINTER(C.c_uint)]
+    L.q35b_debug_gemm_plan.restype = i
+    L.q35b_debug_gemm_plan.argtypes = [i] * 7 + [C.POINTER(C.c_int)] * 4
     L.q35b_debug_gemv_plan.restype = i
     L.q35b_debug_gemv_plan.argtypes = [i, i, C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_int)]
     L.q35b_debug_gemv_batch_wait.restype = i
@@ -399,6 +401,15 @@ def gemv_plan(m: int, max_k: int) -> dict:
     v = [C.c_int(0) for _ in range(4)]
     _check(lib().q35b_debug_gemv_plan(m, max_k, *[C.byref(x) for x in v]))
     return {"ctas_per_sm": v[0].value, "ring_stages": v[1].value, "activation_buffers": v[2].value, "smem_bytes": v[3].value}
+
+
+def gemm_plan(m: int, rows: int, k: int, n_total: int | None = None, sms: int = 148, gather: bool = False,
+              rows_aligned: bool = True) -> dict:
+    """Kernel and order of summation of a prefill projection (q35b_debug_gemm_plan): host arithmetic, needs no device."""
+    v = [C.c_int(0) for _ in range(4)]
+    _check(lib().q35b_debug_gemm_plan(m, rows, rows if n_total is None else n_total, k, sms, int(gather), int(rows_aligned),
+                                      *[C.byref(x) for x in v]))
+    return {"pairs": bool(v[0].value), "tile_cols": v[1].value, "split": v[2].value, "accumulators": v[3].value}
 
 
 def gemm_default_status() -> int:
