@@ -204,11 +204,12 @@ Q35B_API void q35b_gemv_batch_destroy(q35b_gemv_batch * batch);
 Q35B_API int q35b_gemv_batch_status(const q35b_gemv_batch * batch, unsigned int * status_out);
 /* Test hook for the bounded device-side waits of a work list built by q35b_gemv_batch_create: every wait of the
  * following runs (ring barriers, activation hand-over, dependency poll) gives up after `wait_limit_polls` polls
- * instead of 2^22, and a dependent item demands `extra_completions` more completions of the item it runs after than
- * that item can deliver.  With a small limit and one extra completion the dependency poll runs out within
+ * instead of 2^22, and in every other CTA, the first included, a dependent item demands `extra_completions` more
+ * completions of the item it runs after than that item can deliver.  With a small limit and one extra completion the dependency poll runs out within
  * microseconds, 15 lands in the status word, the remaining roles run out on their own waits and the kernel returns:
  * what an item whose producer never finishes looks like, without a kernel that hangs.  (0 extra completions and
- * 1 << 22 polls restore normal operation.)  Also clears the list's status word and completion counts. */
+ * 1 << 22 polls restore normal operation.)  Also clears the list's status word; the counters of a run are at zero
+ * after it, also after one that gave up. */
 Q35B_API int q35b_debug_gemv_batch_wait(q35b_gemv_batch * batch, unsigned int wait_limit_polls,
                                         unsigned int extra_completions);
 /* The shared-memory plan a work list of `m` tokens over weights of at most `max_k` columns would get (host

@@ -201,6 +201,9 @@ __device__ __forceinline__ float ue4m3_to_f32(uint32_t byte) {
 // `slots` is the first part's 512 bytes of this warp's row group, the next part's follow eight row groups on) and the
 // last one of its row group to arrive adds them all in part order and gets true.  Nobody waits.  Out of line: it runs
 // a few times per CTA, and inline it made every other tile slower (2-3 % of a step at four and eight tokens).
+// The counter's low half counts the parts, its high half those whose warp gave up on an expired wait (give_up_parts):
+// then nobody stores.  Either way the last part leaves it at zero for the next run.
+constexpr unsigned int kPartCount = 0xffffu, kGaveUp = 0x10000u;
 __device__ __noinline__ bool meet_parts(float4 & sum, float * slots, unsigned int * arrival, int part, int parts, int lane) {
   float4 * mine = reinterpret_cast<float4 *>(slots) + lane;
   constexpr int kNext = kRowGroups * 32;  // float4s between parts
@@ -209,9 +212,11 @@ __device__ __noinline__ bool meet_parts(float4 & sum, float * slots, unsigned in
   __syncwarp();
   unsigned int before = 0;
   if (lane == 0) before = atomicAdd(arrival, 1u);
-  if (__shfl_sync(0xffffffffu, before, 0) != static_cast<unsigned int>(parts - 1)) return false;
+  before = __shfl_sync(0xffffffffu, before, 0);
+  if ((before & kPartCount) != static_cast<unsigned int>(parts - 1)) return false;
   __threadfence();
-  if (lane == 0) *arrival = 0u;  // for the next run
+  if (lane == 0) *arrival = 0u;
+  if (before >= kGaveUp) return false;
   sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll 4
   for (int p = 0; p < parts; ++p) {
@@ -222,6 +227,15 @@ __device__ __noinline__ bool meet_parts(float4 & sum, float * slots, unsigned in
     sum.w += o.w;
   }
   return true;
+}
+
+// A storing warp that gave up counts itself for its tiles from `tile` to `end` all the same (one thread per warp).
+__device__ __noinline__ void give_up_parts(const GemvTile * tile, const GemvTile * end, unsigned int * arrivals, int rg) {
+  for (; tile < end; ++tile) {
+    if (tile->parts < 2) continue;
+    unsigned int * arrival = arrivals + tile->split * kRowGroups + rg;
+    if ((atomicAdd(arrival, 1u + kGaveUp) & kPartCount) == static_cast<unsigned int>(tile->parts - 1)) *arrival = 0u;
+  }
 }
 
 // MT = number of 4-token groups (1 for M <= 4, 2 for M <= 8).  SHARED: some tiles of the list are shared by several CTAs
@@ -344,7 +358,7 @@ gemv_w4a16_stream_kernel(const GemvItem * __restrict__ items, const GemvTile * _
         // a sixteenth of the budget of the barrier waits: when a dependency cannot be met this poll gives up first and
         // its code (the first one recorded stays) names the cause; the roles waiting on this warp follow
         for (uint32_t i = 0; i < max(wait_limit >> 4, 1u); ++i) {
-          if (*cnt >= tl->wait_count + wait_extra) {
+          if (*cnt >= tl->wait_count + ((blockIdx.x & 1) == 0 ? wait_extra : 0u)) {
             met = 1;
             break;
           }
@@ -429,7 +443,8 @@ gemv_w4a16_stream_kernel(const GemvItem * __restrict__ items, const GemvTile * _
     int prev_item = -1;
     int buf = 0;
     bool ok = true;
-    for (int ti = 0; ti < n_tiles && ok; ++ti) {
+    int ti = 0;
+    for (; ti < n_tiles && ok; ++ti) {
       const GemvTile * tile = tile_at(ti);
       if (tile->item != prev_item) {
         if (prev_item >= 0) {
@@ -723,6 +738,10 @@ gemv_w4a16_stream_kernel(const GemvItem * __restrict__ items, const GemvTile * _
         }
       }
     }
+    if constexpr (SHARED) {
+      // the parts from the tile it gave up in on; a warp leaves that loop only before its tile's parts meet
+      if (!ok && kh == 0 && lane == 0) give_up_parts(tiles + tile_begin + ti, tiles + tile_begin + n_tiles, arrivals, rg);
+    }
     if (ok && prev_item >= 0) {
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(xempty + buf));
@@ -847,7 +866,7 @@ struct q35b_gemv_batch {
   bool shared = false;                       // some tiles are shared by several CTAs
   size_t bytes_per_run = 0;
   uint32_t wait_limit = kWaitLimit;   // polls every device-side wait of a run may take
-  unsigned int wait_extra = 0;        // test hook: completions demanded on top of what a dependency really delivers
+  unsigned int wait_extra = 0;        // test hook: completions that every other CTA demands on top of what a dependency delivers
   q35b::WBatch * tensor = nullptr;   // set: the list runs on the tensor path (gemm_wstream.cu), nothing above is used
 };
 
@@ -1208,10 +1227,8 @@ int gemv_batch_debug_wait(q35b_gemv_batch * b, unsigned int wait_limit, unsigned
   if (b == nullptr || b->tensor != nullptr || wait_limit == 0) return fail(Q35B_ERR_ARGUMENT, "Invalid NVFP4 projection work list.");
   b->wait_limit = wait_limit;
   b->wait_extra = extra_completions;
-  // counts of a run that gave up stay behind: start the next run from zero
-  if (b->item_done != nullptr) {
-    Q35B_CUDA_TRY(cudaMemset(b->status, 0, b->counter_bytes), "cudaMemset(work list counters)");
-  }
+  // only the recorded code: every run leaves its counters at zero, also one that gave up
+  Q35B_CUDA_TRY(cudaMemset(b->status, 0, sizeof(unsigned int)), "cudaMemset(work list status)");
   return Q35B_OK;
 }
 

@@ -77,3 +77,35 @@ def test_mlp_block(engine, oracle, m, hidden, inter):
         graph.replay()
         stream.synchronize()
     assert batch.status() == 0 and torch.equal(y, kept)
+
+
+@pytest.mark.parametrize("m,hidden,inter", [(2, 512, 8192), (8, 512, 8192), (3, 2560, 1280)])
+def test_list_recovers_from_an_expired_wait(engine, m, hidden, inter):
+    """Every other CTA of a run gives up waiting for the gate/up item, so some parts of the down projection's tiles
+    arrive and others do not.  The run reports it, and the next ones, nothing reset but the limit, are right again."""
+    import torch
+
+    _, gc, gs, g2 = make_weight(inter, hidden, seed=1)
+    _, uc, us, u2 = make_weight(inter, hidden, seed=2)
+    _, dc, ds, d2 = make_weight(hidden, inter, seed=3)
+    x = to_torch_bf16(make_activations(m, hidden, seed=4))
+    h = torch.zeros((m, inter), dtype=torch.bfloat16, device="cuda")
+    y = torch.zeros((m, hidden), dtype=torch.bfloat16, device="cuda")
+    batch = engine.GemvBatch([(engine.Nvfp4Weight.gate_up_from_host(gc, gs, g2, uc, us, u2), x, h),
+                              (engine.Nvfp4Weight.from_host(dc, ds, d2), h, y, None, 0)], m)
+    batch.run()
+    assert batch.status() == 0
+    good = y.clone()
+    for _ in range(2):
+        batch.debug_wait(4096, 1)
+        batch.run()
+        assert batch.status() == 15
+        batch.debug_wait(1 << 22, 0)
+        x_kept = x.clone()
+        x.mul_(-3.0)  # stale sums of an earlier run would be those of another input
+        batch.run()
+        x.copy_(x_kept)
+        for _ in range(3):
+            y.zero_()
+            batch.run()
+            assert batch.status() == 0 and torch.equal(y, good)
