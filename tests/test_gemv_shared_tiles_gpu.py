@@ -79,10 +79,11 @@ def test_mlp_block(engine, oracle, m, hidden, inter):
     assert batch.status() == 0 and torch.equal(y, kept)
 
 
-@pytest.mark.parametrize("m,hidden,inter", [(2, 512, 8192), (8, 512, 8192), (3, 2560, 1280)])
+@pytest.mark.parametrize("m,hidden,inter", [(1, 512, 8192), (8, 512, 8192), (3, 512, 4096)])
 def test_list_recovers_from_an_expired_wait(engine, m, hidden, inter):
-    """Every other CTA of a run gives up waiting for the gate/up item, so some parts of the down projection's tiles
-    arrive and others do not.  The run reports it, and the next ones, nothing reset but the limit, are right again."""
+    """Every other CTA of a run gives up waiting for the gate/up item, so some parts of each of the down projection's tiles
+    arrive and others do not.  Such a run reports it and stores none of these tiles, however many of them follow one
+    another, and the next good ones, nothing reset but the limit, are right."""
     import torch
 
     _, gc, gs, g2 = make_weight(inter, hidden, seed=1)
@@ -96,16 +97,13 @@ def test_list_recovers_from_an_expired_wait(engine, m, hidden, inter):
     batch.run()
     assert batch.status() == 0
     good = y.clone()
-    for _ in range(2):
+    for _ in range(4):
         batch.debug_wait(4096, 1)
+        y.zero_()
         batch.run()
-        assert batch.status() == 15
-        batch.debug_wait(1 << 22, 0)
-        x_kept = x.clone()
-        x.mul_(-3.0)  # stale sums of an earlier run would be those of another input
+        assert batch.status() == 15 and not bool(y.any())
+    batch.debug_wait(1 << 22, 0)
+    for _ in range(3):
+        y.zero_()
         batch.run()
-        x.copy_(x_kept)
-        for _ in range(3):
-            y.zero_()
-            batch.run()
-            assert batch.status() == 0 and torch.equal(y, good)
+        assert batch.status() == 0 and torch.equal(y, good)
