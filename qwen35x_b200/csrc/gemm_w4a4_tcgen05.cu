@@ -669,17 +669,17 @@ int launch_gemm_ksplit(const q35b_weight * w, const uint8_t * a_codes, const uin
     {gemm_w4a4_ksplit_kernel<1, kEpiPlain>, gemm_w4a4_ksplit_kernel<2, kEpiPlain>, gemm_w4a4_ksplit_kernel<4, kEpiPlain>, gemm_w4a4_ksplit_kernel<8, kEpiPlain>},
     {gemm_w4a4_ksplit_kernel<1, kEpiGateUp>, gemm_w4a4_ksplit_kernel<2, kEpiGateUp>, gemm_w4a4_ksplit_kernel<4, kEpiGateUp>, gemm_w4a4_ksplit_kernel<8, kEpiGateUp>},
     {gemm_w4a4_ksplit_kernel<1, kEpiNvfp4>, gemm_w4a4_ksplit_kernel<2, kEpiNvfp4>, gemm_w4a4_ksplit_kernel<4, kEpiNvfp4>, gemm_w4a4_ksplit_kernel<8, kEpiNvfp4>}};
-  static std::atomic<bool> attr_set[64];
-  if (!attr_set[w->device & 63].load(std::memory_order_acquire)) {
+  const int epi = ep.q_codes != nullptr ? kEpiNvfp4 : (ep.gate_up ? kEpiGateUp : kEpiPlain), log2_split = split == 8 ? 3 : split >> 1;
+  const Kernel kernel = kernels[epi][log2_split];
+  // Only the instantiation that runs: setting the attribute loads the kernel, and all twelve made the first projection of a
+  // process take 0.93 ms instead of 0.31.
+  static std::atomic<bool> attr_set[64][3][4];
+  std::atomic<bool> & set = attr_set[w->device & 63][epi][log2_split];
+  if (!set.load(std::memory_order_acquire)) {
     // idempotent, so two threads getting here together is harmless
-    for (const auto & row : kernels) {
-      for (const Kernel f : row) {
-        Q35B_CUDA_TRY(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemFull), "cudaFuncSetAttribute(gemm smem)");
-      }
-    }
-    attr_set[w->device & 63].store(true, std::memory_order_release);
+    Q35B_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemFull), "cudaFuncSetAttribute(gemm smem)");
+    set.store(true, std::memory_order_release);
   }
-  const Kernel kernel = kernels[ep.q_codes != nullptr ? kEpiNvfp4 : (ep.gate_up ? kEpiGateUp : kEpiPlain)][split == 8 ? 3 : split >> 1];
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(row_blocks), static_cast<unsigned>(token_tiles), static_cast<unsigned>(split));
   cfg.blockDim = dim3(kThreads);
