@@ -640,9 +640,11 @@ GemmPlan plan_gemm(int m, int rows, int n_total, int k, int sms, bool gather, bo
     const Shape shape = choose_shape(m, (n_total + kRows - 1) / kRows, k_steps, sms, kMaxSplit);
     return {false, shape.tile_cols, shape.split, kMmaPerStage};
   }
-  const long tiles = static_cast<long>(row_blocks) * ((m + kMaxCols - 1) / kMaxCols);
+  const long token_tiles = (m + kMaxCols - 1L) / kMaxCols, tiles = row_blocks * token_tiles;
   const long few = static_cast<long>(sms) * (k_steps <= 4 ? 3 : (k_steps <= 20 ? 2 : 1));
-  if (gemm_2cta_eligible(rows, m, k) && (gather || (tiles > few && rows_aligned))) return {true, 0, 1, 1};
+  // token tiles are the grid's y here, at most 65535 of them; the pairs walk any number
+  const bool pairs = gather || (tiles > few && rows_aligned) || token_tiles > 65535;
+  if (pairs && gemm_2cta_eligible(rows, m, k)) return {true, 0, 1, 1};
   return {false, choose_shape(m, row_blocks, k_steps, sms, 1).tile_cols, 1, 1};
 }
 

@@ -30,6 +30,12 @@ def test_order_of_summation_does_not_depend_on_the_shard(engine):
     assert splits == {1, 2, 4, 8}
 
 
+def test_more_token_tiles_than_a_grid_has_rows(engine):
+    """Rows that are not aligned keep off the kernel of CTA pairs, but not where the other one cannot be launched."""
+    assert not engine.gemm_plan(65535 * 128, 200, 64, rows_aligned=False)["pairs"]
+    assert engine.gemm_plan(65535 * 128 + 1, 200, 64, rows_aligned=False)["pairs"]
+
+
 def test_plan_rejects(engine):
     for args in ((0, 128, 128, 64), (8, 0, 128, 64), (8, 256, 128, 64), (8, 128, 128, 100)):
         with pytest.raises(engine.Q35bError):
