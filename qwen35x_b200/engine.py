@@ -175,8 +175,12 @@ def _torch():
 
 
 def _stream_ptr(torch) -> int:
-    # the raw handle: torch.cuda.current_stream() builds a Stream object first, 3.3 us of the 12 a decode projection took
-    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    # the raw handle: torch.cuda.current_stream() builds a Stream object first, 3.3 us of the 12 a decode projection took;
+    # the names are private, so it is what a torch without them gets
+    try:
+        return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    except AttributeError:
+        return int(torch.cuda.current_stream().cuda_stream)
 
 
 class Nvfp4Weight:
