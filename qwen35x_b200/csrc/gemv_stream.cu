@@ -739,8 +739,12 @@ gemv_w4a16_stream_kernel(const GemvItem * __restrict__ items, const GemvTile * _
       }
     }
     if constexpr (SHARED) {
-      // the parts from the tile it gave up in on; a warp leaves that loop only before its tile's parts meet
-      if (!ok && kh == 0 && lane == 0) give_up_parts(tiles + tile_begin + ti, tiles + tile_begin + n_tiles, arrivals, rg);
+      // the parts from the tile it gave up in on; a warp leaves that loop only before its tile's parts meet.  One that ran
+      // out of polls on its first activations may still be under the run before, whose parts use the same counters.
+      if (!ok && kh == 0) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        if (lane == 0) give_up_parts(tiles + tile_begin + ti, tiles + tile_begin + n_tiles, arrivals, rg);
+      }
     }
     if (ok && prev_item >= 0) {
       __syncwarp();

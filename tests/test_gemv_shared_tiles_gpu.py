@@ -80,10 +80,11 @@ def test_mlp_block(engine, oracle, m, hidden, inter):
 
 
 @pytest.mark.parametrize("m,hidden,inter", [(1, 512, 8192), (8, 512, 8192), (3, 512, 4096)])
-def test_list_recovers_from_an_expired_wait(engine, m, hidden, inter):
+@pytest.mark.parametrize("back_to_back", [False, True])
+def test_list_recovers_from_an_expired_wait(engine, m, hidden, inter, back_to_back):
     """Every other CTA of a run gives up waiting for the gate/up item, so some parts of each of the down projection's tiles
     arrive and others do not.  Such a run reports it and stores none of these tiles, however many of them follow one
-    another, and the next good ones, nothing reset but the limit, are right."""
+    another or start under one another's tail, and the next good ones, nothing reset but the limit, are right."""
     import torch
 
     _, gc, gs, g2 = make_weight(inter, hidden, seed=1)
@@ -100,7 +101,8 @@ def test_list_recovers_from_an_expired_wait(engine, m, hidden, inter):
     for _ in range(4):
         batch.debug_wait(4096, 1)
         y.zero_()
-        batch.run()
+        for _ in range(4 if back_to_back else 1):
+            batch.run()
         assert batch.status() == 15 and not bool(y.any())
     batch.debug_wait(1 << 22, 0)
     for _ in range(3):
