@@ -12,6 +12,10 @@ pytestmark = pytest.mark.gpu
 REL_L2_TOL = 1e-3
 
 
+def _rel_l2_rounded(oracle, got, want):
+    return oracle.rel_l2(oracle.bf16_to_f32(from_torch_bf16(got)), oracle.bf16_to_f32(oracle.bf16_round(want.astype(np.float32))))
+
+
 @pytest.mark.parametrize("m", [1, 2, 4, 5, 8])
 @pytest.mark.parametrize("shapes", [[(1, 256)], [(130, 768)], [(257, 9216)], [(2560, 9216), (100, 512)], [(5000, 1280)] * 12])
 def test_independent_items(engine, oracle, m, shapes):
@@ -38,7 +42,7 @@ def test_independent_items(engine, oracle, m, shapes):
     for (w, x, y, res), (codes, scales, s2, xb) in zip(items, host):
         _, ef = oracle.gemv_bf16(codes, scales, s2, xb, threads=8)
         want = np.asarray(ef) + (res.float().cpu().numpy() if res is not None else 0.0)
-        assert oracle.rel_l2(oracle.bf16_to_f32(from_torch_bf16(y)), want.astype(np.float32)) <= 2.0 ** -9 + REL_L2_TOL
+        assert _rel_l2_rounded(oracle, y, want) <= REL_L2_TOL
 
 
 @pytest.mark.parametrize("m", [1, 3, 8])
@@ -61,11 +65,10 @@ def test_mlp_block(engine, oracle, m, hidden, inter):
     _, gate = oracle.gemv_bf16(gc, gs, g2, xb, threads=8)
     _, up = oracle.gemv_bf16(uc, us, u2, xb, threads=8)
     want_h = gate / (1.0 + np.exp(-gate.astype(np.float64))) * up
-    hb = from_torch_bf16(h)
-    assert oracle.rel_l2(oracle.bf16_to_f32(hb), want_h.astype(np.float32)) <= 2.0 ** -9 + REL_L2_TOL
-    _, ef = oracle.gemv_bf16(dc, ds, d2, hb, threads=8)
+    assert _rel_l2_rounded(oracle, h, want_h) <= REL_L2_TOL
+    _, ef = oracle.gemv_bf16(dc, ds, d2, from_torch_bf16(h), threads=8)
     want = np.asarray(ef) + res.float().cpu().numpy()
-    assert oracle.rel_l2(oracle.bf16_to_f32(from_torch_bf16(y)), want.astype(np.float32)) <= 2.0 ** -9 + REL_L2_TOL
+    assert _rel_l2_rounded(oracle, y, want) <= REL_L2_TOL
     kept = y.clone()
     stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
     with torch.cuda.stream(stream):
