@@ -12,20 +12,21 @@ pytestmark = pytest.mark.gpu
 
 REL_L2_TOL = 1e-3
 
-SHAPES = [
-    # m, n, k
-    (1, 1, 64), (1, 3, 4096), (15, 127, 192), (16, 129, 512), (17, 108, 5760),  # split 1 .. 8, one short K step
-    (63, 512, 2304), (64, 512, 2304), (65, 512, 4672), (127, 250, 9216), (128, 256, 9216),  # 64- and 128-token tiles
-    (129, 2560, 320), (255, 1022, 1024), (300, 1001, 704),  # several token tiles, the last one partial
-    (1000, 3584, 256),  # more tiles than SMs
+SHAPES = [  # m, n, k and the split that the plan picks
+    (1, 1, 64, 1), (1, 3, 4096, 8), (15, 127, 192, 1), (16, 129, 512, 1), (17, 108, 5760, 8), (7, 5001, 2048, 2),  # one short K step
+    (63, 512, 2304, 1), (64, 512, 2304, 1), (65, 512, 4672, 4), (127, 250, 9216, 8), (128, 256, 9216, 8),  # 64- and 128-token tiles
+    (129, 2560, 320, 1), (255, 1022, 1024, 1), (300, 1001, 704, 1),  # several token tiles, the last one partial
+    (1000, 3584, 256, 1),  # more tiles than SMs
 ]
 
 
 @pytest.mark.parametrize("residual", [False, True])
-@pytest.mark.parametrize("m,n,k", SHAPES)
-def test_against_oracle(engine, oracle, m, n, k, residual):
+@pytest.mark.parametrize("m,n,k,split", SHAPES)
+def test_against_oracle(engine, oracle, m, n, k, split, residual):
     import torch
 
+    plan = engine.gemm_plan(m, n, k)
+    assert plan["split"] == split and not plan["pairs"]
     _, codes, scales, s2 = make_weight(n, k, seed=m + n + k)
     xb = make_activations(m, k, m + 1, outlier_frac=0.001)
     w = engine.Nvfp4Weight.from_host(codes, scales, s2)
@@ -45,7 +46,7 @@ def test_against_oracle(engine, oracle, m, n, k, residual):
 
 
 @pytest.mark.parametrize("m", [1, 33, 100, 200, 513])
-@pytest.mark.parametrize("inter,k", [(64, 64), (192, 4096), (1000, 512)])
+@pytest.mark.parametrize("inter,k", [(64, 64), (192, 4096), (1000, 512), (2504, 2048)])  # split in 1, 2, 4 and 8
 def test_gate_up_matches_its_halves(engine, oracle, m, inter, k):
     """silu(gate) * up of the fused epilogue against the two halves projected on their own (BF16 outputs): two roundings of
     2^-9 on its inputs and one on the result, and silu's slope is at most 1.1."""
