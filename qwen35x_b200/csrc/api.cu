@@ -105,8 +105,12 @@ int alloc_weight(int n, int k, int shard_index, int shard_count, float s2, float
 
 using namespace q35b;
 
-// Q35B_GEMV_AUTO sends a single projection to the streaming kernel from this many weight bytes on (measured
-// crossover on B200: the SIMT launch wins at 13 MB, the streaming kernel at 47 MB).
+// Q35B_GEMV_AUTO sends a single projection to the streaming kernel from this many weight bytes on: from about there it
+// is even or ahead for every K and token count.  Measured on B200, us in graph replays, rows kernel / streaming kernel: at 24
+// MiB with K = 1024, 2560 and 9216, one token 11.6 / 10.1, 11.9 / 10.2, 19.2 / 19.2, two 16.2 / 10.4, 15.1 / 10.5, 18.9 / 20.2,
+// eight 40.3 / 11.3, 37.0 / 12.2, 52.1 / 22.9; at 48 MiB one token 21.6 / 14.5, 21.0 / 13.1, 26.9 / 20.5.  Below it who wins
+// depends on both: at 8 MiB one token 5.0 / 5.6, 6.4 / 7.2, 14.6 / 18.6, eight 16.1 / 6.6, 16.7 / 8.6, 41.6 / 22.3, so that with
+// short K or several tokens the streaming kernel would be ahead from 4 to 12 MiB on.
 static constexpr size_t kAutoStreamBytes = 24u << 20;
 
 extern "C" {
@@ -293,9 +297,8 @@ int q35b_gemv_w4a16_bf16(const q35b_weight * w, const void * x_bf16, int m, void
   if (kernel == Q35B_GEMV_AUTO && w != nullptr && m >= 1 && m <= 8 && !w->gate_up &&
       w->codes_bytes + w->scales_bytes >= kAutoStreamBytes && x_bf16 != nullptr &&
       (reinterpret_cast<uintptr_t>(x_bf16) & 15u) == 0 && gemv_stream_eligible(w, m)) {
-    // A weight this large keeps the persistent streaming kernel busy for longer than its set-up costs; below the
-    // threshold the plain SIMT launch finishes first.  The streaming kernel's first use allocates its work list,
-    // which a capturing stream must not do: stay on the SIMT kernel then.
+    // A weight this large keeps the persistent streaming kernel busy for longer than its set-up costs.  Its first use
+    // allocates the work list, which a capturing stream must not do: stay on the rows kernel then.
     bool can_stream = w->stream_batch[m] != nullptr;
     if (!can_stream) {
       cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
