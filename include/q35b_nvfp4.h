@@ -196,7 +196,8 @@ Q35B_API int q35b_gemv_batch_create_tensor(const q35b_gemv_item * items, int cou
  * serialisation: the kernel may begin streaming WEIGHTS while the previous kernel of the stream is still finishing
  * (activations, residuals and outputs are touched only after that kernel is complete).  Weights are therefore
  * treated as constant from q35b_weight_create* on; a host that rewrites weight memory must synchronise the stream
- * before the next run. */
+ * before the next run.  Runs of one list must not overlap, with or without `after` items (counters and partial sums of
+ * a run live in the list): one stream, or an ordering between them. */
 Q35B_API int q35b_gemv_batch_run(const q35b_gemv_batch * batch, q35b_stream stream);
 Q35B_API void q35b_gemv_batch_destroy(q35b_gemv_batch * batch);
 /* Copies the batch's device status word to the host (synchronises): 0, or the code of a bounded device-side wait

@@ -30,9 +30,9 @@ inline void count_launch(unsigned n = 1) { g_launches.fetch_add(n, std::memory_o
 int sm_count();
 
 // Launch with programmatic stream serialisation: the grid may be scheduled while the previous kernel of the stream is
-// still finishing.  Every kernel launched this way executes griddepcontrol.wait before its first access to global
-// memory, which returns only when everything earlier in the stream is complete and visible, so what overlaps is
-// launch latency and the prologue (barrier set-up, TMEM allocation), never data.
+// still finishing.  A kernel launched this way may read what no kernel ever writes (weights and their descriptors,
+// constant from q35b_weight_create* on) before griddepcontrol.wait, which returns only when everything earlier in the
+// stream is complete and visible; what an earlier kernel may have written or may still read it touches only after it.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args &&... args) {
   cudaLaunchConfig_t cfg = {};

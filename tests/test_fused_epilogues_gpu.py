@@ -104,7 +104,7 @@ def test_weight_dequant_bf16_bit_exact(engine, oracle):
 
 @pytest.mark.parametrize("m", [7, 300])
 def test_prefill_gemm_plus_residual(engine, oracle, m):
-    """c = bf16(W4A4 projection + residual) in the GEMM epilogue (1-CTA kernel for m = 7, 2-CTA for m = 300)."""
+    """c = bf16(W4A4 projection + residual) in the GEMM epilogue (K-split kernel)."""
     import torch
 
     n, k = 520, 1024
