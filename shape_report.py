@@ -220,10 +220,7 @@ def gemm_entries(q, torch, device, peaks, n, k, ms, label, row_outliers=False):
             if m <= 128 and name == "gemm_only":
                 # few tokens: the weight stream bounds the cell, not the tensor pipe
                 row[name]["hbm_frac"] = round(alg_bytes / us / 1e3 / peaks["hbm_gbs"], 4)
-        k_steps = (k + 255) // 256
-        few = torch.cuda.get_device_properties(0).multi_processor_count * (3 if k_steps <= 4 else 2 if k_steps <= 20 else 1)
-        pairs = m >= 256 and n >= 192 and n % 16 == 0 and -(-n // 128) * -(-m // 128) > few
-        row["kernel"] = "gemm_w4a4_2cta_kernel" if pairs else "gemm_w4a4_ksplit_kernel"
+        row["kernel"] = "gemm_w4a4_2cta_kernel" if q.gemm_plan(m, n, k, rows_aligned=n % 16 == 0)["pairs"] else "gemm_w4a4_ksplit_kernel"
         out.append(row)
         del data
         torch.cuda.empty_cache()
