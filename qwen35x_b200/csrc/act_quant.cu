@@ -16,10 +16,11 @@
 // (src/runtime/cuda_bench.cu:58-96).  0x7f is never emitted because the
 // tensor-core UE4M3 format reads it as NaN.
 //
-// HBM traffic per [M,K] BF16 call: 2*M*K read by the amax pass, 2*M*K read
-// again (L2-resident for prefill sizes) + M*K/2 + M*K/16 written by the
-// quantise pass.
+// HBM traffic per [M,K] BF16 call: 2*M*K read once (what the second pass does
+// not find in registers it finds in L2) + M*K/2 + M*K/16 written.
 #include <cuda_bf16.h>
+
+#include <algorithm>
 
 #include "engine.h"
 #include "nvfp4_codec.cuh"
@@ -30,49 +31,20 @@ namespace {
 
 constexpr int kThreads = 256;
 
-// Running maximum of |v| over pairs of BF16 values; like fmaxf it skips NaNs.
-__device__ __forceinline__ void abs_max8(const uint4 q, __nv_bfloat162 & best) {
-  const uint32_t r[4] = {q.x & 0x7fff7fffu, q.y & 0x7fff7fffu, q.z & 0x7fff7fffu, q.w & 0x7fff7fffu};
-#pragma unroll
-  for (int j = 0; j < 4; ++j) best = __hmax2(best, *reinterpret_cast<const __nv_bfloat162 *>(&r[j]));
-}
-
-// Pass 1: per-tensor amax -> g.  ws[0] holds the running maximum (fp32 bits),
-// ws[1] counts finished blocks; the last block publishes g and leaves both
-// words zero for the next call.
-template <typename T>
+// Per-tensor amax -> g of a weight.  ws[0] holds the running maximum (fp32 bits), ws[1] counts finished blocks; the last
+// block publishes g and leaves both words zero for the next call.
 __global__ void __launch_bounds__(kThreads)
-amax_to_global_scale_kernel(const T * __restrict__ x, size_t n, unsigned int * __restrict__ ws,
-                            float * __restrict__ g_out) {
+amax_to_global_scale_kernel(const float * __restrict__ x, size_t n, unsigned int * __restrict__ ws, float * __restrict__ g_out) {
   // no early griddepcontrol.launch_dependents here: a dependent grid that became resident early would take the
   // registers this kernel's remaining blocks need; the implicit trigger at block exit overlaps the tail only
   asm volatile("griddepcontrol.wait;" ::: "memory");  // x may come from the kernel before
   float local = 0.0f;
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
-  if constexpr (sizeof(T) == 2) {
-    const uint4 * v = reinterpret_cast<const uint4 *>(x);
-    const size_t nv = n >> 3;
-    size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    // four independent 16-byte loads in flight per thread (eight are no faster); packed maxima, two values per
-    // instruction: [100, 9216] quantised in 5.3 us instead of 6.0, [4096, 2560] in 17.0 instead of 17.7
-    __nv_bfloat162 best = __floats2bfloat162_rn(0.0f, 0.0f);
-    for (; i + 3 * stride < nv; i += 4 * stride) {
-      uint4 q[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) q[j] = __ldg(v + i + j * stride);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) abs_max8(q[j], best);
-    }
-#pragma unroll 4
-    for (; i < nv; i += stride) abs_max8(__ldg(v + i), best);
-    local = fmaxf(__low2float(best), __high2float(best));
-  } else {
-    const float4 * v = reinterpret_cast<const float4 *>(x);
-    const size_t nv = n >> 2;
-    for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < nv; i += stride) {
-      const float4 q = __ldg(v + i);
-      local = fmaxf(local, fmaxf(fmaxf(fabsf(q.x), fabsf(q.y)), fmaxf(fabsf(q.z), fabsf(q.w))));
-    }
+  const float4 * v = reinterpret_cast<const float4 *>(x);
+  const size_t nv = n >> 2;
+  for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < nv; i += stride) {
+    const float4 q = __ldg(v + i);
+    local = fmaxf(local, fmaxf(fmaxf(fabsf(q.x), fabsf(q.y)), fmaxf(fabsf(q.z), fabsf(q.w))));
   }
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) local = fmaxf(local, __shfl_xor_sync(0xffffffffu, local, off));
@@ -180,9 +152,246 @@ quantize_nvfp4_kernel(const T * __restrict__ x, int rows, int rows_padded, int k
   }
 }
 
+// ---- activations: amax, per-tensor scale and quantisation in one launch --------------------------------------------
+
+// What bounds it, once a BF16 value costs one conversion (nvfp4_quant_block.cuh): about 150 instructions per block at 60 %
+// of the issue slots, and for a tensor's own scale the first pass with the meeting at its end.  Four CTAs of 256 threads
+// per SM leave registers for two held blocks and one on its way (five CTAs and one block: [4096, 2560] 15.0 us; three and
+// four: 12.9, but 8.8 instead of 7.0 with a given scale).  us, amax launch + quantise launch with two conversions per
+// value -> now, graph replays over more than L2: [16, 2560] 5.0 -> 3.5, [100, 9216] 6.2 -> 4.9, [4096, 2560] 17.3 -> 13.4,
+// [4096, 9216] 48.7 -> 33.5; with a given scale 1.9 -> 1.6, 2.5 -> 2.1, 10.2 -> 7.0, 30.7 -> 18.9; fp32 [1000, 1024] 7.9 -> 5.4.
+constexpr int kActCtas = 4;          // per SM
+constexpr int kHold = 2;             // blocks a thread keeps in registers between the two passes
+constexpr int kAmaxPolls = 1 << 12;  // looks at the arrival count (a few ms) before a CTA works out the amax alone
+
+// Block slots of a tiled activation: `slots` (a multiple of four) per row, numbered through the rows.
+struct SlotMap {
+  uint32_t slots;
+  uint32_t magic, shift;  // index / slots = umulhi(index, magic) >> shift for indexes below 2^31
+};
+
+__device__ __forceinline__ void locate(uint32_t i, const SlotMap & s, uint32_t & row, uint32_t & b) {
+  row = __umulhi(i, s.magic) >> s.shift;
+  b = i - row * s.slots;
+}
+__device__ __forceinline__ void locate(size_t i, const SlotMap & s, uint32_t & row, uint32_t & b) {
+  row = static_cast<uint32_t>(i / s.slots);
+  b = static_cast<uint32_t>(i % s.slots);
+}
+
+// |values| of 16 bytes into the running maximum; like fmaxf both skip NaNs.
+template <typename T>
+__device__ __forceinline__ float abs_max(const uint4 q, float best);
+template <>
+__device__ __forceinline__ float abs_max<float>(const uint4 q, float best) {
+  return fmaxf(best, fmaxf(fmaxf(fabsf(__uint_as_float(q.x)), fabsf(__uint_as_float(q.y))),
+                           fmaxf(fabsf(__uint_as_float(q.z)), fabsf(__uint_as_float(q.w)))));
+}
+__device__ __forceinline__ uint32_t bf16x2_abs_max(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("max.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+template <>
+__device__ __forceinline__ float abs_max<__nv_bfloat16>(const uint4 q, float best) {
+  // two values per instruction; a pair of NaNs leaves one, which the last step skips
+  const uint32_t m = bf16x2_abs_max(bf16x2_abs_max(q.x, q.y), bf16x2_abs_max(q.z, q.w));
+  return fmaxf(best, fmaxf(fabsf(__uint_as_float(m << 16)), fabsf(__uint_as_float(m & 0xffff0000u))));
+}
+
+// Codes and scale byte of one block.
+template <typename T, bool TABLE>
+__device__ __forceinline__ uint32_t quantize_raw(const uint4 (&r)[sizeof(T)], float g, float rg, const float * table, uint2 & out) {
+  if constexpr (sizeof(T) == 2) {
+    return quantize_block_bf16<TABLE>(r[0], r[1], g, rg, table, out);
+  } else {
+    float v[16];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      v[4 * i] = __uint_as_float(r[i].x);
+      v[4 * i + 1] = __uint_as_float(r[i].y);
+      v[4 * i + 2] = __uint_as_float(r[i].z);
+      v[4 * i + 3] = __uint_as_float(r[i].w);
+    }
+    return quantize_block<kEngine>(v, g, false, out);
+  }
+}
+
+// Codes and scale byte of the block in `slot` (in: not one of the padding).
+template <typename T, bool TABLE, typename Idx>
+__device__ __forceinline__ void emit(Idx slot, bool in, const uint4 (&r)[sizeof(T)], const SlotMap & map, uint32_t scale_cols, Idx total, float g,
+                                     float rg, const float * table, uint8_t * __restrict__ codes, uint8_t * __restrict__ scales) {
+  uint32_t sb = 0, row, b;
+  locate(slot, map, row, b);
+  if (in) {
+    uint2 packed;
+    sb = quantize_raw<T, TABLE>(r, g, rg, table, packed);
+    *(reinterpret_cast<uint2 *>(codes) + (static_cast<Idx>(row) * scale_cols + b)) = packed;
+  }
+  // the quad's four scale bytes (whole quads get here together: slots and kThreads are multiples of four)
+  uint32_t word = sb << (8 * (threadIdx.x & 3));
+  word |= __shfl_xor_sync(0xffffffffu, word, 1);
+  word |= __shfl_xor_sync(0xffffffffu, word, 2);
+  if ((threadIdx.x & 3) == 0 && slot < total) {
+    const uint32_t tile = (row >> 7) * (map.slots >> 2) + (b >> 2);
+    *reinterpret_cast<uint32_t *>(scales + static_cast<size_t>(tile) * 512 + ((row & 31) * 16 + (row >> 5 & 3) * 4)) = word;
+  }
+}
+
+// One thread per 16-element block and turn, so a warp reads 1 KB (fp32: 2 KB) of contiguous activations and writes 256
+// bytes of contiguous codes; the four scale bytes of a 64-element group meet in lane 0 of each quad and leave as one
+// 32-bit word of the tiled layout.  Slots past K and rows past `rows` only produce zero scale bytes.
+// DYNAMIC: the grid (never more CTAs than are resident together) reads everything once, meets at a counter, and quantises
+// what it has kept in registers (the first kHold blocks of a thread) or reads again from L2.  No CTA depends on the others
+// being there: one that has polled kAmaxPolls times for them takes the maximum over the whole tensor by itself.
+// ws: [0] running maximum (fp32 bits), [1] CTAs that have added theirs, [2] CTAs that have read it; all zero between calls.
+// Idx: type of a slot index, 32 bits up to 2^31 slots.
+template <typename T, bool DYNAMIC, typename Idx>
+__global__ void __launch_bounds__(kThreads, kActCtas)
+quantize_activations_kernel(const T * __restrict__ x, uint32_t scale_cols, const SlotMap map, Idx live, Idx total, float g_fixed,
+                            unsigned int parts, unsigned int * ws, float * __restrict__ g_out, uint8_t * __restrict__ codes,
+                            uint8_t * __restrict__ scales) {
+  constexpr int kVecs = sizeof(T);  // 16-byte loads per block
+  constexpr int kHeld = DYNAMIC ? kHold : 1;
+  __shared__ float table[128];
+  __shared__ float red[kThreads / 32];
+  __shared__ float shared_amax;
+  // every CTA of the grid is resident: the next kernel of the stream may move in beside them
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const Idx stride = static_cast<Idx>(gridDim.x) * kThreads, first = static_cast<Idx>(blockIdx.x) * kThreads;
+  const bool even = map.slots == scale_cols;  // no padding slots: a slot's index is its block's
+  float g = g_fixed, rg = 1.0f;
+  // the multipliers pay as a table from the second turn on
+  const bool many = sizeof(T) == 2 && stride < live;
+  if constexpr (!DYNAMIC) {
+    rg = __frcp_rn(g);
+    if (many) {
+      if (threadIdx.x < 127) table[threadIdx.x] = bf16_block_multiplier(threadIdx.x, g);
+      __syncthreads();
+    }
+  }
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // x may come from the kernel before, which may also read the scratch
+
+  // false: a slot of the padding
+  auto load = [&](Idx slot, uint4 (&r)[kVecs]) -> bool {
+    Idx f = slot;
+    bool in = slot < live;
+    if (!even) {
+      uint32_t row, b;
+      locate(slot, map, row, b);
+      f = static_cast<Idx>(row) * scale_cols + b;
+      in = in && b < scale_cols;
+    }
+    const uint4 * src = reinterpret_cast<const uint4 *>(x) + static_cast<size_t>(f) * kVecs;
+#pragma unroll
+    for (int i = 0; i < kVecs; ++i) r[i] = in ? __ldg(src + i) : make_uint4(0u, 0u, 0u, 0u);
+    return in;
+  };
+
+  uint4 held[kHeld][kVecs];
+  bool held_in[kHeld];
+#pragma unroll
+  for (int h = 0; h < kHeld; ++h) held_in[h] = load(first + h * stride + threadIdx.x, held[h]);
+  if constexpr (DYNAMIC) {
+    if (first < live) {  // the other CTAs only write padding
+      float best = 0.0f;
+#pragma unroll
+      for (int h = 0; h < kHeld; ++h) {
+#pragma unroll
+        for (int i = 0; i < kVecs; ++i) best = abs_max<T>(held[h][i], best);
+      }
+#pragma unroll 2
+      for (Idx at = first + kHeld * stride; at < live; at += stride) {
+        uint4 r[kVecs];
+        load(at + threadIdx.x, r);
+#pragma unroll
+        for (int i = 0; i < kVecs; ++i) best = abs_max<T>(r[i], best);
+      }
+      auto block_max = [&](float v) {
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, off));
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+        __syncthreads();
+        float m = red[0];
+#pragma unroll
+        for (int i = 1; i < kThreads / 32; ++i) m = fmaxf(m, red[i]);
+        return m;
+      };
+      best = block_max(best);
+      if (threadIdx.x == 0) {
+        atomicMax(ws, __float_as_uint(best));
+        __threadfence();
+        unsigned int here = atomicAdd(ws + 1, 1u) + 1u;
+        for (int i = 0; here < parts && i < kAmaxPolls; ++i) asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(here) : "l"(ws + 1) : "memory");
+        float amax = -1.0f;
+        if (here >= parts) amax = __uint_as_float(*reinterpret_cast<volatile unsigned int *>(ws));
+        shared_amax = amax;
+        if (atomicAdd(ws + 2, 1u) == parts - 1u) {  // all have added theirs and read the result
+          ws[0] = 0u;
+          ws[1] = 0u;
+          ws[2] = 0u;
+        }
+      }
+      __syncthreads();
+      float amax = shared_amax;
+      if (amax < 0.0f) {
+        best = 0.0f;
+        for (Idx at = threadIdx.x; at < live; at += kThreads) {
+          uint4 r[kVecs];
+          load(at, r);
+#pragma unroll
+          for (int i = 0; i < kVecs; ++i) best = abs_max<T>(r[i], best);
+        }
+        amax = block_max(best);
+      }
+      g = amax > 0.0f ? __fdiv_rn(amax, 6.0f * 448.0f) : 1.0f;
+      rg = __frcp_rn(g);
+      if (many) {
+        if (threadIdx.x < 127) table[threadIdx.x] = bf16_block_multiplier(threadIdx.x, g);
+        __syncthreads();
+      }
+    }
+  }
+  if (g_out != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *g_out = g;
+
+  if (!many) {
+#pragma unroll
+    for (int h = 0; h < kHeld; ++h) {
+      if (first + h * stride < total) emit<T, false>(first + h * stride + threadIdx.x, held_in[h], held[h], map, scale_cols, total, g, rg, table, codes, scales);
+    }
+    for (Idx at = first + kHeld * stride; at < total; at += stride) {  // padding, or fp32
+      uint4 r[kVecs];
+      const bool in = load(at + threadIdx.x, r);
+      emit<T, false>(at + threadIdx.x, in, r, map, scale_cols, total, g, rg, table, codes, scales);
+    }
+    return;
+  }
+  if constexpr (sizeof(T) == 2) {
+    // the next block is on its way while one is quantised
+    uint4 next[kVecs];
+    Idx at = first + kHeld * stride;
+    bool next_in = at < total && load(at + threadIdx.x, next);
+#pragma unroll
+    for (int h = 0; h < kHeld; ++h) {
+      if (first + h * stride < total) emit<T, true>(first + h * stride + threadIdx.x, held_in[h], held[h], map, scale_cols, total, g, rg, table, codes, scales);
+    }
+#pragma unroll 1
+    while (at < total) {
+      uint4 r[kVecs];
+#pragma unroll
+      for (int i = 0; i < kVecs; ++i) r[i] = next[i];
+      const bool in = next_in;
+      const Idx slot = at + threadIdx.x;
+      at += stride;
+      next_in = at < total && load(at + threadIdx.x, next);
+      emit<T, true>(slot, in, r, map, scale_cols, total, g, rg, table, codes, scales);
+    }
+  }
+}
+
 __global__ void __launch_bounds__(kThreads)
 tile_scales_kernel(const uint8_t * __restrict__ src, int rows, int rows_padded, int scale_cols,
-                   uint8_t * __restrict__ tiled, unsigned int * __restrict__ sign_flag) {
+                   uint8_t * __restrict__ tiled, unsigned int * __restrict__ flags) {
   const int groups = (scale_cols + 3) >> 2;
   const size_t idx = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (idx >= static_cast<size_t>(rows_padded) * groups) return;
@@ -197,7 +406,11 @@ tile_scales_kernel(const uint8_t * __restrict__ src, int rows, int rows_padded, 
     }
   }
   *reinterpret_cast<uint32_t *>(tiled + tiled_scale_offset(row, grp * 4, groups * 4)) = sbytes;
-  if (sign_flag != nullptr && (sbytes & 0x80808080u) != 0u) atomicOr(sign_flag, 1u);
+  if (flags != nullptr) {
+    // some byte has its sign bit set; some byte is 0x7f or 0xff: adding one to the low seven bits carries into the eighth
+    const uint32_t found = ((sbytes & 0x80808080u) != 0u ? 1u : 0u) | ((((sbytes & 0x7f7f7f7fu) + 0x01010101u) & 0x80808080u) != 0u ? 2u : 0u);
+    if (found != 0u) atomicOr(flags, found);
+  }
 }
 
 int check_quant_args(const void * x, int m, int k, const void * codes, const void * scales) {
@@ -213,38 +426,35 @@ int check_quant_args(const void * x, int m, int k, const void * codes, const voi
 }
 
 template <typename T>
-int launch_amax(const T * x, size_t n, unsigned int * ws, float * g_out, cudaStream_t s) {
-  // few blocks (every one ends with two atomics on the same pair of words), each with plenty of loads in flight
-  const size_t per_block = static_cast<size_t>(kThreads) * 8 * 4;
-  int blocks = static_cast<int>(std::min<size_t>((n + per_block - 1) / per_block, static_cast<size_t>(sm_count()) * 4));
-  if (blocks < 1) blocks = 1;
-  const cudaError_t le = launch_pdl(amax_to_global_scale_kernel<T>, dim3(blocks), dim3(kThreads), 0, s, x, n, ws, g_out);
-  count_launch();
-  Q35B_CUDA_TRY(le, "amax_to_global_scale_kernel launch");
-  return Q35B_OK;
-}
-
-}  // namespace
-
-namespace {
-
-template <typename T>
 int launch_quantize_activations(const T * x, int m, int k, float global_scale, uint8_t * codes, uint8_t * scales_tiled,
                                 float * g_dev, void * workspace, cudaStream_t s) {
   if (const int st = check_quant_args(x, m, k, codes, scales_tiled)) return st;
   if (g_dev == nullptr) return fail(Q35B_ERR_ARGUMENT, "NVFP4 quantisation needs a device word for the input scale.");
   const bool dynamic = !(global_scale > 0.0f);
-  if (dynamic) {
-    if (workspace == nullptr) return fail(Q35B_ERR_ARGUMENT, "Dynamic NVFP4 quantisation needs its workspace.");
-    if (const int st = launch_amax(x, static_cast<size_t>(m) * k, static_cast<unsigned int *>(workspace), g_dev, s)) return st;
-  }
+  if (dynamic && workspace == nullptr) return fail(Q35B_ERR_ARGUMENT, "Dynamic NVFP4 quantisation needs its workspace.");
   const int rows_padded = round_up_int(m, 128);
-  const size_t threads = static_cast<size_t>(rows_padded) * ((((k >> 4) + 3) >> 2) << 2);
-  const unsigned blocks = static_cast<unsigned>((threads + kThreads - 1) / kThreads);
-  const cudaError_t le = launch_pdl(quantize_nvfp4_kernel<T, kEngine, true>, dim3(blocks), dim3(kThreads), 0, s, x, m, rows_padded, k,
-                                    dynamic ? g_dev : nullptr, global_scale, dynamic ? nullptr : g_dev, 0, codes, scales_tiled);
+  SlotMap map = {static_cast<uint32_t>((((k >> 4) + 3) >> 2) << 2), 0u, 0u};
+  const size_t total = static_cast<size_t>(rows_padded) * map.slots, live = static_cast<size_t>(m) * map.slots;
+  const size_t per_turn = static_cast<size_t>(sm_count()) * kActCtas * kThreads;
+  const unsigned grid = static_cast<unsigned>(std::min((total + kThreads - 1) / kThreads, per_turn / kThreads));
+  const unsigned parts = static_cast<unsigned>(std::min<size_t>(grid, (live + kThreads - 1) / kThreads));
+  cudaError_t le;
+  if (total + (kHold + 1) * per_turn < (1u << 31)) {
+    // ceil(2^(31 + l) / slots) with 2^(l - 1) < slots <= 2^l divides every index below 2^31 exactly; slots >= 4, so l >= 2
+    int l = 2;
+    while ((1u << l) < map.slots) ++l;
+    map.magic = static_cast<uint32_t>(((1ull << (31 + l)) + map.slots - 1) / map.slots);
+    map.shift = static_cast<uint32_t>(l - 1);
+    le = launch_pdl(dynamic ? quantize_activations_kernel<T, true, uint32_t> : quantize_activations_kernel<T, false, uint32_t>, dim3(grid),
+                    dim3(kThreads), 0, s, x, static_cast<uint32_t>(k >> 4), map, live, total, global_scale, parts,
+                    static_cast<unsigned int *>(workspace), g_dev, codes, scales_tiled);
+  } else {
+    le = launch_pdl(dynamic ? quantize_activations_kernel<T, true, size_t> : quantize_activations_kernel<T, false, size_t>, dim3(grid),
+                    dim3(kThreads), 0, s, x, static_cast<uint32_t>(k >> 4), map, live, total, global_scale, parts,
+                    static_cast<unsigned int *>(workspace), g_dev, codes, scales_tiled);
+  }
   count_launch();
-  Q35B_CUDA_TRY(le, "quantize_nvfp4_kernel launch");
+  Q35B_CUDA_TRY(le, "quantize_activations_kernel launch");
   return Q35B_OK;
 }
 
@@ -280,7 +490,13 @@ int launch_quantize_weight_f32(const float * w, int n, int k, uint8_t * codes, u
     return fail(Q35B_ERR_ARGUMENT, "NVFP4 weight quantisation received a null buffer.");
   }
   if (n <= 0 || k <= 0 || (k % 16) != 0) return fail(Q35B_ERR_SHAPE, "Invalid dimensions for NVFP4 weight quantisation.");
-  if (const int st = launch_amax(w, static_cast<size_t>(n) * k, static_cast<unsigned int *>(workspace), s2_dev, s)) return st;
+  // few blocks (every one ends with two atomics on the same pair of words), each with plenty of loads in flight
+  const size_t elements = static_cast<size_t>(n) * k, per_block = static_cast<size_t>(kThreads) * 8 * 4;
+  const int amax_blocks = static_cast<int>(std::min<size_t>((elements + per_block - 1) / per_block, static_cast<size_t>(sm_count()) * 4));
+  const cudaError_t le = launch_pdl(amax_to_global_scale_kernel, dim3(amax_blocks), dim3(kThreads), 0, s, w, elements,
+                                    static_cast<unsigned int *>(workspace), s2_dev);
+  count_launch();
+  Q35B_CUDA_TRY(le, "amax_to_global_scale_kernel launch");
   const size_t threads = static_cast<size_t>(n) * ((((k >> 4) + 3) >> 2) << 2);
   const unsigned blocks = static_cast<unsigned>((threads + kThreads - 1) / kThreads);
   quantize_nvfp4_kernel<float, kEngine, false><<<blocks, kThreads, 0, s>>>(w, n, n, k, s2_dev, 1.0f, nullptr, 0, codes,
@@ -291,11 +507,11 @@ int launch_quantize_weight_f32(const float * w, int n, int k, uint8_t * codes, u
 }
 
 int launch_tile_scales(const uint8_t * scales_rowmajor, int rows, int scale_cols, uint8_t * tiled,
-                       unsigned int * sign_flag, cudaStream_t s) {
+                       unsigned int * flags, cudaStream_t s) {
   const int rows_padded = round_up_int(rows, 128);
   const size_t threads = static_cast<size_t>(rows_padded) * ((scale_cols + 3) >> 2);
   const unsigned blocks = static_cast<unsigned>((threads + kThreads - 1) / kThreads);
-  tile_scales_kernel<<<blocks, kThreads, 0, s>>>(scales_rowmajor, rows, rows_padded, scale_cols, tiled, sign_flag);
+  tile_scales_kernel<<<blocks, kThreads, 0, s>>>(scales_rowmajor, rows, rows_padded, scale_cols, tiled, flags);
   count_launch();
   Q35B_CUDA_TRY(cudaGetLastError(), "tile_scales_kernel launch");
   return Q35B_OK;

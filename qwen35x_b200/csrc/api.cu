@@ -159,10 +159,8 @@ int q35b_weight_create(const uint8_t * codes_host, const uint8_t * scales_host, 
     }
   }
   for (size_t i = 0; i < w->scales_bytes; ++i) {
-    if (src_scales[i] & 0x80u) {
-      w->negative_scales = true;
-      break;
-    }
+    w->negative_scales = w->negative_scales || (src_scales[i] & 0x80u) != 0;
+    w->nan_scales = w->nan_scales || (src_scales[i] & 0x7fu) == 0x7fu;
   }
   cudaError_t e = cudaSuccess;
   if (w->rows > 0) {
@@ -224,7 +222,8 @@ int q35b_weight_create_from_device(const uint8_t * codes_dev, const uint8_t * sc
     q35b_weight_destroy(w);
     return fail_cuda(e, "cudaStreamSynchronize(nvfp4 weight)");
   }
-  w->negative_scales = flag != 0;
+  w->negative_scales = (flag & 1u) != 0;
+  w->nan_scales = (flag & 2u) != 0;
   if (const int st = finish_weight(w)) {
     q35b_weight_destroy(w);
     return st;

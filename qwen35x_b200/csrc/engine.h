@@ -71,6 +71,7 @@ struct q35b_weight {
   uint8_t * scales = nullptr;       // [rows, k/16] row-major (decode kernels)
   uint8_t * scales_tiled = nullptr; // [ceil128(rows), ceil4(k/16)] 128x4 tiles (UMMA scale factors)
   size_t codes_bytes = 0, scales_bytes = 0, scales_tiled_bytes = 0;
+  bool nan_scales = false;           // some block scale is 0x7f (480 here, NaN to the tensor cores)
   bool negative_scales = false;      // some block scale has its sign bit set (only the SIMT decode kernel takes those)
   // Single-projection work lists of the streaming decode kernel, by token count: built on first use under
   // batch_mutex (the only state of a weight that changes after q35b_weight_create*).
@@ -101,7 +102,7 @@ int launch_quantize_reference_recipe(const void * x, int m, int k, int swap, uin
 int launch_quantize_weight_f32(const float * w, int n, int k, uint8_t * codes, uint8_t * scales_rowmajor,
                                float * s2_dev, void * workspace, cudaStream_t s);
 int launch_tile_scales(const uint8_t * scales_rowmajor, int rows, int scale_cols, uint8_t * tiled,
-                       unsigned int * sign_flag, cudaStream_t s);
+                       unsigned int * flags, cudaStream_t s);
 
 // gemv_stream.cu
 bool gemv_stream_eligible(const q35b_weight * w, int m);

@@ -138,41 +138,48 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
   return *reinterpret_cast<const uint32_t *>(&h);
 }
 
+// The NVFP4 output's per-tensor scale, its correctly rounded reciprocal and the table of block multipliers (NULL: none), read
+// or built once per warp or CTA: thousands of warps loading that one word per chunk would queue up on a single L2 slice.
+struct GemmQuantScale {
+  float g = 1.0f, rg = 1.0f;
+  const float * table = nullptr;
+};
+
 // gate/up -> NVFP4: 32 accumulator columns (8 gate, 8 up, 8 gate, 8 up) of row `row` -> one block of 16 outputs.
+template <bool TABLE>
 __device__ __forceinline__ void store_nvfp4_chunk32(const uint32_t (&r)[32], int row, int col0, float alpha, float alpha_up,
-                                                    const GemmEpilogue & ep, float q_g) {
-  float v[16];
+                                                    const GemmEpilogue & ep, const GemmQuantScale & q) {
+  uint32_t v[8];
 #pragma unroll
   for (int j = 0; j < 2; ++j) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const float gv = __uint_as_float(r[16 * j + i]) * alpha;
-      const float uv = __uint_as_float(r[16 * j + 8 + i]) * alpha_up;
-      v[8 * j + i] = __bfloat162float(__float2bfloat16_rn(silu_mul(gv, uv)));
+    for (int i = 0; i < 8; i += 2) {
+      v[4 * j + (i >> 1)] = pack_bf16(silu_mul(__uint_as_float(r[16 * j + i]) * alpha, __uint_as_float(r[16 * j + 8 + i]) * alpha_up),
+                                      silu_mul(__uint_as_float(r[16 * j + i + 1]) * alpha, __uint_as_float(r[16 * j + 9 + i]) * alpha_up));
     }
   }
   uint2 packed;
-  const uint32_t sb = quantize_block<kEngine>(v, q_g, false, packed);
+  const uint32_t sb = quantize_block_bf16<TABLE>(make_uint4(v[0], v[1], v[2], v[3]), make_uint4(v[4], v[5], v[6], v[7]), q.g, q.rg, q.table, packed);
   *reinterpret_cast<uint2 *>(ep.q_codes + static_cast<size_t>(row) * ep.q_ld + (col0 >> 2)) = packed;
   ep.q_scales[tiled_scale_offset(row, ep.q_slot0 + (col0 >> 5), ep.q_slots)] = static_cast<uint8_t>(sb);
 }
 
 // r: 32 accumulator columns starting at global column col0 (a multiple of 32) of row `row`; n = accumulator columns
 // of the whole problem (weight rows); g = the activation tensor's scale.
+// GATE_UP: the weight may be a gate/up one (false keeps that code out of a kernel that never sees one).
 // to_peers: also repeat every store on the other ranks (one 32-byte piece per lane); a caller that forwards whole
 // rows afterwards (gemm_forward_rows_to_peers) passes false.
-// q_g: value of *ep.q_g (the NVFP4 output's per-tensor scale), read once per warp by the caller: thousands of warps
-// loading that one word per chunk would queue up on a single L2 slice.
+template <bool GATE_UP>
 __device__ __forceinline__ void gemm_store_chunk32(const uint32_t (&r)[32], int row, int col0, int n, float g,
                                                    const GemmEpilogue & ep, __nv_bfloat16 * __restrict__ c, int ldc,
-                                                   bool to_peers = true, float q_g = 1.0f) {
+                                                   bool to_peers, const GemmQuantScale & q) {
   if (col0 >= n) return;  // a chunk wholly past the last column of a partial tile
   const int n_peers = to_peers ? ep.n_peers : 0;
   const float alpha = g * ep.s2;
-  if (ep.gate_up) {
+  if (GATE_UP && ep.gate_up) {
     const float alpha_up = g * ep.s2_up;
     if (ep.q_codes != nullptr) {
-      store_nvfp4_chunk32(r, row, col0, alpha, alpha_up, ep, q_g);  // n % 32 == 0 is checked on the host: the chunk is whole
+      store_nvfp4_chunk32<true>(r, row, col0, alpha, alpha_up, ep, q);  // n % 32 == 0 is checked on the host: the chunk is whole
       return;
     }
     __nv_bfloat16 * dst = c + static_cast<size_t>(row) * ldc + (col0 >> 1);

@@ -348,7 +348,18 @@ gemm_w4a4_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     const int quarter = warp & 3;                 // TMEM lanes 32 * quarter .. + 31 (fixed by the warp's index)
     const int col_base = ((warp - 2) >> 2) * kEpiCols;
     const float g = __ldg(g_dev);
-    const float q_g = ep.q_g != nullptr ? __ldg(ep.q_g) : 1.0f;
+    GemmQuantScale q;
+    if constexpr (kEpilogueWarps == kEpiWarpsWide) {
+      __shared__ float q_table[128];
+      if (ep.q_codes != nullptr) {
+        q.g = __ldg(ep.q_g);
+        q.rg = __frcp_rn(q.g);
+        q.table = q_table;
+        const int at = threadIdx.x - 64;
+        if (at < 127) q_table[at] = bf16_block_multiplier(at, q.g);
+        asm volatile("bar.sync 1, %0;" ::"n"(kEpilogueWarps * 32) : "memory");  // the epilogue warps only
+      }
+    }
     uint32_t li = 0;
     bool ok = !aborted;
     for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, ++li) {
@@ -377,7 +388,7 @@ gemm_w4a4_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       if (row < m) {
 #pragma unroll
         for (int j = 0; j < kEpiCols / 32; ++j) {
-          gemm_store_chunk32(r[j], row, tn * kTileN + col_base + 32 * j, n, g, ep, c, ldc, !forward, q_g);
+          gemm_store_chunk32<kEpilogueWarps == kEpiWarpsWide>(r[j], row, tn * kTileN + col_base + 32 * j, n, g, ep, c, ldc, !forward, q);
         }
       }
       if (forward) {

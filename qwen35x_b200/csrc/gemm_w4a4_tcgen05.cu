@@ -475,6 +475,7 @@ gemm_w4a4_ksplit_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
       // one thread per token and 32 weight rows = one block of 16 outputs (n % 128 == 0 is checked on the host);
       // lanes along the tokens, whose pitch spreads them over the banks
       const float q_g = __ldg(ep.q_g);
+      const GemmQuantScale q = {q_g, __frcp_rn(q_g), nullptr};
       const int live = __any_sync(0xffffffffu, stop_lane) ? 0 : t_end - t_begin;
       for (int u = threadIdx.x; u < live * (kRows / 32); u += kThreads) {
         const int t = t_begin + u % live, blk = u / live;
@@ -484,7 +485,7 @@ gemm_w4a4_ksplit_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
           const float4 a = sum4<SPLIT>(src, static_cast<uint32_t>(t * kPitch + 32 * blk + i) * 4u);
           r[i] = __float_as_uint(a.x); r[i + 1] = __float_as_uint(a.y); r[i + 2] = __float_as_uint(a.z); r[i + 3] = __float_as_uint(a.w);
         }
-        store_nvfp4_chunk32(r, token0 + t, row0 + 32 * blk, alpha, alpha_up, ep, q_g);
+        store_nvfp4_chunk32<false>(r, token0 + t, row0 + 32 * blk, alpha, alpha_up, ep, q);
       }
     } else {
       // one warp per token, four consecutive weight rows per lane

@@ -138,4 +138,109 @@ __device__ __forceinline__ uint32_t quantize_block(const float (&v)[16], float g
   return sb;
 }
 
+// ---- sixteen BF16 values, engine recipe -------------------------------------------------------------------------
+//
+// A BF16 value has eight significant bits, so with one divisor d the BF16 values next to b * d for a rounding boundary b are
+// 2^-8 of it apart: one of them at most lies closer than 2^-21, and whether its correctly rounded quotient is above b (or
+// on it, a tie that goes down) can be worked out beforehand.  If no such value has to go up, one multiplication by a
+// reciprocal that is a little too small (1 - 2^-22) puts every quotient on its side of every boundary; if none has to go
+// down, one that is a little too large does.  The hardware converter then finishes the job: one conversion per pair where
+// quantize_block needs two and a comparison.  The choice depends on the block's scale byte and the tensor's scale only, so
+// there are 127 multipliers per tensor: bf16_block_multiplier gives one of them, or 0 for "use quantize_block", and a
+// kernel that quantises many blocks per CTA keeps them in a table.  (Such close values are no rarity: under the scale of
+// a tensor, amax / 2688, an eighth of the scale bytes have divisors that are thirds of BF16 values.)
+
+// The multiplier for scale byte sb (0..0x7e) under per-tensor scale g.
+__device__ __forceinline__ float bf16_block_multiplier(uint32_t sb, float g) {
+  if (!(g >= 0x1p-60f && g <= 0x1p60f)) return 0.0f;
+  const float d = __fmul_rn(fmaxf(decode_e4m3(static_cast<uint8_t>(sb)), 1.0e-8f), g);
+  if (!(d <= 0x1p15f)) return 0.0f;  // beyond, a quotient may round to zero, which loses its sign
+  // The boundaries are 1, 1.25, 1.5 and 1.75 times powers of two.  p: d times one of these, in quarters of d's last bit;
+  // BF16 values are 2^18 of them apart in the binade of d, 2^19 in the next one.
+  const uint32_t mant = (__float_as_uint(d) & 0x7fffffu) | 0x800000u;
+  bool up = false, down = false;
+#pragma unroll 1
+  for (uint32_t n = 4; n < 8; ++n) {
+    const uint32_t p = mant * n, spacing = p < (1u << 26) ? (1u << 18) : (1u << 19);
+    const uint32_t near = (p + (spacing >> 1)) & ~(spacing - 1);
+    if (static_cast<uint32_t>(abs(static_cast<int>(near - p))) <= (p >> 21) + 1u) {
+      const bool above = __fdiv_rn(static_cast<float>(near) * 0.25f, static_cast<float>(mant)) > static_cast<float>(n) * 0.25f;
+      up = up || above;
+      down = down || !above;
+    }
+  }
+  if (up && down) return 0.0f;
+  // errors of the reciprocal, the product and the quotient's own rounding are 2^-24 each: the sum stays below 2^-22, and
+  // 2^-22 and all of them below 2^-21
+  return __fmul_rn(__frcp_rn(d), up ? 1.0f + 0x1p-22f : 1.0f - 0x1p-22f);
+}
+
+__device__ __forceinline__ uint32_t bf16x2_abs_max_nan(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("max.NaN.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+
+// quantize_block for what the multipliers do not cover (NaN, infinities, extreme scales, boundaries of both kinds), out of
+// line.
+static __device__ __noinline__ uint3 quantize_block_bf16_general(uint4 a, uint4 b, float g) {
+  const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  float v[16];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    v[2 * i] = __uint_as_float(w[i] << 16);
+    v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+  }
+  uint2 packed;
+  const uint32_t sb = quantize_block<kEngine>(v, g, false, packed);
+  return make_uint3(packed.x, packed.y, sb);
+}
+
+// Two BF16 values of a register times m as fp32 (+ 0: a negative zero becomes positive, as (value < 0) has it).
+__device__ __forceinline__ void bf16x2_scaled(uint32_t w, float m, float & lo, float & hi) {
+  asm("{\n\t.reg .b32 l, h;\n\t.reg .b64 v, mm, z;\n\t"
+      "shl.b32 l, %2, 16;\n\tand.b32 h, %2, 0xffff0000;\n\t"
+      "mov.b64 v, {l, h};\n\tmov.b64 mm, {%3, %3};\n\tmov.b64 z, {%4, %4};\n\t"
+      "fma.rn.f32x2 v, v, mm, z;\n\tmov.b64 {%0, %1}, v;\n\t}"
+      : "=f"(lo), "=f"(hi)
+      : "r"(w), "f"(m), "f"(0.0f));
+}
+
+// The bytes of quantize_block<kEngine> for sixteen BF16 values, two per register.  rg = 1 / g correctly rounded;
+// TABLE: `table` holds the multipliers of this tensor by scale byte; else the one needed is worked out here.
+template <bool TABLE>
+__device__ __forceinline__ uint32_t quantize_block_bf16(const uint4 a, const uint4 b, float g, float rg, const float * table, uint2 & out) {
+  uint32_t am = bf16x2_abs_max_nan(bf16x2_abs_max_nan(bf16x2_abs_max_nan(a.x, a.y), bf16x2_abs_max_nan(a.z, a.w)),
+                                   bf16x2_abs_max_nan(bf16x2_abs_max_nan(b.x, b.y), bf16x2_abs_max_nan(b.z, b.w)));
+  am = max((am << 16) & 0x7fffffffu, am & 0x7fff0000u);
+  // amax / 6 / g: with a correctly rounded reciprocal the second correction delivers the rounded quotient (Markstein 1990)
+  const float t = div_by_shared(__uint_as_float(am), 6.0f, 1.0f / 6.0f);
+  const float s = div_by_shared(t, g, rg);
+  const uint32_t u = __float_as_uint(s);
+  // encode_ue4m3 up to 2^24, without its branches
+  const uint32_t normal = min(((u + 0x7ffffu) >> 20) - 960u, 0x7eu);
+  const uint32_t small = static_cast<uint32_t>(max(__float2int_ru(fmaf(s, 512.0f, -0.5f)), 0));
+  const uint32_t sb = u < 0x3c800000u ? small : normal;
+  float m;
+  if constexpr (TABLE) m = table[sb]; else m = bf16_block_multiplier(sb, g);
+  const bool in_range = am - 0x21800000u <= 0x5d800000u - 0x21800000u || am == 0u;  // 2^-60 .. 2^60: no rounding above is off
+  if (!in_range || u >= 0x4b800000u || m == 0.0f) {
+    const uint3 r = quantize_block_bf16_general(a, b, g);
+    out = make_uint2(r.x, r.y);
+    return r.z;
+  }
+  float q[8];
+  bf16x2_scaled(a.x, m, q[0], q[1]);
+  bf16x2_scaled(a.y, m, q[2], q[3]);
+  bf16x2_scaled(a.z, m, q[4], q[5]);
+  bf16x2_scaled(a.w, m, q[6], q[7]);
+  out.x = cvt_e2m1x8(q);
+  bf16x2_scaled(b.x, m, q[0], q[1]);
+  bf16x2_scaled(b.y, m, q[2], q[3]);
+  bf16x2_scaled(b.z, m, q[4], q[5]);
+  bf16x2_scaled(b.w, m, q[6], q[7]);
+  out.y = cvt_e2m1x8(q);
+  return sb;
+}
+
 }  // namespace q35b
