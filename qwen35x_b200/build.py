@@ -10,6 +10,7 @@ from __future__ import annotations
 import shutil
 import subprocess
 import sys
+import sysconfig
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
@@ -17,6 +18,7 @@ CSRC = PKG / "csrc"
 LIB_DIR = PKG / "_lib"
 LIB = LIB_DIR / "libq35b.so"
 CLI = LIB_DIR / "q35b"
+BINDING = LIB_DIR / "q35b_torch.so"
 
 SOURCES = ["api.cu", "gemv_w4a16.cu", "gemv_stream.cu", "act_quant.cu", "gemm_w4a4_tcgen05.cu", "gemm_w4a4_2cta.cu", "gemm_wstream.cu", "static_prefill.cu", "peer_gather.cu"]
 NVCC_FLAGS = [
@@ -62,7 +64,24 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         cmd = [_nvcc(), "-shared", "-o", str(LIB), *map(str, objs), "-cudart", "static", "-lpthread", "-ldl"]
         subprocess.run(cmd, check=True)
     build_cli(force=force or bool(procs))
+    build_binding(force=force)
     return LIB
+
+
+def build_binding(force: bool = False) -> Path:
+    """The extension module of the Python binding's hot calls (qwen35x_b200/_lib/q35b_torch.so)."""
+    src = CSRC / "host" / "q35b_torch.cpp"
+    if force or _stale(BINDING, [src, PKG.parent / "include" / "q35b_nvfp4.h"]):
+        import torch
+
+        root = Path(torch.__file__).resolve().parent
+        cuda = Path(_nvcc()).resolve().parent.parent
+        cmd = ["g++", "-std=c++17", "-O2", "-fPIC", "-shared", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+               f"-I{root / 'include'}", f"-I{root / 'include' / 'torch' / 'csrc' / 'api' / 'include'}", f"-I{cuda / 'include'}",
+               f"-I{sysconfig.get_paths()['include']}", str(src), "-o", str(BINDING), f"-L{LIB_DIR}", "-lq35b", f"-L{root / 'lib'}",
+               "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python", "-Wl,-rpath,$ORIGIN"]
+        subprocess.run(cmd, check=True)
+    return BINDING
 
 
 def build_cli(force: bool = False) -> Path:

@@ -6,12 +6,14 @@ CUDA device is present, calls raise."""
 from __future__ import annotations
 
 import ctypes as C
+import importlib.util
 from pathlib import Path
 
 import numpy as np
 
 _PKG = Path(__file__).resolve().parent
 _LIB_PATH = _PKG / "_lib" / "libq35b.so"
+_NATIVE_PATH = _PKG / "_lib" / "q35b_torch.so"
 _lib = None
 
 GEMV_AUTO, GEMV_SIMT, GEMV_STREAM = -1, 10, 11
@@ -174,6 +176,26 @@ def _torch():
     return _torch_module
 
 
+_native_module = None
+
+
+def _native():
+    """The extension module of the hot calls (csrc/host/q35b_torch.cpp).  Its functions answer NotImplemented for a call
+    that is not in their plain form; the caller then goes the general way below."""
+    global _native_module
+    if _native_module is None:
+        _torch()
+        lib()
+        if not _NATIVE_PATH.is_file():
+            raise FileNotFoundError(f"{_NATIVE_PATH} is missing: run `python -m qwen35x_b200.build` (needs nvcc and torch)")
+        spec = importlib.util.spec_from_file_location("q35b_torch", _NATIVE_PATH)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        module.setup(Q35bError, _workspaces)
+        _native_module = module
+    return _native_module
+
+
 def _stream_ptr(torch) -> int:
     # the raw handle: torch.cuda.current_stream() builds a Stream object first, 3.3 us of the 12 a decode projection took;
     # the names are private, so it is what a torch without them gets
@@ -191,6 +213,7 @@ class Nvfp4Weight:
 
     def __init__(self, handle: int, n: int, k: int, s2: float, input_scale: float):
         self._h = C.c_void_p(handle)
+        self._ptr = handle
         self.n_total, self.k, self.s2, self.input_scale = n, k, s2, input_scale
         L = lib()
         self.row_begin = L.q35b_weight_row_begin(self._h)
@@ -255,6 +278,7 @@ class Nvfp4Weight:
 
     def close(self) -> None:
         if self._h is not None and self._h.value:
+            self._ptr = 0
             lib().q35b_weight_destroy(self._h)
             self._h = None
 
@@ -267,6 +291,9 @@ class Nvfp4Weight:
 
 def gemv_w4a16(weight: Nvfp4Weight, x, out=None, kernel: int = GEMV_AUTO):
     """Decode projection: x [m, K] bf16 (m = 1..8) -> y [m, rows] bf16."""
+    y = (_native_module or _native()).gemv(weight._ptr, x, out, kernel)
+    if y is not NotImplemented:
+        return y
     torch = _torch()
     if x.dim() == 1:
         x = x.unsqueeze(0)
@@ -280,6 +307,10 @@ def gemv_w4a16(weight: Nvfp4Weight, x, out=None, kernel: int = GEMV_AUTO):
 
 def gemv_w4a16_f32(weight: Nvfp4Weight, x, input_scale: float = 1.0, out=None, kernel: int = GEMV_AUTO):
     """The reference benchmark's contract: fp32 x [K], fp32 y [rows], x scaled by input_scale."""
+    if out is None:
+        y = (_native_module or _native()).gemv_f32(weight._ptr, x, input_scale, kernel)
+        if y is not NotImplemented:
+            return y
     torch = _torch()
     assert x.is_cuda and x.dtype == torch.float32 and x.is_contiguous() and x.numel() == weight.k
     if out is None:
@@ -326,11 +357,14 @@ class GemvBatch:
         else:
             _check(lib().q35b_gemv_batch_create(arr, len(self._keep), m, C.byref(h)))
         self._h = h
+        self._ptr = h.value
         self.digits = digits
         self.m = m
         self.stream_bytes = int(lib().q35b_gemv_batch_stream_bytes(h))
 
     def run(self) -> None:
+        if (_native_module or _native()).batch_run(self._ptr) is None:
+            return
         _check(lib().q35b_gemv_batch_run(self._h, _stream_ptr(_torch())))
 
     def status(self) -> int:
@@ -344,6 +378,7 @@ class GemvBatch:
 
     def close(self) -> None:
         if self._h is not None and self._h.value:
+            self._ptr = 0
             lib().q35b_gemv_batch_destroy(self._h)
             self._h = None
 
@@ -396,7 +431,8 @@ def quantize_activations(x, global_scale: float = 0.0, scratch=None):
     assert x.is_cuda and x.dim() == 2
     m, k = x.shape
     codes, scales, g = scratch if scratch is not None else act_scratch(m, k, x.device)
-    _quantize(torch, x, global_scale, codes, scales, g, _stream_ptr(torch))
+    if (_native_module or _native()).quantize(x, codes, scales, g, global_scale) is NotImplemented:
+        _quantize(torch, x, global_scale, codes, scales, g, _stream_ptr(torch))
     return codes.view(m, k // 2), scales, g
 
 
@@ -474,6 +510,10 @@ def _gemm(torch, weight, a_codes, a_scales_tiled, g, m, out, status, residual, s
 def gemm_w4a4(weight: Nvfp4Weight, a_codes, a_scales_tiled, g, m: int, out=None, status=None, residual=None):
     """Prefill projection on quantised activations: -> c [m, rows] bf16; with `residual` [m, rows] bf16 the sum is
     rounded once; a gate/up weight gives silu(gate) * up, [m, rows/2]."""
+    if status is None:
+        c = (_native_module or _native()).gemm(weight._ptr, a_codes, a_scales_tiled, g, m, out, residual)
+        if c is not NotImplemented:
+            return c
     torch = _torch()
     return _gemm(torch, weight, a_codes, a_scales_tiled, g, m, out, status, residual, _stream_ptr(torch))
 
@@ -603,6 +643,9 @@ def project_prefill(weight: Nvfp4Weight, x, out=None, scratch=None, global_scale
     assert x.is_cuda and x.dim() == 2
     m, k = x.shape
     codes, scales, g = scratch if scratch is not None else act_scratch(m, k, x.device)
+    c = (_native_module or _native()).project_prefill(weight._ptr, x, out, codes, scales, g, global_scale, residual)
+    if c is not NotImplemented:
+        return c
     stream = _stream_ptr(torch)
     _quantize(torch, x, global_scale, codes, scales, g, stream)
     return _gemm(torch, weight, codes, scales, g, m, out, None, residual, stream)

@@ -1,0 +1,71 @@
+"""The binding's native calls take the plain form of a call only; every other form goes the general way with the results and
+errors it always had.  Both ways on the same inputs have to give the same bits."""
+import numpy as np
+import pytest
+
+from helpers import make_activations, make_weight, to_torch_bf16
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def weight(engine):
+    _, codes, scales, s2 = make_weight(384, 512, seed=3)
+    return engine.Nvfp4Weight.from_host(codes, scales, s2)
+
+
+def _general(engine, monkeypatch, call):
+    """The call with every native function declining."""
+    class Declines:
+        def __getattr__(self, name):
+            return lambda *a: NotImplemented
+
+    with monkeypatch.context() as mp:
+        mp.setattr(engine.engine if hasattr(engine, "engine") else engine, "_native_module", Declines())
+        return call()
+
+
+@pytest.mark.parametrize("m", [1, 8])
+def test_same_bits_either_way(engine, weight, monkeypatch, m):
+    import torch
+
+    x = to_torch_bf16(make_activations(m, 512, seed=m))
+    res = torch.randn((m, 384), device="cuda").to(torch.bfloat16)
+    scratch = engine.act_scratch(m, 512, x.device)
+    calls = [lambda: engine.gemv_w4a16(weight, x), lambda: engine.gemv_w4a16(weight, x, kernel=engine.GEMV_SIMT),
+             lambda: engine.gemv_w4a16_f32(weight, x[0].float(), 0.5), lambda: engine.project_prefill(weight, x),
+             lambda: engine.project_prefill(weight, x, scratch=scratch, global_scale=0.01, residual=res),
+             lambda: engine.project_prefill(weight, x.float(), scratch=scratch),
+             lambda: engine.gemm_w4a4(weight, *engine.quantize_activations(x), m)]
+    for call in calls:
+        a, b = call().clone(), _general(engine, monkeypatch, call)
+        assert a.dtype == b.dtype and a.shape == b.shape and torch.equal(a, b)
+
+
+def test_other_forms(engine, weight):
+    import torch
+
+    x = to_torch_bf16(make_activations(2, 512, seed=9))
+    want = engine.gemv_w4a16(weight, x)
+    assert torch.equal(engine.gemv_w4a16(weight, x[0]), want[:1])          # a vector: one row comes back
+    out = torch.zeros(2 * 384, dtype=torch.bfloat16, device="cuda")
+    assert engine.gemv_w4a16(weight, x, out=out) is out and torch.equal(out.view(2, 384), want)
+    assert torch.equal(engine.gemv_w4a16(weight, torch.nn.Parameter(x, requires_grad=False)), want)
+    wide = torch.zeros((2, 400), dtype=torch.bfloat16, device="cuda")
+    got = engine.project_prefill(weight, x, out=wide[:, :384])
+    assert got.data_ptr() == wide.data_ptr() and torch.equal(wide[:, :384], engine.project_prefill(weight, x))
+    for bad in (x.float(), x[:, :256], x.t()):
+        with pytest.raises(AssertionError):
+            engine.gemv_w4a16(weight, bad)
+    with pytest.raises(engine.Q35bError):
+        engine.gemv_w4a16(weight, x.repeat(5, 1))                            # ten tokens
+    with pytest.raises(RuntimeError):
+        engine.quantize_activations(x, scratch=engine.act_scratch(4, 512, x.device))
+    with torch.cuda.stream(torch.cuda.Stream()):
+        other = engine.gemv_w4a16(weight, x)
+        torch.cuda.current_stream().synchronize()
+    assert torch.equal(other, want)
+    w2 = engine.Nvfp4Weight.from_host(np.zeros((128, 128), dtype=np.uint8), np.zeros((128, 16), dtype=np.uint8), 1.0)
+    w2.close()
+    with pytest.raises(Exception):
+        engine.gemv_w4a16(w2, x[:, :256].contiguous())
