@@ -152,11 +152,13 @@ int launch_gemm_w4a4(const q35b_weight * w, const uint8_t * a_codes, const uint8
 
 // gemm_wstream.cu: decode work lists on the tensor cores
 struct WBatch;  // decode work list on the tensor path (digit-expanded activations)
-int wbatch_build(const q35b_gemv_item * items, int count, int m, int digits, WBatch ** out);
+// propagate: infinities and NaNs of the activations reach the outputs (else they count as zero)
+int wbatch_build(const q35b_gemv_item * items, int count, int m, int digits, bool propagate, WBatch ** out);
 int wbatch_launch(const WBatch * b, cudaStream_t s);
 void wbatch_free(WBatch * b);
 int wbatch_status(const WBatch * b, unsigned int * out);
 size_t wbatch_bytes(const WBatch * b);
+int wbatch_debug_wait(WBatch * b, unsigned int wait_limit);
 
 // gemm_w4a4_2cta.cu
 bool gemm_2cta_eligible(int rows, int m, int k);

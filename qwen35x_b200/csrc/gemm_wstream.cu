@@ -15,15 +15,15 @@
 // a tile runs under the MMAs of the next, and four epilogue warps that turn accumulator lanes into BF16 outputs
 // y[token, row].
 //
-// Decode (W4A16, 1..8 tokens): every token is expanded into `digits` operand rows, an NVFP4 digit expansion of
-// its BF16 activations (expand_digits_kernel below): digit j quantises what digits 0..j-1 left over, so the sum
-// of the rows reproduces the activation to 6^-digits of its block's amax (digits = 5: 1.3e-4, far below BF16's
-// own 2^-9), and the epilogue adds the digits' accumulator columns.  Replaces nvfp4_row_dot / matvec_nvfp4_bf16
-// (src/kernels/cuda/decode_layers.cuh:200-284) with the FP4 decode done by the tensor core instead of by
-// conversion instructions.
+// Decode (W4A16, 1..8 tokens): every token enters as `digits` operand rows, the octal digits of its BF16 activations
+// (split_digits_kernel below).  Eight digits leave 2^-23 of a block's largest value, which is all that fp32 sums keep, and
+// the epilogue adds the digits' accumulator columns.  Replaces nvfp4_row_dot / matvec_nvfp4_bf16
+// (src/kernels/cuda/decode_layers.cuh:200-284) with the FP4 decode done by the tensor core instead of by conversion
+// instructions: a fifth of gemv_stream.cu's instructions, so a long run of steps does not meet the power cap.
 //
 // Every wait is bounded; an expired wait records a code in *status and the role stops; the CTA still frees TMEM.
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 
 #include <algorithm>
 #include <vector>
@@ -42,10 +42,11 @@ constexpr int kABytes = kRows * kStepBytes;          // 16 KB
 constexpr int kSfBytes = kMmaPerStage * kSfChunk;    // 2 KB (weights, and activations: at most 128 operand rows)
 constexpr int kMaxCols = 128;
 constexpr int kMaxStages = 8;
-constexpr int kThreads = 7 * 32;         // warp 0 weight producer, 1 MMA, 2 activation producer, 3..6 epilogue
-constexpr int kTmemCols = 512;           // two accumulator buffers of up to 240 columns + 16 + 16 scale-factor columns
+constexpr int kEpilogueWarps = 8;        // two per quarter of the TMEM lanes, each taking every other token
+constexpr int kThreads = (3 + kEpilogueWarps) * 32;  // warp 0 weight producer, 1 MMA, 2 activation producer
+constexpr int kTmemCols = 512;           // two accumulator buffers ...
 constexpr int kAccBufCols = 224;
-constexpr int kSfaCol = 2 * kAccBufCols;   // two sets of scale-factor columns (A 16 + B 16 each), used by stages in turn,
+constexpr int kSfaCol = 2 * kAccBufCols;   // ... and two sets of scale-factor columns (A 16 + B 16 each), used by stages in turn,
 constexpr int kSfbCol = kSfaCol + 16;      // so that the copies of one stage do not wait for the MMAs of the one before
 constexpr int kSfSetCols = 32;
 constexpr uint32_t kWaitLimit = 1u << 22;
@@ -57,10 +58,12 @@ enum Epilogue : int { kEpiPlain = 0, kEpiGateUp = 1 };
 // One projection of the list, in device memory; the tensor maps are read by the TMA unit from there.
 struct alignas(128) WItem {
   CUtensorMap tmap_w;            // weight codes [rows, K/2], box 128 rows x 128 bytes, 128B swizzle
-  CUtensorMap tmap_x;            // operand codes [operand rows, K/2], box n_cols rows x 128 bytes, 128B swizzle
   const uint8_t * w_scales;      // weight scale tiles
-  const uint8_t * x_scales;      // operand scale tiles (one 128-row block)
-  const float * x_g;             // the operand's scale, one per token
+  const uint8_t * x_ops;         // the operand, one run of bytes per K step: codes as they lie in shared memory (n_cols rows of
+                                 // 128 bytes, 128B swizzle), then four scale tiles
+  const float * x_g;             // the operand's scale, one per token (NaN: the token has infinities or NaNs, see exact_dot)
+  const uint8_t * w_codes;       // for such tokens: weight codes and the activations themselves
+  const __nv_bfloat16 * x;
   __nv_bfloat16 * y;             // [tokens, ldy]
   const __nv_bfloat16 * residual;  // NULL or [tokens, ldr]
   int rows;                      // weight rows
@@ -82,10 +85,10 @@ struct alignas(8) WTile {
 // pointers through global memory at a tile boundary (a 128-row x 1024-column tile lasts under two microseconds).
 struct alignas(16) STile {
   const CUtensorMap * tmap_w;
-  const CUtensorMap * tmap_x;
   const uint8_t * w_scales;      // scale tiles of this row block
-  const uint8_t * x_scales;
+  const uint8_t * x_ops;
   const float * x_g;
+  const WItem * item;
   __nv_bfloat16 * y;
   const __nv_bfloat16 * residual;
   int row_block, rows, k_steps, n_cols, tokens, digits, ldy, ldr, epilogue;
@@ -103,8 +106,8 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-  for (uint32_t i = 0; i < kWaitLimit; ++i) {
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t limit) {
+  for (uint32_t i = 0; i < limit; ++i) {
     uint32_t ok;
     asm volatile(
       "{\n\t.reg .pred p;\n\t"
@@ -116,6 +119,15 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
     if (ok) return true;
   }
   return false;
+}
+__device__ __forceinline__ bool elect_one() {
+  uint32_t pred;
+  asm volatile(
+    "{\n\t.reg .pred p;\n\t"
+    "elect.sync _|p, 0xffffffff;\n\t"
+    "selp.u32 %0, 1, 0, p;\n\t}"
+    : "=r"(pred));
+  return pred != 0;
 }
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap * map, uint32_t bar, int x, int y) {
   asm volatile(
@@ -176,29 +188,51 @@ __device__ __forceinline__ void utccp_sf(uint32_t tmem_dst, uint64_t sdesc) {
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-    "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-    "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-    : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-      "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-    : "r"(taddr)
-    : "memory");
+// Waits for the loads before it.  The registers are operands, or the compiler might use them before the wait.
+__device__ __forceinline__ void tmem_wait_ld(uint32_t (&r)[4][8]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0][0]), "+r"(r[0][1]), "+r"(r[0][2]), "+r"(r[0][3]), "+r"(r[0][4]), "+r"(r[0][5]), "+r"(r[0][6]), "+r"(r[0][7]),
+                 "+r"(r[1][0]), "+r"(r[1][1]), "+r"(r[1][2]), "+r"(r[1][3]), "+r"(r[1][4]), "+r"(r[1][5]), "+r"(r[1][6]), "+r"(r[1][7]),
+                 "+r"(r[2][0]), "+r"(r[2][1]), "+r"(r[2][2]), "+r"(r[2][3]), "+r"(r[2][4]), "+r"(r[2][5]), "+r"(r[2][6]), "+r"(r[2][7]),
+                 "+r"(r[3][0]), "+r"(r[3][1]), "+r"(r[3][2]), "+r"(r[3][3]), "+r"(r[3][4]), "+r"(r[3][5]), "+r"(r[3][6]), "+r"(r[3][7])
+               :
+               : "memory");
+}
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
 }
 
-__device__ __forceinline__ float silu_mul(float g, float u) { return __fdividef(g, 1.0f + __expf(-g)) * u; }
+// One output of a token with infinities or NaNs, as fp32 arithmetic over the activations themselves gives it.
+__device__ __noinline__ float exact_dot(const WItem * it, int row, int token) {
+  const int k = it->k_steps * 256, row_block = row >> 7;
+  const uint8_t * codes = it->w_codes + static_cast<size_t>(row) * (k >> 1);
+  const __nv_bfloat16 * x = it->x + static_cast<size_t>(token) * k;
+  float sum = 0.0f;
+  for (int blk = 0; blk < k >> 4; ++blk) {
+    float dot = 0.0f;
+    for (int i = 0; i < 16; ++i) {
+      const uint32_t code = codes[blk * 8 + (i >> 1)] >> (4 * (i & 1));
+      dot = fmaf(decode_e2m1(static_cast<uint8_t>(code & 15u)), __bfloat162float(x[blk * 16 + i]), dot);
+    }
+    sum = fmaf(dot, decode_e4m3(it->w_scales[tiled_scale_offset(row_block * kRows + (row & 127), blk, k >> 4)]), sum);
+  }
+  return sum;
+}
+
 
 // CTA b walks tiles[cta_begin[b] .. cta_begin[b + 1]).
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__ tiles, const int * __restrict__ cta_begin,
-                    int stages, int b_slot_bytes, unsigned int * status) {
+                    int stages, int b_slot_bytes, unsigned int * status, uint32_t wait_limit) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t * smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint8_t * smem_a = smem;
   uint8_t * smem_b = smem_a + stages * kABytes;
-  uint8_t * smem_sfa = smem_b + stages * b_slot_bytes;
-  uint8_t * smem_sfb = smem_sfa + stages * kSfBytes;
-  uint64_t * bars = reinterpret_cast<uint64_t *>(smem_sfb + stages * kSfBytes);
+  uint8_t * smem_sfa = smem_b + stages * b_slot_bytes;     // a slot of smem_b holds a step's operand codes and scale tiles
+  uint64_t * bars = reinterpret_cast<uint64_t *>(smem_sfa + stages * kSfBytes);
   uint64_t * full = bars;                           // [stages]: both producers' bytes have landed
   uint64_t * empty = bars + kMaxStages;             // [stages]: the MMAs that read the stage have retired
   uint64_t * tmem_full = bars + 2 * kMaxStages;     // [2]: accumulator complete
@@ -213,11 +247,11 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
     const WTile t = tiles[tile_begin + ti];
     const int rb = t.row_block;
     const WItem * it = items + t.item;
+    d.item = it;
     d.tmap_w = &it->tmap_w;
-    d.tmap_x = &it->tmap_x;
     d.k_steps = it->k_steps;
     d.w_scales = it->w_scales + static_cast<size_t>(rb) * d.k_steps * kSfBytes;
-    d.x_scales = it->x_scales;
+    d.x_ops = it->x_ops;
     d.x_g = it->x_g;
     d.y = it->y;
     d.residual = it->residual;
@@ -233,7 +267,12 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
     d.s2_up = it->s2_up;
   };
   // tile descriptors are constant for the life of a work list (and of a launch): read them before anything else
-  for (int ti = threadIdx.x; ti < min(n_tiles, kMaxTilesInSmem); ti += kThreads) describe(ti, stile[ti]);
+  for (int ti = threadIdx.x; ti < min(n_tiles, kMaxTilesInSmem); ti += kThreads) {
+    describe(ti, stile[ti]);
+    if (ti == 0 || tiles[tile_begin + ti - 1].item != tiles[tile_begin + ti].item) {
+      asm volatile("prefetch.tensormap [%0];" ::"l"(stile[ti].tmap_w) : "memory");
+    }
+  }
   // tiles beyond the staged ones (a CTA with a very long list) are described on the fly
   auto tile_at = [&](int ti, STile & spill) -> const STile * {
     if (ti < kMaxTilesInSmem) return stile + ti;
@@ -248,7 +287,7 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(tmem_full + i), 1);
-      mbar_init(smem_u32(tmem_empty + i), 4);
+      mbar_init(smem_u32(tmem_empty + i), kEpilogueWarps);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -268,7 +307,7 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
 
   if (warp == 0) {
     // ------------------------------------------------------------ weight producer (constant data: no wait)
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -278,7 +317,7 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
         const int k_steps = it->k_steps, rb = it->row_block;
         const uint8_t * sf = it->w_scales;
         for (int ks = 0; ks < k_steps; ++ks) {
-          if (!mbar_wait(smem_u32(empty + stage), phase ^ 1)) {
+          if (!mbar_wait(smem_u32(empty + stage), phase ^ 1, wait_limit)) {
             atomicExch(status, kWeightWait);
             ok = false;
             break;
@@ -296,7 +335,7 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
     }
   } else if (warp == 2) {
     // ------------------------------------------------------------ activation producer
-    if (lane == 0) {
+    if (elect_one()) {
       asm volatile("griddepcontrol.wait;" ::: "memory");
       int stage = 0;
       uint32_t phase = 0;
@@ -305,17 +344,16 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
       for (int ti = 0; ti < n_tiles && ok; ++ti) {
         const STile * it = tile_at(ti, spill);
         const int k_steps = it->k_steps;
-        const uint32_t b_bytes = static_cast<uint32_t>(it->n_cols) * kStepBytes;
+        const uint8_t * ops = it->x_ops;
         for (int ks = 0; ks < k_steps; ++ks) {
-          if (!mbar_wait(smem_u32(empty + stage), phase ^ 1)) {
+          if (!mbar_wait(smem_u32(empty + stage), phase ^ 1, wait_limit)) {
             atomicExch(status, kActWait);
             ok = false;
             break;
           }
           const uint32_t bar = smem_u32(full + stage);
-          mbar_expect_tx(bar, b_bytes + kSfBytes);
-          tma_load_2d(smem_u32(smem_b + stage * b_slot_bytes), it->tmap_x, bar, ks * kStepBytes, 0);
-          bulk_load(smem_u32(smem_sfb + stage * kSfBytes), it->x_scales + static_cast<size_t>(ks) * kSfBytes, kSfBytes, bar);
+          mbar_expect_tx(bar, static_cast<uint32_t>(b_slot_bytes));
+          bulk_load(smem_u32(smem_b + stage * b_slot_bytes), ops + static_cast<size_t>(ks) * b_slot_bytes, static_cast<uint32_t>(b_slot_bytes), bar);
           if (++stage == stages) {
             stage = 0;
             phase ^= 1;
@@ -325,11 +363,10 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    // Per stage: eight scale-factor copies into one of two TMEM column sets, then four MMAs.  With operand tiles this
-    // narrow the MMAs are far shorter than the copy-to-MMA turnaround of the tensor pipe (about 500 cycles per stage,
-    // measured by switching copies and MMAs off in turn: 49 us per 0.8B-class step without either, 52 with copies
-    // only, 51 with MMAs only, 73 with both); issuing the copies a stage ahead of their MMAs did not hide it (83 us).
-    if (lane == 0) {
+    // Per stage: eight scale-factor copies into one of two TMEM column sets, then four MMAs; a stage's turn takes about 500
+    // cycles, its bytes 800 to come from HBM.  The issuing threads are chosen with elect.sync: by a test of the lane number
+    // the same code took 600 ns per stage (0.8B-class step of one token 73 us instead of 44).
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0, sf_turn = 0;
       bool ok = true;
@@ -339,7 +376,7 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
         const int k_steps = it->k_steps;
         const uint32_t idesc = instr_desc(it->n_cols);
         const uint32_t ab = ti & 1;
-        if (!mbar_wait(smem_u32(tmem_empty + ab), ((ti >> 1) & 1) ^ 1)) {
+        if (!mbar_wait(smem_u32(tmem_empty + ab), ((ti >> 1) & 1) ^ 1, wait_limit)) {
           atomicExch(status, kMmaDrainWait);
           break;
         }
@@ -347,7 +384,7 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
         const uint32_t acc = tmem_base + ab * kAccBufCols;
         const int n_cols = it->n_cols, parts = partial_accumulators(n_cols);
         for (int ks = 0; ks < k_steps; ++ks) {
-          if (!mbar_wait(smem_u32(full + stage), phase)) {
+          if (!mbar_wait(smem_u32(full + stage), phase, wait_limit)) {
             atomicExch(status, kMmaWait);
             ok = false;
             break;
@@ -356,7 +393,7 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
           const uint64_t a_desc = desc_k_sw128(smem_u32(smem_a + stage * kABytes));
           const uint64_t b_desc = desc_k_sw128(smem_u32(smem_b + stage * b_slot_bytes));
           const uint64_t sfa_desc = desc_sf(smem_u32(smem_sfa + stage * kSfBytes));
-          const uint64_t sfb_desc = desc_sf(smem_u32(smem_sfb + stage * kSfBytes));
+          const uint64_t sfb_desc = desc_sf(smem_u32(smem_b + (stage + 1) * b_slot_bytes - kSfBytes));
           const uint32_t sf_set = tmem_base + (sf_turn ^= 1u) * kSfSetCols;
 #pragma unroll
           for (int j = 0; j < kMmaPerStage; ++j) {
@@ -380,74 +417,72 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
   } else {
     // ------------------------------------------------------------ epilogue: lane = weight row, column = operand row
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int quarter = warp & 3;
+    const int quarter = warp & 3, first_token = (warp - 3) >> 2;
     const int row_in_tile = quarter * 32 + lane;
     STile spill;
     for (int ti = 0; ti < n_tiles; ++ti) {
       const STile * it = tile_at(ti, spill);
-      const int rb = it->row_block;
       const uint32_t ab = ti & 1;
-      if (!mbar_wait(smem_u32(tmem_full + ab), (ti >> 1) & 1)) {
+      if (!mbar_wait(smem_u32(tmem_full + ab), (ti >> 1) & 1, wait_limit)) {
         if (lane == 0) atomicExch(status, kEpilogueWait);
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const int rows = it->rows, tokens = it->tokens, digits = it->digits, n_cols = it->n_cols;
-      const int row = rb * kRows + row_in_tile;
-      const float * x_g = it->x_g;
+      const int row = it->row_block * kRows + row_in_tile;
       const bool gate_up = it->epilogue == kEpiGateUp;
       const float s2 = it->s2, s2_up = it->s2_up;
-      __nv_bfloat16 * y = it->y;
-      const __nv_bfloat16 * residual = it->residual;
-      const int ldy = it->ldy, ldr = it->ldr;
       const uint32_t taddr = tmem_base + ab * kAccBufCols + (static_cast<uint32_t>(quarter * 32) << 16);
       const int parts = partial_accumulators(n_cols);
-      float sum = 0.0f;
-      int jc = 0, token = 0;
-      for (int c0 = 0; c0 < n_cols; c0 += 16) {
-        uint32_t r[16];
-        tmem_ld16(taddr + c0, r);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        for (int p = 1; p < parts; ++p) {
-          uint32_t r2[16];
-          tmem_ld16(taddr + p * n_cols + c0, r2);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-          for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) + __uint_as_float(r2[i]));
+      // One token at a time, in a compact loop: a small part of a tile's time as long as its code stays resident (with all
+      // columns unrolled a 0.8B-class step of eight tokens took 99 us instead of 54).
+#pragma unroll 1
+      for (int token = first_token; token < tokens; token += 2) {
+        uint32_t r[4][8] = {};
+        tmem_ld8(taddr + token * digits, r[0]);  // digits <= 8: what lies behind them is not used
+        if (parts > 1) tmem_ld8(taddr + n_cols + token * digits, r[1]);
+        if (parts > 2) {
+          tmem_ld8(taddr + 2 * n_cols + token * digits, r[2]);
+          tmem_ld8(taddr + 3 * n_cols + token * digits, r[3]);
         }
-        if (c0 + 16 >= n_cols) {
-          // the accumulator is in registers: hand it back before the stores
-          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-          __syncwarp();
-          if (lane == 0) mbar_arrive(smem_u32(tmem_empty + ab));
-        }
+        float g = __ldg(it->x_g + token);
+        tmem_wait_ld(r);
+        float sum = 0.0f, weight = 1.0f;  // of digit j: 8^-j
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          sum += __uint_as_float(r[i]);
-          if (++jc == digits) {
-            // one output value per (token, weight row); all lanes take the same path
-            const float gval = token < tokens ? __ldg(x_g + token) : 0.0f;
-            const float alpha = gval * s2, alpha_up = gval * s2_up;
-            if (gate_up) {
-              // rows alternate 8 gate / 8 up: lane l holds gate row j, lane l ^ 8 the matching up row
-              const float other = __shfl_xor_sync(0xffffffffu, sum, 8);
-              if ((row & 8) == 0 && token < tokens && row + 8 < rows) {
-                const int j = (row >> 4) * 8 + (row & 7);
-                y[static_cast<size_t>(token) * ldy + j] = __float2bfloat16_rn(silu_mul(sum * alpha, other * alpha_up));
-              }
-            } else if (token < tokens && row < rows) {
-              const float rv = residual != nullptr ? __bfloat162float(residual[static_cast<size_t>(token) * ldr + row]) : 0.0f;
-              y[static_cast<size_t>(token) * ldy + row] = __float2bfloat16_rn(fmaf(sum, alpha, rv));
-            }
-            sum = 0.0f;
-            jc = 0;
-            ++token;
+        for (int j = 0; j < 8; ++j) {
+          if (j < digits) {
+            sum = fmaf((__uint_as_float(r[0][j]) + __uint_as_float(r[1][j])) + (__uint_as_float(r[2][j]) + __uint_as_float(r[3][j])), weight, sum);
+            weight *= 0.125f;
           }
         }
+        if (g != g) {
+          sum = row < rows ? exact_dot(it->item, row, token) : 0.0f;
+          g = 1.0f;
+        }
+        // g is a power of two, possibly a subnormal one: it comes last, so that nothing underflows before the result does
+        if (gate_up) {
+          // rows alternate 8 gate / 8 up: lane l holds gate row j, lane l ^ 8 the matching up row
+          const float other = __shfl_xor_sync(0xffffffffu, sum, 8);
+          if ((row & 8) == 0 && row + 8 < rows) {
+            const int j = (row >> 4) * 8 + (row & 7);
+            const float gate = sum * s2 * g, up = other * s2_up * g;
+            it->y[static_cast<size_t>(token) * it->ldy + j] = __float2bfloat16_rn(gate / (1.0f + expf(-gate)) * up);
+          }
+        } else if (row < rows) {
+          const float rv = it->residual != nullptr ? __bfloat162float(it->residual[static_cast<size_t>(token) * it->ldr + row]) : 0.0f;
+          it->y[static_cast<size_t>(token) * it->ldy + row] = __float2bfloat16_rn(fmaf(sum * s2, g, rv));
+        }
       }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(tmem_empty + ab));
     }
   }
 
+  // after an expired wait some of this CTA's copies may still be under way: give them 100 us before its memory is let go
+  if (threadIdx.x == 0 && *reinterpret_cast<volatile unsigned int *>(status) != 0u) {
+    for (int i = 0; i < 1000; ++i) __nanosleep(100);
+  }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 1) {
@@ -457,9 +492,10 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
   }
 }
 
-// ---- decode: BF16 activations -> NVFP4 digit expansion ---------------------------------------------------------
+// ---- decode: BF16 activations -> octal digits in NVFP4 ----------------------------------------------------------
 
-__device__ __forceinline__ uint32_t cvt_e2m1x8_w(const float (&q)[8]) {
+// Eight fp32 values -> one word of eight E2M1 codes, nearest; element 2j in the low nibble of byte j.
+__device__ __forceinline__ uint32_t to_e2m1x8(const float (&q)[8]) {
   uint32_t w;
   asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\t"
       "cvt.rn.satfinite.e2m1x2.f32 b0, %2, %1;\n\t"
@@ -471,106 +507,117 @@ __device__ __forceinline__ uint32_t cvt_e2m1x8_w(const float (&q)[8]) {
       : "f"(q[0]), "f"(q[1]), "f"(q[2]), "f"(q[3]), "f"(q[4]), "f"(q[5]), "f"(q[6]), "f"(q[7]));
   return w;
 }
+// The two E2M1 codes of a byte (low nibble first) -> fp32.
+__device__ __forceinline__ void from_e2m1x2(uint32_t byte, float & lo, float & hi) {
+  asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\t.reg .b32 h;\n\t.reg .b16 l, u;\n\t"
+      "mov.b32 {b0, b1, b2, b3}, %2;\n\t"
+      "cvt.rn.f16x2.e2m1x2 h, b0;\n\t"
+      "mov.b32 {l, u}, h;\n\t"
+      "cvt.f32.f16 %0, l;\n\t"
+      "cvt.f32.f16 %1, u;\n\t}"
+      : "=f"(lo), "=f"(hi)
+      : "r"(byte));
+}
 
 struct ExpandItem {
-  const __nv_bfloat16 * x;   // [tokens, k]
-  uint8_t * codes;           // [tokens * digits, k / 2], operand row = token * digits + digit
-  uint8_t * scales;          // tiled scales of one 128-row block: 128 * roundup(k / 16, 4) bytes
+  const __nv_bfloat16 * x;   // [tokens, k], k a multiple of 256
+  uint8_t * ops;             // see WItem::x_ops; operand row = token * digits + digit
   float * g;                 // [tokens]: scale of each token's expansion
   int k;
+  int code_bytes;            // of a K step: n_cols * 128
 };
 
-// One CTA per (projection, token).  g = amax / (6 * 448) over the token's activations; per 16-element block, digit j
-// takes the block's current residual r_j (r_0 = x): scale byte sb_j = UE4M3(amax(r_j) / 6 / g), d_j = decode(sb_j) * g,
-// codes q_j = E2M1(r_j / d_j) (nearest), r_{j+1} = r_j - q_j * d_j.  |r_{j+1}| <= max(d_j, amax(r_j) / 16), so each
-// digit shrinks the residual by about six; digits whose scale would underflow E4M3 stay zero.  Every scale byte of a
-// real (row, block) is written by every run; the padding of the tiled layout was zeroed when the list was built.
-__global__ void __launch_bounds__(128) expand_digits_kernel(const ExpandItem * __restrict__ items, int digits) {
-  asm volatile("griddepcontrol.wait;" ::: "memory");  // the activations may come from the kernel before
+constexpr int kSplitThreads = 256;
+
+// One CTA per (projection, token).  A block of sixteen values whose largest has exponent e is counted in units of
+// 2^(e - 1), which makes every value less than 4: digit 0 is the nearest E2M1 number (up to 4 the grid is no coarser than
+// 1, so at most half a unit is left over), digit 1 the nearest to eight times the rest, and so on; all of it is exact in
+// fp32.  The unit goes into the block's scale byte, a power of two relative to the token's largest exponent (down to 2^-17
+// of it, the range of E4M3), and 8^-j into the epilogue.  Eight digits leave at most 2^-24 of the block's binade.
+// A token with an infinity or a NaN gets NaN for its scale if `propagate`, and the epilogue works its outputs out from the
+// activations; else such elements count as zero.
+__global__ void __launch_bounds__(kSplitThreads) split_digits_kernel(const ExpandItem * __restrict__ items, int digits, int propagate) {
+  // small CTAs that are soon all resident: the projection kernel may start streaming its weights
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const ExpandItem it = items[blockIdx.x];
-  const int token = blockIdx.y;
-  const int k = it.k, blocks_per_row = k >> 4, slots = ((blocks_per_row + 3) >> 2) << 2;
-  const __nv_bfloat16 * xt = it.x + static_cast<size_t>(token) * k;
-  __shared__ float red[4];
-  __shared__ float g_shared;
-  float amax = 0.0f;
-  for (int b = threadIdx.x; b < blocks_per_row * 2; b += blockDim.x) {
-    const uint4 q = __ldg(reinterpret_cast<const uint4 *>(xt) + b);
-    const uint32_t r[4] = {q.x, q.y, q.z, q.w};
+  const int token = blockIdx.y, k = it.k, chunks = k >> 3;
+  const uint4 * src = reinterpret_cast<const uint4 *>(it.x + static_cast<size_t>(token) * k);
+  __shared__ uint32_t red[kSplitThreads / 32];
+  auto load = [&](int c) {
+    uint4 q = __ldg(src + c);
+    if (!propagate) {
+      uint32_t * r = reinterpret_cast<uint32_t *>(&q);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float lo = fabsf(__uint_as_float(r[j] << 16)), hi = fabsf(__uint_as_float(r[j] & 0xffff0000u));
-      if (lo < 3.0e38f) amax = fmaxf(amax, lo);  // NaN and inf do not take part
-      if (hi < 3.0e38f) amax = fmaxf(amax, hi);
+      for (int i = 0; i < 4; ++i) {
+        if ((r[i] & 0x7f80u) == 0x7f80u) r[i] &= 0xffff0000u;
+        if ((r[i] & 0x7f800000u) == 0x7f800000u) r[i] &= 0xffffu;
+      }
     }
-  }
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
+    return q;
+  };
+  // largest of the magnitudes' bit patterns
+  auto abs_max = [](const uint4 & q) {
+    const uint32_t a = __vmaxu2(__vmaxu2(q.x & 0x7fff7fffu, q.y & 0x7fff7fffu), __vmaxu2(q.z & 0x7fff7fffu, q.w & 0x7fff7fffu));
+    return max(a & 0xffffu, a >> 16);
+  };
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // the activations may come from the kernel before
+  uint32_t best = 0;
+  for (int c = threadIdx.x; c < chunks; c += kSplitThreads) best = max(best, abs_max(load(c)));
+  best = __reduce_max_sync(0xffffffffu, best);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = best;
   __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kSplitThreads / 32; ++i) best = max(best, red[i]);
+  const int top = max(static_cast<int>(best >> 7), 1);  // exponent field of the token's largest value
   if (threadIdx.x == 0) {
-    const float m = fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3]));
-    const float g = m > 0.0f ? m / (6.0f * 448.0f) : 1.0f;
-    g_shared = g;
-    it.g[token] = g;
+    // 2^(top - 136): the unit of a block at the token's largest exponent is 2^(top - 128), and its scale byte stands for 2^8
+    const uint32_t bits = top > 9 ? static_cast<uint32_t>(top - 9) << 23 : 1u << (top + 13);
+    it.g[token] = best >= 0x7f80u ? __uint_as_float(0x7fffffffu) : __uint_as_float(bits);
   }
-  __syncthreads();
-  const float g = g_shared;
-  const float inv_g6 = 1.0f / (6.0f * g);
-  for (int blk = threadIdx.x; blk < blocks_per_row; blk += blockDim.x) {
-    float v[16];
-    {
-      const uint4 * src = reinterpret_cast<const uint4 *>(xt + blk * 16);
+  for (int c = threadIdx.x; c < chunks; c += kSplitThreads) {  // whole warps: chunks is a multiple of 32
+    const uint4 q = load(c);
+    uint32_t b = abs_max(q);
+    b = max(b, __shfl_xor_sync(0xffffffffu, b, 1));
+    const int e = max(max(static_cast<int>(b >> 7), top - 17), 1);
+    const float scale = __uint_as_float(static_cast<uint32_t>(255 - e) << 23);  // 2^(128 - e)
+    const uint32_t r[4] = {q.x, q.y, q.z, q.w};
+    float v[8];
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const uint4 q = __ldg(src + h);
-        const uint32_t r[4] = {q.x, q.y, q.z, q.w};
+    for (int i = 0; i < 4; ++i) {
+      v[2 * i] = __uint_as_float(r[i] << 16) * scale;
+      v[2 * i + 1] = __uint_as_float(r[i] & 0xffff0000u) * scale;
+    }
+    uint8_t * step = it.ops + static_cast<size_t>(c >> 5) * (it.code_bytes + kSfBytes);
+    int row = token * digits;
+    for (int j = 0; j < digits; ++j) {
+      const uint32_t w = to_e2m1x8(v);
+      *reinterpret_cast<uint32_t *>(step + row * kStepBytes + ((((c >> 2) ^ row) & 7) << 4) + ((c & 3) << 2)) = w;
+      ++row;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float lo = __uint_as_float(r[j] << 16), hi = __uint_as_float(r[j] & 0xffff0000u);
-          // NaN and inf have no digit expansion: they contribute zero (the exact decode kernel propagates them)
-          v[h * 8 + 2 * j] = fabsf(lo) < 3.0e38f ? lo : 0.0f;
-          v[h * 8 + 2 * j + 1] = fabsf(hi) < 3.0e38f ? hi : 0.0f;
-        }
+      for (int i = 0; i < 4; ++i) {
+        float d0, d1;
+        from_e2m1x2(w >> (8 * i), d0, d1);
+        v[2 * i] = (v[2 * i] - d0) * 8.0f;
+        v[2 * i + 1] = (v[2 * i + 1] - d1) * 8.0f;
       }
     }
-    for (int dgt = 0; dgt < digits; ++dgt) {
-      float bmax = 0.0f;
-#pragma unroll
-      for (int i = 0; i < 16; ++i) bmax = fmaxf(bmax, fabsf(v[i]));
-      uint32_t sb = encode_ue4m3(bmax * inv_g6);
-      sb = sb > 0x7eu ? 0x7eu : sb;
-      const int op_row = token * digits + dgt;
-      uint2 packed = make_uint2(0u, 0u);
-      if (sb != 0u) {
-        const float d = decode_e4m3(static_cast<uint8_t>(sb)) * g;
-        const float r = 1.0f / d;
-        float q0[8], q1[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          q0[i] = v[i] * r;
-          q1[i] = v[8 + i] * r;
-        }
-        packed.x = cvt_e2m1x8_w(q0);
-        packed.y = cvt_e2m1x8_w(q1);
-        const uint32_t w[2] = {packed.x, packed.y};
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const uint32_t c = (w[i >> 3] >> (4 * (i & 7))) & 0xfu;
-          v[i] = fmaf(-decode_e2m1(static_cast<uint8_t>(c)), d, v[i]);
-        }
-      }
-      *reinterpret_cast<uint2 *>(it.codes + (static_cast<size_t>(op_row) * k + blk * 16) / 2) = packed;
-      it.scales[tiled_scale_offset(op_row, blk, slots)] = static_cast<uint8_t>(sb);
-    }
+    // E4M3 byte of 2^(8 + e - top); the four blocks of eight lanes make one word of the tiled layout, the same for every digit
+    const int s = 8 + e - top;
+    const uint32_t byte = s >= -6 ? static_cast<uint32_t>(s + 7) << 3 : 8u >> (-6 - s);
+    uint32_t word = byte << (8 * ((threadIdx.x >> 1) & 3));
+    word |= __shfl_xor_sync(0xffffffffu, word, 2);
+    word |= __shfl_xor_sync(0xffffffffu, word, 4);
+    const int j = threadIdx.x & 7;
+    row = token * digits + j;
+    if (j < digits) *reinterpret_cast<uint32_t *>(step + it.code_bytes + ((c >> 3) & 3) * kSfChunk + (row & 31) * 16 + (row >> 5) * 4) = word;
   }
 }
 
 int plan_stages(int b_slot_bytes) {
-  const int stage = kABytes + b_slot_bytes + 2 * kSfBytes;
+  const int stage = kABytes + kSfBytes + b_slot_bytes;
   return std::max(2, std::min(kMaxStages, (kSmemBudget - 1024 - 256) / stage));
 }
-int smem_for(int stages, int b_slot_bytes) { return stages * (kABytes + b_slot_bytes + 2 * kSfBytes) + 1024 + 256; }
+int smem_for(int stages, int b_slot_bytes) { return stages * (kABytes + kSfBytes + b_slot_bytes) + 1024 + 256; }
 
 int ensure_attr() {
   static std::atomic<bool> attr_set[64];
@@ -597,9 +644,11 @@ struct WBatch {
   ExpandItem * expand = nullptr;
   unsigned int * status = nullptr;
   size_t bytes_per_run = 0;
+  bool propagate = false;   // infinities and NaNs of the activations reach the outputs
+  uint32_t wait_limit = kWaitLimit;
 };
 
-int wbatch_build(const q35b_gemv_item * items, int count, int m, int digits, WBatch ** out) {
+int wbatch_build(const q35b_gemv_item * items, int count, int m, int digits, bool propagate, WBatch ** out) {
   if (items == nullptr || out == nullptr || count <= 0) return fail(Q35B_ERR_ARGUMENT, "Invalid NVFP4 projection work list.");
   *out = nullptr;
   if (m < 1 || m > 8) return fail(Q35B_ERR_SHAPE, "NVFP4 decode projection supports 1..8 tokens.");
@@ -631,9 +680,10 @@ int wbatch_build(const q35b_gemv_item * items, int count, int m, int digits, WBa
   b->count = count;
   b->m = m;
   b->digits = digits;
+  b->propagate = propagate;
   const int op_rows = m * digits;
   const int n_cols = round_up_int(op_rows, 16);
-  b->b_slot = n_cols * kStepBytes;
+  b->b_slot = n_cols * kStepBytes + kSfBytes;
   b->stages = plan_stages(b->b_slot);
   b->smem = smem_for(b->stages, b->b_slot);
 
@@ -669,13 +719,10 @@ int wbatch_build(const q35b_gemv_item * items, int count, int m, int digits, WBa
   const size_t o_expand = up(o_begin + sizeof(int) * (grid + 1), 256);
   const size_t o_status = up(o_expand + sizeof(ExpandItem) * count, 256);
   size_t o_data = o_status + 256;
-  std::vector<size_t> o_codes(count), o_scales(count), o_g(count);
+  std::vector<size_t> o_ops(count), o_g(count);
   for (int i = 0; i < count; ++i) {
-    const int k = items[i].weight->k;
-    o_codes[i] = o_data;
-    o_data = up(o_data + static_cast<size_t>(op_rows) * (k / 2), 256);
-    o_scales[i] = o_data;
-    o_data = up(o_data + static_cast<size_t>(128) * round_up_int(k / 16, 4), 256);
+    o_ops[i] = o_data;
+    o_data = up(o_data + static_cast<size_t>(items[i].weight->k / 256) * b->b_slot, 256);
     o_g[i] = o_data;
     o_data += 256;
   }
@@ -697,14 +744,11 @@ int wbatch_build(const q35b_gemv_item * items, int count, int m, int digits, WBa
     WItem & it = h_items[i];
     it = WItem{};
     it.tmap_w = w->tmap_codes_128;
-    if (const int st = make_code_map(&it.tmap_x, base + o_codes[i], op_rows, w->k / 2, n_cols)) {
-      cudaFree(b->dev_base);
-      delete b;
-      return st;
-    }
     it.w_scales = w->scales_tiled;
-    it.x_scales = base + o_scales[i];
+    it.x_ops = base + o_ops[i];
     it.x_g = reinterpret_cast<const float *>(base + o_g[i]);
+    it.w_codes = w->codes;
+    it.x = static_cast<const __nv_bfloat16 *>(items[i].x_bf16);
     it.y = static_cast<__nv_bfloat16 *>(items[i].y_bf16);
     it.residual = static_cast<const __nv_bfloat16 *>(items[i].residual_bf16);
     it.rows = w->rows;
@@ -717,8 +761,8 @@ int wbatch_build(const q35b_gemv_item * items, int count, int m, int digits, WBa
     it.s2 = w->s2;
     it.s2_up = w->s2_up;
     it.epilogue = w->gate_up ? kEpiGateUp : kEpiPlain;
-    h_expand[i] = ExpandItem{static_cast<const __nv_bfloat16 *>(items[i].x_bf16), base + o_codes[i], base + o_scales[i],
-                             reinterpret_cast<float *>(base + o_g[i]), w->k};
+    h_expand[i] = ExpandItem{static_cast<const __nv_bfloat16 *>(items[i].x_bf16), base + o_ops[i], reinterpret_cast<float *>(base + o_g[i]),
+                             w->k, n_cols * kStepBytes};
   }
   e = cudaMemset(b->dev_base, 0, o_data);
   if (e == cudaSuccess) e = cudaMemcpy(b->items, h_items.data(), sizeof(WItem) * count, cudaMemcpyHostToDevice);
@@ -737,13 +781,13 @@ int wbatch_build(const q35b_gemv_item * items, int count, int m, int digits, WBa
 int wbatch_launch(const WBatch * b, cudaStream_t s) {
   // 1. digit expansion of every item's activations (one CTA per item); 2. the streaming kernel, whose weight
   // producer starts at once while its activation producer waits for the expansion
-  cudaError_t le = launch_pdl(expand_digits_kernel, dim3(b->count, b->m), dim3(128), 0, s, static_cast<const ExpandItem *>(b->expand),
-                              b->digits);
+  cudaError_t le = launch_pdl(split_digits_kernel, dim3(b->count, b->m), dim3(kSplitThreads), 0, s,
+                              static_cast<const ExpandItem *>(b->expand), b->digits, b->propagate ? 1 : 0);
   count_launch();
-  Q35B_CUDA_TRY(le, "expand_digits_kernel launch");
+  Q35B_CUDA_TRY(le, "split_digits_kernel launch");
   le = launch_pdl(gemm_wstream_kernel, dim3(b->grid), dim3(kThreads), static_cast<size_t>(b->smem), s,
                   static_cast<const WItem *>(b->items), static_cast<const WTile *>(b->tiles), static_cast<const int *>(b->cta_begin),
-                  b->stages, b->b_slot, b->status);
+                  b->stages, b->b_slot, b->status, b->wait_limit);
   count_launch();
   Q35B_CUDA_TRY(le, "gemm_wstream_kernel launch");
   return Q35B_OK;
@@ -757,6 +801,12 @@ void wbatch_free(WBatch * b) {
 
 int wbatch_status(const WBatch * b, unsigned int * out) {
   Q35B_CUDA_TRY(cudaMemcpy(out, b->status, sizeof(unsigned int), cudaMemcpyDeviceToHost), "cudaMemcpy(work list status)");
+  return Q35B_OK;
+}
+
+int wbatch_debug_wait(WBatch * b, unsigned int wait_limit) {
+  b->wait_limit = wait_limit;
+  Q35B_CUDA_TRY(cudaMemset(b->status, 0, sizeof(unsigned int)), "cudaMemset(work list status)");
   return Q35B_OK;
 }
 

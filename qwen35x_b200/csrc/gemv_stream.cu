@@ -1001,6 +1001,27 @@ Assignment assign_tiles(const std::vector<GemvTile> & all, const std::vector<int
   return out;
 }
 
+// Whether a list runs on the tensor cores (gemm_wstream.cu): independent items, block scales the tensor cores read as this
+// kernel does, and enough weights.  That path puts one more launch in front of every run (5 us for one token, 10 for eight,
+// under which the next weights fill the rings), issues a fifth of the instructions and, in runs long enough to meet the
+// power cap, keeps its clock.  Measured in graph replays of 0.2 s and more, us, this kernel / tensor cores: 223 MiB of
+// 1024-column projections one token 50.5 / 44.2, four 52.1 / 50.8, eight 62.0 / 55.4; 461 MiB of 2560-column ones 98 / 88,
+// 111 / 91, 124 / 98; 1.8 GiB 348 / 304, 395 / 332, 443 / 359.  The line: 115 MiB one token 29.8 / 31.3, two 31.1 / 31.4,
+// four 34.9 / 31.9, eight 35.4 / 33.4; 111 MiB one token 26.4 / 24.9; 56 MiB one token 16.2 / 15.7, four 17.6 / 17.0, eight
+// 21.6 / 19.6.
+constexpr int kTensorDigits = 8;  // three bits each: BF16's eight below the largest value of a block and sixteen further down
+constexpr size_t kTensorBytes = 128u << 20, kTensorBytesFrom4 = 48u << 20;  // up to three tokens, and from four on
+
+bool tensor_list(const q35b_gemv_item * items, int count, int m) {
+  size_t bytes = 0;
+  for (int i = 0; i < count; ++i) {
+    const q35b_weight * w = items[i].weight;
+    if (items[i].after != 0 || w->rows <= 0 || !w->has_maps || w->nan_scales || items[i].x_bf16 == nullptr || items[i].y_bf16 == nullptr) return false;
+    bytes += w->codes_bytes + w->scales_bytes;
+  }
+  return bytes >= (m >= 4 ? kTensorBytesFrom4 : kTensorBytes);
+}
+
 }  // namespace
 
 int gemv_batch_build(const q35b_gemv_item * items, int count, int m, bool share_tiles, q35b_gemv_batch ** out) {
@@ -1023,6 +1044,17 @@ int gemv_batch_build(const q35b_gemv_item * items, int count, int m, bool share_
       return fail(Q35B_ERR_ARGUMENT, "An NVFP4 projection work list item can only run after an earlier item of the list.");
     }
     max_k = std::max(max_k, w->k);
+  }
+  if (share_tiles && tensor_list(items, count, m)) {
+    WBatch * t = nullptr;
+    if (const int st = wbatch_build(items, count, m, kTensorDigits, true, &t)) return st;
+    auto * b = new q35b_gemv_batch();
+    b->count = count;
+    b->m = m;
+    b->tensor = t;
+    b->bytes_per_run = wbatch_bytes(t);
+    *out = b;
+    return Q35B_OK;
   }
   auto * b = new q35b_gemv_batch();
   b->count = count;
@@ -1172,7 +1204,7 @@ int gemv_batch_build_tensor(const q35b_gemv_item * items, int count, int m, int 
   if (out == nullptr) return fail(Q35B_ERR_ARGUMENT, "Invalid NVFP4 projection work list.");
   *out = nullptr;
   WBatch * t = nullptr;
-  if (const int st = wbatch_build(items, count, m, digits, &t)) return st;
+  if (const int st = wbatch_build(items, count, m, digits, false, &t)) return st;
   auto * b = new q35b_gemv_batch();
   b->count = count;
   b->m = m;
@@ -1228,7 +1260,8 @@ int gemv_batch_read_status(const q35b_gemv_batch * b, unsigned int * out) {
 size_t gemv_batch_bytes(const q35b_gemv_batch * b) { return b ? b->bytes_per_run : 0; }
 
 int gemv_batch_debug_wait(q35b_gemv_batch * b, unsigned int wait_limit, unsigned int extra_completions) {
-  if (b == nullptr || b->tensor != nullptr || wait_limit == 0) return fail(Q35B_ERR_ARGUMENT, "Invalid NVFP4 projection work list.");
+  if (b == nullptr || wait_limit == 0) return fail(Q35B_ERR_ARGUMENT, "Invalid NVFP4 projection work list.");
+  if (b->tensor != nullptr) return wbatch_debug_wait(b->tensor, wait_limit);
   b->wait_limit = wait_limit;
   b->wait_extra = extra_completions;
   // only the recorded code: every run leaves its counters at zero, also one that gave up

@@ -1,0 +1,129 @@
+"""Large decode lists run on the tensor cores with every BF16 activation split into eight octal NVFP4 digits
+(gemm_wstream.cu).  A value keeps all it has within 2^-23 of its block's largest, so the outputs are those of 64-bit sums of
+the same products to fp32 accuracy: after the BF16 rounding they differ in flipped roundings only, relative L2 below 2e-4
+(a result flips where the fp32 error, some 2^-22 of the terms' size, spans a rounding boundary 2^-9 wide: a few in 10^4
+values by one step of 2^-8)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+E2M1 = [0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0]
+
+
+def _random_weight(engine, torch, gen, n, k, nan_scale=False):
+    codes = torch.randint(0, 256, (n, k // 2), dtype=torch.uint8, device="cuda", generator=gen)
+    scales = torch.randint(0, 0x7f, (n, k // 16), dtype=torch.uint8, device="cuda", generator=gen)
+    if nan_scale:
+        scales[n // 2, 1] = 0x7f
+    table = torch.tensor(E2M1 + [-v for v in E2M1], dtype=torch.float64, device="cuda")
+    sb = scales.to(torch.int64)
+    decoded = torch.where(sb < 8, (sb & 7) * 2.0 ** -9, (8 + (sb & 7)) * torch.pow(2.0, ((sb >> 3) - 10).double()))
+    w = torch.stack([table[(codes & 15).long()], table[(codes >> 4).long()]], dim=2).view(n, k) * decoded.repeat_interleave(16, dim=1)
+    return engine.Nvfp4Weight.from_device(codes, scales, 2.0 ** -12), w * 2.0 ** -12
+
+
+def _filler(engine, torch, gen, m):
+    """What makes a list large enough for the tensor cores: 144 MiB of weights nobody looks at."""
+    n, k = 16384, 16384
+    w = engine.Nvfp4Weight.from_device(torch.randint(0, 256, (n, k // 2), dtype=torch.uint8, device="cuda", generator=gen),
+                                       torch.full((n, k // 16), 0x30, dtype=torch.uint8, device="cuda"), 1e-3)
+    return w, torch.randn((m, k), device="cuda", generator=gen).to(torch.bfloat16), torch.empty((m, n), dtype=torch.bfloat16, device="cuda")
+
+
+def _run(engine, torch, items, m, launches=2):
+    batch = engine.GemvBatch(items, m)
+    before = engine.launch_count()
+    batch.run()
+    assert engine.launch_count() - before == launches
+    batch.run()
+    torch.cuda.synchronize()
+    assert batch.status() == 0
+
+
+def _rel(y, want):
+    import torch
+
+    want = want.to(torch.bfloat16).double()
+    return ((y.double() - want).norm() / want.norm()).item()
+
+
+@pytest.mark.parametrize("m", [1, 2, 3, 5, 8])
+def test_outputs(engine, m):
+    """Rows around a tile, one and many K steps, a residual, activations over the whole range of a token, zeros."""
+    import torch
+
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    items, want = [_filler(engine, torch, gen, m)], [None]
+    for j, (n, k) in enumerate([(1, 256), (127, 512), (129, 2560), (640, 9216), (256, 1024), (300, 768)]):
+        w, wd = _random_weight(engine, torch, gen, n, k)
+        x = torch.randn((m, k), device="cuda", generator=gen)
+        if j == 2:
+            x *= torch.exp2(torch.randint(-30, 30, (m, k), device="cuda", generator=gen).float())
+        if j == 4:
+            x[0] *= 0.0 if m > 1 else 1.0
+            x[:, 16:32] *= 2.0 ** -100
+        if j == 5:
+            x *= 2.0 ** -110
+        x = x.to(torch.bfloat16)
+        res = torch.randn((m, n), device="cuda", generator=gen).to(torch.bfloat16) if j == 3 else None
+        y = torch.zeros((m, n), dtype=torch.bfloat16, device="cuda")
+        items.append((w, x, y, res))
+        want.append(x.double() @ wd.T + (res.double() if res is not None else 0.0))
+    _run(engine, torch, items, m)
+    for item, e in list(zip(items, want))[1:]:
+        assert _rel(item[2], e) <= 2e-4, item[0].rows
+
+
+@pytest.mark.parametrize("m", [1, 4])
+def test_infinities_and_nans(engine, m):
+    import torch
+
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    w, wd = _random_weight(engine, torch, gen, 200, 512)
+    for value in (float("inf"), float("-inf"), float("nan")):
+        x = torch.randn((m, 512), device="cuda", generator=gen).to(torch.bfloat16)
+        x[m - 1, 37] = value
+        y = torch.zeros((m, 200), dtype=torch.bfloat16, device="cuda")
+        _run(engine, torch, [_filler(engine, torch, gen, m), (w, x, y)], m)
+        want = (x.double() @ wd.T).to(torch.bfloat16)
+        same = (y == want) | (torch.isnan(y) & torch.isnan(want))
+        assert bool(same[m - 1].all())
+        if m > 1:
+            assert _rel(y[: m - 1], want[: m - 1].double()) <= 2e-4
+
+
+def test_gate_up(engine):
+    import torch
+
+    m, k, half = 3, 1024, 200
+    gen = torch.Generator(device="cuda").manual_seed(11)
+    gu, parts = [], []
+    for _ in range(2):
+        c = torch.randint(0, 256, (half, k // 2), dtype=torch.uint8, device="cuda", generator=gen)
+        s = torch.full((half, k // 16), 0x38, dtype=torch.uint8, device="cuda")
+        table = torch.tensor(E2M1 + [-v for v in E2M1], dtype=torch.float64, device="cuda")
+        parts.append(torch.stack([table[(c & 15).long()], table[(c >> 4).long()]], dim=2).view(half, k) * 2.0 ** -6)
+        gu += [c.cpu().numpy(), s.cpu().numpy(), 2.0 ** -6]
+    x = torch.randn((m, k), device="cuda", generator=gen).to(torch.bfloat16)
+    y = torch.zeros((m, half), dtype=torch.bfloat16, device="cuda")
+    _run(engine, torch, [_filler(engine, torch, gen, m), (engine.Nvfp4Weight.gate_up_from_host(*gu), x, y)], m)
+    gate, up = x.double() @ parts[0].T, x.double() @ parts[1].T
+    assert _rel(y, gate / (1 + torch.exp(-gate)) * up) <= 3e-4
+
+
+@pytest.mark.parametrize("what", ["0x7f", "after", "small"])
+def test_lists_that_stay_on_the_other_kernel(engine, what):
+    """A scale byte that is NaN to the tensor cores (480 here), an item that waits for another one, few weights."""
+    import torch
+
+    m, gen = 2, torch.Generator(device="cuda").manual_seed(5)
+    w, wd = _random_weight(engine, torch, gen, 256, 512, nan_scale=what == "0x7f")
+    x = torch.randn((m, 512), device="cuda", generator=gen).to(torch.bfloat16)
+    y = torch.zeros((m, 256), dtype=torch.bfloat16, device="cuda")
+    items = [(w, x, y)] if what == "small" else [_filler(engine, torch, gen, m), (w, x, y)]
+    if what == "after":
+        w2, _ = _random_weight(engine, torch, gen, 128, 256)
+        items.append((w2, y, torch.zeros((m, 128), dtype=torch.bfloat16, device="cuda"), None, 1))
+    _run(engine, torch, items, m, launches=1)
+    assert _rel(y, x.double() @ wd.T) <= 1e-3
