@@ -779,7 +779,7 @@ int wbatch_build(const q35b_gemv_item * items, int count, int m, int digits, boo
 }
 
 int wbatch_launch(const WBatch * b, cudaStream_t s) {
-  // 1. digit expansion of every item's activations (one CTA per item); 2. the streaming kernel, whose weight
+  // 1. the digits of every item's activations (one CTA per item and token); 2. the streaming kernel, whose weight
   // producer starts at once while its activation producer waits for the expansion
   cudaError_t le = launch_pdl(split_digits_kernel, dim3(b->count, b->m), dim3(kSplitThreads), 0, s,
                               static_cast<const ExpandItem *>(b->expand), b->digits, b->propagate ? 1 : 0);

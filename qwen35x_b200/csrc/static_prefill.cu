@@ -74,7 +74,7 @@ int q35b_project_prefill_bf16_static(const q35b_weight * w, const void * x_bf16,
   unsigned char * base = nullptr;
   if (const int st = scratch_for_current_device(&base)) return st;
   auto s = static_cast<cudaStream_t>(stream);
-  // Control block: [0,8) quantiser workspace, [16,20) per-tensor scale, [32,36) GEMM status.  The array keeps
+  // Control block: [0,12) quantiser workspace, [16,20) per-tensor scale, [32,36) GEMM status.  The array keeps
   // whatever the previous call left, so everything that must start at zero is cleared here.
   Q35B_CUDA_TRY(cudaMemsetAsync(base, 0, kControlBytes, s), "cudaMemsetAsync(prefill scratch control block)");
   auto * workspace = base;
