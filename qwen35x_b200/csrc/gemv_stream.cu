@@ -1045,7 +1045,8 @@ int gemv_batch_build(const q35b_gemv_item * items, int count, int m, bool share_
     }
     max_k = std::max(max_k, w->k);
   }
-  if (share_tiles && tensor_list(items, count, m)) {
+  // only what the plan below takes too: a list whose activations do not fit it is refused whatever its size
+  if (Plan fits_plan; share_tiles && tensor_list(items, count, m) && make_plan(m, max_k, &fits_plan)) {
     WBatch * t = nullptr;
     if (const int st = wbatch_build(items, count, m, kTensorDigits, true, &t)) return st;
     auto * b = new q35b_gemv_batch();

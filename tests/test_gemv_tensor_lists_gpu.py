@@ -24,8 +24,8 @@ def _random_weight(engine, torch, gen, n, k, nan_scale=False):
 
 
 def _filler(engine, torch, gen, m):
-    """What makes a list large enough for the tensor cores: 144 MiB of weights nobody looks at."""
-    n, k = 16384, 16384
+    """What makes a list large enough for the tensor cores: 142 MiB of weights nobody looks at."""
+    n, k = 28672, 9216
     w = engine.Nvfp4Weight.from_device(torch.randint(0, 256, (n, k // 2), dtype=torch.uint8, device="cuda", generator=gen),
                                        torch.full((n, k // 16), 0x30, dtype=torch.uint8, device="cuda"), 1e-3)
     return w, torch.randn((m, k), device="cuda", generator=gen).to(torch.bfloat16), torch.empty((m, n), dtype=torch.bfloat16, device="cuda")
@@ -127,3 +127,16 @@ def test_lists_that_stay_on_the_other_kernel(engine, what):
         items.append((w2, y, torch.zeros((m, 128), dtype=torch.bfloat16, device="cuda"), None, 1))
     _run(engine, torch, items, m, launches=1)
     assert _rel(y, x.double() @ wd.T) <= 1e-3
+
+
+def test_activations_too_large_for_the_other_kernel_stay_refused(engine):
+    import torch
+
+    n, k, m = 8192, 32768, 8
+    w = engine.Nvfp4Weight.from_device(torch.zeros((n, k // 2), dtype=torch.uint8, device="cuda"),
+                                       torch.full((n, k // 16), 0x30, dtype=torch.uint8, device="cuda"), 1.0)
+    x, y = torch.zeros((m, k), dtype=torch.bfloat16, device="cuda"), torch.zeros((m, n), dtype=torch.bfloat16, device="cuda")
+    items = [(w, x, y)] * 5  # 320 tiles of 128 steps: whole ones
+    with pytest.raises(engine.Q35bError) as e:
+        engine.GemvBatch(items, m)
+    assert e.value.status == 2
