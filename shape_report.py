@@ -105,6 +105,10 @@ def decode_entries(q, torch, device, peaks, shapes, layers, ms, label, row_outli
         graphs = None
         try:
             batches = [q.GemvBatch(list(zip(ws, xs, ys)), m) for ws in weights]
+            launched = q.launch_count()
+            batches[0].run()
+            if q.launch_count() - launched > 1:
+                kernel = "gemm_wstream_kernel (work list, tensor cores)"
         except q.Q35bError as e:
             # activations too large for the streaming kernel's shared memory: per-projection SIMT launches
             kernel = f"gemv_w4a16_rows_kernel per projection ({e})"
