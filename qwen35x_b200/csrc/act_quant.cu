@@ -43,7 +43,7 @@ amax_to_global_scale_kernel(const float * __restrict__ x, size_t n, unsigned int
   const float4 * v = reinterpret_cast<const float4 *>(x);
   const size_t nv = n >> 2;
   for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < nv; i += stride) {
-    const float4 q = __ldg(v + i);
+    const float4 q = __ldcg(v + i);
     local = fmaxf(local, fmaxf(fmaxf(fabsf(q.x), fabsf(q.y)), fmaxf(fabsf(q.z), fabsf(q.w))));
   }
 #pragma unroll
@@ -75,7 +75,7 @@ __device__ __forceinline__ void load16<__nv_bfloat16>(const __nv_bfloat16 * p, f
   const uint4 * q = reinterpret_cast<const uint4 *>(p);
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
-    const uint4 a = __ldg(q + i);
+    const uint4 a = __ldcg(q + i);
     const uint32_t r[4] = {a.x, a.y, a.z, a.w};
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -90,7 +90,7 @@ __device__ __forceinline__ void load16<float>(const float * p, float (&v)[16]) {
   const float4 * q = reinterpret_cast<const float4 *>(p);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const float4 a = __ldg(q + i);
+    const float4 a = __ldcg(q + i);
     v[i * 4] = a.x;
     v[i * 4 + 1] = a.y;
     v[i * 4 + 2] = a.z;
@@ -284,7 +284,7 @@ quantize_activations_kernel(const T * __restrict__ x, uint32_t scale_cols, const
     }
     const uint4 * src = reinterpret_cast<const uint4 *>(x) + static_cast<size_t>(f) * kVecs;
 #pragma unroll
-    for (int i = 0; i < kVecs; ++i) r[i] = in ? __ldg(src + i) : make_uint4(0u, 0u, 0u, 0u);
+    for (int i = 0; i < kVecs; ++i) r[i] = in ? __ldcg(src + i) : make_uint4(0u, 0u, 0u, 0u);
     return in;
   };
 

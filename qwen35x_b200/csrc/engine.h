@@ -33,6 +33,9 @@ int sm_count();
 // still finishing.  A kernel launched this way may read what no kernel ever writes (weights and their descriptors,
 // constant from q35b_weight_create* on) before griddepcontrol.wait, which returns only when everything earlier in the
 // stream is complete and visible; what an earlier kernel may have written or may still read it touches only after it.
+// Since the kernel before may still be writing when such a grid starts, nothing it writes is read-only for the grid's whole
+// life: activations, scales of tensors and residuals are loaded with __ldcg or __ldca and never with __ldg, whose
+// non-coherent path may answer from a line fetched before the write (a scale word has the same address in every call).
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args &&... args) {
   cudaLaunchConfig_t cfg = {};

@@ -347,12 +347,12 @@ gemm_w4a4_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     // ---------------- epilogue (both CTAs): this CTA's 128 rows of the pair's tile ----------------
     const int quarter = warp & 3;                 // TMEM lanes 32 * quarter .. + 31 (fixed by the warp's index)
     const int col_base = ((warp - 2) >> 2) * kEpiCols;
-    const float g = __ldg(g_dev);
+    const float g = __ldcg(g_dev);
     GemmQuantScale q;
     if constexpr (kEpilogueWarps == kEpiWarpsWide) {
       __shared__ float q_table[128];
       if (ep.q_codes != nullptr) {
-        q.g = __ldg(ep.q_g);
+        q.g = __ldcg(ep.q_g);
         q.rg = __frcp_rn(q.g);
         q.table = q_table;
         const int at = threadIdx.x - 64;

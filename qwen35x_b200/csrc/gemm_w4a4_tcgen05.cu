@@ -463,7 +463,7 @@ gemm_w4a4_ksplit_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   {
     // this CTA's share of the tokens
     const int t_begin = rank * n_cols / SPLIT, t_end = min((rank + 1) * n_cols / SPLIT, tokens);
-    const float g = __ldg(g_dev);
+    const float g = __ldcg(g_dev);
     const float alpha = g * ep.s2, alpha_up = g * ep.s2_up;
     uint32_t src[SPLIT];
 #pragma unroll
@@ -474,7 +474,7 @@ gemm_w4a4_ksplit_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
     if constexpr (EPI == kEpiNvfp4) {
       // one thread per token and 32 weight rows = one block of 16 outputs (n % 128 == 0 is checked on the host);
       // lanes along the tokens, whose pitch spreads them over the banks
-      const float q_g = __ldg(ep.q_g);
+      const float q_g = __ldcg(ep.q_g);
       const GemmQuantScale q = {q_g, __frcp_rn(q_g), nullptr};
       const int live = __any_sync(0xffffffffu, stop_lane) ? 0 : t_end - t_begin;
       for (int u = threadIdx.x; u < live * (kRows / 32); u += kThreads) {
@@ -512,7 +512,7 @@ gemm_w4a4_ksplit_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
           float rv[4] = {0.0f, 0.0f, 0.0f, 0.0f};
           if (ep.residual != nullptr) {
             if (whole) {
-              const uint2 p = __ldg(reinterpret_cast<const uint2 *>(res));
+              const uint2 p = __ldcg(reinterpret_cast<const uint2 *>(res));
               rv[0] = __uint_as_float(p.x << 16); rv[1] = __uint_as_float(p.x & 0xffff0000u);
               rv[2] = __uint_as_float(p.y << 16); rv[3] = __uint_as_float(p.y & 0xffff0000u);
             } else {

@@ -420,9 +420,15 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
     const int quarter = warp & 3, first_token = (warp - 3) >> 2;
     const int row_in_tile = quarter * 32 + lane;
     STile spill;
+    const float * scales_of = nullptr;
+    float scales = 0.0f;  // of token `lane`, read once per projection and before the wait (one load per token cost 1 us a tile)
     for (int ti = 0; ti < n_tiles; ++ti) {
       const STile * it = tile_at(ti, spill);
       const uint32_t ab = ti & 1;
+      if (it->x_g != scales_of) {
+        scales_of = it->x_g;
+        scales = lane < it->tokens ? __ldcg(scales_of + lane) : 0.0f;
+      }
       if (!mbar_wait(smem_u32(tmem_full + ab), (ti >> 1) & 1, wait_limit)) {
         if (lane == 0) atomicExch(status, kEpilogueWait);
         break;
@@ -445,7 +451,7 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
           tmem_ld8(taddr + 2 * n_cols + token * digits, r[2]);
           tmem_ld8(taddr + 3 * n_cols + token * digits, r[3]);
         }
-        float g = __ldg(it->x_g + token);
+        float g = __shfl_sync(0xffffffffu, scales, token);
         tmem_wait_ld(r);
         float sum = 0.0f, weight = 1.0f;  // of digit j: 8^-j
 #pragma unroll
@@ -544,7 +550,7 @@ __global__ void __launch_bounds__(kSplitThreads) split_digits_kernel(const Expan
   const uint4 * src = reinterpret_cast<const uint4 *>(it.x + static_cast<size_t>(token) * k);
   __shared__ uint32_t red[kSplitThreads / 32];
   auto load = [&](int c) {
-    uint4 q = __ldg(src + c);
+    uint4 q = __ldca(src + c);
     if (!propagate) {
       uint32_t * r = reinterpret_cast<uint32_t *>(&q);
 #pragma unroll

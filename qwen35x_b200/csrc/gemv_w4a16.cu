@@ -81,7 +81,7 @@ struct XLoad;
 template <>
 struct XLoad<__nv_bfloat16> {
   static __device__ __forceinline__ void load8(const __nv_bfloat16 * p, float, float2 (&x)[4]) {
-    const uint4 q = __ldg(reinterpret_cast<const uint4 *>(p));
+    const uint4 q = __ldca(reinterpret_cast<const uint4 *>(p));
     x[0] = make_float2(__uint_as_float(q.x << 16), __uint_as_float(q.x & 0xffff0000u));
     x[1] = make_float2(__uint_as_float(q.y << 16), __uint_as_float(q.y & 0xffff0000u));
     x[2] = make_float2(__uint_as_float(q.z << 16), __uint_as_float(q.z & 0xffff0000u));
@@ -91,7 +91,7 @@ struct XLoad<__nv_bfloat16> {
 template <>
 struct XLoad<float> {
   static __device__ __forceinline__ void load8(const float * p, float scale, float2 (&x)[4]) {
-    const float4 a = __ldg(reinterpret_cast<const float4 *>(p)), b = __ldg(reinterpret_cast<const float4 *>(p) + 1);
+    const float4 a = __ldca(reinterpret_cast<const float4 *>(p)), b = __ldca(reinterpret_cast<const float4 *>(p) + 1);
     x[0] = make_float2(a.x * scale, a.y * scale);
     x[1] = make_float2(a.z * scale, a.w * scale);
     x[2] = make_float2(b.x * scale, b.y * scale);
