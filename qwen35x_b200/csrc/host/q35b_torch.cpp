@@ -29,6 +29,25 @@ PyObject * raise_status(int status) {
   return nullptr;
 }
 
+// An int (kernel numbers) or a float or int (scales), as the general path takes them: anything else is left to it.
+bool int_arg(PyObject * o, int * out) {
+  if (!PyLong_Check(o)) return false;
+  const long v = PyLong_AsLong(o);
+  if (v < INT32_MIN || v > INT32_MAX || PyErr_Occurred() != nullptr) {
+    PyErr_Clear();
+    return false;
+  }
+  *out = static_cast<int>(v);
+  return true;
+}
+bool float_arg(PyObject * o, float * out) {
+  if (!PyFloat_Check(o) && !PyLong_Check(o)) return false;
+  *out = static_cast<float>(PyFloat_AsDouble(o));
+  if (PyErr_Occurred() == nullptr) return true;
+  PyErr_Clear();
+  return false;
+}
+
 // A tensor of exactly torch.Tensor on the current CUDA device, strided and with memory behind it.
 bool plain_cuda(PyObject * o, at::ScalarType type, c10::DeviceIndex device, const at::Tensor ** out) {
   if (!THPVariable_CheckExact(o)) return false;
@@ -79,13 +98,14 @@ PyObject * gemv(PyObject *, PyObject * const * args, Py_ssize_t n) {
   if (!plain_cuda(args[1], at::kBFloat16, device, &x) || !x->is_contiguous() || x->dim() < 1 || x->dim() > 2) return not_plain();
   const int64_t m = x->dim() == 2 ? x->size(0) : 1;
   if (x->size(-1) != q35b_weight_cols(w) || m < 1 || m > 8) return not_plain();
-  const long kernel = PyLong_AsLong(args[3]);
+  int kernel = 0;
+  if (!int_arg(args[3], &kernel)) return not_plain();
   at::Tensor made;
   const at::Tensor * y = output(args[2], m, q35b_weight_rows(w), device, made);
   if (y == nullptr || !y->is_contiguous()) return not_plain();
   const void * xp = x->const_data_ptr();
   void * yp = y->mutable_data_ptr(), * stream = stream_of(device);
-  if (const int st = without_gil([&] { return q35b_gemv_w4a16_bf16(w, xp, static_cast<int>(m), yp, static_cast<int>(kernel), stream); })) return raise_status(st);
+  if (const int st = without_gil([&] { return q35b_gemv_w4a16_bf16(w, xp, static_cast<int>(m), yp, kernel, stream); })) return raise_status(st);
   return returned(args[2], made);
   END_HANDLE_TH_ERRORS
 }
@@ -98,14 +118,14 @@ PyObject * gemv_f32(PyObject *, PyObject * const * args, Py_ssize_t n) {
   const c10::DeviceIndex device = c10::cuda::current_device();
   const at::Tensor * x = nullptr;
   if (!plain_cuda(args[1], at::kFloat, device, &x) || !x->is_contiguous() || x->numel() != q35b_weight_cols(w)) return not_plain();
-  const float scale = static_cast<float>(PyFloat_AsDouble(args[2]));
-  const long kernel = PyLong_AsLong(args[3]);
-  if (PyErr_Occurred() != nullptr) return nullptr;
+  float scale = 0.0f;
+  int kernel = 0;
+  if (!float_arg(args[2], &scale) || !int_arg(args[3], &kernel)) return not_plain();
   at::Tensor y = at::empty({q35b_weight_rows(w)}, x->options());
   const float * xp = x->const_data_ptr<float>();
   float * yp = y.mutable_data_ptr<float>();
   void * stream = stream_of(device);
-  if (const int st = without_gil([&] { return q35b_gemv_w4a16_f32(w, xp, scale, yp, static_cast<int>(kernel), stream); })) return raise_status(st);
+  if (const int st = without_gil([&] { return q35b_gemv_w4a16_f32(w, xp, scale, yp, kernel, stream); })) return raise_status(st);
   return THPVariable_Wrap(std::move(y));
   END_HANDLE_TH_ERRORS
 }
@@ -139,11 +159,7 @@ struct Activations {
       return false;
     }
     if (!codes->is_contiguous() || codes->numel() != static_cast<int64_t>(m) * (k / 2)) return false;
-    scale = static_cast<float>(PyFloat_AsDouble(global_scale));
-    if (PyErr_Occurred() != nullptr) {
-      PyErr_Clear();
-      return false;
-    }
+    if (!float_arg(global_scale, &scale)) return false;
     PyObject * key = Py_BuildValue("(iK)", static_cast<int>(device), static_cast<unsigned long long>(reinterpret_cast<uintptr_t>(stream)));
     if (key == nullptr) {
       PyErr_Clear();
@@ -228,14 +244,14 @@ PyObject * gemm(PyObject *, PyObject * const * args, Py_ssize_t n) {
   const c10::DeviceIndex device = c10::cuda::current_device();
   const at::Tensor * codes = nullptr, * scales = nullptr, * g = nullptr, * residual = nullptr;
   if (!plain_cuda(args[1], at::kByte, device, &codes) || !plain_cuda(args[2], at::kByte, device, &scales) || !plain_cuda(args[3], at::kFloat, device, &g)) return not_plain();
-  const long m = PyLong_Check(args[4]) ? PyLong_AsLong(args[4]) : 0;
+  int m = 0;
   const int rows = q35b_weight_rows(w);
-  if (m < 1 || m > INT32_MAX || !residual_arg(args[6], static_cast<int>(m), rows, device, &residual)) return not_plain();
+  if (!int_arg(args[4], &m) || m < 1 || !residual_arg(args[6], m, rows, device, &residual)) return not_plain();
   at::Tensor made;
   const at::Tensor * out = output(args[5], m, q35b_weight_is_gate_up(w) != 0 ? rows / 2 : rows, device, made);
   if (out == nullptr || out->stride(0) > INT32_MAX) return not_plain();
   void * stream = stream_of(device);
-  if (const int st = without_gil([&] { return gemm_call(w, *codes, *scales, *g, static_cast<int>(m), residual, *out, stream); })) return raise_status(st);
+  if (const int st = without_gil([&] { return gemm_call(w, *codes, *scales, *g, m, residual, *out, stream); })) return raise_status(st);
   return returned(args[5], made);
   END_HANDLE_TH_ERRORS
 }
