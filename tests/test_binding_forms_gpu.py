@@ -1,5 +1,7 @@
 """The binding's native calls take the plain form of a call only; every other form goes the general way with the results and
 errors it always had.  Both ways on the same inputs have to give the same bits."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -69,3 +71,19 @@ def test_other_forms(engine, weight):
     w2.close()
     with pytest.raises(Exception):
         engine.gemv_w4a16(w2, x[:, :256].contiguous())
+
+
+@pytest.mark.parametrize("bad", [None, "1", 1.5, np.int64(1)])
+def test_kernel_numbers_and_scales_of_other_types_stay_refused(engine, weight, bad):
+    """What ctypes refuses on the general path is not converted by the native one."""
+    import torch
+
+    x = to_torch_bf16(make_activations(1, 512, seed=2))
+    scratch = engine.act_scratch(1, 512, x.device)
+    with pytest.raises(ctypes.ArgumentError):
+        engine.gemv_w4a16(weight, x, kernel=bad)
+    if bad != 1.5:
+        with pytest.raises(ctypes.ArgumentError):
+            engine.gemv_w4a16_f32(weight, x[0].float(), bad)
+        with pytest.raises(ctypes.ArgumentError):
+            engine.quantize_activations(x, torch.ones(1) if bad is None else bad, scratch)
