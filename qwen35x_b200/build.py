@@ -7,6 +7,7 @@ entry points it needs at run time, so it loads on a machine without a GPU
 (every compute call then fails with Q35B_ERR_CUDA)."""
 from __future__ import annotations
 
+import importlib.util
 import shutil
 import subprocess
 import sys
@@ -19,6 +20,7 @@ LIB_DIR = PKG / "_lib"
 LIB = LIB_DIR / "libq35b.so"
 CLI = LIB_DIR / "q35b"
 BINDING = LIB_DIR / "q35b_torch.so"
+BINDING_STAMP = LIB_DIR / "q35b_torch.built_for"
 
 SOURCES = ["api.cu", "gemv_w4a16.cu", "gemv_stream.cu", "act_quant.cu", "gemm_w4a4_tcgen05.cu", "gemm_w4a4_2cta.cu", "gemm_wstream.cu", "static_prefill.cu", "peer_gather.cu"]
 NVCC_FLAGS = [
@@ -64,16 +66,27 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         cmd = [_nvcc(), "-shared", "-o", str(LIB), *map(str, objs), "-cudart", "static", "-lpthread", "-ldl"]
         subprocess.run(cmd, check=True)
     build_cli(force=force or bool(procs))
-    build_binding(force=force)
+    if importlib.util.find_spec("torch") is None or shutil.which("g++") is None:
+        print("q35b_torch.so is left out: it needs torch and g++ (the library and the command line need neither)", file=sys.stderr)
+        return LIB
+    try:
+        build_binding(force=force)
+    except subprocess.CalledProcessError as e:  # a torch without its headers or CUDA libraries
+        print(f"q35b_torch.so could not be built ({e}): the Python binding goes its general way for every call", file=sys.stderr)
     return LIB
 
 
 def build_binding(force: bool = False) -> Path:
-    """The extension module of the Python binding's hot calls (qwen35x_b200/_lib/q35b_torch.so)."""
-    src = CSRC / "host" / "q35b_torch.cpp"
-    if force or _stale(BINDING, [src, PKG.parent / "include" / "q35b_nvfp4.h"]):
-        import torch
+    """The extension module of the Python binding's hot calls (qwen35x_b200/_lib/q35b_torch.so), for the torch and the Python
+    that run this."""
+    import torch
 
+    from .engine import native_stamp
+
+    src, stamp = CSRC / "host" / "q35b_torch.cpp", native_stamp(torch)
+    stale = _stale(BINDING, [src, PKG.parent / "include" / "q35b_nvfp4.h"]) or not BINDING_STAMP.is_file() or BINDING_STAMP.read_text() != stamp
+    if force or stale:
+        BINDING_STAMP.unlink(missing_ok=True)
         root = Path(torch.__file__).resolve().parent
         cuda = Path(_nvcc()).resolve().parent.parent
         cmd = ["g++", "-std=c++17", "-O2", "-fPIC", "-shared", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
@@ -81,6 +94,7 @@ def build_binding(force: bool = False) -> Path:
                f"-I{sysconfig.get_paths()['include']}", str(src), "-o", str(BINDING), f"-L{LIB_DIR}", "-lq35b", f"-L{root / 'lib'}",
                "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python", "-Wl,-rpath,$ORIGIN"]
         subprocess.run(cmd, check=True)
+        BINDING_STAMP.write_text(stamp)
     return BINDING
 
 

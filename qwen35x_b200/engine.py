@@ -7,6 +7,8 @@ from __future__ import annotations
 
 import ctypes as C
 import importlib.util
+import sys
+import warnings
 from pathlib import Path
 
 import numpy as np
@@ -14,6 +16,7 @@ import numpy as np
 _PKG = Path(__file__).resolve().parent
 _LIB_PATH = _PKG / "_lib" / "libq35b.so"
 _NATIVE_PATH = _PKG / "_lib" / "q35b_torch.so"
+_NATIVE_STAMP = _PKG / "_lib" / "q35b_torch.built_for"  # native_stamp of the torch and Python it was built for
 _lib = None
 
 GEMV_AUTO, GEMV_SIMT, GEMV_STREAM = -1, 10, 11
@@ -179,21 +182,41 @@ def _torch():
 _native_module = None
 
 
+class _NoNative:
+    """In the place of an extension module that is not there: every call goes the general way."""
+
+    def __getattr__(self, name):
+        return lambda *args: NotImplemented
+
+
 def _native():
     """The extension module of the hot calls (csrc/host/q35b_torch.cpp).  Its functions answer NotImplemented for a call
-    that is not in their plain form; the caller then goes the general way below."""
+    that is not in their plain form; the caller then goes the general way below, as it does for every call where the
+    module has not been built (the library itself needs neither torch nor a C++ compiler) or was built for another torch."""
     global _native_module
     if _native_module is None:
-        _torch()
+        torch = _torch()
         lib()
-        if not _NATIVE_PATH.is_file():
-            raise FileNotFoundError(f"{_NATIVE_PATH} is missing: run `python -m qwen35x_b200.build` (needs nvcc and torch)")
-        spec = importlib.util.spec_from_file_location("q35b_torch", _NATIVE_PATH)
-        module = importlib.util.module_from_spec(spec)
-        spec.loader.exec_module(module)
-        module.setup(Q35bError, _workspaces)
+        stamp = _NATIVE_STAMP.read_text() if _NATIVE_STAMP.is_file() and _NATIVE_PATH.is_file() else None
+        try:
+            if stamp != native_stamp(torch):
+                raise ImportError("not built" if stamp is None else f"built for {stamp.split()[0]}")
+            spec = importlib.util.spec_from_file_location("q35b_torch", _NATIVE_PATH)
+            module = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(module)
+        except ImportError as e:
+            warnings.warn(f"{_NATIVE_PATH.name} is not used ({e}): every call spends 3 to 4 us more in the interpreter; "
+                          "`python -m qwen35x_b200.build` builds it for this torch", RuntimeWarning, stacklevel=3)
+            module = _NoNative()
+        else:
+            module.setup(Q35bError, _workspaces)
         _native_module = module
     return _native_module
+
+
+def native_stamp(torch) -> str:
+    """What the extension module of the hot calls has to have been built for."""
+    return f"torch-{torch.__version__} python-{sys.version_info[0]}.{sys.version_info[1]}"
 
 
 def _stream_ptr(torch) -> int:
