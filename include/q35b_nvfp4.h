@@ -175,14 +175,20 @@ typedef struct q35b_gemv_item {
 Q35B_API size_t q35b_gemv_item_bytes(void);
 
 typedef struct q35b_gemv_batch q35b_gemv_batch;
-/* Builds the tile schedule and uploads the descriptors (allocates, synchronises). */
+/* Builds the tile schedule and uploads the descriptors (allocates, synchronises).
+ * How exact a list is does not depend on what is in it: sums are fp32, and of a BF16 activation nothing is lost above 2^-39
+ * of its token's largest one.  Lists with dependent items, and small ones, convert every token to fp16 with one power of two;
+ * large lists of independent items run on the tensor cores (see below) with as many octal digits as that takes: eight in
+ * every K step, and six more in the steps of 256 columns where a value has bits below 2^-16 of the largest of its sixteen
+ * neighbours.  Infinities and NaNs reach the outputs as fp32 arithmetic has it, on either path. */
 Q35B_API int q35b_gemv_batch_create(const q35b_gemv_item * items, int count, int m, q35b_gemv_batch ** out);
 /* The same work list on the tensor cores (no counterpart in the reference, whose decode dequantises in registers,
  * src/kernels/cuda/decode_layers.cuh:200-261): the weight streams through tcgen05.mma as the 128-row operand and
  * every token's BF16 activations enter as `digits` rows of NVFP4, their octal digits, computed on the device before
  * each run (16-element blocks, power-of-two block scale, one fp32 scale per token): what `digits` digits leave of a
- * value is at most 2^(1 - 3 digits) of its block's largest element.  q35b_gemv_batch_create itself takes this path with
- * eight digits (2^-23) for large lists of independent items, where it is the faster one.  Here items must be independent
+ * value is at most 2^(1 - 3 digits) of its block's largest element, or of 2^-17 of its token's largest element where that
+ * is more.  q35b_gemv_batch_create itself takes this path, with digits as they are needed, for large lists of independent
+ * items, where it is the faster one.  Here the digits are the caller's choice, items must be independent
  * (after = 0), and non-finite activations count as zero.  digits: 1..8 with m * digits <= 128.  q35b_gemv_batch_run
  * launches two kernels (the digits, then the projection, whose weight stream starts at once). */
 Q35B_API int q35b_gemv_batch_create_tensor(const q35b_gemv_item * items, int count, int m, int digits,

@@ -155,8 +155,8 @@ int launch_gemm_w4a4(const q35b_weight * w, const uint8_t * a_codes, const uint8
 
 // gemm_wstream.cu: decode work lists on the tensor cores
 struct WBatch;  // decode work list on the tensor path (digit-expanded activations)
-// propagate: infinities and NaNs of the activations reach the outputs (else they count as zero)
-int wbatch_build(const q35b_gemv_item * items, int count, int m, int digits, bool propagate, WBatch ** out);
+// exact: all bits of the activations, their infinities and NaNs too, reach the outputs (else what `digits` digits hold)
+int wbatch_build(const q35b_gemv_item * items, int count, int m, int digits, bool exact, WBatch ** out);
 int wbatch_launch(const WBatch * b, cudaStream_t s);
 void wbatch_free(WBatch * b);
 int wbatch_status(const WBatch * b, unsigned int * out);

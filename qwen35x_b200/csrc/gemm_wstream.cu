@@ -16,8 +16,10 @@
 // y[token, row].
 //
 // Decode (W4A16, 1..8 tokens): every token enters as `digits` operand rows, the octal digits of its BF16 activations
-// (split_digits_kernel below).  Eight digits leave 2^-23 of a block's largest value, which is all that fp32 sums keep, and
-// the epilogue adds the digits' accumulator columns.  Replaces nvfp4_row_dot / matvec_nvfp4_bf16
+// (split_digits_kernel below), and the epilogue adds the digits' accumulator columns.  Eight digits hold all eight bits of a
+// value down to about 2^-16 of its block's largest one; smaller values need up to six more, the deep digits.  They are rows
+// of a second operand that is loaded and multiplied only in the K steps where some value has them (one in 60,000 normal
+// values does), with sums of their own; with one token they fit into the padding of the first.  Replaces nvfp4_row_dot / matvec_nvfp4_bf16
 // (src/kernels/cuda/decode_layers.cuh:200-284) with the FP4 decode done by the tensor core instead of by conversion
 // instructions: a fifth of gemv_stream.cu's instructions, so a long run of steps does not meet the power cap.
 //
@@ -45,7 +47,7 @@ constexpr int kMaxStages = 8;
 constexpr int kEpilogueWarps = 8;        // two per quarter of the TMEM lanes, each taking every other token
 constexpr int kThreads = (3 + kEpilogueWarps) * 32;  // warp 0 weight producer, 1 MMA, 2 activation producer
 constexpr int kTmemCols = 512;           // two accumulator buffers ...
-constexpr int kAccBufCols = 224;
+constexpr int kAccBufCols = 224;         // partial accumulators of the operand rows, then those of the deep digits' rows
 constexpr int kSfaCol = 2 * kAccBufCols;   // ... and two sets of scale-factor columns (A 16 + B 16 each), used by stages in turn,
 constexpr int kSfbCol = kSfaCol + 16;      // so that the copies of one stage do not wait for the MMAs of the one before
 constexpr int kSfSetCols = 32;
@@ -55,12 +57,15 @@ constexpr int kSmemBudget = 220 * 1024;   // dynamic part; the staged tile descr
 enum StatusCode : unsigned { kWeightWait = 41, kActWait = 42, kMmaWait = 43, kMmaDrainWait = 44, kEpilogueWait = 45 };
 enum Epilogue : int { kEpiPlain = 0, kEpiGateUp = 1 };
 
+constexpr int kDeepDigits = 6;           // of a list that takes the activations exactly (see split_digits_kernel)
+
 // One projection of the list, in device memory; the tensor maps are read by the TMA unit from there.
 struct alignas(128) WItem {
   CUtensorMap tmap_w;            // weight codes [rows, K/2], box 128 rows x 128 bytes, 128B swizzle
   const uint8_t * w_scales;      // weight scale tiles
   const uint8_t * x_ops;         // the operand, one run of bytes per K step: codes as they lie in shared memory (n_cols rows of
-                                 // 128 bytes, 128B swizzle), then four scale tiles
+                                 // 128 bytes, 128B swizzle) and four scale tiles, then the same of the deep digits' rows
+  const uint32_t * x_deep;       // NULL (no deep digits), or for every 32 K steps a word per token (eight): the steps where it has them
   const float * x_g;             // the operand's scale, one per token (NaN: the token has infinities or NaNs, see exact_dot)
   const uint8_t * w_codes;       // for such tokens: weight codes and the activations themselves
   const __nv_bfloat16 * x;
@@ -69,6 +74,8 @@ struct alignas(128) WItem {
   int rows;                      // weight rows
   int k_steps;                   // K / 256
   int n_cols;                    // operand rows padded to a multiple of 16 (UMMA N)
+  int deep_cols;                 // the same of the deep digits' rows; 0: there are none, or they are
+  int deep_rows;                 // rows of the operand itself, from this one on
   int tokens;
   int digits;                    // operand rows per token
   int ldy, ldr;
@@ -87,11 +94,12 @@ struct alignas(16) STile {
   const CUtensorMap * tmap_w;
   const uint8_t * w_scales;      // scale tiles of this row block
   const uint8_t * x_ops;
+  const uint32_t * x_deep;
   const float * x_g;
   const WItem * item;
   __nv_bfloat16 * y;
   const __nv_bfloat16 * residual;
-  int row_block, rows, k_steps, n_cols, tokens, digits, ldy, ldr, epilogue;
+  int row_block, rows, k_steps, n_cols, deep_cols, deep_rows, tokens, digits, ldy, ldr, epilogue;
   float s2, s2_up;
 };
 constexpr int kMaxTilesInSmem = 40;
@@ -162,7 +170,11 @@ __device__ __forceinline__ uint64_t desc_sf(uint32_t saddr) {
 // against 900 for the stage's bytes to arrive from HBM).  So the MMAs of a stage go to different partial
 // accumulators (as many as fit beside each other in a buffer), each of which then sees one MMA per stage, and the
 // epilogue adds the partials.
-__device__ __forceinline__ int partial_accumulators(int n_cols) { return 4 * n_cols <= kAccBufCols ? 4 : (2 * n_cols <= kAccBufCols ? 2 : 1); }
+__device__ __forceinline__ int partial_accumulators(int n_cols, int deep_cols) {
+  return 4 * n_cols + deep_cols <= kAccBufCols ? 4 : (2 * n_cols + deep_cols <= kAccBufCols ? 2 : 1);
+}
+// ... and of the deep digits' rows behind them
+__device__ __forceinline__ int deep_accumulators(int used, int deep_cols) { return used + 2 * deep_cols <= kAccBufCols ? 2 : 1; }
 
 // kind::mxf4nvf4: E2M1 x E2M1, K-major, UE4M3 scales, M = 128, N = n_cols.
 __device__ __forceinline__ uint32_t instr_desc(int n_cols) {
@@ -226,12 +238,13 @@ __device__ __noinline__ float exact_dot(const WItem * it, int row, int token) {
 // CTA b walks tiles[cta_begin[b] .. cta_begin[b + 1]).
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__ tiles, const int * __restrict__ cta_begin,
-                    int stages, int b_slot_bytes, unsigned int * status, uint32_t wait_limit) {
+                    int stages, int b_slot_bytes, int deep_bytes, unsigned int * status, uint32_t wait_limit) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t * smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint8_t * smem_a = smem;
   uint8_t * smem_b = smem_a + stages * kABytes;
-  uint8_t * smem_sfa = smem_b + stages * b_slot_bytes;     // a slot of smem_b holds a step's operand codes and scale tiles
+  uint8_t * smem_sfa = smem_b + stages * b_slot_bytes;     // a slot of smem_b holds a step's operand codes and scale tiles,
+                                                           // its last deep_bytes those of the deep digits
   uint64_t * bars = reinterpret_cast<uint64_t *>(smem_sfa + stages * kSfBytes);
   uint64_t * full = bars;                           // [stages]: both producers' bytes have landed
   uint64_t * empty = bars + kMaxStages;             // [stages]: the MMAs that read the stage have retired
@@ -239,6 +252,7 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
   uint64_t * tmem_empty = tmem_full + 2;            // [2]: the epilogue warps have read the accumulator out
   uint32_t * tmem_slot = reinterpret_cast<uint32_t *>(tmem_empty + 2);
   __shared__ STile stile[kMaxTilesInSmem];
+  __shared__ uint32_t stage_deep[kMaxStages];              // the stage's step has deep digits; set before its bytes are asked for
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -252,12 +266,15 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
     d.k_steps = it->k_steps;
     d.w_scales = it->w_scales + static_cast<size_t>(rb) * d.k_steps * kSfBytes;
     d.x_ops = it->x_ops;
+    d.x_deep = it->x_deep;
     d.x_g = it->x_g;
     d.y = it->y;
     d.residual = it->residual;
     d.row_block = rb;
     d.rows = it->rows;
     d.n_cols = it->n_cols;
+    d.deep_cols = it->deep_cols;
+    d.deep_rows = it->deep_rows;
     d.tokens = it->tokens;
     d.digits = it->digits;
     d.ldy = it->ldy;
@@ -335,30 +352,46 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
     }
   } else if (warp == 2) {
     // ------------------------------------------------------------ activation producer
-    if (elect_one()) {
-      asm volatile("griddepcontrol.wait;" ::: "memory");
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      STile spill;
-      for (int ti = 0; ti < n_tiles && ok; ++ti) {
-        const STile * it = tile_at(ti, spill);
-        const int k_steps = it->k_steps;
-        const uint8_t * ops = it->x_ops;
-        for (int ks = 0; ks < k_steps; ++ks) {
-          if (!mbar_wait(smem_u32(empty + stage), phase ^ 1, wait_limit)) {
-            atomicExch(status, kActWait);
-            ok = false;
-            break;
-          }
-          const uint32_t bar = smem_u32(full + stage);
-          mbar_expect_tx(bar, static_cast<uint32_t>(b_slot_bytes));
-          bulk_load(smem_u32(smem_b + stage * b_slot_bytes), ops + static_cast<size_t>(ks) * b_slot_bytes, static_cast<uint32_t>(b_slot_bytes), bar);
-          if (++stage == stages) {
-            stage = 0;
-            phase ^= 1;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    STile spill;
+    const uint32_t * deep_of = nullptr;
+    int deep_block = 0;
+    uint32_t masks = 0;  // of token lane & 7, steps 128 * deep_block + 32 * (lane >> 3) and on; read once per projection
+    for (int ti = 0; ti < n_tiles && ok; ++ti) {
+      const STile * it = tile_at(ti, spill);
+      const int k_steps = it->k_steps;
+      for (int base = 0; base < k_steps && ok; base += 32) {
+        if (deep_bytes > 0 && (it->x_deep != deep_of || base >> 7 != deep_block)) {
+          deep_of = it->x_deep;
+          deep_block = base >> 7;
+          const int word = 4 * deep_block + (lane >> 3);
+          masks = 32 * word < k_steps ? __ldcg(deep_of + 8 * word + (lane & 7)) : 0u;
+        }
+        const uint32_t deep = __reduce_or_sync(0xffffffffu, lane >> 3 == (base >> 5 & 3) ? masks : 0u);
+        const uint8_t * ops = it->x_ops + static_cast<size_t>(base) * b_slot_bytes;
+        if (elect_one()) {
+          for (int i = 0; i < min(k_steps - base, 32); ++i) {
+            if (!mbar_wait(smem_u32(empty + stage), phase ^ 1, wait_limit)) {
+              atomicExch(status, kActWait);
+              ok = false;
+              break;
+            }
+            const uint32_t bar = smem_u32(full + stage), has = deep >> i & 1u;
+            const uint32_t bytes = static_cast<uint32_t>(has != 0u ? b_slot_bytes : b_slot_bytes - deep_bytes);
+            stage_deep[stage] = has;
+            mbar_expect_tx(bar, bytes);
+            bulk_load(smem_u32(smem_b + stage * b_slot_bytes), ops + static_cast<size_t>(i) * b_slot_bytes, bytes, bar);
+            if (++stage == stages) {
+              stage = 0;
+              phase ^= 1;
+            }
           }
         }
+        // the elected lane is the same one every time and keeps the ring's position; whether it gave up, all have to know
+        ok = __all_sync(0xffffffffu, ok);
       }
     }
   } else if (warp == 1) {
@@ -374,7 +407,8 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
       for (int ti = 0; ti < n_tiles && ok; ++ti) {
         const STile * it = tile_at(ti, spill);
         const int k_steps = it->k_steps;
-        const uint32_t idesc = instr_desc(it->n_cols);
+        const uint32_t idesc = instr_desc(it->n_cols), idesc_deep = instr_desc(it->deep_cols);
+        uint32_t deep_seen = 0;
         const uint32_t ab = ti & 1;
         if (!mbar_wait(smem_u32(tmem_empty + ab), ((ti >> 1) & 1) ^ 1, wait_limit)) {
           atomicExch(status, kMmaDrainWait);
@@ -382,7 +416,8 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t acc = tmem_base + ab * kAccBufCols;
-        const int n_cols = it->n_cols, parts = partial_accumulators(n_cols);
+        const int n_cols = it->n_cols, deep_cols = it->deep_cols, parts = partial_accumulators(n_cols, deep_cols);
+        const int deep_parts = deep_accumulators(parts * n_cols, deep_cols);
         for (int ks = 0; ks < k_steps; ++ks) {
           if (!mbar_wait(smem_u32(full + stage), phase, wait_limit)) {
             atomicExch(status, kMmaWait);
@@ -393,7 +428,7 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
           const uint64_t a_desc = desc_k_sw128(smem_u32(smem_a + stage * kABytes));
           const uint64_t b_desc = desc_k_sw128(smem_u32(smem_b + stage * b_slot_bytes));
           const uint64_t sfa_desc = desc_sf(smem_u32(smem_sfa + stage * kSfBytes));
-          const uint64_t sfb_desc = desc_sf(smem_u32(smem_b + (stage + 1) * b_slot_bytes - kSfBytes));
+          const uint64_t sfb_desc = desc_sf(smem_u32(smem_b + (stage + 1) * b_slot_bytes - deep_bytes - kSfBytes));
           const uint32_t sf_set = tmem_base + (sf_turn ^= 1u) * kSfSetCols;
 #pragma unroll
           for (int j = 0; j < kMmaPerStage; ++j) {
@@ -404,6 +439,19 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
           for (int j = 0; j < kMmaPerStage; ++j) {
             umma(acc + (j & (parts - 1)) * n_cols, a_desc + j * 2, b_desc + j * 2, idesc, sf_set + kSfaCol + j * 4,
                  sf_set + kSfbCol + j * 4, (ks * kMmaPerStage + j) >= parts ? 1u : 0u);
+          }
+          if (stage_deep[stage] != 0u) {
+            // The copies overwrite the scale columns of the MMAs above, behind which they stand in the tensor pipe.
+            const uint64_t bd_desc = desc_k_sw128(smem_u32(smem_b + (stage + 1) * b_slot_bytes - deep_bytes));
+            const uint64_t sfd_desc = desc_sf(smem_u32(smem_b + (stage + 1) * b_slot_bytes - kSfBytes));
+#pragma unroll
+            for (int j = 0; j < kMmaPerStage; ++j) utccp_sf(sf_set + kSfbCol + j * 4, sfd_desc + j * (kSfChunk >> 4));
+#pragma unroll
+            for (int j = 0; j < kMmaPerStage; ++j) {
+              umma(acc + parts * n_cols + (j & (deep_parts - 1)) * deep_cols, a_desc + j * 2, bd_desc + j * 2, idesc_deep, sf_set + kSfaCol + j * 4,
+                   sf_set + kSfbCol + j * 4, deep_seen != 0u || j >= deep_parts ? 1u : 0u);
+            }
+            deep_seen = 1;
           }
           umma_commit(smem_u32(empty + stage));
           if (++stage == stages) {
@@ -421,45 +469,68 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
     const int row_in_tile = quarter * 32 + lane;
     STile spill;
     const float * scales_of = nullptr;
-    float scales = 0.0f;  // of token `lane`, read once per projection and before the wait (one load per token cost 1 us a tile)
+    float scales = 0.0f;      // of token `lane`, read once per projection and before the wait (one load per token cost 1 us a tile)
+    uint32_t deep_tokens = 0; // tokens with deep digits; the sums of the others have nothing in those rows
     for (int ti = 0; ti < n_tiles; ++ti) {
       const STile * it = tile_at(ti, spill);
       const uint32_t ab = ti & 1;
       if (it->x_g != scales_of) {
         scales_of = it->x_g;
-        scales = lane < it->tokens ? __ldcg(scales_of + lane) : 0.0f;
+        uint32_t any = 0;
+        if (lane < it->tokens) {
+          scales = __ldcg(scales_of + lane);
+          if (it->x_deep != nullptr) {
+            for (int w = 0; 32 * w < it->k_steps; ++w) any |= __ldcg(it->x_deep + 8 * w + lane);
+          }
+        }
+        deep_tokens = __ballot_sync(0xffffffffu, any != 0u);
       }
       if (!mbar_wait(smem_u32(tmem_full + ab), (ti >> 1) & 1, wait_limit)) {
         if (lane == 0) atomicExch(status, kEpilogueWait);
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const int rows = it->rows, tokens = it->tokens, digits = it->digits, n_cols = it->n_cols;
+      const int rows = it->rows, tokens = it->tokens, digits = it->digits, n_cols = it->n_cols, deep_cols = it->deep_cols;
       const int row = it->row_block * kRows + row_in_tile;
       const bool gate_up = it->epilogue == kEpiGateUp;
       const float s2 = it->s2, s2_up = it->s2_up;
       const uint32_t taddr = tmem_base + ab * kAccBufCols + (static_cast<uint32_t>(quarter * 32) << 16);
-      const int parts = partial_accumulators(n_cols);
+      const int parts = partial_accumulators(n_cols, deep_cols);
+      // the deep digits' sums: columns among the others', or accumulators of their own behind them
+      const uint32_t deep_addr = taddr + (deep_cols > 0 ? parts * n_cols : it->deep_rows);
+      const int deep_stride = deep_cols > 0 ? deep_cols : n_cols, deep_parts = deep_cols > 0 ? deep_accumulators(parts * n_cols, deep_cols) : parts;
       // One token at a time, in a compact loop: a small part of a tile's time as long as its code stays resident (with all
       // columns unrolled a 0.8B-class step of eight tokens took 99 us instead of 54).
 #pragma unroll 1
       for (int token = first_token; token < tokens; token += 2) {
-        uint32_t r[4][8] = {};
-        tmem_ld8(taddr + token * digits, r[0]);  // digits <= 8: what lies behind them is not used
-        if (parts > 1) tmem_ld8(taddr + n_cols + token * digits, r[1]);
-        if (parts > 2) {
-          tmem_ld8(taddr + 2 * n_cols + token * digits, r[2]);
-          tmem_ld8(taddr + 3 * n_cols + token * digits, r[3]);
-        }
+        uint32_t col = taddr + token * digits;
+        int stride = n_cols, count = digits, sums = parts;
         float g = __shfl_sync(0xffffffffu, scales, token);
-        tmem_wait_ld(r);
         float sum = 0.0f, weight = 1.0f;  // of digit j: 8^-j
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          if (j < digits) {
-            sum = fmaf((__uint_as_float(r[0][j]) + __uint_as_float(r[1][j])) + (__uint_as_float(r[2][j]) + __uint_as_float(r[3][j])), weight, sum);
-            weight *= 0.125f;
+#pragma unroll 1
+        for (bool again = (deep_tokens >> token & 1u) != 0u;; again = false) {
+          uint32_t r[4][8] = {};
+          tmem_ld8(col, r[0]);  // digits <= 8: what lies behind them is not used
+          if (sums > 1) tmem_ld8(col + stride, r[1]);
+          if (sums > 2) {
+            tmem_ld8(col + 2 * stride, r[2]);
+            tmem_ld8(col + 3 * stride, r[3]);
           }
+          tmem_wait_ld(r);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            if (j < count) {
+              sum = fmaf((__uint_as_float(r[0][j]) + __uint_as_float(r[1][j])) + (__uint_as_float(r[2][j]) + __uint_as_float(r[3][j])), weight, sum);
+              weight *= 0.125f;
+            }
+          }
+          if (!again) break;
+          // the same code once more for the deep digits: code of its own, seldom run, is fetched from afar every time
+          // (out of line a 0.8B-class step of eight tokens took 71 us)
+          col = deep_addr + token * kDeepDigits;
+          stride = deep_stride;
+          count = kDeepDigits;
+          sums = deep_parts;
         }
         if (g != g) {
           sum = row < rows ? exact_dot(it->item, row, token) : 0.0f;
@@ -527,19 +598,32 @@ __device__ __forceinline__ void from_e2m1x2(uint32_t byte, float & lo, float & h
 
 struct ExpandItem {
   const __nv_bfloat16 * x;   // [tokens, k], k a multiple of 256
-  uint8_t * ops;             // see WItem::x_ops; operand row = token * digits + digit
+  uint8_t * ops;             // see WItem::x_ops; operand row = token * digits + digit, and likewise of the deep digits
+  uint32_t * deep;           // see WItem::x_deep
   float * g;                 // [tokens]: scale of each token's expansion
   int k;
-  int code_bytes;            // of a K step: n_cols * 128
+  int step_bytes;            // of a K step of ops
+  int scales_at;             // its scale tiles
+  int deep_row, deep_at, deep_scales_at;  // the deep digits' first operand row, their codes and scale tiles
 };
 
 constexpr int kSplitThreads = 256;
+constexpr int kDeepWords = 64;   // of 32 K steps each: 524288 columns, more than a list on either path can have
 
 // One CTA per (projection, token).  A block of sixteen values whose largest has exponent e is counted in units of
 // 2^(e - 1), which makes every value less than 4: digit 0 is the nearest E2M1 number (up to 4 the grid is no coarser than
 // 1, so at most half a unit is left over), digit 1 the nearest to eight times the rest, and so on; all of it is exact in
 // fp32.  The unit goes into the block's scale byte, a power of two relative to the token's largest exponent (down to 2^-17
-// of it, the range of E4M3), and 8^-j into the epilogue.  Eight digits leave at most 2^-24 of the block's binade.
+// of it, the range of E4M3), and 8^-j into the epilogue.  d digits leave at most 2^(e + 1 - 3 d), and nothing of a value
+// whose last bit is not below 2^(e + 2 - 3 d).
+// With deep digits (a list that has to be as exact as BF16 activations converted to fp16 by one power of two per token,
+// which keep multiples of 2^-38 of the token's largest binade): where the first eight leave something of any value of a K
+// step, six more are written, fourteen in all, which hold multiples of 2^-40 of the block's largest binade; the step is
+// marked in the token's mask.  A step that was marked in the run before and is not any more gets zero scales there, since
+// another token's deep digits may be used in it.  A warp takes one K step at a time.
+// The deep digits cost one microsecond here with one token (4.9 -> 5.9 us; with eight the wider unrolling gives it back, 9.9
+// -> 9.1) and about one in the projection.  In runs of 0.2 s, us: 0.8B-class step one token 44.2 -> 45.5, eight 54.4 -> 54.9,
+// 4B-class one 305 -> 308, four 335 -> 339; always fourteen digits: 45.7, 68, 308 and 362.
 // A token with an infinity or a NaN gets NaN for its scale if `propagate`, and the epilogue works its outputs out from the
 // activations; else such elements count as zero.
 __global__ void __launch_bounds__(kSplitThreads) split_digits_kernel(const ExpandItem * __restrict__ items, int digits, int propagate) {
@@ -549,6 +633,8 @@ __global__ void __launch_bounds__(kSplitThreads) split_digits_kernel(const Expan
   const int token = blockIdx.y, k = it.k, chunks = k >> 3;
   const uint4 * src = reinterpret_cast<const uint4 *>(it.x + static_cast<size_t>(token) * k);
   __shared__ uint32_t red[kSplitThreads / 32];
+  __shared__ uint32_t deep_now[kDeepWords], deep_before[kDeepWords];
+  const int words = (chunks + 1023) >> 10;
   auto load = [&](int c) {
     uint4 q = __ldca(src + c);
     if (!propagate) {
@@ -567,10 +653,15 @@ __global__ void __launch_bounds__(kSplitThreads) split_digits_kernel(const Expan
     return max(a & 0xffffu, a >> 16);
   };
   asm volatile("griddepcontrol.wait;" ::: "memory");  // the activations may come from the kernel before
-  uint32_t best = 0;
+  uint32_t best = 0, before = 0;
+  if (it.deep != nullptr && static_cast<int>(threadIdx.x) < words) before = __ldcg(it.deep + 8 * threadIdx.x + token);
   for (int c = threadIdx.x; c < chunks; c += kSplitThreads) best = max(best, abs_max(load(c)));
   best = __reduce_max_sync(0xffffffffu, best);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = best;
+  if (threadIdx.x < kDeepWords) {
+    deep_before[threadIdx.x] = before;
+    deep_now[threadIdx.x] = 0u;
+  }
   __syncthreads();
 #pragma unroll
   for (int i = 0; i < kSplitThreads / 32; ++i) best = max(best, red[i]);
@@ -593,12 +684,11 @@ __global__ void __launch_bounds__(kSplitThreads) split_digits_kernel(const Expan
       v[2 * i] = __uint_as_float(r[i] << 16) * scale;
       v[2 * i + 1] = __uint_as_float(r[i] & 0xffff0000u) * scale;
     }
-    uint8_t * step = it.ops + static_cast<size_t>(c >> 5) * (it.code_bytes + kSfBytes);
-    int row = token * digits;
-    for (int j = 0; j < digits; ++j) {
+    uint8_t * step = it.ops + static_cast<size_t>(c >> 5) * it.step_bytes;
+    // writes the next digit as an operand row
+    auto write_digit = [&](uint8_t * codes, int row) {
       const uint32_t w = to_e2m1x8(v);
-      *reinterpret_cast<uint32_t *>(step + row * kStepBytes + ((((c >> 2) ^ row) & 7) << 4) + ((c & 3) << 2)) = w;
-      ++row;
+      *reinterpret_cast<uint32_t *>(codes + row * kStepBytes + ((((c >> 2) ^ row) & 7) << 4) + ((c & 3) << 2)) = w;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         float d0, d1;
@@ -606,7 +696,7 @@ __global__ void __launch_bounds__(kSplitThreads) split_digits_kernel(const Expan
         v[2 * i] = (v[2 * i] - d0) * 8.0f;
         v[2 * i + 1] = (v[2 * i + 1] - d1) * 8.0f;
       }
-    }
+    };
     // E4M3 byte of 2^(8 + e - top); the four blocks of eight lanes make one word of the tiled layout, the same for every digit
     const int s = 8 + e - top;
     const uint32_t byte = s >= -6 ? static_cast<uint32_t>(s + 7) << 3 : 8u >> (-6 - s);
@@ -614,8 +704,31 @@ __global__ void __launch_bounds__(kSplitThreads) split_digits_kernel(const Expan
     word |= __shfl_xor_sync(0xffffffffu, word, 2);
     word |= __shfl_xor_sync(0xffffffffu, word, 4);
     const int j = threadIdx.x & 7;
-    row = token * digits + j;
-    if (j < digits) *reinterpret_cast<uint32_t *>(step + it.code_bytes + ((c >> 3) & 3) * kSfChunk + (row & 31) * 16 + (row >> 5) * 4) = word;
+    auto write_scales = [&](uint8_t * tiles, int row, int count, uint32_t value) {
+      if (j < count) *reinterpret_cast<uint32_t *>(tiles + ((c >> 3) & 3) * kSfChunk + ((row + j) & 31) * 16 + ((row + j) >> 5) * 4) = value;
+    };
+    for (int i = 0; i < digits; ++i) write_digit(step, token * digits + i);
+    write_scales(step + it.scales_at, token * digits, digits, word);
+    if (it.deep != nullptr) {
+      uint32_t rest = 0;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) rest |= __float_as_uint(v[i]);
+      const int row = it.deep_row + token * kDeepDigits;
+      const int at = c >> 10, bit = c >> 5 & 31;
+      if (__any_sync(0xffffffffu, (rest & 0x7fffffffu) != 0u)) {
+#pragma unroll 1
+        for (int i = 0; i < kDeepDigits; ++i) write_digit(step + it.deep_at, row + i);
+        write_scales(step + it.deep_scales_at, row, kDeepDigits, word);
+        if ((threadIdx.x & 31) == 0) atomicOr(deep_now + at, 1u << bit);
+      } else if ((deep_before[at] >> bit & 1u) != 0u) {
+        // zero scales again: in this step another token's deep digits may be used
+        write_scales(step + it.deep_scales_at, row, kDeepDigits, 0u);
+      }
+    }
+  }
+  if (it.deep != nullptr) {
+    __syncthreads();
+    if (static_cast<int>(threadIdx.x) < words && deep_now[threadIdx.x] != before) it.deep[8 * threadIdx.x + token] = deep_now[threadIdx.x];
   }
 }
 
@@ -642,7 +755,7 @@ int ensure_attr() {
 // ---- decode work list on the tensor path ------------------------------------------------------------------------
 
 struct WBatch {
-  int count = 0, m = 0, digits = 0, grid = 0, stages = 0, b_slot = 0, smem = 0;
+  int count = 0, m = 0, digits = 0, grid = 0, stages = 0, b_slot = 0, deep_bytes = 0, smem = 0;
   void * dev_base = nullptr;
   WItem * items = nullptr;
   WTile * tiles = nullptr;
@@ -650,11 +763,11 @@ struct WBatch {
   ExpandItem * expand = nullptr;
   unsigned int * status = nullptr;
   size_t bytes_per_run = 0;
-  bool propagate = false;   // infinities and NaNs of the activations reach the outputs
+  bool exact = false;       // all bits of the activations, their infinities and NaNs too, reach the outputs
   uint32_t wait_limit = kWaitLimit;
 };
 
-int wbatch_build(const q35b_gemv_item * items, int count, int m, int digits, bool propagate, WBatch ** out) {
+int wbatch_build(const q35b_gemv_item * items, int count, int m, int digits, bool exact, WBatch ** out) {
   if (items == nullptr || out == nullptr || count <= 0) return fail(Q35B_ERR_ARGUMENT, "Invalid NVFP4 projection work list.");
   *out = nullptr;
   if (m < 1 || m > 8) return fail(Q35B_ERR_SHAPE, "NVFP4 decode projection supports 1..8 tokens.");
@@ -686,10 +799,13 @@ int wbatch_build(const q35b_gemv_item * items, int count, int m, int digits, boo
   b->count = count;
   b->m = m;
   b->digits = digits;
-  b->propagate = propagate;
+  b->exact = exact;
   const int op_rows = m * digits;
   const int n_cols = round_up_int(op_rows, 16);
-  b->b_slot = n_cols * kStepBytes + kSfBytes;
+  const bool inside = exact && m * (digits + kDeepDigits) <= n_cols;  // the deep digits' rows fit into the padding (one token)
+  const int deep_cols = exact && !inside ? round_up_int(m * kDeepDigits, 16) : 0;
+  b->deep_bytes = deep_cols > 0 ? deep_cols * kStepBytes + kSfBytes : 0;
+  b->b_slot = n_cols * kStepBytes + kSfBytes + b->deep_bytes;
   b->stages = plan_stages(b->b_slot);
   b->smem = smem_for(b->stages, b->b_slot);
 
@@ -725,12 +841,14 @@ int wbatch_build(const q35b_gemv_item * items, int count, int m, int digits, boo
   const size_t o_expand = up(o_begin + sizeof(int) * (grid + 1), 256);
   const size_t o_status = up(o_expand + sizeof(ExpandItem) * count, 256);
   size_t o_data = o_status + 256;
-  std::vector<size_t> o_ops(count), o_g(count);
+  std::vector<size_t> o_ops(count), o_g(count), o_deep(count);
   for (int i = 0; i < count; ++i) {
     o_ops[i] = o_data;
     o_data = up(o_data + static_cast<size_t>(items[i].weight->k / 256) * b->b_slot, 256);
     o_g[i] = o_data;
     o_data += 256;
+    o_deep[i] = o_data;
+    if (exact) o_data = up(o_data + static_cast<size_t>((items[i].weight->k / 256 + 31) / 32) * 32, 256);
   }
   cudaError_t e = cudaMalloc(&b->dev_base, o_data);
   if (e != cudaSuccess) {
@@ -752,6 +870,7 @@ int wbatch_build(const q35b_gemv_item * items, int count, int m, int digits, boo
     it.tmap_w = w->tmap_codes_128;
     it.w_scales = w->scales_tiled;
     it.x_ops = base + o_ops[i];
+    it.x_deep = exact ? reinterpret_cast<const uint32_t *>(base + o_deep[i]) : nullptr;
     it.x_g = reinterpret_cast<const float *>(base + o_g[i]);
     it.w_codes = w->codes;
     it.x = static_cast<const __nv_bfloat16 *>(items[i].x_bf16);
@@ -760,6 +879,8 @@ int wbatch_build(const q35b_gemv_item * items, int count, int m, int digits, boo
     it.rows = w->rows;
     it.k_steps = w->k / 256;
     it.n_cols = n_cols;
+    it.deep_cols = deep_cols;
+    it.deep_rows = inside ? op_rows : 0;
     it.tokens = m;
     it.digits = digits;
     it.ldy = w->gate_up ? w->rows / 2 : w->rows;
@@ -767,8 +888,11 @@ int wbatch_build(const q35b_gemv_item * items, int count, int m, int digits, boo
     it.s2 = w->s2;
     it.s2_up = w->s2_up;
     it.epilogue = w->gate_up ? kEpiGateUp : kEpiPlain;
-    h_expand[i] = ExpandItem{static_cast<const __nv_bfloat16 *>(items[i].x_bf16), base + o_ops[i], reinterpret_cast<float *>(base + o_g[i]),
-                             w->k, n_cols * kStepBytes};
+    h_expand[i] = ExpandItem{static_cast<const __nv_bfloat16 *>(items[i].x_bf16), base + o_ops[i],
+                             exact ? reinterpret_cast<uint32_t *>(base + o_deep[i]) : nullptr,
+                             reinterpret_cast<float *>(base + o_g[i]), w->k, b->b_slot, n_cols * kStepBytes, inside ? op_rows : 0,
+                             inside ? 0 : n_cols * kStepBytes + kSfBytes,
+                             inside ? n_cols * kStepBytes : (n_cols + deep_cols) * kStepBytes + kSfBytes};
   }
   e = cudaMemset(b->dev_base, 0, o_data);
   if (e == cudaSuccess) e = cudaMemcpy(b->items, h_items.data(), sizeof(WItem) * count, cudaMemcpyHostToDevice);
@@ -788,12 +912,12 @@ int wbatch_launch(const WBatch * b, cudaStream_t s) {
   // 1. the digits of every item's activations (one CTA per item and token); 2. the streaming kernel, whose weight
   // producer starts at once while its activation producer waits for the expansion
   cudaError_t le = launch_pdl(split_digits_kernel, dim3(b->count, b->m), dim3(kSplitThreads), 0, s,
-                              static_cast<const ExpandItem *>(b->expand), b->digits, b->propagate ? 1 : 0);
+                              static_cast<const ExpandItem *>(b->expand), b->digits, b->exact ? 1 : 0);
   count_launch();
   Q35B_CUDA_TRY(le, "split_digits_kernel launch");
   le = launch_pdl(gemm_wstream_kernel, dim3(b->grid), dim3(kThreads), static_cast<size_t>(b->smem), s,
                   static_cast<const WItem *>(b->items), static_cast<const WTile *>(b->tiles), static_cast<const int *>(b->cta_begin),
-                  b->stages, b->b_slot, b->status, b->wait_limit);
+                  b->stages, b->b_slot, b->deep_bytes, b->status, b->wait_limit);
   count_launch();
   Q35B_CUDA_TRY(le, "gemm_wstream_kernel launch");
   return Q35B_OK;

@@ -1009,7 +1009,7 @@ Assignment assign_tiles(const std::vector<GemvTile> & all, const std::vector<int
 // 111 / 91, 124 / 98; 1.8 GiB 348 / 304, 395 / 332, 443 / 359.  The line: 115 MiB one token 29.8 / 31.3, two 31.1 / 31.4,
 // four 34.9 / 31.9, eight 35.4 / 33.4; 111 MiB one token 26.4 / 24.9; 56 MiB one token 16.2 / 15.7, four 17.6 / 17.0, eight
 // 21.6 / 19.6.
-constexpr int kTensorDigits = 8;  // three bits each: BF16's eight below the largest value of a block and sixteen further down
+constexpr int kTensorDigits = 8;  // three bits each, and more of them where a value needs them (gemm_wstream.cu)
 constexpr size_t kTensorBytes = 128u << 20, kTensorBytesFrom4 = 48u << 20;  // up to three tokens, and from four on
 
 bool tensor_list(const q35b_gemv_item * items, int count, int m) {

@@ -358,7 +358,8 @@ class GemvBatch:
 
     def __init__(self, items, m: int, digits: int = 0):
         """digits > 0: run the list on the tensor cores with every token's activations expanded into that many NVFP4
-        digit rows (q35b_gemv_batch_create_tensor; 5 is the intended setting); 0: BF16 activations carried exactly."""
+        digit rows, 2^(1 - 3 digits) of a block's largest value (q35b_gemv_batch_create_tensor); 0: the library chooses the
+        path, and the activations are exact down to 2^-39 of a token's largest value (q35b_gemv_batch_create)."""
         torch = _torch()
         self._keep = list(items)
         arr = (_GemvItem * len(self._keep))()

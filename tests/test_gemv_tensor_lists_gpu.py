@@ -1,8 +1,8 @@
-"""Large decode lists run on the tensor cores with every BF16 activation split into eight octal NVFP4 digits
-(gemm_wstream.cu).  A value keeps all it has within 2^-23 of its block's largest, so the outputs are those of 64-bit sums of
-the same products to fp32 accuracy: after the BF16 rounding they differ in flipped roundings only, relative L2 below 2e-4
-(a result flips where the fp32 error, some 2^-22 of the terms' size, spans a rounding boundary 2^-9 wide: a few in 10^4
-values by one step of 2^-8)."""
+"""Large decode lists run on the tensor cores with every BF16 activation split into octal NVFP4 digits (gemm_wstream.cu): eight
+of them, and six deep ones in the K steps where a value needs them.  No value loses anything down to 2^-38 of its token's
+largest, so the outputs are those of 64-bit sums of the same products to fp32 accuracy: after the BF16 rounding they differ
+in flipped roundings only, relative L2 below 2e-4 (a result flips where the fp32 error, some 2^-22 of the terms' size, spans
+a rounding boundary 2^-9 wide: a few in 10^4 values by one step of 2^-8)."""
 import numpy as np
 import pytest
 
@@ -73,6 +73,63 @@ def test_outputs(engine, m):
     _run(engine, torch, items, m)
     for item, e in list(zip(items, want))[1:]:
         assert _rel(item[2], e) <= 2e-4, item[0].rows
+
+
+def _below(torch, gen, m, k, where, depth):
+    """Activations N(0, 1) whose columns `where` are 2^-depth of the token's largest value, which is a power of two."""
+    x = torch.randn((m, k), device="cuda", generator=gen).clamp_(-3.9, 3.9)
+    x[:, 0] = 4.0
+    x[:, where] = torch.sign(x[:, where]) * (1.0 + torch.rand((m, len(where)), device="cuda", generator=gen)) * 2.0 ** (2 - depth)
+    return x.to(torch.bfloat16)
+
+
+# depth: of the values that decide the outputs, in powers of two below the token's largest; two K steps, and so many that the
+# words that name the deep ones are more than one and more than a producer's 128 steps
+@pytest.mark.parametrize("m", range(1, 9))
+@pytest.mark.parametrize("k", [512, 9216, 33280])
+def test_small_values_beside_large_ones_keep_their_bits(engine, m, k):
+    """Weight rows that are zero except at small activations, which stand in the blocks of the large ones or in blocks of
+    their own: every output for itself, against 64 bits.  An output is exact up to fp32 sums of a few terms, 2^-20 of their
+    magnitudes, and its own BF16 rounding, half of a step of 2^-7 of its binade and so 2^-8 of it at most.  Some tokens of a list have such values and others have not, in this run and the one before."""
+    import torch
+
+    if m * (k + 32) * 2 > 150_000:
+        k = 9216 - 256
+    gen = torch.Generator(device="cuda").manual_seed(100 * m + k)
+    blocks = k // 16
+    inside = torch.arange(5, k, 16, device="cuda")[torch.randperm(blocks, device="cuda", generator=gen)[: blocks // 2]]
+    alone = torch.arange(32, 48, device="cuda")
+    rows = 130
+    items, checks = [_filler(engine, torch, gen, m)], []
+    for depth in (9, 15, 16, 17, 20, 24, 28, 31):
+        for where in (inside, alone):
+            codes = torch.zeros((rows, k), dtype=torch.uint8, device="cuda")
+            # one to three of the small columns per row, in places that no other row shares
+            pick = torch.randint(0, len(where), (rows, 3), device="cuda", generator=gen)
+            codes.scatter_(1, where[pick], torch.randint(1, 8, (rows, 3), dtype=torch.uint8, device="cuda", generator=gen))
+            packed = codes[:, 0::2] | codes[:, 1::2] << 4
+            scales = torch.full((rows, k // 16), 0x38, dtype=torch.uint8, device="cuda")
+            w = engine.Nvfp4Weight.from_device(packed.contiguous(), scales, 1.0)
+            x = _below(torch, gen, m, k, where, depth)
+            if m > 1:
+                x[1::2] = torch.randint(-3, 4, (len(range(1, m, 2)), k), device="cuda", generator=gen).to(torch.bfloat16)
+            y = torch.zeros((m, rows), dtype=torch.bfloat16, device="cuda")
+            items.append((w, x, y))
+            table = torch.tensor(E2M1, dtype=torch.float64, device="cuda")
+            checks.append((x, y, table[codes.long()]))
+    batch = engine.GemvBatch(items, m)
+    before = engine.launch_count()
+    for turn in range(3):
+        batch.run()
+        torch.cuda.synchronize()
+        assert engine.launch_count() - before == 2 * (turn + 1) and batch.status() == 0
+        for x, y, wd in checks:
+            want = x.double() @ wd.T
+            # the few terms of an output have the same size, so it is not far below their sum of magnitudes
+            bound = 2.0 ** -8 * want.abs() + 2.0 ** -20 * (x.double().abs() @ wd.T)
+            assert bool(((y.double() - want).abs() <= bound).all()), (turn, (y.double() - want).abs().max().item())
+            if m > 1:
+                x.copy_(x.roll(1, 0))  # other tokens have the small values in the next run
 
 
 @pytest.mark.parametrize("m", [1, 4])
