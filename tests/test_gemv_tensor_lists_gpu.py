@@ -197,3 +197,74 @@ def test_activations_too_large_for_the_other_kernel_stay_refused(engine):
     with pytest.raises(engine.Q35bError) as e:
         engine.GemvBatch(items, m)
     assert e.value.status == 2
+
+
+@pytest.mark.parametrize("m", [1, 3, 8])
+def test_outputs_of_infinities(engine, m):
+    """An infinity times a weight is one of that sign, or a NaN where the weight or its block's scale is zero; two of opposite
+    signs are a NaN.  Rows around a warp's 32, the first and last columns, infinities in every column, one and two K steps."""
+    import torch
+
+    gen = torch.Generator(device="cuda").manual_seed(17 + m)
+    inf = float("inf")
+    items, want = [_filler(engine, torch, gen, m)], []
+    for j, (n, k) in enumerate([(33, 256), (127, 512), (160, 2560), (65, 512)]):
+        codes = torch.randint(0, 256, (n, k // 2), dtype=torch.uint8, device="cuda", generator=gen)
+        scales = torch.randint(0, 0x7f, (n, k // 16), dtype=torch.uint8, device="cuda", generator=gen)
+        x = torch.randn((m, k), device="cuda", generator=gen)
+        if j == 0:
+            x[0, 0], x[m - 1, k - 1] = inf, -inf
+        elif j == 1:
+            codes = codes % 7 * 16 + codes % 5 + 0x11 & 0x77  # no weight is zero or negative
+            scales.clamp_(min=1)
+            x[m - 1] = inf
+            x[0, 300:] = -inf
+        elif j == 2:
+            scales[:, ::3] = 0
+            x[m // 2, torch.randint(0, k, (3,), device="cuda", generator=gen)] = inf
+            x[m // 2, 16 * 3] = -inf                           # under a scale of zero
+        else:
+            x[m - 1, 5], x[m - 1, 6], x[0, 7] = inf, float("nan"), -inf
+        if j == 1 and m == 1:
+            x[0] = inf
+        table = torch.tensor(E2M1 + [-v for v in E2M1], dtype=torch.float64, device="cuda")
+        sb = scales.to(torch.int64)
+        decoded = torch.where(sb < 8, (sb & 7) * 2.0 ** -9, (8 + (sb & 7)) * torch.pow(2.0, ((sb >> 3) - 10).double()))
+        w = torch.stack([table[(codes & 15).long()], table[(codes >> 4).long()]], dim=2).view(n, k)
+        x = x.to(torch.bfloat16)
+        y = torch.zeros((m, n), dtype=torch.bfloat16, device="cuda")
+        items.append((engine.Nvfp4Weight.from_device(codes.contiguous(), scales, 1.0), x, y))
+        # products one by one: a matrix product may skip what it multiplies by zero
+        want.append(((x.double()[:, None] * w[None]) * decoded.repeat_interleave(16, dim=1)[None]).sum(2))
+    _run(engine, torch, items, m)
+    for (_, x, y), e in zip(items[1:], want):
+        bad = ~torch.isfinite(e)
+        assert bool(bad.any()) and bool(torch.equal(torch.isnan(e), torch.isnan(y)))
+        assert bool((y.double()[bad & ~torch.isnan(e)] == e[bad & ~torch.isnan(e)]).all())
+        for t in range(m):
+            if not bool(bad[t].any()):
+                assert _rel(y[t], e[t]) <= 2e-4
+
+
+def test_infinities_and_nans_cost_little(engine):
+    """A list with such tokens takes about as long as one without; a serial sum over all columns per output took 10 times that."""
+    import torch
+
+    m, gen = 8, torch.Generator(device="cuda").manual_seed(3)
+    w, x, y = _filler(engine, torch, gen, m)
+    batch = engine.GemvBatch([(w, x, y)], m)
+
+    def run():
+        a, b = torch.cuda.Event(True), torch.cuda.Event(True)
+        batch.run()
+        a.record()
+        for _ in range(20):
+            batch.run()
+        b.record()
+        b.synchronize()
+        return a.elapsed_time(b)
+
+    finite = min(run() for _ in range(3))
+    x[:, 1000] = float("inf")
+    x[0, 1000] = float("nan")
+    assert min(run() for _ in range(3)) <= 4 * finite and batch.status() == 0
