@@ -23,7 +23,8 @@
 // (src/kernels/cuda/decode_layers.cuh:200-284) with the FP4 decode done by the tensor core instead of by conversion
 // instructions: a fifth of gemv_stream.cu's instructions, so a long run of steps does not meet the power cap.
 //
-// Every wait is bounded; an expired wait records a code in *status and the role stops; the CTA still frees TMEM.
+// Every wait is bounded; an expired wait records a code in *status and the role stops.  The CTA then waits (again with a
+// limit) for the copies and MMAs that it has under way, and frees its TMEM.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -52,6 +53,7 @@ constexpr int kSfaCol = 2 * kAccBufCols;   // ... and two sets of scale-factor c
 constexpr int kSfbCol = kSfaCol + 16;      // so that the copies of one stage do not wait for the MMAs of the one before
 constexpr int kSfSetCols = 32;
 constexpr uint32_t kWaitLimit = 1u << 22;
+constexpr uint32_t kDrainLimit = 1u << 22;  // polls for what is still under way after an expired wait, however short that one's limit was
 constexpr int kSmemBudget = 220 * 1024;   // dynamic part; the staged tile descriptors are static shared memory
 
 enum StatusCode : unsigned { kWeightWait = 41, kActWait = 42, kMmaWait = 43, kMmaDrainWait = 44, kEpilogueWait = 45 };
@@ -273,9 +275,13 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
   uint64_t * empty = bars + kMaxStages;             // [stages]: the MMAs that read the stage have retired
   uint64_t * tmem_full = bars + 2 * kMaxStages;     // [2]: accumulator complete
   uint64_t * tmem_empty = tmem_full + 2;            // [2]: the epilogue warps have read the accumulator out
-  uint32_t * tmem_slot = reinterpret_cast<uint32_t *>(tmem_empty + 2);
+  uint64_t * mma_done = tmem_empty + 2;             // after an expired wait: every MMA issued has retired
+  uint32_t * tmem_slot = reinterpret_cast<uint32_t *>(mma_done + 1);
   __shared__ STile stile[kMaxTilesInSmem];
   __shared__ uint32_t stage_deep[kMaxStages];              // the stage's step has deep digits; set before its bytes are asked for
+
+  __shared__ uint32_t gave_up;                             // some role of this CTA has
+  __shared__ uint32_t issued[2];                           // K steps whose weights, and whose activations, were asked for
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -329,6 +335,9 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
       mbar_init(smem_u32(tmem_full + i), 1);
       mbar_init(smem_u32(tmem_empty + i), kEpilogueWarps);
     }
+    mbar_init(smem_u32(mma_done), 1);
+    gave_up = 0;
+    issued[0] = issued[1] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -349,7 +358,7 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
     // ------------------------------------------------------------ weight producer (constant data: no wait)
     if (elect_one()) {
       int stage = 0;
-      uint32_t phase = 0;
+      uint32_t phase = 0, steps = 0;
       bool ok = true;
       STile spill;
       for (int ti = 0; ti < n_tiles && ok; ++ti) {
@@ -359,6 +368,7 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
         for (int ks = 0; ks < k_steps; ++ks) {
           if (!mbar_wait(smem_u32(empty + stage), phase ^ 1, wait_limit)) {
             atomicExch(status, kWeightWait);
+            gave_up = 1;
             ok = false;
             break;
           }
@@ -366,6 +376,7 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
           mbar_expect_tx(bar, kABytes + kSfBytes);
           tma_load_2d(smem_u32(smem_a + stage * kABytes), it->tmap_w, bar, ks * kStepBytes, rb * kRows);
           bulk_load(smem_u32(smem_sfa + stage * kSfBytes), sf + static_cast<size_t>(ks) * kSfBytes, kSfBytes, bar);
+          issued[0] = ++steps;
           if (++stage == stages) {
             stage = 0;
             phase ^= 1;
@@ -377,7 +388,7 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
     // ------------------------------------------------------------ activation producer
     asm volatile("griddepcontrol.wait;" ::: "memory");
     int stage = 0;
-    uint32_t phase = 0;
+    uint32_t phase = 0, steps = 0;
     bool ok = true;
     STile spill;
     const uint32_t * deep_of = nullptr;
@@ -399,6 +410,7 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
           for (int i = 0; i < min(k_steps - base, 32); ++i) {
             if (!mbar_wait(smem_u32(empty + stage), phase ^ 1, wait_limit)) {
               atomicExch(status, kActWait);
+              gave_up = 1;
               ok = false;
               break;
             }
@@ -407,6 +419,7 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
             stage_deep[stage] = has;
             mbar_expect_tx(bar, bytes);
             bulk_load(smem_u32(smem_b + stage * b_slot_bytes), ops + static_cast<size_t>(i) * b_slot_bytes, bytes, bar);
+            issued[1] = ++steps;
             if (++stage == stages) {
               stage = 0;
               phase ^= 1;
@@ -435,6 +448,7 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
         const uint32_t ab = ti & 1;
         if (!mbar_wait(smem_u32(tmem_empty + ab), ((ti >> 1) & 1) ^ 1, wait_limit)) {
           atomicExch(status, kMmaDrainWait);
+          gave_up = 1;
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -444,6 +458,7 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
         for (int ks = 0; ks < k_steps; ++ks) {
           if (!mbar_wait(smem_u32(full + stage), phase, wait_limit)) {
             atomicExch(status, kMmaWait);
+            gave_up = 1;
             ok = false;
             break;
           }
@@ -509,7 +524,10 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
         deep_tokens = __ballot_sync(0xffffffffu, any != 0u);
       }
       if (!mbar_wait(smem_u32(tmem_full + ab), (ti >> 1) & 1, wait_limit)) {
-        if (lane == 0) atomicExch(status, kEpilogueWait);
+        if (lane == 0) {
+          atomicExch(status, kEpilogueWait);
+          gave_up = 1;
+        }
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -580,12 +598,22 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
     }
   }
 
-  // after an expired wait some of this CTA's copies may still be under way: give them 100 us before its memory is let go
-  if (threadIdx.x == 0 && *reinterpret_cast<volatile unsigned int *>(status) != 0u) {
-    for (int i = 0; i < 1000; ++i) __nanosleep(100);
-  }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (gave_up != 0) {
+    // Nothing is issued any more.  What was issued lands in this CTA's memory, so it has to land before the CTA ends: the
+    // thread that issued the MMAs waits for them, and another one for the copies.  A step that one producer asked for and the
+    // other did not lacks an arrival at its barrier; the ring is never more than one turn ahead of the slower producer.
+    if (warp == 1 && elect_one()) {
+      umma_commit(smem_u32(mma_done));
+      mbar_wait(smem_u32(mma_done), 0, kDrainLimit);
+    } else if (warp == 0 && elect_one()) {
+      const int first = static_cast<int>(min(issued[0], issued[1])), last = static_cast<int>(max(issued[0], issued[1]));
+      for (int n = first; n < last; ++n) mbar_arrive(smem_u32(full + n % stages));
+      for (int n = max(last - stages, 0); n < last; ++n) mbar_wait(smem_u32(full + n % stages), (n / stages) & 1, kDrainLimit);
+    }
+    __syncthreads();
+  }
   if (warp == 1) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
                  "r"(static_cast<uint32_t>(kTmemCols))
