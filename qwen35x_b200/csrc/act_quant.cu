@@ -323,10 +323,15 @@ quantize_activations_kernel(const T * __restrict__ x, uint32_t scale_cols, const
         __threadfence();
         unsigned int here = atomicAdd(ws + 1, 1u) + 1u;
         for (int i = 0; here < parts && i < kAmaxPolls; ++i) asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(here) : "l"(ws + 1) : "memory");
+        // the counts only order what a fence stands on either side of: every maximum comes before its arrival and this read
+        // after all arrivals (the last to arrive has not polled), and this read before leaving and the reset after all have left
+        __threadfence();
         float amax = -1.0f;
         if (here >= parts) amax = __uint_as_float(*reinterpret_cast<volatile unsigned int *>(ws));
         shared_amax = amax;
+        __threadfence();
         if (atomicAdd(ws + 2, 1u) == parts - 1u) {  // all have added theirs and read the result
+          __threadfence();
           ws[0] = 0u;
           ws[1] = 0u;
           ws[2] = 0u;
