@@ -366,6 +366,9 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
         const int k_steps = it->k_steps, rb = it->row_block;
         const uint8_t * sf = it->w_scales;
         for (int ks = 0; ks < k_steps; ++ks) {
+          // the first turn of the ring was free; from here on it depends on the activations, which an earlier kernel may take
+          // any time to deliver, and a bounded wait must not
+          if (steps == static_cast<uint32_t>(stages)) asm volatile("griddepcontrol.wait;" ::: "memory");
           if (!mbar_wait(smem_u32(empty + stage), phase ^ 1, wait_limit)) {
             atomicExch(status, kWeightWait);
             gave_up = 1;
@@ -436,6 +439,7 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
     // cycles, its bytes 800 to come from HBM.  The issuing threads are chosen with elect.sync: by a test of the lane number
     // the same code took 600 ns per stage (0.8B-class step of one token 73 us instead of 44).
     if (elect_one()) {
+      asm volatile("griddepcontrol.wait;" ::: "memory");  // no bounded wait for activations before they can be there
       int stage = 0;
       uint32_t phase = 0, sf_turn = 0;
       bool ok = true;
