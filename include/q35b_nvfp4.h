@@ -231,6 +231,11 @@ Q35B_API size_t q35b_gemv_batch_stream_bytes(const q35b_gemv_batch * batch);
  * src/runtime/cuda_bench.cu:2616-2619). */
 Q35B_API size_t q35b_act_codes_bytes(int m, int k);
 Q35B_API size_t q35b_act_scales_bytes(int m, int k);
+/* Test hook: q35b_quantize_nvfp4_bf16 with global_scale 0 whose CTAs look `polls` times for the others' maxima, of which there
+ * are `absent` fewer than they wait for, and then `help_polls` times for the CTAs that work the absent ones' shares out.  The
+ * bytes are the same whatever these are. */
+Q35B_API int q35b_debug_quantize_wait(const void * x_bf16, int m, int k, uint8_t * codes, uint8_t * scales_tiled, float * input_scale_dev,
+                                      void * workspace, int polls, int help_polls, unsigned int absent, q35b_stream stream);
 /* Bytes of the quantiser's workspace; must be zero before its first use and
  * is left zero by every call. */
 Q35B_API size_t q35b_quant_workspace_bytes(void);

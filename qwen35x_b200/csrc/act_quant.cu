@@ -162,7 +162,11 @@ quantize_nvfp4_kernel(const T * __restrict__ x, int rows, int rows_padded, int k
 // [4096, 9216] 48.7 -> 33.5; with a given scale 1.9 -> 1.6, 2.5 -> 2.1, 10.2 -> 7.0, 30.7 -> 18.9; fp32 [1000, 1024] 7.9 -> 5.4.
 constexpr int kActCtas = 4;          // per SM
 constexpr int kHold = 2;             // blocks a thread keeps in registers between the two passes
-constexpr int kAmaxPolls = 1 << 12;  // looks at the arrival count (a few ms) before a CTA works out the amax alone
+// Looks at the arrival counts, some 0.7 us each, before a CTA stops waiting for the others, and then for the ones that help.
+struct AmaxWait {
+  int polls = 64, help_polls = 1 << 12;
+  unsigned int absent = 0;  // test hook: arrivals demanded on top of what the grid delivers
+};
 
 // Block slots of a tiled activation: `slots` (a multiple of four) per row, numbered through the rows.
 struct SlotMap {
@@ -243,19 +247,23 @@ __device__ __forceinline__ void emit(Idx slot, bool in, const uint4 (&r)[sizeof(
 // 32-bit word of the tiled layout.  Slots past K and rows past `rows` only produce zero scale bytes.
 // DYNAMIC: the grid (never more CTAs than are resident together) reads everything once, meets at a counter, and quantises
 // what it has kept in registers (the first kHold blocks of a thread) or reads again from L2.  No CTA depends on the others
-// being there: one that has polled kAmaxPolls times for them takes the maximum over the whole tensor by itself.
-// ws: [0] running maximum (fp32 bits), [1] CTAs that have added theirs, [2] CTAs that have read it; all zero between calls.
+// being there (kernels of other streams may hold their places for as long as they like): those that have waited some 45 us
+// deal the whole tensor out among themselves, a CTA's share at a time, so that the amax costs one more pass over it and not
+// one per CTA; and one that has waited much longer for these takes the maximum over everything by itself.
+// ws: [0] running maximum (fp32 bits), [1] CTAs that have added theirs, [2] CTAs that have read it, [3] shares dealt out,
+// [4] shares added; all zero between calls.
 // Idx: type of a slot index, 32 bits up to 2^31 slots.
 template <typename T, bool DYNAMIC, typename Idx>
 __global__ void __launch_bounds__(kThreads, kActCtas)
 quantize_activations_kernel(const T * __restrict__ x, uint32_t scale_cols, const SlotMap map, Idx live, Idx total, float g_fixed,
-                            unsigned int parts, unsigned int * ws, float * __restrict__ g_out, uint8_t * __restrict__ codes,
+                            unsigned int parts, const AmaxWait wait, unsigned int * ws, float * __restrict__ g_out, uint8_t * __restrict__ codes,
                             uint8_t * __restrict__ scales) {
   constexpr int kVecs = sizeof(T);  // 16-byte loads per block
   constexpr int kHeld = DYNAMIC ? kHold : 1;
   __shared__ float table[128];
   __shared__ float red[kThreads / 32];
   __shared__ float shared_amax;
+  __shared__ unsigned int shared_share;
   // every CTA of the grid is resident: the next kernel of the stream may move in beside them
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const Idx stride = static_cast<Idx>(gridDim.x) * kThreads, first = static_cast<Idx>(blockIdx.x) * kThreads;
@@ -318,36 +326,68 @@ quantize_activations_kernel(const T * __restrict__ x, uint32_t scale_cols, const
         return m;
       };
       best = block_max(best);
+      // whether all have added theirs, or those who wait have added every share, within `polls` looks (one thread)
+      auto all_there = [&](int polls) {
+        const unsigned int all = parts + wait.absent;
+        for (int i = 0; i < polls; ++i) {
+          unsigned int here, shares;
+          asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(here) : "l"(ws + 1) : "memory");
+          asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(shares) : "l"(ws + 4) : "memory");
+          if (here >= all || shares >= parts) return true;
+        }
+        return false;
+      };
+      // The counts only order what a fence stands on either side of: every maximum comes before its arrival, reading the
+      // result comes after all arrivals (the last to arrive need not have polled) and before leaving, the reset after all
+      // have left.
+      auto read_amax = [&] {
+        __threadfence();
+        return __uint_as_float(*reinterpret_cast<volatile unsigned int *>(ws));
+      };
       if (threadIdx.x == 0) {
         atomicMax(ws, __float_as_uint(best));
         __threadfence();
-        unsigned int here = atomicAdd(ws + 1, 1u) + 1u;
-        for (int i = 0; here < parts && i < kAmaxPolls; ++i) asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(here) : "l"(ws + 1) : "memory");
-        // the counts only order what a fence stands on either side of: every maximum comes before its arrival and this read
-        // after all arrivals (the last to arrive has not polled), and this read before leaving and the reset after all have left
-        __threadfence();
-        float amax = -1.0f;
-        if (here >= parts) amax = __uint_as_float(*reinterpret_cast<volatile unsigned int *>(ws));
-        shared_amax = amax;
-        __threadfence();
-        if (atomicAdd(ws + 2, 1u) == parts - 1u) {  // all have added theirs and read the result
-          __threadfence();
-          ws[0] = 0u;
-          ws[1] = 0u;
-          ws[2] = 0u;
-        }
+        const unsigned int here = atomicAdd(ws + 1, 1u) + 1u;
+        shared_amax = here >= parts + wait.absent || all_there(wait.polls) ? read_amax() : -1.0f;
       }
       __syncthreads();
       float amax = shared_amax;
       if (amax < 0.0f) {
-        best = 0.0f;
-        for (Idx at = threadIdx.x; at < live; at += kThreads) {
-          uint4 r[kVecs];
-          load(at, r);
+        auto share_max = [&](Idx from, Idx step) {
+          float m = 0.0f;
+          for (Idx at = from + threadIdx.x; at < live; at += step) {
+            uint4 r[kVecs];
+            load(at, r);
 #pragma unroll
-          for (int i = 0; i < kVecs; ++i) best = abs_max<T>(r[i], best);
+            for (int i = 0; i < kVecs; ++i) m = abs_max<T>(r[i], m);
+          }
+          __syncthreads();  // the words that hold the warps' maxima are free
+          return block_max(m);
+        };
+        while (true) {
+          if (threadIdx.x == 0) shared_share = atomicAdd(ws + 3, 1u);
+          __syncthreads();
+          const unsigned int share = shared_share;
+          if (share >= parts) break;
+          const float m = share_max(static_cast<Idx>(share) * kThreads, stride);
+          if (threadIdx.x == 0) {
+            atomicMax(ws, __float_as_uint(m));
+            __threadfence();
+            atomicAdd(ws + 4, 1u);
+          }
         }
-        amax = block_max(best);
+        if (threadIdx.x == 0) shared_amax = all_there(wait.help_polls) ? read_amax() : -1.0f;
+        __syncthreads();
+        amax = shared_amax;
+        if (amax < 0.0f) amax = share_max(0, kThreads);
+      }
+      if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(ws + 2, 1u) == parts - 1u) {
+          __threadfence();
+#pragma unroll
+          for (int i = 0; i < kQuantWorkspaceWords; ++i) ws[i] = 0u;
+        }
       }
       g = amax > 0.0f ? __fdiv_rn(amax, 6.0f * 448.0f) : 1.0f;
       rg = __frcp_rn(g);
@@ -432,7 +472,7 @@ int check_quant_args(const void * x, int m, int k, const void * codes, const voi
 
 template <typename T>
 int launch_quantize_activations(const T * x, int m, int k, float global_scale, uint8_t * codes, uint8_t * scales_tiled,
-                                float * g_dev, void * workspace, cudaStream_t s) {
+                                float * g_dev, void * workspace, cudaStream_t s, const AmaxWait & wait = AmaxWait()) {
   if (const int st = check_quant_args(x, m, k, codes, scales_tiled)) return st;
   if (g_dev == nullptr) return fail(Q35B_ERR_ARGUMENT, "NVFP4 quantisation needs a device word for the input scale.");
   const bool dynamic = !(global_scale > 0.0f);
@@ -451,11 +491,11 @@ int launch_quantize_activations(const T * x, int m, int k, float global_scale, u
     map.magic = static_cast<uint32_t>(((1ull << (31 + l)) + map.slots - 1) / map.slots);
     map.shift = static_cast<uint32_t>(l - 1);
     le = launch_pdl(dynamic ? quantize_activations_kernel<T, true, uint32_t> : quantize_activations_kernel<T, false, uint32_t>, dim3(grid),
-                    dim3(kThreads), 0, s, x, static_cast<uint32_t>(k >> 4), map, live, total, global_scale, parts,
+                    dim3(kThreads), 0, s, x, static_cast<uint32_t>(k >> 4), map, live, total, global_scale, parts, wait,
                     static_cast<unsigned int *>(workspace), g_dev, codes, scales_tiled);
   } else {
     le = launch_pdl(dynamic ? quantize_activations_kernel<T, true, size_t> : quantize_activations_kernel<T, false, size_t>, dim3(grid),
-                    dim3(kThreads), 0, s, x, static_cast<uint32_t>(k >> 4), map, live, total, global_scale, parts,
+                    dim3(kThreads), 0, s, x, static_cast<uint32_t>(k >> 4), map, live, total, global_scale, parts, wait,
                     static_cast<unsigned int *>(workspace), g_dev, codes, scales_tiled);
   }
   count_launch();
@@ -469,6 +509,15 @@ int launch_quantize_bf16(const void * x, int m, int k, float global_scale, uint8
                          float * g_dev, void * workspace, cudaStream_t s) {
   return launch_quantize_activations(static_cast<const __nv_bfloat16 *>(x), m, k, global_scale, codes, scales_tiled, g_dev,
                                      workspace, s);
+}
+
+int launch_quantize_bf16_wait(const void * x, int m, int k, uint8_t * codes, uint8_t * scales_tiled, float * g_dev, void * workspace,
+                              int polls, int help_polls, unsigned int absent, cudaStream_t s) {
+  AmaxWait wait;
+  wait.polls = polls;
+  wait.help_polls = help_polls;
+  wait.absent = absent;
+  return launch_quantize_activations(static_cast<const __nv_bfloat16 *>(x), m, k, 0.0f, codes, scales_tiled, g_dev, workspace, s, wait);
 }
 
 int launch_quantize_f32(const float * x, int m, int k, float global_scale, uint8_t * codes, uint8_t * scales_tiled,

@@ -382,6 +382,12 @@ int q35b_quantize_nvfp4_bf16(const void * x_bf16, int m, int k, float global_sca
                               static_cast<cudaStream_t>(stream));
 }
 
+int q35b_debug_quantize_wait(const void * x_bf16, int m, int k, uint8_t * codes, uint8_t * scales_tiled, float * input_scale_dev,
+                             void * workspace, int polls, int help_polls, unsigned int absent, q35b_stream stream) {
+  return launch_quantize_bf16_wait(x_bf16, m, k, codes, scales_tiled, input_scale_dev, workspace, polls, help_polls, absent,
+                                   static_cast<cudaStream_t>(stream));
+}
+
 int q35b_quantize_nvfp4_f32(const float * x_f32, int m, int k, float global_scale, uint8_t * codes, uint8_t * scales_tiled,
                             float * input_scale_dev, void * workspace, q35b_stream stream) {
   return launch_quantize_f32(x_f32, m, k, global_scale, codes, scales_tiled, input_scale_dev, workspace,

@@ -98,6 +98,9 @@ int launch_gemv_f32(const q35b_weight * w, const float * x, float input_scale, f
 // act_quant.cu
 int launch_quantize_bf16(const void * x, int m, int k, float global_scale, uint8_t * codes, uint8_t * scales_tiled,
                          float * g_dev, void * workspace, cudaStream_t s);
+constexpr int kQuantWorkspaceWords = 5;  // of the workspace's 256 bytes: what quantize_activations_kernel counts in
+int launch_quantize_bf16_wait(const void * x, int m, int k, uint8_t * codes, uint8_t * scales_tiled, float * g_dev, void * workspace,
+                              int polls, int help_polls, unsigned int absent, cudaStream_t s);
 int launch_quantize_f32(const float * x, int m, int k, float global_scale, uint8_t * codes, uint8_t * scales_tiled,
                         float * g_dev, void * workspace, cudaStream_t s);
 int launch_quantize_reference_recipe(const void * x, int m, int k, int swap, uint8_t * codes, uint8_t * scales_tiled,

@@ -21,6 +21,8 @@ namespace {
 // reference runs (4096 tokens x 9216 columns): 18 MiB of codes + 2.25 MiB of
 // scales, plus one 256-byte control block.
 constexpr size_t kControlBytes = 256;
+constexpr size_t kScaleAt = 64, kStatusAt = 96;  // in the control block; the quantiser's workspace words are in front of them
+static_assert(kQuantWorkspaceWords * sizeof(unsigned int) <= kScaleAt, "the per-tensor scale stands behind the workspace");
 constexpr size_t kStaticScratchBytes = static_cast<size_t>(24) << 20;
 
 static __device__ __align__(256) unsigned char g_prefill_scratch[kStaticScratchBytes];
@@ -74,12 +76,12 @@ int q35b_project_prefill_bf16_static(const q35b_weight * w, const void * x_bf16,
   unsigned char * base = nullptr;
   if (const int st = scratch_for_current_device(&base)) return st;
   auto s = static_cast<cudaStream_t>(stream);
-  // Control block: [0,12) quantiser workspace, [16,20) per-tensor scale, [32,36) GEMM status.  The array keeps
+  // Control block: quantiser workspace, per-tensor scale, GEMM status.  The array keeps
   // whatever the previous call left, so everything that must start at zero is cleared here.
   Q35B_CUDA_TRY(cudaMemsetAsync(base, 0, kControlBytes, s), "cudaMemsetAsync(prefill scratch control block)");
   auto * workspace = base;
-  auto * g_dev = reinterpret_cast<float *>(base + 16);
-  auto * status = reinterpret_cast<unsigned int *>(base + 32);
+  auto * g_dev = reinterpret_cast<float *>(base + kScaleAt);
+  auto * status = reinterpret_cast<unsigned int *>(base + kStatusAt);
   uint8_t * codes = base + kControlBytes;
   uint8_t * scales = codes + codes_bytes;
   if (const int st = launch_quantize_bf16(x_bf16, m, w->k, global_scale, codes, scales, g_dev, workspace, s)) return st;
@@ -90,7 +92,7 @@ int q35b_static_prefill_status(unsigned int * status_out) {
   if (status_out == nullptr) return fail(Q35B_ERR_ARGUMENT, "Null status pointer.");
   unsigned char * base = nullptr;
   if (const int st = scratch_for_current_device(&base)) return st;
-  Q35B_CUDA_TRY(cudaMemcpy(status_out, base + 32, sizeof(unsigned int), cudaMemcpyDeviceToHost), "cudaMemcpy(prefill scratch status)");
+  Q35B_CUDA_TRY(cudaMemcpy(status_out, base + kStatusAt, sizeof(unsigned int), cudaMemcpyDeviceToHost), "cudaMemcpy(prefill scratch status)");
   return Q35B_OK;
 }
 
