@@ -160,6 +160,8 @@ int launch_gemm_w4a4(const q35b_weight * w, const uint8_t * a_codes, const uint8
 struct WBatch;  // decode work list on the tensor path (digit-expanded activations)
 // exact: all bits of the activations, their infinities and NaNs too, reach the outputs (else what `digits` digits hold)
 int wbatch_build(const q35b_gemv_item * items, int count, int m, int digits, bool exact, WBatch ** out);
+// the longest CTA's share of a list's K steps, whole tiles dealt out, over an SM's even share of them
+double wbatch_longest_share(const q35b_gemv_item * items, int count);
 int wbatch_launch(const WBatch * b, cudaStream_t s);
 void wbatch_free(WBatch * b);
 int wbatch_status(const WBatch * b, unsigned int * out);

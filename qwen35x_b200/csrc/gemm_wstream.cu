@@ -823,6 +823,46 @@ struct WBatch {
   uint32_t wait_limit = kWaitLimit;
 };
 
+namespace {
+
+// K steps of every tile of a list, and one for what a tile costs besides.
+std::vector<long> tile_costs(const q35b_gemv_item * items, int count) {
+  std::vector<long> cost;
+  for (int i = 0; i < count; ++i) cost.insert(cost.end(), (items[i].weight->rows + kRows - 1) / kRows, items[i].weight->k / 256 + 1);
+  return cost;
+}
+
+// Contiguous runs of about equal cost: a tile goes to the CTA in whose share of the total its midpoint falls.
+std::vector<int> deal_tiles(const std::vector<long> & cost, int grid) {
+  std::vector<int> begin(grid + 1, 0);
+  long total = 0, done = 0;
+  for (long c : cost) total += c;
+  int c = 0;
+  for (size_t t = 0; t < cost.size(); ++t) {
+    while (c + 1 < grid && (done + cost[t] / 2) * grid >= static_cast<long>(c + 1) * total) begin[++c] = static_cast<int>(t);
+    done += cost[t];
+  }
+  while (c + 1 <= grid) begin[++c] = static_cast<int>(cost.size());
+  return begin;
+}
+
+}  // namespace
+
+double wbatch_longest_share(const q35b_gemv_item * items, int count) {
+  const std::vector<long> cost = tile_costs(items, count);
+  if (cost.empty()) return 0.0;
+  const int grid = std::min<int>(sm_count(), static_cast<int>(cost.size()));
+  const std::vector<int> begin = deal_tiles(cost, grid);
+  long total = 0, longest = 0;
+  for (int c = 0; c < grid; ++c) {
+    long share = 0;
+    for (int t = begin[c]; t < begin[c + 1]; ++t) share += cost[t];
+    longest = std::max(longest, share);
+    total += share;
+  }
+  return static_cast<double>(longest) * sm_count() / total;
+}
+
 int wbatch_build(const q35b_gemv_item * items, int count, int m, int digits, bool exact, WBatch ** out) {
   if (items == nullptr || out == nullptr || count <= 0) return fail(Q35B_ERR_ARGUMENT, "Invalid NVFP4 projection work list.");
   *out = nullptr;
@@ -867,30 +907,15 @@ int wbatch_build(const q35b_gemv_item * items, int count, int m, int digits, boo
 
   // layout of the one allocation: items | tiles | cta_begin | expand items | status | per-item digit buffers
   std::vector<WTile> all;
-  std::vector<long> cost;
+  const std::vector<long> cost = tile_costs(items, count);
   for (int i = 0; i < count; ++i) {
     const q35b_weight * w = items[i].weight;
-    for (int rb = 0; rb < (w->rows + kRows - 1) / kRows; ++rb) {
-      all.push_back(WTile{i, rb});
-      cost.push_back(w->k / 256 + 1);
-    }
+    for (int rb = 0; rb < (w->rows + kRows - 1) / kRows; ++rb) all.push_back(WTile{i, rb});
     b->bytes_per_run += w->codes_bytes + w->scales_bytes;
   }
   const int grid = std::max(1, std::min<int>(sm_count(), static_cast<int>(all.size())));
   b->grid = grid;
-  // contiguous runs of about equal cost: a tile goes to the CTA in whose share of the total its midpoint falls
-  std::vector<int> h_begin(grid + 1, 0);
-  {
-    long total = 0;
-    for (long c : cost) total += c;
-    long done = 0;
-    int c = 0;
-    for (size_t t = 0; t < all.size(); ++t) {
-      while (c + 1 < grid && (done + cost[t] / 2) * grid >= static_cast<long>(c + 1) * total) h_begin[++c] = static_cast<int>(t);
-      done += cost[t];
-    }
-    while (c + 1 <= grid) h_begin[++c] = static_cast<int>(all.size());
-  }
+  const std::vector<int> h_begin = deal_tiles(cost, grid);
   auto up = [](size_t v, size_t a) { return (v + a - 1) / a * a; };
   const size_t o_tiles = up(sizeof(WItem) * count, 256);
   const size_t o_begin = up(o_tiles + sizeof(WTile) * all.size(), 256);

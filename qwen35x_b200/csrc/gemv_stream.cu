@@ -1002,24 +1002,28 @@ Assignment assign_tiles(const std::vector<GemvTile> & all, const std::vector<int
 }
 
 // Whether a list runs on the tensor cores (gemm_wstream.cu): independent items, block scales the tensor cores read as this
-// kernel does, and enough weights.  That path puts one more launch in front of every run (5 us for one token, 10 for eight,
-// under which the next weights fill the rings), issues a fifth of the instructions and, in runs long enough to meet the
-// power cap, keeps its clock.  Measured in graph replays of 0.2 s and more, us, this kernel / tensor cores: 223 MiB of
-// 1024-column projections one token 50.5 / 44.2, four 52.1 / 50.8, eight 62.0 / 55.4; 461 MiB of 2560-column ones 98 / 88,
-// 111 / 91, 124 / 98; 1.8 GiB 348 / 304, 395 / 332, 443 / 359.  The line: 115 MiB one token 29.8 / 31.3, two 31.1 / 31.4,
-// four 34.9 / 31.9, eight 35.4 / 33.4; 111 MiB one token 26.4 / 24.9; 56 MiB one token 16.2 / 15.7, four 17.6 / 17.0, eight
-// 21.6 / 19.6.
+// kernel does, enough weights, and whole tiles that come out even.  That path puts one more launch in front of every run (5 us
+// for one token, 9 for eight, under which the next weights fill the rings), issues a fifth of the instructions and, in runs
+// long enough to meet the power cap, keeps its clock; and it never splits a tile.  us, this kernel / tensor cores, one, four and
+// eight tokens.  In runs of 0.2 s and more: 223 MiB of 1024-column projections 49 / 45, -, 61 / 55; 1.8 GiB 358 / 308, 405 / 339.
+// In runs of 80 ms, by the longest CTA's share of the K steps over an even share:
+//   1.0 to 1.4: 231 MiB 53 / 48, 51 / 50, 61 / 52; 202 MiB 55 / 49, 53 / 51, 55 / 53; 180 MiB 35.4 / 34.5, 37.0 / 36.3, 41.9 / 37.8;
+//               142 MiB (1.3) 31 / 35, 36 / 37, 39 / 38; 111 MiB 26.0 / 26.5, 28.0 / 29.8, 32.1 / 32.7; 90 MiB 19.3 / 20.7, 20.2 / 21.9,
+//               25.2 / 23.4; 72 MiB 17.4 / 16.4, 18.1 / 18.1, 20.2 / 22.4; 56 MiB 16.3 / 17.3, 17.7 / 18.7, 21.7 / 22.6
+//   1.55: 115 MiB 30 / 33, 35 / 34, 35 / 36; 58 MiB 17 / 20, 19 / 22, 22 / 24
+//   1.85: 101 MiB 24 / 34, 38 / 36, 31 / 37; 51 MiB 16 / 20, 18 / 21, 21 / 23; 2.3: 72 MiB 21 / 30, 23 / 31
 constexpr int kTensorDigits = 8;  // three bits each, and more of them where a value needs them (gemm_wstream.cu)
-constexpr size_t kTensorBytes = 128u << 20, kTensorBytesFrom4 = 48u << 20;  // up to three tokens, and from four on
+constexpr size_t kTensorBytes = 128u << 20;
+constexpr double kTensorLongest = 1.45;
 
-bool tensor_list(const q35b_gemv_item * items, int count, int m) {
+bool tensor_list(const q35b_gemv_item * items, int count) {
   size_t bytes = 0;
   for (int i = 0; i < count; ++i) {
     const q35b_weight * w = items[i].weight;
     if (items[i].after != 0 || w->rows <= 0 || !w->has_maps || w->nan_scales || items[i].x_bf16 == nullptr || items[i].y_bf16 == nullptr) return false;
     bytes += w->codes_bytes + w->scales_bytes;
   }
-  return bytes >= (m >= 4 ? kTensorBytesFrom4 : kTensorBytes);
+  return bytes >= kTensorBytes && wbatch_longest_share(items, count) <= kTensorLongest;
 }
 
 }  // namespace
@@ -1046,7 +1050,7 @@ int gemv_batch_build(const q35b_gemv_item * items, int count, int m, bool share_
     max_k = std::max(max_k, w->k);
   }
   // only what the plan below takes too: a list whose activations do not fit it is refused whatever its size
-  if (Plan fits_plan; share_tiles && tensor_list(items, count, m) && make_plan(m, max_k, &fits_plan)) {
+  if (Plan fits_plan; share_tiles && tensor_list(items, count) && make_plan(m, max_k, &fits_plan)) {
     WBatch * t = nullptr;
     if (const int st = wbatch_build(items, count, m, kTensorDigits, true, &t)) return st;
     auto * b = new q35b_gemv_batch();

@@ -100,7 +100,7 @@ def test_small_values_beside_large_ones_keep_their_bits(engine, m, k):
     inside = torch.arange(5, k, 16, device="cuda")[torch.randperm(blocks, device="cuda", generator=gen)[: blocks // 2]]
     alone = torch.arange(32, 48, device="cuda")
     rows = 130
-    items, checks = [_filler(engine, torch, gen, m)], []
+    items, checks = [_filler(engine, torch, gen, m)] * (3 if k > 9216 else 1), []  # a share of the GPU has room for the long tiles
     for depth in (9, 15, 16, 17, 20, 24, 28, 31):
         for where in (inside, alone):
             codes = torch.zeros((rows, k), dtype=torch.uint8, device="cuda")
@@ -268,3 +268,19 @@ def test_infinities_and_nans_cost_little(engine):
     x[:, 1000] = float("inf")
     x[0, 1000] = float("nan")
     assert min(run() for _ in range(3)) <= 4 * finite and batch.status() == 0
+
+
+# few long tiles, of which whole ones come out uneven over the SMs, and many; 128 MiB of weights and less
+@pytest.mark.parametrize("shapes,launches", [([(20480, 16384)], 1), ([(8192, 16384)], 1), ([(2560, 9216)] * 16, 2),
+                                             ([(32768, 2560)] * 4, 2), ([(32768, 2560)] * 2, 1), ([(1000, 4096)] * 64, 2)])
+def test_lists_whose_whole_tiles_come_out_uneven_stay_on_the_other_kernel(engine, shapes, launches):
+    import torch
+
+    m, gen = 4, torch.Generator(device="cuda").manual_seed(4)
+    items = []
+    for n, k in shapes:
+        w = engine.Nvfp4Weight.from_device(torch.randint(0, 256, (n, k // 2), dtype=torch.uint8, device="cuda", generator=gen),
+                                           torch.full((n, k // 16), 0x30, dtype=torch.uint8, device="cuda"), 1e-3)
+        items.append((w, torch.randn((m, k), device="cuda", generator=gen).to(torch.bfloat16),
+                      torch.empty((m, n), dtype=torch.bfloat16, device="cuda")))
+    _run(engine, torch, items, m, launches=launches)
