@@ -75,7 +75,7 @@ __device__ __forceinline__ void load16<__nv_bfloat16>(const __nv_bfloat16 * p, f
   const uint4 * q = reinterpret_cast<const uint4 *>(p);
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
-    const uint4 a = __ldcg(q + i);
+    const uint4 a = __ldca(q + i);
     const uint32_t r[4] = {a.x, a.y, a.z, a.w};
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -90,7 +90,7 @@ __device__ __forceinline__ void load16<float>(const float * p, float (&v)[16]) {
   const float4 * q = reinterpret_cast<const float4 *>(p);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const float4 a = __ldcg(q + i);
+    const float4 a = __ldca(q + i);
     v[i * 4] = a.x;
     v[i * 4 + 1] = a.y;
     v[i * 4 + 2] = a.z;
@@ -291,8 +291,9 @@ quantize_activations_kernel(const T * __restrict__ x, uint32_t scale_cols, const
       in = in && b < scale_cols;
     }
     const uint4 * src = reinterpret_cast<const uint4 *>(x) + static_cast<size_t>(f) * kVecs;
+    // through L1: a lane's loads share sectors, which each of them would fetch from L2 anew
 #pragma unroll
-    for (int i = 0; i < kVecs; ++i) r[i] = in ? __ldcg(src + i) : make_uint4(0u, 0u, 0u, 0u);
+    for (int i = 0; i < kVecs; ++i) r[i] = in ? __ldca(src + i) : make_uint4(0u, 0u, 0u, 0u);
     return in;
   };
 

@@ -222,8 +222,8 @@ __device__ __forceinline__ void gemm_store_chunk32(const uint32_t (&r)[32], int 
       uint32_t p[8];
       uint32_t rr[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
       if (res != nullptr) {
-        const uint4 a = __ldcg(reinterpret_cast<const uint4 *>(res + v * 16));
-        const uint4 b = __ldcg(reinterpret_cast<const uint4 *>(res + v * 16 + 8));
+        const uint4 a = __ldca(reinterpret_cast<const uint4 *>(res + v * 16));
+        const uint4 b = __ldca(reinterpret_cast<const uint4 *>(res + v * 16 + 8));
         rr[0] = a.x; rr[1] = a.y; rr[2] = a.z; rr[3] = a.w;
         rr[4] = b.x; rr[5] = b.y; rr[6] = b.z; rr[7] = b.w;
       }

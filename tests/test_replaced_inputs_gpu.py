@@ -100,3 +100,30 @@ def test_single_projection(engine, m):
         x.copy_(v)
         got.append(engine.gemv_w4a16(w, x))
     assert all(_same(torch, a, b) for a, b in zip(got, want * 5))
+
+
+@pytest.mark.parametrize("m", [16, 300])
+def test_prefill_reading_what_the_call_before_wrote(engine, m):
+    """Two projections in a row, the second quantising the first one's output: nothing of it may be read before the first one's
+    kernel, which lets its successor start early, is complete."""
+    import torch
+
+    k, n = 2560, 2048
+    w1, w2 = _weight(engine, torch, n, k, 8), _weight(engine, torch, 512, n, 9)
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    xs = [(torch.randn((m, k), device="cuda", generator=gen) * 4.0 ** i).to(torch.bfloat16) for i in range(8)]
+    s1, s2 = engine.act_scratch(m, k, "cuda"), engine.act_scratch(m, n, "cuda")
+    between = torch.empty((m, n), dtype=torch.bfloat16, device="cuda")
+    want = []
+    for x in xs:
+        torch.cuda.synchronize()
+        engine.project_prefill(w1, x, out=between, scratch=s1)
+        torch.cuda.synchronize()
+        want.append(engine.project_prefill(w2, between, scratch=s2).clone())
+    for _ in range(20):
+        torch.cuda.synchronize()
+        got = []
+        for x in xs:
+            engine.project_prefill(w1, x, out=between, scratch=s1)
+            got.append(engine.project_prefill(w2, between, scratch=s2))
+        assert all(_same(torch, a, b) for a, b in zip(got, want))
