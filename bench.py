@@ -241,7 +241,7 @@ def capture(torch, stream, fn):
 
 def time_decode_step(torch, timer, stream, batches, steps: int, warmup: int):
     """Per-step milliseconds of a work-list step: (back-to-back launches issued from CUDA graphs of up to 64
-    consecutive steps, programmatic edges between the kernel nodes), (one-kernel graph replays, no overlap)."""
+    consecutive steps, programmatic edges between the kernel nodes), (one-step graph replays, no overlap)."""
     sets = len(batches)
     chunk = min(steps, 64)
     if chunk > 1 and sets > 1:
@@ -312,7 +312,7 @@ def run_engine(args, rank: int, world: int, local_rank: int) -> dict | None:
         sampler.start()
     # Device-resident steps: back-to-back stream launches.  The kernel is launched with programmatic stream
     # serialisation, so a step's weight stream starts under the tail of the previous step (its activations and
-    # outputs still wait for the previous kernel to complete); one-kernel graph replays cannot overlap that way and
+    # outputs still wait for the previous kernel to complete); one-step graph replays cannot overlap that way and
     # are reported beside it.
     ms_per_step, ms_graph_step = time_decode_step(torch, timer, stream, batches, args.steps, args.warmup)
 
@@ -357,7 +357,7 @@ def run_engine(args, rank: int, world: int, local_rank: int) -> dict | None:
                              "consecutive steps)",
                    "graph_replay": {"ms_per_step": round(ms_graph_step, 5), "value": round(world * achieved_graph, 2),
                                     "frac_of_hbm_peak": round(achieved_graph / pk["hbm_gbs"], 4),
-                                    "note": "same step as one-kernel CUDA graph replays (no overlap between replays): "
+                                    "note": "same step as one-step CUDA graph replays (no overlap between replays): "
                                             "what a step with other work between its projections sees"},
                    "per_projection_launches": {"ms_per_step": round(ms_pp, 5),
                                                "value": round(world * step_bytes / (ms_pp * 1e-3) / 1e9, 2),

@@ -180,7 +180,9 @@ typedef struct q35b_gemv_batch q35b_gemv_batch;
  * of its token's largest one.  Lists with dependent items, and small ones, convert every token to fp16 with one power of two;
  * large lists of independent items run on the tensor cores (see below) with as many octal digits as that takes: eight in
  * every K step, and six more in the steps of 256 columns where a value has bits below 2^-16 of the largest of its sixteen
- * neighbours.  Infinities and NaNs reach the outputs as fp32 arithmetic has it, on either path. */
+ * neighbours.  Infinities and NaNs reach the outputs as fp32 arithmetic has it, on either path.
+ * Device memory a list owns: descriptors and counters, some hundred KB; on the tensor cores also the operand rows, per 256
+ * columns of every item 4 KB for one token, 8 KB for two, 12 KB for four and 18 KB for eight (a 4B-class step 9 and 41 MB). */
 Q35B_API int q35b_gemv_batch_create(const q35b_gemv_item * items, int count, int m, q35b_gemv_batch ** out);
 /* The same work list on the tensor cores (no counterpart in the reference, whose decode dequantises in registers,
  * src/kernels/cuda/decode_layers.cuh:200-261): the weight streams through tcgen05.mma as the 128-row operand and
