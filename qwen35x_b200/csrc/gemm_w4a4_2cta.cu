@@ -3,22 +3,24 @@
 // Same contract as gemm_w4a4_tcgen05.cu (C[M,N] bf16 = (Aq . Wq^T) * g * s2, replacing
 // run_nvfp4_cublaslt_prefill_projection_device, src/runtime/cuda_bench.cu:1056-1167), built for large M:
 //
-//   - a pair of CTAs on neighbouring SMs (cluster of 2) computes one 256 x 192 output tile with
-//     tcgen05.mma.cta_group::2: each CTA stages only its own 128 rows of A and its own 96 rows of B.  No TMA
+//   - a pair of CTAs on neighbouring SMs (cluster of 2) computes one 256 x 256 output tile with
+//     tcgen05.mma.cta_group::2: each CTA stages only its own 128 rows of A and its own 128 rows of B.  No TMA
 //     multicast is used: every load lands in the issuing CTA's own shared memory;
-//   - N = 192 leaves room in TMEM (2 x 192 accumulator columns + 48 scale-factor columns <= 512) for TWO
-//     accumulators, so the epilogue of one tile overlaps the MMAs of the next;
 //   - persistent: 74 pairs walk the tile list (M-tiles fastest, so the pairs in flight share B tiles in L2);
 //     barriers, TMEM and tensor maps are set up once per CTA, not once per tile;
-//   - per K step (256 FP4 columns) a CTA lands A 16 KB + B 12 KB (128B-swizzled TMA boxes) and the scale
-//     factors SFA 2 KB + SFB 4 KB (TMA boxes over the 512-byte scale tiles); 6-stage ring.  A 192-row tile
-//     starts either on a 128-row scale tile or 64 rows into one: it always takes two scale tiles, and the MMA's
-//     SFB address is moved by two TMEM columns (= 64 rows) in the second case;
+//   - per K step (256 FP4 columns) a CTA lands A 16 KB + B 16 KB (128B-swizzled TMA boxes) and the scale
+//     factors SFA 2 KB + SFB 4 KB (TMA boxes over the 512-byte scale tiles); 5-stage ring;
 //   - the leader CTA's MMA thread copies scale factors to TMEM in both CTAs (tcgen05.cp.cta_group::2) and
-//     issues four M=256, N=192, K=64 block-scaled MMAs per K step; tcgen05.commit multicasts stage release and
+//     issues four M=256, N=256, K=64 block-scaled MMAs per K step; tcgen05.commit multicasts stage release and
 //     accumulator-ready to both CTAs;
-//   - four epilogue warps per CTA drain that CTA's 128 x 192 fp32 accumulator half from TMEM, scale, convert
-//     and store BF16.
+//   - two accumulators alternate, so that a tile's MMAs run while the one before is converted and stored.  Beside 48
+//     columns of scale factors 512 columns of TMEM do not hold two of 256: the second starts at column 208 and shares 48
+//     with the first (OVERLAP below).  The 64 columns of a tile that hold them are read out first, and the next tile's MMAs
+//     wait for these alone; all others have a tile's time to leave.
+//
+// What bounds it: the power cap.  At [4096, 2560] x [18432, 2560] the SM clock falls to 1.5 GHz within a millisecond and to
+// 1.35 GHz in a loop.  A K step takes some 560 cycles (542 at the tensor cores' nominal rate); with one accumulator 1900 of a
+// tile's 8300 cycles went by between its last MMA and the next tile's first one.
 //
 // Every mbarrier wait is bounded; an expired wait records a code in *status and the role stops, the kernel
 // still runs to its cluster barrier and frees TMEM.
@@ -31,14 +33,9 @@
 namespace q35b {
 namespace {
 
-#ifndef Q35B_TILE_N
-#define Q35B_TILE_N 256
-#endif
 constexpr int kCtaRows = 128;            // rows of A staged per CTA
 constexpr int kTileM = 256;              // output tile of the pair: 256 tokens ...
-constexpr int kTileN = Q35B_TILE_N;      // ... by 192 (two accumulators in TMEM) or 256 (one) weight rows
-static_assert(kTileN == 192 || kTileN == 256, "tile width");
-constexpr int kAccs = kTileN == 192 ? 2 : 1;  // accumulators that fit beside the scale factors in 512 TMEM columns
+constexpr int kTileN = 256;              // ... by 256 weight rows
 constexpr int kCtaBRows = kTileN / 2;    // rows of B staged per CTA
 constexpr int kStepBytes = 128;          // 256 FP4 columns
 constexpr int kMmaPerStage = 4;
@@ -47,23 +44,24 @@ constexpr int kABytes = kCtaRows * kStepBytes;
 constexpr int kBBytes = kCtaBRows * kStepBytes;
 constexpr int kSfaBytes = kMmaPerStage * kSfChunk;
 constexpr int kSfbBytes = 2 * kMmaPerStage * kSfChunk;
-constexpr int kStageBytes = kABytes + kBBytes + kSfaBytes + kSfbBytes;   // 34816
-#ifndef Q35B_STAGES
-#define Q35B_STAGES (Q35B_TILE_N == 192 ? 6 : 5)
-#endif
-constexpr int kStages = Q35B_STAGES;
+constexpr int kStageBytes = kABytes + kBBytes + kSfaBytes + kSfbBytes;   // 38912
+constexpr int kStages = 5;
 // Epilogue warps per CTA (template parameter of the kernel), a multiple of four: kEpilogueWarps / 4 per TMEM lane
-// quarter, each draining a column slice of the accumulator.  Sixteen for the epilogues that do arithmetic on what they
-// drain (SiLU, NVFP4 output) and for launches that forward rows to peers (their 64-column grain); eight for the plain
-// and the residual epilogue, which measured 1-5 % faster with fewer, wider warps.
-constexpr int kEpiWarpsWide = kTileN == 192 ? 12 : 16;
-constexpr int kEpiWarpsPlain = kTileN == 192 ? 12 : 8;
+// quarter, which take turns at the 64-column units of the accumulator.  Sixteen for the epilogues that do arithmetic on what
+// they drain (SiLU, NVFP4 output) and for launches that forward rows to peers; eight for the plain and the residual epilogue,
+// which measured 1-5 % faster with fewer warps.
+constexpr int kEpiWarpsWide = 16;
+constexpr int kEpiWarpsPlain = 8;
+constexpr int kUnitCols = 64;
+constexpr int kUnits = kTileN / kUnitCols;
 constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 256;
 static_assert(kStages * kStageBytes + 1024 + 256 <= 227 * 1024, "shared memory");
-constexpr int kAccCols = kAccs * kTileN;
 constexpr int kSfaCols = kMmaPerStage * 4;
 constexpr int kSfbCols = kMmaPerStage * 8;
 constexpr int kTmemCols = 512;
+// OVERLAP: the second accumulator ends where the scale factors begin.
+constexpr int kAcc1 = kTmemCols - kSfaCols - kSfbCols - kTileN;  // its first column, 208
+static_assert(kAcc1 < kTileN && kTileN - kAcc1 <= kUnitCols, "the shared columns lie in the first accumulator's last unit and the second one's first");
 constexpr uint32_t kWaitLimit = 1u << 20;
 constexpr uint32_t kPeerMask = 0xFEFFFFFFu;  // clears the CTA-rank bit of a shared::cluster address: the pair's leader
 
@@ -77,14 +75,11 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-// Arrive on the barrier at the same offset in CTA `cta` of the cluster.
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar, uint32_t cta) {
-  uint32_t remote;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(bar), "r"(cta));
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+// Arrive on the barrier at this offset in the pair's leader.  What it tells is that registers hold what TMEM held
+// (tcgen05.wait::ld), so no scope beyond the CTA is asked for: with .release.cluster the arrival waits for the output
+// stores under way, 1400 cycles in which the tensor cores had nothing to do.
+__device__ __forceinline__ void mbar_arrive_leader(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar & kPeerMask) : "memory");
 }
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   for (uint32_t i = 0; i < kWaitLimit; ++i) {
@@ -132,7 +127,7 @@ __device__ __forceinline__ uint64_t desc_sf(uint32_t saddr) {
   d |= static_cast<uint64_t>(1) << 46;
   return d;
 }
-// kind::mxf4nvf4 instruction descriptor: E2M1 x E2M1, K-major, UE4M3 scales, M = 256 (pair), N = 192.
+// kind::mxf4nvf4 instruction descriptor: E2M1 x E2M1, K-major, UE4M3 scales, M = 256 (pair), N = 256.
 __device__ __forceinline__ uint32_t instr_desc_pair() {
   uint32_t d = 0;
   d |= 1u << 7;
@@ -181,8 +176,8 @@ gemm_w4a4_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                       const __grid_constant__ CUtensorMap tmap_sfa, const __grid_constant__ CUtensorMap tmap_sfb,
                       const float * __restrict__ g_dev, const GemmEpilogue ep, int m, int n, int k_bytes, int m_tiles, int num_tiles,
                       __nv_bfloat16 * __restrict__ c, int ldc, unsigned int * status) {
-  constexpr int kEpiCols = kTileN / (kEpilogueWarps / 4);  // columns drained by one epilogue warp
-  static_assert(kEpilogueWarps % 4 == 0 && kEpiCols % 32 == 0 && kEpiCols * (kEpilogueWarps / 4) == kTileN, "epilogue column split");
+  constexpr int kTurns = kUnits / (kEpilogueWarps / 4);  // units of a tile that one epilogue warp takes
+  static_assert(kEpilogueWarps % 4 == 0 && kTurns * (kEpilogueWarps / 4) == kUnits, "epilogue column split");
   extern __shared__ uint8_t smem_raw[];
   uint8_t * smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint8_t * smem_a = smem;
@@ -192,10 +187,9 @@ gemm_w4a4_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
   uint64_t * bars = reinterpret_cast<uint64_t *>(smem_sfb + kStages * kSfbBytes);
   uint64_t * full = bars;                       // used in the leader: bytes of both CTAs
   uint64_t * empty = bars + kStages;            // in each CTA: its own stages are free
-  uint64_t * tmem_full = bars + 2 * kStages;    // [2] in each CTA: accumulator b is complete
-  uint64_t * drained = tmem_full + 2;           // [2] in each CTA: its epilogue warps have read accumulator b out of TMEM
-  uint64_t * peer_drained = drained + 2;        // [2] used in the leader: the partner CTA has drained accumulator b
-  uint32_t * tmem_slot = reinterpret_cast<uint32_t *>(peer_drained + 2);
+  uint64_t * tmem_full = bars + 2 * kStages;    // in each CTA: the tile's accumulator is complete
+  uint64_t * drained = tmem_full + 1;           // used in the leader: both CTAs' epilogue warps have read the columns that the next tile's accumulator shares
+  uint32_t * tmem_slot = reinterpret_cast<uint32_t *>(drained + 1);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -211,11 +205,8 @@ gemm_w4a4_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       mbar_init(smem_u32(full + i), 1);
       mbar_init(smem_u32(empty + i), 1);
     }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(smem_u32(tmem_full + i), 1);
-      mbar_init(smem_u32(drained + i), kEpilogueWarps);
-      mbar_init(smem_u32(peer_drained + i), 1);
-    }
+    mbar_init(smem_u32(tmem_full), 1);
+    mbar_init(smem_u32(drained), 2 * kEpilogueWarps);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -230,7 +221,7 @@ gemm_w4a4_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tmem_acc = tmem_base;
-  const uint32_t tmem_sfa = tmem_base + kAccCols;
+  const uint32_t tmem_sfa = tmem_base + kAcc1 + kTileN;
   const uint32_t tmem_sfb = tmem_sfa + kSfaCols;
   // Launched with programmatic stream serialisation: everything above (barriers, TMEM, the pair's rendezvous) may run
   // under the tail of the previous kernel; nothing below touches global memory before that kernel is complete.
@@ -251,7 +242,7 @@ gemm_w4a4_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         const int a_row = tm * kTileM + static_cast<int>(rank) * kCtaRows;
         const int b_row = tn * kTileN + static_cast<int>(rank) * kCtaBRows;
         const int sfa_chunk0 = (tm * 2 + static_cast<int>(rank)) * sf_col_blocks;
-        const int sfb_rb = (tn * kTileN) >> 7;  // first 128-row scale tile the 192 rows touch
+        const int sfb_rb = (tn * kTileN) >> 7;  // first of the two 128-row scale tiles
         const int sfb_chunk0 = sfb_rb * sf_col_blocks;
         const int sfb_chunk1 = (sfb_rb + 1) * sf_col_blocks;
         for (int ks = 0; ks < k_steps; ++ks) {
@@ -284,15 +275,13 @@ gemm_w4a4_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       uint32_t li = 0;
       bool ok = true;
       for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, ++li) {
-        const uint32_t ab = li % kAccs;
-        const uint32_t acc_phase = (li / kAccs) & 1;
-        if (!mbar_wait(smem_u32(drained + ab), acc_phase ^ 1) || !mbar_wait(smem_u32(peer_drained + ab), acc_phase ^ 1)) {
+        // the shared columns of the tile before are read out, and with them all of the one before that
+        if (!mbar_wait(smem_u32(drained), (li & 1) ^ 1)) {
           atomicExch(status, kMmaDrainWait);
           ok = false;
           break;
         }
-        const uint32_t acc = tmem_acc + ab * kTileN;
-        const uint32_t sfb_off = ((static_cast<uint32_t>(tile / m_tiles) * kTileN) & 127u) >> 5;  // 0 or 2 columns
+        const uint32_t acc = tmem_acc + (li & 1) * kAcc1;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         for (int ks = 0; ks < k_steps; ++ks) {
           if (!mbar_wait(smem_u32(full + stage), phase)) {
@@ -318,7 +307,7 @@ gemm_w4a4_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
 #pragma unroll
           for (int j = 0; j < kMmaPerStage; ++j) {
             if (j < valid) {
-              umma_pair(acc, a_desc + j * 2, b_desc + j * 2, idesc, tmem_sfa + j * 4, tmem_sfb + j * 8 + sfb_off,
+              umma_pair(acc, a_desc + j * 2, b_desc + j * 2, idesc, tmem_sfa + j * 4, tmem_sfb + j * 8,
                         (ks | j) != 0 ? 1u : 0u);
             }
           }
@@ -328,25 +317,13 @@ gemm_w4a4_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             phase ^= 1;
           }
         }
-        if (ok) umma_commit_pair(smem_u32(tmem_full + ab));
-      }
-    } else if (rank == 1 && elect_one() && !aborted) {
-      // ---------------- drain forwarder (partner CTA): tells the leader when this CTA's epilogue warps have
-      // read an accumulator out, so that none of them spends a cluster round trip on it ----------------
-      uint32_t li = 0;
-      for (int tile = pair; tile < num_tiles; tile += num_pairs, ++li) {
-        const uint32_t ab = li % kAccs;
-        if (!mbar_wait(smem_u32(drained + ab), (li / kAccs) & 1)) {
-          atomicExch(status, kEpilogueWait);
-          break;
-        }
-        mbar_arrive_cluster(smem_u32(peer_drained + ab), 0);
+        if (ok) umma_commit_pair(smem_u32(tmem_full));
       }
     }
   } else {
     // ---------------- epilogue (both CTAs): this CTA's 128 rows of the pair's tile ----------------
     const int quarter = warp & 3;                 // TMEM lanes 32 * quarter .. + 31 (fixed by the warp's index)
-    const int col_base = ((warp - 2) >> 2) * kEpiCols;
+    const int turn0 = (warp - 2) >> 2;
     const float g = __ldcg(g_dev);
     GemmQuantScale q;
     if constexpr (kEpilogueWarps == kEpiWarpsWide) {
@@ -365,35 +342,44 @@ gemm_w4a4_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, ++li) {
       const int tm = tile % m_tiles;
       const int tn = tile / m_tiles;
-      const uint32_t ab = li % kAccs;
-      if (!mbar_wait(smem_u32(tmem_full + ab), (li / kAccs) & 1)) {
+      if (!mbar_wait(smem_u32(tmem_full), li & 1)) {
         if (lane == 0) atomicExch(status, kEpilogueWait);
         ok = false;
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const int row = tm * kTileM + static_cast<int>(rank) * kCtaRows + quarter * 32 + lane;
-      const uint32_t taddr = tmem_acc + ab * kTileN + col_base + (static_cast<uint32_t>(quarter * 32) << 16);
-      // read the warp's whole share into registers, give the accumulator back at once, then convert and store
-      uint32_t r[kEpiCols / 32][32];
-#pragma unroll
-      for (int j = 0; j < kEpiCols / 32; ++j) tmem_ld32(taddr + 32 * j, r[j]);
+      const int row0 = tm * kTileM + static_cast<int>(rank) * kCtaRows + quarter * 32;
+      const uint32_t taddr = tmem_acc + (li & 1) * kAcc1 + (static_cast<uint32_t>(quarter * 32) << 16);
+      // the unit with the shared columns comes first: the last of the first accumulator, the first of the second
+      auto unit = [&](int turn) { return static_cast<int>((turn0 + turn * (kEpilogueWarps / 4) + ((li & 1) != 0u ? 0 : kUnits - 1)) % kUnits) * kUnitCols; };
+      uint32_t r[kTurns][2][32];
+      auto load = [&](int turn) {
+        tmem_ld32(taddr + unit(turn), r[turn][0]);
+        tmem_ld32(taddr + unit(turn) + 32, r[turn][1]);
+      };
+      load(0);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(drained + ab));
+      if (lane == 0) mbar_arrive_leader(smem_u32(drained));
       // plain BF16 output of a gathering launch: store locally, then forward whole rows; the fused epilogues (and a
       // launch without peers) store per lane
       const bool forward = ep.n_peers > 0 && !ep.gate_up && ep.forward_rows != 0;
-      if (row < m) {
 #pragma unroll
-        for (int j = 0; j < kEpiCols / 32; ++j) {
-          gemm_store_chunk32<kEpilogueWarps == kEpiWarpsWide>(r[j], row, tn * kTileN + col_base + 32 * j, n, g, ep, c, ldc, !forward, q);
+      for (int turn = 0; turn < kTurns; ++turn) {
+        const int col0 = tn * kTileN + unit(turn);
+        if (turn + 1 < kTurns) load(turn + 1);  // on its way while this one is stored
+        if (row0 + lane < m) {
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            gemm_store_chunk32<kEpilogueWarps == kEpiWarpsWide>(r[turn][j], row0 + lane, col0 + 32 * j, n, g, ep, c, ldc, !forward, q);
+          }
         }
-      }
-      if (forward) {
-        gemm_forward_rows_to_peers<kEpiCols>(ep, c, ldc, tm * kTileM + static_cast<int>(rank) * kCtaRows + quarter * 32, m,
-                                             tn * kTileN + col_base, n, lane);
+        if (forward) gemm_forward_rows_to_peers<kUnitCols>(ep, c, ldc, row0, m, col0, n, lane);
+        if (turn + 1 < kTurns) {
+          __syncwarp();
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        }
       }
     }
   }
