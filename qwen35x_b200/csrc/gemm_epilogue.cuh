@@ -166,17 +166,15 @@ __device__ __forceinline__ void store_nvfp4_chunk32(const uint32_t (&r)[32], int
 
 // r: 32 accumulator columns starting at global column col0 (a multiple of 32) of row `row`; n = accumulator columns
 // of the whole problem (weight rows); g = the activation tensor's scale.
-// GATE_UP: the weight may be a gate/up one (false keeps that code out of a kernel that never sees one).
 // to_peers: also repeat every store on the other ranks (one 32-byte piece per lane); a caller that forwards whole
 // rows afterwards (gemm_forward_rows_to_peers) passes false.
-template <bool GATE_UP>
 __device__ __forceinline__ void gemm_store_chunk32(const uint32_t (&r)[32], int row, int col0, int n, float g,
                                                    const GemmEpilogue & ep, __nv_bfloat16 * __restrict__ c, int ldc,
                                                    bool to_peers, const GemmQuantScale & q) {
   if (col0 >= n) return;  // a chunk wholly past the last column of a partial tile
   const int n_peers = to_peers ? ep.n_peers : 0;
   const float alpha = g * ep.s2;
-  if (GATE_UP && ep.gate_up) {
+  if (ep.gate_up) {
     const float alpha_up = g * ep.s2_up;
     if (ep.q_codes != nullptr) {
       store_nvfp4_chunk32<true>(r, row, col0, alpha, alpha_up, ep, q);  // n % 32 == 0 is checked on the host: the chunk is whole

@@ -15,7 +15,7 @@
 //     accumulator-ready to both CTAs;
 //   - two accumulators alternate, so that a tile's MMAs run while the one before is converted and stored.  Beside 48
 //     columns of scale factors 512 columns of TMEM do not hold two of 256: the second starts at column 208 and shares 48
-//     with the first (OVERLAP below).  The 64 columns of a tile that hold them are read out first, and the next tile's MMAs
+//     with the first (OVERLAP below).  The 64 columns that hold them are read out of a tile first, and the next tile's MMAs
 //     wait for these alone; all others have a tile's time to leave.
 //
 // What bounds it: the power cap.  At [4096, 2560] x [18432, 2560] the SM clock falls to 1.5 GHz within a millisecond and to
@@ -47,21 +47,27 @@ constexpr int kSfbBytes = 2 * kMmaPerStage * kSfChunk;
 constexpr int kStageBytes = kABytes + kBBytes + kSfaBytes + kSfbBytes;   // 38912
 constexpr int kStages = 5;
 // Epilogue warps per CTA (template parameter of the kernel), a multiple of four: kEpilogueWarps / 4 per TMEM lane
-// quarter, which take turns at the 64-column units of the accumulator.  Sixteen for the epilogues that do arithmetic on what
-// they drain (SiLU, NVFP4 output) and for launches that forward rows to peers; eight for the plain and the residual epilogue,
-// which measured 1-5 % faster with fewer warps.
+// quarter, which take turns at the 32-column chunks of the accumulator.  Eight for the plain and the residual epilogue,
+// whose chunks leave through shared memory as TMA boxes of 32 x 32 values, two per warp in turn; sixteen for the epilogues that do
+// arithmetic on what they drain (SiLU, NVFP4 output) and for launches that forward rows to peers, which store per lane.
+// Either is a loop of few instructions: unrolled over the chunks it fetched them anew for every tile, 3900 cycles for 128
+// columns, and pushed the MMA issuer's out of the instruction cache.  With loop and boxes [4096, 2560] x [18432, 2560] went
+// from 81.5 to 80.5 us, and quantise + GEMM in a loop at the power cap from 113.3 to 110.7.
 constexpr int kEpiWarpsWide = 16;
 constexpr int kEpiWarpsPlain = 8;
-constexpr int kUnitCols = 64;
-constexpr int kUnits = kTileN / kUnitCols;
-constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 256;
-static_assert(kStages * kStageBytes + 1024 + 256 <= 227 * 1024, "shared memory");
+constexpr int kChunkCols = 32;
+constexpr int kChunks = kTileN / kChunkCols;
+constexpr int kBoxBytes = 32 * kChunkCols * 2;
+constexpr int kBoxOffset = kStages * kStageBytes + 512;  // of the boxes, behind the barriers; the swizzle repeats every 512 bytes
+constexpr int kSmemBytes = 1024 + kBoxOffset;
+constexpr int kSmemBytesPlain = kSmemBytes + kEpiWarpsPlain * 2 * kBoxBytes;
+static_assert(kSmemBytesPlain <= 227 * 1024 && kBoxOffset % 512 == 0, "shared memory");
 constexpr int kSfaCols = kMmaPerStage * 4;
 constexpr int kSfbCols = kMmaPerStage * 8;
 constexpr int kTmemCols = 512;
 // OVERLAP: the second accumulator ends where the scale factors begin.
 constexpr int kAcc1 = kTmemCols - kSfaCols - kSfbCols - kTileN;  // its first column, 208
-static_assert(kAcc1 < kTileN && kTileN - kAcc1 <= kUnitCols, "the shared columns lie in the first accumulator's last unit and the second one's first");
+static_assert(kAcc1 < kTileN && kTileN - kAcc1 <= 2 * kChunkCols, "the shared columns lie in the first accumulator's last two chunks and the second one's first two");
 constexpr uint32_t kWaitLimit = 1u << 20;
 constexpr uint32_t kPeerMask = 0xFEFFFFFFu;  // clears the CTA-rank bit of a shared::cluster address: the pair's leader
 
@@ -170,14 +176,32 @@ __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+// The first `count` (below eight) of eight BF16 values, as a register each two: the ragged end of a residual's row.
+__device__ __noinline__ uint4 load_bf16_tail(const __nv_bfloat16 * p, int count) {
+  uint64_t w[2] = {0u, 0u};
+  for (int i = 0; i < count; ++i) w[i >> 2] |= static_cast<uint64_t>(__ldca(reinterpret_cast<const unsigned short *>(p) + i)) << (16 * (i & 3));
+  return make_uint4(static_cast<uint32_t>(w[0]), static_cast<uint32_t>(w[0] >> 32), static_cast<uint32_t>(w[1]), static_cast<uint32_t>(w[1] >> 32));
+}
+
+// The first `count` (up to eight) of eight BF16 values into 16-byte aligned memory.
+__device__ __noinline__ void store_bf16_tail(__nv_bfloat16 * p, uint4 v, int count) {
+  if (count >= 8) {
+    *reinterpret_cast<uint4 *>(p) = v;
+    return;
+  }
+  const uint64_t w[2] = {v.x | static_cast<uint64_t>(v.y) << 32, v.z | static_cast<uint64_t>(v.w) << 32};
+  for (int i = 0; i < count; ++i) reinterpret_cast<unsigned short *>(p)[i] = static_cast<unsigned short>(w[i >> 2] >> (16 * (i & 3)));
+}
+
 template <int kEpilogueWarps>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((2 + kEpilogueWarps) * 32, 1)
 gemm_w4a4_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                       const __grid_constant__ CUtensorMap tmap_sfa, const __grid_constant__ CUtensorMap tmap_sfb,
+                      const __grid_constant__ CUtensorMap tmap_c,  // of the output, for the plain epilogue
                       const float * __restrict__ g_dev, const GemmEpilogue ep, int m, int n, int k_bytes, int m_tiles, int num_tiles,
                       __nv_bfloat16 * __restrict__ c, int ldc, unsigned int * status) {
-  constexpr int kTurns = kUnits / (kEpilogueWarps / 4);  // units of a tile that one epilogue warp takes
-  static_assert(kEpilogueWarps % 4 == 0 && kTurns * (kEpilogueWarps / 4) == kUnits, "epilogue column split");
+  constexpr int kColWarps = kEpilogueWarps / 4, kTurns = kChunks / kColWarps;  // chunks of a tile that one epilogue warp takes
+  static_assert(kEpilogueWarps % 4 == 0 && kColWarps >= 2 && kTurns * kColWarps == kChunks, "epilogue column split");
   extern __shared__ uint8_t smem_raw[];
   uint8_t * smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint8_t * smem_a = smem;
@@ -323,8 +347,9 @@ gemm_w4a4_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
   } else {
     // ---------------- epilogue (both CTAs): this CTA's 128 rows of the pair's tile ----------------
     const int quarter = warp & 3;                 // TMEM lanes 32 * quarter .. + 31 (fixed by the warp's index)
-    const int turn0 = (warp - 2) >> 2;
+    const int col_warp = (warp - 2) >> 2;
     const float g = __ldcg(g_dev);
+    const float alpha = g * ep.s2;
     GemmQuantScale q;
     if constexpr (kEpilogueWarps == kEpiWarpsWide) {
       __shared__ float q_table[128];
@@ -342,46 +367,99 @@ gemm_w4a4_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, ++li) {
       const int tm = tile % m_tiles;
       const int tn = tile / m_tiles;
-      if (!mbar_wait(smem_u32(tmem_full), li & 1)) {
-        if (lane == 0) atomicExch(status, kEpilogueWait);
-        ok = false;
-        break;
-      }
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const int row0 = tm * kTileM + static_cast<int>(rank) * kCtaRows + quarter * 32;
       const uint32_t taddr = tmem_acc + (li & 1) * kAcc1 + (static_cast<uint32_t>(quarter * 32) << 16);
-      // the unit with the shared columns comes first: the last of the first accumulator, the first of the second
-      auto unit = [&](int turn) { return static_cast<int>((turn0 + turn * (kEpilogueWarps / 4) + ((li & 1) != 0u ? 0 : kUnits - 1)) % kUnits) * kUnitCols; };
-      uint32_t r[kTurns][2][32];
-      auto load = [&](int turn) {
-        tmem_ld32(taddr + unit(turn), r[turn][0]);
-        tmem_ld32(taddr + unit(turn) + 32, r[turn][1]);
-      };
-      load(0);
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) mbar_arrive_leader(smem_u32(drained));
-      // plain BF16 output of a gathering launch: store locally, then forward whole rows; the fused epilogues (and a
-      // launch without peers) store per lane
-      const bool forward = ep.n_peers > 0 && !ep.gate_up && ep.forward_rows != 0;
+      // the chunks with the shared columns come first: the last two of the first accumulator, the first two of the second
+      const int chunk0 = (li & 1) != 0u ? col_warp : col_warp + kChunks - 2;
+      if constexpr (kEpilogueWarps == kEpiWarpsPlain) {
+        const uint32_t box0 = smem_u32(smem + kBoxOffset) + (warp - 2) * 2 * kBoxBytes;
+        const __nv_bfloat16 * res = ep.residual != nullptr && row0 + lane < m ? ep.residual + static_cast<size_t>(row0 + lane) * ep.ldr : nullptr;
+#pragma unroll 1
+        for (int turn = 0; turn < kTurns; ++turn) {
+          const int chunk = (chunk0 + turn * kColWarps) & (kChunks - 1);
+          const int col0 = tn * kTileN + chunk * kChunkCols;
+          uint4 rr[4] = {};
+          if (res != nullptr) {  // asked for before the sums are there
 #pragma unroll
-      for (int turn = 0; turn < kTurns; ++turn) {
-        const int col0 = tn * kTileN + unit(turn);
-        if (turn + 1 < kTurns) load(turn + 1);  // on its way while this one is stored
-        if (row0 + lane < m) {
+            for (int i = 0; i < 4; ++i) {
+              if (col0 + 8 * i + 8 <= n) {
+                rr[i] = __ldca(reinterpret_cast<const uint4 *>(res + col0 + 8 * i));
+              } else if (col0 + 8 * i < n) {
+                rr[i] = load_bf16_tail(res + col0 + 8 * i, n - col0 - 8 * i);
+              }
+            }
+          }
+          if (turn == 0) {
+            ok = mbar_wait(smem_u32(tmem_full), li & 1);
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          }
+          uint32_t r[32];
+          tmem_ld32(taddr + chunk * kChunkCols, r);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          if (turn == 0) {
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive_leader(smem_u32(drained));
+          }
+          // the box before last has been read
+          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+          __syncwarp();
+          const uint32_t box = box0 + (turn & 1) * kBoxBytes;
+          const bool whole = col0 + kChunkCols <= n;  // a box that is cut off in the middle of 16 bytes writes them all
 #pragma unroll
-          for (int j = 0; j < 2; ++j) {
-            gemm_store_chunk32<kEpilogueWarps == kEpiWarpsWide>(r[turn][j], row0 + lane, col0 + 32 * j, n, g, ep, c, ldc, !forward, q);
+          for (int i = 0; i < 4; ++i) {
+            const uint32_t rw[4] = {rr[i].x, rr[i].y, rr[i].z, rr[i].w};
+            uint32_t p[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              p[e] = pack_bf16(fmaf(__uint_as_float(r[8 * i + 2 * e]), alpha, __uint_as_float(rw[e] << 16)),
+                               fmaf(__uint_as_float(r[8 * i + 2 * e + 1]), alpha, __uint_as_float(rw[e] & 0xffff0000u)));
+            }
+            if (!whole) {
+              if (row0 + lane < m && col0 + 8 * i < n) store_bf16_tail(c + static_cast<size_t>(row0 + lane) * ldc + col0 + 8 * i, make_uint4(p[0], p[1], p[2], p[3]), n - col0 - 8 * i);
+              continue;
+            }
+            // 64-byte swizzle: eight lanes' pieces lie in eight different sixteenths of the 128-byte span of the banks
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(box + lane * 64 + ((i ^ (lane >> 1 & 3)) << 4)), "r"(p[0]), "r"(p[1]), "r"(p[2]), "r"(p[3]) : "memory");
+          }
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) {
+            // rows past m are not written
+            if (whole && row0 < m) {
+              asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(&tmap_c), "r"(box), "r"(col0), "r"(row0) : "memory");
+            }
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
           }
         }
-        if (forward) gemm_forward_rows_to_peers<kUnitCols>(ep, c, ldc, row0, m, col0, n, lane);
-        if (turn + 1 < kTurns) {
-          __syncwarp();
+      } else {
+        // plain BF16 output of a gathering launch: store locally, then forward whole rows, whose chunks are neighbours then;
+        // the fused epilogues (and a launch without peers) store per lane
+        const bool forward = ep.n_peers > 0 && !ep.gate_up && ep.forward_rows != 0;
+        ok = mbar_wait(smem_u32(tmem_full), li & 1);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll 1
+        for (int turn = 0; turn < kTurns; ++turn) {
+          const int chunk = forward ? col_warp * kTurns + turn : (chunk0 + turn * kColWarps) & (kChunks - 1);
+          uint32_t r[32];
+          tmem_ld32(taddr + chunk * kChunkCols, r);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          if (turn == (forward ? kTurns - 1 : 0)) {
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive_leader(smem_u32(drained));
+          }
+          if (row0 + lane < m) gemm_store_chunk32(r, row0 + lane, tn * kTileN + chunk * kChunkCols, n, g, ep, c, ldc, !forward, q);
+          __syncwarp();
         }
+        if (forward) gemm_forward_rows_to_peers<kTurns * kChunkCols>(ep, c, ldc, row0, m, tn * kTileN + col_warp * kTurns * kChunkCols, n, lane);
       }
     }
+    if (!ok && !aborted && lane == 0) atomicExch(status, kEpilogueWait);
+    // the boxes stay until they have been stored
+    if (kEpilogueWarps == kEpiWarpsPlain && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
 
   gemm_signal_peers(ep, status);
@@ -397,8 +475,9 @@ gemm_w4a4_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
 
 }  // namespace
 
-// 2-D map over a tiled scale array seen as [chunks, 128 x u32]: box = 4 consecutive 512-byte chunks.
-int make_sf_map(CUtensorMap * map, const void * base, long long chunks) {
+namespace {
+int encode_map(CUtensorMap * map, CUtensorMapDataType type, const void * base, cuuint64_t inner, cuuint64_t outer, cuuint64_t stride, cuuint32_t box_inner,
+               cuuint32_t box_outer, CUtensorMapSwizzle swizzle, const char * what) {
   using Fn = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
                           const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
                           CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -411,17 +490,28 @@ int make_sf_map(CUtensorMap * map, const void * base, long long chunks) {
     }
     fn = reinterpret_cast<Fn>(p);
   }
-  const cuuint64_t dims[2] = {128, static_cast<cuuint64_t>(chunks)};
-  const cuuint64_t strides[1] = {512};
-  const cuuint32_t box[2] = {128, 4};
+  const cuuint64_t dims[2] = {inner, outer};
+  const cuuint64_t strides[1] = {stride};
+  const cuuint32_t box[2] = {box_inner, box_outer};
   const cuuint32_t elem[2] = {1, 1};
-  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void *>(base), dims, strides, box, elem,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  const CUresult r = fn(map, type, 2, const_cast<void *>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
-    return fail(Q35B_ERR_CUDA, "cuTensorMapEncodeTiled(scale factors) failed with CUresult " + std::to_string(static_cast<int>(r)) + ".");
+    return fail(Q35B_ERR_CUDA, std::string("cuTensorMapEncodeTiled(") + what + ") failed with CUresult " + std::to_string(static_cast<int>(r)) + ".");
   }
   return Q35B_OK;
+}
+
+// 2-D map over the BF16 output [m, n] with rows ldc apart: boxes of 32 x 32 values.
+int make_output_map(CUtensorMap * map, const void * c, int m, int n, int ldc) {
+  return encode_map(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, c, static_cast<cuuint64_t>(n), static_cast<cuuint64_t>(m), static_cast<cuuint64_t>(ldc) * 2,
+                    kChunkCols, 32, CU_TENSOR_MAP_SWIZZLE_64B, "output");
+}
+}  // namespace
+
+// 2-D map over a tiled scale array seen as [chunks, 128 x u32]: box = 4 consecutive 512-byte chunks.
+int make_sf_map(CUtensorMap * map, const void * base, long long chunks) {
+  return encode_map(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, base, 128, static_cast<cuuint64_t>(chunks), 512, 128, 4, CU_TENSOR_MAP_SWIZZLE_NONE, "scale factors");
 }
 
 int build_weight_maps(q35b_weight * w) {
@@ -443,7 +533,7 @@ int launch_gemm_w4a4_2cta(const q35b_weight * w, const uint8_t * a_codes, const 
   if (!attr_set[w->device & 63].load(std::memory_order_acquire)) {
     Q35B_CUDA_TRY(cudaFuncSetAttribute(gemm_w4a4_2cta_kernel<kEpiWarpsWide>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes),
                   "cudaFuncSetAttribute(2-CTA gemm smem)");
-    Q35B_CUDA_TRY(cudaFuncSetAttribute(gemm_w4a4_2cta_kernel<kEpiWarpsPlain>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes),
+    Q35B_CUDA_TRY(cudaFuncSetAttribute(gemm_w4a4_2cta_kernel<kEpiWarpsPlain>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytesPlain),
                   "cudaFuncSetAttribute(2-CTA gemm smem)");
     attr_set[w->device & 63].store(true, std::memory_order_release);
   }
@@ -454,12 +544,17 @@ int launch_gemm_w4a4_2cta(const q35b_weight * w, const uint8_t * a_codes, const 
   const int n_tiles = (w->rows + kTileN - 1) / kTileN;
   const int num_tiles = m_tiles * n_tiles;
   const int pairs = std::max(1, std::min(num_tiles, sm_count() / 2));
-  // plain and residual epilogues without peers: the narrow set of epilogue warps
-  const bool plain = !ep.gate_up && ep.q_codes == nullptr && ep.n_peers == 0;
+  // plain and residual epilogues without peers whose rows a TMA box can be stored to
+  const bool plain = !ep.gate_up && ep.q_codes == nullptr && ep.n_peers == 0 && (ldc % 8) == 0 && (reinterpret_cast<uintptr_t>(c_bf16) & 15u) == 0 &&
+                     (ep.residual == nullptr || ((ep.ldr % 8) == 0 && (reinterpret_cast<uintptr_t>(ep.residual) & 15u) == 0));
+  CUtensorMap tmap_c = tmap_a;
+  if (plain) {
+    if (const int st = make_output_map(&tmap_c, c_bf16, m, w->rows, ldc)) return st;
+  }
   const int epi_warps = plain ? kEpiWarpsPlain : kEpiWarpsWide;
   const auto kernel = plain ? gemm_w4a4_2cta_kernel<kEpiWarpsPlain> : gemm_w4a4_2cta_kernel<kEpiWarpsWide>;
-  const cudaError_t le = launch_pdl(kernel, dim3(2 * pairs), dim3((2 + epi_warps) * 32), kSmemBytes, s, tmap_a, w->tmap2_codes,
-                                    tmap_sfa, w->tmap2_sf, g_dev, ep, m, w->rows, w->k / 2, m_tiles, num_tiles,
+  const cudaError_t le = launch_pdl(kernel, dim3(2 * pairs), dim3((2 + epi_warps) * 32), plain ? kSmemBytesPlain : kSmemBytes, s, tmap_a, w->tmap2_codes,
+                                    tmap_sfa, w->tmap2_sf, tmap_c, g_dev, ep, m, w->rows, w->k / 2, m_tiles, num_tiles,
                                     static_cast<__nv_bfloat16 *>(c_bf16), ldc, status_dev);
   count_launch();
   Q35B_CUDA_TRY(le, "gemm_w4a4_2cta_kernel launch");
