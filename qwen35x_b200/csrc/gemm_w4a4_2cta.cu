@@ -109,6 +109,9 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
     "l"(map), "r"(leader_bar), "r"(x), "r"(y)
     : "memory");
 }
+__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap * map, int x, int y) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
+}
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred;
   asm volatile(
@@ -269,6 +272,16 @@ gemm_w4a4_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         const int sfb_rb = (tn * kTileN) >> 7;  // first of the two 128-row scale tiles
         const int sfb_chunk0 = sfb_rb * sf_col_blocks;
         const int sfb_chunk1 = (sfb_rb + 1) * sf_col_blocks;
+        // The weights of the pair's next tile come from HBM, where they queue up behind the output that is being written (waits
+        // of up to 1700 cycles, longer than the ring): into L2 with them now, the K steps shared out among the pairs that
+        // will read them.  With the order of waits in the MMA issuer 80.5 -> 75.4 us.
+        if (const int next = tile + num_pairs; next < num_tiles) {
+          const int next_row = next / m_tiles * kTileN;
+          for (int ks = next % m_tiles; ks < k_steps; ks += m_tiles) {
+            tma_prefetch_2d(&tmap_b, ks * kStepBytes, next_row + static_cast<int>(rank) * kCtaBRows);
+            tma_prefetch_2d(&tmap_sfb, 0, ((next_row >> 7) + static_cast<int>(rank)) * sf_col_blocks + ks * kMmaPerStage);
+          }
+        }
         for (int ks = 0; ks < k_steps; ++ks) {
           if (!mbar_wait(smem_u32(empty + stage), phase ^ 1)) {
             atomicExch(status, kProducerWait);
@@ -299,14 +312,7 @@ gemm_w4a4_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       uint32_t li = 0;
       bool ok = true;
       for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, ++li) {
-        // the shared columns of the tile before are read out, and with them all of the one before that
-        if (!mbar_wait(smem_u32(drained), (li & 1) ^ 1)) {
-          atomicExch(status, kMmaDrainWait);
-          ok = false;
-          break;
-        }
         const uint32_t acc = tmem_acc + (li & 1) * kAcc1;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         for (int ks = 0; ks < k_steps; ++ks) {
           if (!mbar_wait(smem_u32(full + stage), phase)) {
             atomicExch(status, kMmaWait);
@@ -327,6 +333,16 @@ gemm_w4a4_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
               utccp_sf_pair(tmem_sfb + j * 8, sfb_desc + j * (kSfChunk >> 4));
               utccp_sf_pair(tmem_sfb + j * 8 + 4, sfb_desc + (kSfaBytes >> 4) + j * (kSfChunk >> 4));
             }
+          }
+          // the scale factors are on their way; the shared columns of the tile before are read out, and with them all of
+          // the one before that
+          if (ks == 0) {
+            if (!mbar_wait(smem_u32(drained), (li & 1) ^ 1)) {
+              atomicExch(status, kMmaDrainWait);
+              ok = false;
+              break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           }
 #pragma unroll
           for (int j = 0; j < kMmaPerStage; ++j) {
