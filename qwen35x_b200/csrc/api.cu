@@ -113,6 +113,25 @@ using namespace q35b;
 // short K or several tokens the streaming kernel would be ahead from 4 to 12 MiB on.
 static constexpr size_t kAutoStreamBytes = 24u << 20;
 
+// Q35B_GEMV_AUTO sends one to the resident tensor-core kernel (gemm_resident.cu) where the estimates, fitted to graph replays,
+// are more than 0.7 us apart: long K or several tokens, for which the rows kernel's warps unpack one piece after the other.
+// us, rows or streaming kernel / resident kernel, one, two and four tokens: [2560, 9216] 17.1 / 6.6, 18.3 / 7.5, 26.9 / 10.2;
+// [2560, 2560] 5.6 / 4.9, 5.8 / 5.2, 8.6 / 6.3; [32768, 1024] 8.2 / 6.1, 11.3 / 7.0, 16.7 / 9.6; [16000, 4096] 14.7 / 9.7, 15.1 / 12.8, -;
+// left where they were [3584, 1024] 2.6 / 4.6, 2.8 / 5.0, 4.3 / 5.4 and [300, 4096] 2.0 / 4.5, 2.3 / 4.5, 2.9 / 5.0.
+static bool resident_projection(const q35b_weight * w, int m) {
+  double other;
+  if (w->codes_bytes + w->scales_bytes >= kAutoStreamBytes && gemv_stream_eligible(w, m)) {
+    // whole tiles, one or two to an SM at a time, and so much per K step
+    const int tiles = (w->rows + 127) / 128, sms = sm_count();
+    other = 2000.0 + w->k / 256 * (tiles <= sms ? 780.0 : 960.0) * ((tiles + 2 * sms - 1) / (2 * sms));
+  } else {
+    other = gemv_rows_ns(w, m);
+  }
+  if (other < 5500.0) return false;
+  const double ns = decode_resident_ns(w, m);
+  return ns > 0.0 && ns + 700.0 < other;
+}
+
 extern "C" {
 
 const char * q35b_last_error(void) { return t_error.c_str(); }
@@ -293,6 +312,13 @@ size_t q35b_weight_stream_bytes(const q35b_weight * w) { return w ? w->codes_byt
 
 int q35b_gemv_w4a16_bf16(const q35b_weight * w, const void * x_bf16, int m, void * y_bf16, int kernel,
                          q35b_stream stream) {
+  if (kernel == Q35B_GEMV_AUTO && w != nullptr && x_bf16 != nullptr && y_bf16 != nullptr && m >= 1 && m <= 8 && w->rows > 0 && !w->gate_up &&
+      (reinterpret_cast<uintptr_t>(x_bf16) & 15u) == 0 && resident_projection(w, m)) {
+    if (const int st = check_weight_device(w)) return st;
+    unsigned int * status = nullptr;
+    if (const int st = default_status_word(&status)) return st;
+    return launch_decode_resident(w, x_bf16, m, y_bf16, nullptr, false, nullptr, status, 1u << 20, static_cast<cudaStream_t>(stream));
+  }
   if (kernel == Q35B_GEMV_AUTO && w != nullptr && m >= 1 && m <= 8 && !w->gate_up &&
       w->codes_bytes + w->scales_bytes >= kAutoStreamBytes && x_bf16 != nullptr &&
       (reinterpret_cast<uintptr_t>(x_bf16) & 15u) == 0 && gemv_stream_eligible(w, m)) {

@@ -93,6 +93,7 @@ namespace q35b {
 // gemv_w4a16.cu
 int launch_dequant_bf16(const q35b_weight * w, void * w_bf16, cudaStream_t s);
 int launch_gemv_bf16(const q35b_weight * w, const void * x_bf16, int m, void * y_bf16, int kernel, cudaStream_t s);
+double gemv_rows_ns(const q35b_weight * w, int m);  // estimate for the kernel of any shape
 int launch_gemv_f32(const q35b_weight * w, const float * x, float input_scale, float * y, int kernel, cudaStream_t s);
 
 // act_quant.cu
@@ -154,8 +155,6 @@ int default_status_word(unsigned int ** out);
 int launch_gemm_w4a4(const q35b_weight * w, const uint8_t * a_codes, const uint8_t * a_scales_tiled, const float * g_dev,
                      int m, void * c_bf16, int ldc, const void * residual_bf16, int ldr, unsigned int * status_dev,
                      cudaStream_t s, const GemmQuantOut * qout = nullptr, const GemmGather * gather = nullptr);
-
-
 // gemm_wstream.cu: decode work lists on the tensor cores
 struct WBatch;  // decode work list on the tensor path (digit-expanded activations)
 // exact: all bits of the activations, their infinities and NaNs too, reach the outputs (else what `digits` digits hold)
@@ -167,6 +166,16 @@ void wbatch_free(WBatch * b);
 int wbatch_status(const WBatch * b, unsigned int * out);
 size_t wbatch_bytes(const WBatch * b);
 int wbatch_debug_wait(WBatch * b, unsigned int wait_limit);
+
+// gemm_resident.cu: few tokens, the operand made in shared memory
+bool decode_resident_chain(const q35b_weight * w, int m);  // fits as one launch of several
+double decode_resident_ns(const q35b_weight * w, int m);  // estimate for one projection; 0: it does not fit
+// next: the weight that the launch after this one streams (brought into L2 under this one), or NULL
+int launch_decode_resident(const q35b_weight * w, const void * x_bf16, int m, void * y_bf16, const void * residual_bf16, bool chain,
+                           const q35b_weight * next, unsigned int * status, unsigned int wait_limit, cudaStream_t s);
+bool prefill_resident_shape(const q35b_weight * w, int m, float scale, int split, int * stages, int * smem);
+int launch_prefill_resident(const q35b_weight * w, const void * x, bool f32, int m, float scale, uint8_t * codes, uint8_t * scales, float * g_dev, int split, int stages,
+                            int smem, const void * residual, int ldr, void * c, int ldc, unsigned int * status, cudaStream_t s);
 
 // gemm_w4a4_2cta.cu
 bool gemm_2cta_eligible(int rows, int m, int k);

@@ -31,6 +31,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "digits.cuh"
 #include "engine.h"
 #include "nvfp4_codec.cuh"
 
@@ -58,8 +59,6 @@ constexpr int kSmemBudget = 220 * 1024;   // dynamic part; the staged tile descr
 
 enum StatusCode : unsigned { kWeightWait = 41, kActWait = 42, kMmaWait = 43, kMmaDrainWait = 44, kEpilogueWait = 45 };
 enum Epilogue : int { kEpiPlain = 0, kEpiGateUp = 1 };
-
-constexpr int kDeepDigits = 6;           // of a list that takes the activations exactly (see split_digits_kernel)
 
 // One projection of the list, in device memory; the tensor maps are read by the TMA unit from there.
 struct alignas(128) WItem {
@@ -217,47 +216,6 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                : "r"(taddr)
                : "memory");
-}
-
-// The outputs (one per lane, weight row `row`) of a token that has infinities but no NaN.  Next to an infinity the finite
-// activations do not matter, so a warp looks for the infinities, 256 columns at a time, and takes only their products: an
-// infinity, or a NaN where the weight is zero.  It stops as soon as every output is a NaN, which opposite signs bring about
-// within a few infinities.  A 4B-class step with an infinity in one token, in all of eight tokens: 0.49 and 1.7 ms, against
-// 0.31 and 0.35 without; a serial sum over all columns for each output took 9.3 and 58.
-__device__ __noinline__ float infinite_dot(const WItem * it, int row, int token, int lane) {
-  const int k = it->k_steps * 256, row_block = row / kRows;
-  const bool live = row < it->rows;
-  const uint8_t * codes = it->w_codes + static_cast<size_t>(live ? row : 0) * (k >> 1);
-  const uint4 * x = reinterpret_cast<const uint4 *>(it->x + static_cast<size_t>(token) * k);
-  float sum = 0.0f;
-#pragma unroll 1
-  for (int base = 0; base < k; base += 256) {
-    const uint4 q = __ldcg(x + (base >> 3) + lane);
-    const uint32_t r[4] = {q.x, q.y, q.z, q.w};
-    uint32_t found = 0;  // bit i: this lane's value i is infinite; bit 8 + i: and negative
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const uint32_t v = r[i >> 1] >> (16 * (i & 1)) & 0xffffu;
-      if ((v & 0x7fffu) == 0x7f80u) found |= (v >> 15 != 0u ? 0x101u : 1u) << i;
-    }
-    uint32_t lanes = __ballot_sync(0xffffffffu, found != 0u);
-    while (lanes != 0u) {
-      const int src = __ffs(lanes) - 1;
-      lanes &= lanes - 1;
-      const uint32_t f = __shfl_sync(0xffffffffu, found, src);
-      const int c = (base >> 3) + src;  // eight columns of one block
-      const uint32_t word = *reinterpret_cast<const uint32_t *>(codes + c * 4);
-      const float scale = live ? decode_e4m3(it->w_scales[tiled_scale_offset(row_block * kRows + (row & (kRows - 1)), c >> 1, k >> 4)]) : 0.0f;
-#pragma unroll 1
-      for (int i = 0; i < 8; ++i) {
-        if ((f >> i & 1u) == 0u) continue;
-        const float inf = __uint_as_float((f >> (8 + i) & 1u) != 0u ? 0xff800000u : 0x7f800000u);
-        sum = fmaf(decode_e2m1(static_cast<uint8_t>(word >> (4 * i) & 15u)) * inf, scale, sum);
-      }
-      if (__all_sync(0xffffffffu, sum != sum || !live)) return sum;
-    }
-  }
-  return sum;
 }
 
 // CTA b walks tiles[cta_begin[b] .. cta_begin[b + 1]).
@@ -579,7 +537,7 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
         }
         if (!(g < INFINITY)) {
           // a token with NaNs has nothing else to give: a NaN times anything is one
-          sum = g != g ? g : infinite_dot(it->item, row, token, lane);
+          sum = g != g ? g : infinite_dot(it->item->w_codes, it->item->w_scales, it->item->x + static_cast<size_t>(token) * it->k_steps * 256, rows, it->k_steps * 256, 0, it->k_steps * 256, row, lane);
           g = 1.0f;
         }
         // g is a power of two, possibly a subnormal one: it comes last, so that nothing underflows before the result does
@@ -627,31 +585,6 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
 
 // ---- decode: BF16 activations -> octal digits in NVFP4 ----------------------------------------------------------
 
-// Eight fp32 values -> one word of eight E2M1 codes, nearest; element 2j in the low nibble of byte j.
-__device__ __forceinline__ uint32_t to_e2m1x8(const float (&q)[8]) {
-  uint32_t w;
-  asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\t"
-      "cvt.rn.satfinite.e2m1x2.f32 b0, %2, %1;\n\t"
-      "cvt.rn.satfinite.e2m1x2.f32 b1, %4, %3;\n\t"
-      "cvt.rn.satfinite.e2m1x2.f32 b2, %6, %5;\n\t"
-      "cvt.rn.satfinite.e2m1x2.f32 b3, %8, %7;\n\t"
-      "mov.b32 %0, {b0, b1, b2, b3};\n\t}"
-      : "=r"(w)
-      : "f"(q[0]), "f"(q[1]), "f"(q[2]), "f"(q[3]), "f"(q[4]), "f"(q[5]), "f"(q[6]), "f"(q[7]));
-  return w;
-}
-// The two E2M1 codes of a byte (low nibble first) -> fp32.
-__device__ __forceinline__ void from_e2m1x2(uint32_t byte, float & lo, float & hi) {
-  asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\t.reg .b32 h;\n\t.reg .b16 l, u;\n\t"
-      "mov.b32 {b0, b1, b2, b3}, %2;\n\t"
-      "cvt.rn.f16x2.e2m1x2 h, b0;\n\t"
-      "mov.b32 {l, u}, h;\n\t"
-      "cvt.f32.f16 %0, l;\n\t"
-      "cvt.f32.f16 %1, u;\n\t}"
-      : "=f"(lo), "=f"(hi)
-      : "r"(byte));
-}
-
 struct ExpandItem {
   const __nv_bfloat16 * x;   // [tokens, k], k a multiple of 256
   uint8_t * ops;             // see WItem::x_ops; operand row = token * digits + digit, and likewise of the deep digits
@@ -666,12 +599,7 @@ struct ExpandItem {
 constexpr int kSplitThreads = 256;
 constexpr int kDeepWords = 64;   // of 32 K steps each: 524288 columns, more than a list on either path can have
 
-// One CTA per (projection, token).  A block of sixteen values whose largest has exponent e is counted in units of
-// 2^(e - 1), which makes every value less than 4: digit 0 is the nearest E2M1 number (up to 4 the grid is no coarser than
-// 1, so at most half a unit is left over), digit 1 the nearest to eight times the rest, and so on; all of it is exact in
-// fp32.  The unit goes into the block's scale byte, a power of two relative to the token's largest exponent (down to 2^-17
-// of it, the range of E4M3), and 8^-j into the epilogue.  d digits leave at most 2^(e + 1 - 3 d), and nothing of a value
-// whose last bit is not below 2^(e + 2 - 3 d).
+// One CTA per (projection, token); digits.cuh has what they are.
 // With deep digits (a list that has to be as exact as BF16 activations converted to fp16 by one power of two per token,
 // which keep multiples of 2^-38 of the token's largest binade): where the first eight leave something of any value of a K
 // step, six more are written, fourteen in all, which hold multiples of 2^-40 of the block's largest binade; the step is
@@ -703,15 +631,10 @@ __global__ void __launch_bounds__(kSplitThreads) split_digits_kernel(const Expan
     }
     return q;
   };
-  // largest of the magnitudes' bit patterns
-  auto abs_max = [](const uint4 & q) {
-    const uint32_t a = __vmaxu2(__vmaxu2(q.x & 0x7fff7fffu, q.y & 0x7fff7fffu), __vmaxu2(q.z & 0x7fff7fffu, q.w & 0x7fff7fffu));
-    return max(a & 0xffffu, a >> 16);
-  };
   asm volatile("griddepcontrol.wait;" ::: "memory");  // the activations may come from the kernel before
   uint32_t best = 0, before = 0;
   if (it.deep != nullptr && static_cast<int>(threadIdx.x) < words) before = __ldcg(it.deep + 8 * threadIdx.x + token);
-  for (int c = threadIdx.x; c < chunks; c += kSplitThreads) best = max(best, abs_max(load(c)));
+  for (int c = threadIdx.x; c < chunks; c += kSplitThreads) best = max(best, bf16x8_abs_max(load(c)));
   best = __reduce_max_sync(0xffffffffu, best);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = best;
   if (threadIdx.x < kDeepWords) {
@@ -723,39 +646,22 @@ __global__ void __launch_bounds__(kSplitThreads) split_digits_kernel(const Expan
   for (int i = 0; i < kSplitThreads / 32; ++i) best = max(best, red[i]);
   const int top = max(static_cast<int>(best >> 7), 1);  // exponent field of the token's largest value
   if (threadIdx.x == 0) {
-    // 2^(top - 136): the unit of a block at the token's largest exponent is 2^(top - 128), and its scale byte stands for 2^8
-    const uint32_t bits = top > 9 ? static_cast<uint32_t>(top - 9) << 23 : 1u << (top + 13);
-    it.g[token] = __uint_as_float(best > 0x7f80u ? 0x7fffffffu : (best == 0x7f80u ? 0x7f800000u : bits));
+    it.g[token] = best > 0x7f80u ? __uint_as_float(0x7fffffffu) : (best == 0x7f80u ? __uint_as_float(0x7f800000u) : digits_scale(top));
   }
   for (int c = threadIdx.x; c < chunks; c += kSplitThreads) {  // whole warps: chunks is a multiple of 32
     const uint4 q = best < 0x7f80u ? load(c) : make_uint4(0u, 0u, 0u, 0u);  // the epilogue has no use for the digits then
-    uint32_t b = abs_max(q);
+    uint32_t b = bf16x8_abs_max(q);
     b = max(b, __shfl_xor_sync(0xffffffffu, b, 1));
-    const int e = max(max(static_cast<int>(b >> 7), top - 17), 1);
-    const float scale = __uint_as_float(static_cast<uint32_t>(255 - e) << 23);  // 2^(128 - e)
-    const uint32_t r[4] = {q.x, q.y, q.z, q.w};
+    const int e = digits_exponent(b, top);
     float v[8];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      v[2 * i] = __uint_as_float(r[i] << 16) * scale;
-      v[2 * i + 1] = __uint_as_float(r[i] & 0xffff0000u) * scale;
-    }
+    digits_begin(q, e, v);
     uint8_t * step = it.ops + static_cast<size_t>(c >> 5) * it.step_bytes;
     // writes the next digit as an operand row
     auto write_digit = [&](uint8_t * codes, int row) {
-      const uint32_t w = to_e2m1x8(v);
-      *reinterpret_cast<uint32_t *>(codes + row * kStepBytes + ((((c >> 2) ^ row) & 7) << 4) + ((c & 3) << 2)) = w;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        float d0, d1;
-        from_e2m1x2(w >> (8 * i), d0, d1);
-        v[2 * i] = (v[2 * i] - d0) * 8.0f;
-        v[2 * i + 1] = (v[2 * i + 1] - d1) * 8.0f;
-      }
+      *reinterpret_cast<uint32_t *>(codes + row * kStepBytes + ((((c >> 2) ^ row) & 7) << 4) + ((c & 3) << 2)) = digits_next(v);
     };
-    // E4M3 byte of 2^(8 + e - top); the four blocks of eight lanes make one word of the tiled layout, the same for every digit
-    const int s = 8 + e - top;
-    const uint32_t byte = s >= -6 ? static_cast<uint32_t>(s + 7) << 3 : 8u >> (-6 - s);
+    // the scale bytes of eight lanes' four blocks make one word of the tiled layout, the same for every digit
+    const uint32_t byte = digits_scale_byte(e, top);
     uint32_t word = byte << (8 * ((threadIdx.x >> 1) & 3));
     word |= __shfl_xor_sync(0xffffffffu, word, 2);
     word |= __shfl_xor_sync(0xffffffffu, word, 4);

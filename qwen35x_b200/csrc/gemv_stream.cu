@@ -872,6 +872,7 @@ struct q35b_gemv_batch {
   uint32_t wait_limit = kWaitLimit;   // polls every device-side wait of a run may take
   unsigned int wait_extra = 0;        // test hook: completions that every other CTA demands on top of what a dependency delivers
   q35b::WBatch * tensor = nullptr;   // set: the list runs on the tensor path (gemm_wstream.cu), nothing above is used
+  std::vector<q35b_gemv_item> chain;  // set: it runs as one launch per item, in this order (gemm_resident.cu)
 };
 
 namespace q35b {
@@ -1026,6 +1027,21 @@ bool tensor_list(const q35b_gemv_item * items, int count) {
   return bytes >= kTensorBytes && wbatch_longest_share(items, count) <= kTensorLongest;
 }
 
+// Whether a list runs as one launch per item in which the operand is made in shared memory (gemm_resident.cu): a chain, so
+// that the launches follow one another as the items would.
+// Up to six tokens: every row block makes the operand anew, and from seven on that costs more than the dependent items'
+// conversions in one launch do.  us, one launch / one per item, MLP blocks [2560, 9216], [1024, 3584], [512, 1280], one token 25.3 /
+// 15.9, 14.9 / 9.9, 9.8 / 8.9; two 26.2 / 17.1, 15.5 / 10.5, 10.4 / 9.5; four 26.8 / 22.5, 15.7 / 11.9, 10.7 / 9.9; six 28.5 / 28.7, 16.5 /
+// 14.0, 11.3 / 11.6; eight 28.9 / 29.2, 16.8 / 17.6, 11.5 / 11.7.
+constexpr int kResidentTokens = 6;
+bool resident_chain(const q35b_gemv_item * items, const std::vector<int> & level, int m) {
+  if (m > kResidentTokens) return false;
+  for (size_t i = 0; i < level.size(); ++i) {
+    if (level[i] != static_cast<int>(i) || items[i].x_bf16 == nullptr || items[i].y_bf16 == nullptr || !decode_resident_chain(items[i].weight, m)) return false;
+  }
+  return true;
+}
+
 }  // namespace
 
 int gemv_batch_build(const q35b_gemv_item * items, int count, int m, bool share_tiles, q35b_gemv_batch ** out) {
@@ -1130,6 +1146,7 @@ int gemv_batch_build(const q35b_gemv_item * items, int count, int m, bool share_
     if (items[i].after > 0) level[i] = level[items[i].after - 1] + 1;
     max_level = std::max(max_level, level[i]);
   }
+  const bool callers_list = share_tiles;
   const int most = share_tiles ? static_cast<int>(std::min<long>(total_steps, 1 << 20)) : static_cast<int>(all.size());
   auto grid_for = [&](int ksplit) { return std::max(1, std::min(sm_count() * ctas_per_sm(ksplit), most)); };
   int grid = grid_for(b->plan.ksplit);
@@ -1201,6 +1218,7 @@ int gemv_batch_build(const q35b_gemv_item * items, int count, int m, bool share_
     delete b;
     return fail_cuda(e, "uploading the projection work list");
   }
+  if (callers_list && resident_chain(items, level, m)) b->chain.assign(items, items + count);
   *out = b;
   return Q35B_OK;
 }
@@ -1222,6 +1240,14 @@ int gemv_batch_build_tensor(const q35b_gemv_item * items, int count, int m, int 
 int gemv_batch_launch(const q35b_gemv_batch * b, const void * x_override, void * y_override, cudaStream_t s) {
   if (b == nullptr) return fail(Q35B_ERR_ARGUMENT, "Null NVFP4 projection work list.");
   if (b->tensor != nullptr) return wbatch_launch(b->tensor, s);
+  if (!b->chain.empty() && b->wait_extra == 0) {
+    for (size_t i = 0; i < b->chain.size(); ++i) {
+      const q35b_gemv_item & it = b->chain[i];
+      const q35b_weight * next = i + 1 < b->chain.size() ? b->chain[i + 1].weight : nullptr;
+      if (const int st = launch_decode_resident(it.weight, it.x_bf16, b->m, it.y_bf16, it.residual_bf16, true, next, b->status, b->wait_limit, s)) return st;
+    }
+    return Q35B_OK;
+  }
   const auto * xo = static_cast<const __nv_bfloat16 *>(x_override);
   auto * yo = static_cast<__nv_bfloat16 *>(y_override);
   const int counted = b->has_dependencies ? b->count : 0;

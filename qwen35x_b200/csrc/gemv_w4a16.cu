@@ -362,6 +362,15 @@ int launch_gemv_bf16(const q35b_weight * w, const void * x_bf16, int m, void * y
                     kernel, s);
 }
 
+// The rows kernel, from a fit to graph replays: so much per 256 columns and turn of the warps that the SMs hold.
+double gemv_rows_ns(const q35b_weight * w, int m) {
+  static constexpr int per_piece[9] = {0, 480, 480, 620, 720, 950, 1100, 1000, 840};
+  const int sms = sm_count(), pieces = (w->k + kPiece - 1) / kPiece;
+  const bool four = w->rows < kWarpsPerBlock * sms && w->k > pieces_ahead(m) * kPiece;  // as launch_simt deals them out
+  const double warps = four ? 4.0 * w->rows : (w->rows < 2 * kWarpsPerBlock * sms ? w->rows : 0.5 * w->rows);
+  return 1000.0 + per_piece[m] * std::max(1.0, pieces / (four ? 4.0 : 1.0)) * std::max(1.0, warps / (sms * (m == 1 ? 32.0 : 18.0)));
+}
+
 int launch_gemv_f32(const q35b_weight * w, const float * x, float input_scale, float * y, int kernel, cudaStream_t s) {
   return launch_any(w, x, 1, y, input_scale, kernel, s);
 }

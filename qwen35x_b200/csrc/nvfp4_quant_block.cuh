@@ -8,6 +8,8 @@
 //   code_i = E2M1(x_i / d), element 2j in the low nibble (or swapped for the reference's cuBLASLt order)
 #pragma once
 
+#include <cuda_bf16.h>
+
 #include <cstdint>
 
 #include "nvfp4_codec.cuh"
@@ -241,6 +243,46 @@ __device__ __forceinline__ uint32_t quantize_block_bf16(const uint4 a, const uin
   bf16x2_scaled(b.w, m, q[6], q[7]);
   out.y = cvt_e2m1x8(q);
   return sb;
+}
+
+// ---- as the kernels that quantise activations use them: values as they lie in memory ----------------------------
+
+// |values| of 16 bytes into the running maximum; like fmaxf both skip NaNs.
+template <typename T>
+__device__ __forceinline__ float abs_max(const uint4 q, float best);
+template <>
+__device__ __forceinline__ float abs_max<float>(const uint4 q, float best) {
+  return fmaxf(best, fmaxf(fmaxf(fabsf(__uint_as_float(q.x)), fabsf(__uint_as_float(q.y))),
+                           fmaxf(fabsf(__uint_as_float(q.z)), fabsf(__uint_as_float(q.w)))));
+}
+__device__ __forceinline__ uint32_t bf16x2_abs_max(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("max.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+template <>
+__device__ __forceinline__ float abs_max<__nv_bfloat16>(const uint4 q, float best) {
+  // two values per instruction; a pair of NaNs leaves one, which the last step skips
+  const uint32_t m = bf16x2_abs_max(bf16x2_abs_max(q.x, q.y), bf16x2_abs_max(q.z, q.w));
+  return fmaxf(best, fmaxf(fabsf(__uint_as_float(m << 16)), fabsf(__uint_as_float(m & 0xffff0000u))));
+}
+
+// Codes and scale byte of one block.
+template <typename T, bool TABLE>
+__device__ __forceinline__ uint32_t quantize_raw(const uint4 (&r)[sizeof(T)], float g, float rg, const float * table, uint2 & out) {
+  if constexpr (sizeof(T) == 2) {
+    return quantize_block_bf16<TABLE>(r[0], r[1], g, rg, table, out);
+  } else {
+    float v[16];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      v[4 * i] = __uint_as_float(r[i].x);
+      v[4 * i + 1] = __uint_as_float(r[i].y);
+      v[4 * i + 2] = __uint_as_float(r[i].z);
+      v[4 * i + 3] = __uint_as_float(r[i].w);
+    }
+    return quantize_block<kEngine>(v, g, false, out);
+  }
 }
 
 }  // namespace q35b

@@ -1,0 +1,179 @@
+"""Projections whose operand is made in shared memory (gemm_resident.cu): chains of a decode work list and single decode
+projections, activations as octal digits.  Against 64-bit sums of the same products: the sums are fp32, so after the BF16
+rounding an output differs by a flipped rounding at most, relative L2 below 2e-4 over many outputs (a few in 10^4 values by one
+step of 2^-8) and below 2^-8 for one."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+E2M1 = [0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0]
+
+
+def _weight(engine, torch, gen, n, k, gate_up=False):
+    codes = torch.randint(0, 256, (n, k // 2), dtype=torch.uint8, device="cuda", generator=gen)
+    scales = torch.randint(0, 0x7f, (n, k // 16), dtype=torch.uint8, device="cuda", generator=gen)
+    table = torch.tensor(E2M1 + [-v for v in E2M1], dtype=torch.float64, device="cuda")
+    sb = scales.to(torch.int64)
+    decoded = torch.where(sb < 8, (sb & 7) * 2.0 ** -9, (8 + (sb & 7)) * torch.pow(2.0, ((sb >> 3) - 10).double()))
+    w = torch.stack([table[(codes & 15).long()], table[(codes >> 4).long()]], dim=2).view(n, k) * decoded.repeat_interleave(16, dim=1)
+    return (codes, scales), w * 2.0 ** -12
+
+
+def _rel(y, want):
+    import torch
+
+    want = want.to(torch.bfloat16).double()
+    return ((y.double() - want).norm() / want.norm().clamp_min(1e-300)).item()
+
+
+def _limit(count):
+    return 2e-4 if count >= 1000 else 2.0 ** -8
+
+
+def _run(engine, torch, items, m, launches):
+    batch = engine.GemvBatch(items, m)
+    before = engine.launch_count()
+    batch.run()
+    assert engine.launch_count() - before == launches
+    first = [it[2].clone() for it in items]
+    batch.run()
+    torch.cuda.synchronize()
+    assert batch.status() == 0 and all(torch.equal(a.view(torch.int16), it[2].view(torch.int16)) for a, it in zip(first, items))
+    return batch
+
+
+@pytest.mark.parametrize("m", [1, 2, 3, 4, 5, 6])
+@pytest.mark.parametrize("n,k", [(1, 256), (127, 512), (130, 1280), (640, 9216), (2600, 2560)])
+def test_one_item(engine, m, n, k):
+    """Rows around a tile, splits from one to eight CTAs (also uneven ones), a residual, activations over the range of a token."""
+    import torch
+
+    gen = torch.Generator(device="cuda").manual_seed(m + n)
+    (codes, scales), wd = _weight(engine, torch, gen, n, k)
+    w = engine.Nvfp4Weight.from_device(codes, scales, 2.0 ** -12)
+    for kind in range(4):
+        x = torch.randn((m, k), device="cuda", generator=gen)
+        if kind == 1:
+            x *= torch.exp2(torch.randint(-30, 30, (m, k), device="cuda", generator=gen).float())
+        if kind == 2:
+            x *= 2.0 ** -110
+            x[0] *= 0.0 if m > 1 else 1.0
+        if kind == 3:
+            x[:, k // 2:] *= 2.0 ** -60  # CTAs of a cluster that count in units far apart
+        x = x.to(torch.bfloat16)
+        res = torch.randn((m, n), device="cuda", generator=gen).to(torch.bfloat16) if kind == 0 else None
+        y = torch.zeros((m, n), dtype=torch.bfloat16, device="cuda")
+        _run(engine, torch, [(w, x, y, res)], m, 1)
+        assert _rel(y, x.double() @ wd.T + (res.double() if res is not None else 0.0)) <= _limit(m * n), kind
+
+
+@pytest.mark.parametrize("m", [1, 2, 4, 6])
+@pytest.mark.parametrize("hidden,inter", [(256, 256), (768, 2304), (2560, 3584)])
+def test_chain(engine, m, hidden, inter):
+    """Gate/up, then down reading its output: one launch each, replayed from a graph too."""
+    import torch
+
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    (gc, gs), gd = _weight(engine, torch, gen, inter, hidden)
+    (uc, us), ud = _weight(engine, torch, gen, inter, hidden)
+    (dc, ds), dd = _weight(engine, torch, gen, hidden, inter)
+    gate_up = engine.Nvfp4Weight.gate_up_from_host(*(t.cpu().numpy() for t in (gc, gs)), 2.0 ** -12, *(t.cpu().numpy() for t in (uc, us)), 2.0 ** -13)
+    x = (torch.randn((m, hidden), device="cuda", generator=gen) * 2.0 ** -4).to(torch.bfloat16)
+    res = torch.randn((m, hidden), device="cuda", generator=gen).to(torch.bfloat16)
+    h = torch.zeros((m, inter), dtype=torch.bfloat16, device="cuda")
+    y = torch.zeros((m, hidden), dtype=torch.bfloat16, device="cuda")
+    batch = _run(engine, torch, [(gate_up, x, h), (engine.Nvfp4Weight.from_device(dc, ds, 2.0 ** -12), h, y, res, 0)], m, 2)
+    gate, up = x.double() @ gd.T, x.double() @ ud.T / 2
+    assert _rel(h, gate / (1 + torch.exp(-gate)) * up) <= 1e-3  # the sigmoid in fp32 before the product is rounded
+    assert _rel(y, h.double() @ dd.T + res.double()) <= _limit(m * hidden)
+    kept = y.clone()
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    with torch.cuda.stream(stream):
+        with torch.cuda.graph(graph, stream=stream):
+            for _ in range(3):
+                batch.run()
+        y.zero_()
+        graph.replay()
+        stream.synchronize()
+    assert batch.status() == 0 and torch.equal(y, kept)
+
+
+@pytest.mark.parametrize("m", [1, 2, 4, 8])
+@pytest.mark.parametrize("n,k", [(2500, 4160), (1300, 7232), (9000, 2624), (2560, 9216)])
+def test_single_projections(engine, m, n, k):
+    """What AUTO chooses, K ending anywhere in a K step."""
+    import torch
+
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    (codes, scales), wd = _weight(engine, torch, gen, n, k)
+    w = engine.Nvfp4Weight.from_device(codes, scales, 2.0 ** -12)
+    x = torch.randn((m, k), device="cuda", generator=gen).to(torch.bfloat16)
+    want = x.double() @ wd.T
+    assert _rel(engine.gemv_w4a16(w, x), want) <= 2e-4
+    assert _rel(engine.gemv_w4a16(w, x, kernel=engine.GEMV_SIMT), want) <= 2e-4
+
+
+@pytest.mark.parametrize("depth", [18, 24, 37])
+@pytest.mark.parametrize("m", [1, 3, 6])
+def test_small_values_beside_large_ones(engine, m, depth):
+    """Where the weights of a row are zero at the large values of every block, the small ones are all it has."""
+    import torch
+
+    gen = torch.Generator(device="cuda").manual_seed(depth)
+    n, k = 300, 2560
+    (codes, scales), wd = _weight(engine, torch, gen, n, k)
+    codes[:, ::8] &= 0xf0  # the first element of every block
+    wd[:, ::16] = 0.0
+    w = engine.Nvfp4Weight.from_device(codes, scales, 2.0 ** -12)
+    x = torch.randn((m, k), device="cuda", generator=gen) * 2.0 ** -depth
+    x[:, ::16] = 1.0
+    x = x.to(torch.bfloat16)
+    y = torch.zeros((m, n), dtype=torch.bfloat16, device="cuda")
+    _run(engine, torch, [(w, x, y)], m, 1)
+    # multiples of 2^-40 of the block's largest binade: half of one per value, against values of 2^-depth
+    assert _rel(y, x.double() @ wd.T) <= max(4e-3, 2.0 ** (depth - 39))
+
+
+@pytest.mark.parametrize("m", [1, 4])
+def test_infinities_and_nans(engine, m):
+    import torch
+
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    n, k = 400, 2560
+    (codes, scales), wd = _weight(engine, torch, gen, n, k)
+    codes[:200, 350] &= 0xf0  # zero weights at column 700
+    w = engine.Nvfp4Weight.from_device(codes, scales, 2.0 ** -12)
+    for places in ([(700, float("inf"))], [(5, float("-inf")), (2500, float("inf"))], [(1000, float("nan"))]):
+        x = torch.randn((m, k), device="cuda", generator=gen).to(torch.bfloat16)
+        for at, v in places:
+            x[m - 1, at] = v
+        y = torch.zeros((m, n), dtype=torch.bfloat16, device="cuda")
+        _run(engine, torch, [(w, x, y)], m, 1)
+        want = engine.gemv_w4a16(w, x, kernel=engine.GEMV_SIMT)
+        assert torch.equal(y.isnan(), want.isnan()) and torch.equal(y[want.isinf()], want[want.isinf()])
+        assert _rel(y[want.isfinite()], want[want.isfinite()].double()) <= 4e-3 if bool(want.isfinite().any()) else True
+
+
+@pytest.mark.parametrize("m,hidden,inter", [(1, 256, 256), (2, 2560, 9216), (5, 512, 4096)])
+def test_a_run_that_gives_up_leaves_a_list_that_works(engine, m, hidden, inter):
+    import torch
+
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    (uc, us), _ = _weight(engine, torch, gen, inter, hidden)
+    (dc, ds), _ = _weight(engine, torch, gen, hidden, inter)
+    x = torch.randn((m, hidden), device="cuda", generator=gen).to(torch.bfloat16)
+    h = torch.zeros((m, inter), dtype=torch.bfloat16, device="cuda")
+    y = torch.zeros((m, hidden), dtype=torch.bfloat16, device="cuda")
+    batch = _run(engine, torch, [(engine.Nvfp4Weight.from_device(uc, us, 2.0 ** -16), x, h), (engine.Nvfp4Weight.from_device(dc, ds, 2.0 ** -16), h, y, None, 0)], m, 2)
+    good = y.clone()
+    for limit in (1, 2, 5, 20, 100):
+        batch.debug_wait(limit, 0)
+        for _ in range(3):
+            batch.run()
+        torch.cuda.synchronize()
+        assert batch.status() == 0 or 51 <= batch.status() <= 56
+        batch.debug_wait(1 << 22, 0)
+        y.zero_()
+        batch.run()
+        torch.cuda.synchronize()
+        assert batch.status() == 0 and torch.equal(y, good)
