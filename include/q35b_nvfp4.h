@@ -305,6 +305,13 @@ Q35B_API int q35b_gemm_w4a4_bf16_residual(const q35b_weight * w, const uint8_t *
                                           const float * input_scale_dev, int m, const void * residual_bf16, int ldr,
                                           void * c_bf16, int ldc, unsigned int * status_dev, q35b_stream stream);
 
+/* q35b_quantize_nvfp4_bf16 (x_is_f32: _f32) of x [m, cols] followed by q35b_gemm_w4a4_bf16 or, with a residual,
+ * q35b_gemm_w4a4_bf16_residual: the same outputs, codes, scales and scale word, in one launch where the activation is
+ * small enough for every CTA to quantise the columns that it multiplies.  `workspace` as for the quantisation. */
+Q35B_API int q35b_project_prefill(const q35b_weight * w, const void * x, int x_is_f32, int m, float global_scale, uint8_t * codes,
+                                  uint8_t * scales_tiled, float * input_scale_dev, void * workspace, const void * residual_bf16,
+                                  int ldr, void * c_bf16, int ldc, unsigned int * status_dev, q35b_stream stream);
+
 /* Gate/up GEMM whose epilogue writes silu(gate) * up as an NVFP4 activation (codes [m, rows/4] bytes, tiled block
  * scales sized by q35b_act_scales_bytes(m, rows/2)), ready to be the A operand of the down projection's
  * q35b_gemm_w4a4_bf16(_residual) with out_scale_dev as its input_scale_dev.  Replaces pf_silu_mul_bf16 plus the

@@ -454,6 +454,13 @@ int q35b_gemm_w4a4_bf16_residual(const q35b_weight * w, const uint8_t * a_codes,
                           residual_bf16, ldr, status_dev, static_cast<cudaStream_t>(stream));
 }
 
+int q35b_project_prefill(const q35b_weight * w, const void * x, int x_is_f32, int m, float global_scale, uint8_t * codes, uint8_t * scales_tiled,
+                         float * input_scale_dev, void * workspace, const void * residual_bf16, int ldr, void * c_bf16, int ldc, unsigned int * status_dev,
+                         q35b_stream stream) {
+  return launch_project_prefill(w, x, x_is_f32 != 0, m, global_scale, codes, scales_tiled, input_scale_dev, workspace, residual_bf16, ldr, c_bf16, ldc, status_dev,
+                                static_cast<cudaStream_t>(stream));
+}
+
 int q35b_debug_gemm_plan(int m, int rows, int n_total, int k, int sms, int gather, int rows_aligned, int * pairs,
                          int * tile_cols, int * split, int * accumulators) {
   return gemm_plan_debug(m, rows, n_total, k, sms, gather != 0, rows_aligned != 0, pairs, tile_cols, split, accumulators);

@@ -155,6 +155,10 @@ int default_status_word(unsigned int ** out);
 int launch_gemm_w4a4(const q35b_weight * w, const uint8_t * a_codes, const uint8_t * a_scales_tiled, const float * g_dev,
                      int m, void * c_bf16, int ldc, const void * residual_bf16, int ldr, unsigned int * status_dev,
                      cudaStream_t s, const GemmQuantOut * qout = nullptr, const GemmGather * gather = nullptr);
+// Quantisation and projection of an activation, in one launch where it is small; codes, scales and scale word are written either way.
+int launch_project_prefill(const q35b_weight * w, const void * x, bool f32, int m, float global_scale, uint8_t * codes, uint8_t * scales_tiled, float * g_dev,
+                           void * workspace, const void * residual_bf16, int ldr, void * c_bf16, int ldc, unsigned int * status_dev, cudaStream_t s);
+
 // gemm_wstream.cu: decode work lists on the tensor cores
 struct WBatch;  // decode work list on the tensor path (digit-expanded activations)
 // exact: all bits of the activations, their infinities and NaNs too, reach the outputs (else what `digits` digits hold)

@@ -881,7 +881,7 @@ int launch_decode_resident(const q35b_weight * w, const void * x_bf16, int m, vo
 // two launches.  It pays where the two launches would meet twice (a scale from the tensor) and the quantising, which every row
 // block does anew, is one block of sixteen per thread; and only if the ring holds the weights, or they come when the operand
 // has been waited for.  us, two launches / one: [3, 5184] x [169, 5184] 9.1 / 6.1, [2, 2688] x [2077, 2688] 8.8 / 6.1, [4, 1664] x
-// [8025, 1664] 9.1 / 7.4, [13, 2432] x [1059, 2432] 8.6 / 7.0; more than one block per thread: [16, 2560] x [9216, 2560] 9.6 / 10.7, [20, 1280] x
+// [8025, 1664] 9.1 / 7.4, [11, 1920] x [973, 1920] 8.5 / 6.2; more than one block per thread: [16, 2560] x [9216, 2560] 9.6 / 10.7, [20, 1280] x
 // [870, 1280] 8.5 / 11.9; a given scale: [3, 2048] x [133, 2048] 4.9 / 4.8, [5, 3136] x [273, 3136] 5.3 / 5.5; weights that come later: [1, 3008] x
 // [22014, 3008] 12.5 / 13.3.
 bool prefill_resident_shape(const q35b_weight * w, int m, float scale, int split, int * stages, int * smem) {

@@ -830,4 +830,30 @@ int launch_gemm_w4a4(const q35b_weight * w, const uint8_t * a_codes, const uint8
   return launch_gemm_ksplit(w, a_codes, a_scales_tiled, g_dev, m, c_bf16, ldc, ep, plan, status_dev, s);
 }
 
+int launch_project_prefill(const q35b_weight * w, const void * x, bool f32, int m, float global_scale, uint8_t * codes, uint8_t * scales_tiled, float * g_dev,
+                           void * workspace, const void * residual_bf16, int ldr, void * c_bf16, int ldc, unsigned int * status_dev, cudaStream_t s) {
+  // One launch where the operand is made in shared memory (gemm_resident.cu); whatever is not in order goes the general way,
+  // which says so.
+  auto aligned = [](const void * p) { return p != nullptr && (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
+  if (w != nullptr && m >= 1 && m <= kSplitTokens && w->rows > 0 && w->has_maps && (w->k % 64) == 0 && aligned(x) && aligned(codes) && aligned(scales_tiled) && g_dev != nullptr &&
+      (global_scale > 0.0f || workspace != nullptr) && c_bf16 != nullptr && ldc >= (w->gate_up ? w->rows / 2 : w->rows) &&
+      (residual_bf16 == nullptr || (!w->gate_up && ldr >= w->rows))) {
+    const GemmPlan plan = plan_gemm(m, w->rows, w->n_total, w->k, sm_count(), false, true);
+    int stages = 0, smem = 0;
+    if (!plan.pairs && plan.tile_cols >= m && prefill_resident_shape(w, m, global_scale, plan.split, &stages, &smem)) {
+      if (const int st = check_weight_device(w)) return st;
+      if (status_dev == nullptr) {
+        if (const int st = default_status_word(&status_dev)) return st;
+      }
+      return launch_prefill_resident(w, x, f32, m, global_scale, codes, scales_tiled, g_dev, plan.split, stages, smem, residual_bf16, ldr, c_bf16, ldc, status_dev, s);
+    }
+  }
+  const int k = w != nullptr ? w->k : 0;
+  if (const int st = f32 ? launch_quantize_f32(static_cast<const float *>(x), m, k, global_scale, codes, scales_tiled, g_dev, workspace, s)
+                         : launch_quantize_bf16(x, m, k, global_scale, codes, scales_tiled, g_dev, workspace, s)) {
+    return st;
+  }
+  return launch_gemm_w4a4(w, codes, scales_tiled, g_dev, m, c_bf16, ldc, residual_bf16, ldr, status_dev, s);
+}
+
 }  // namespace q35b

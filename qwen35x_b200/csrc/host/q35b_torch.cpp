@@ -214,9 +214,13 @@ PyObject * project_prefill(PyObject *, PyObject * const * args, Py_ssize_t n) {
   at::Tensor made;
   const at::Tensor * out = output(args[2], a.m, q35b_weight_is_gate_up(w) != 0 ? rows / 2 : rows, device, made);
   if (out == nullptr || out->stride(0) > INT32_MAX) return not_plain();
+  auto * codes = static_cast<uint8_t *>(a.codes->mutable_data_ptr()), * scales = static_cast<uint8_t *>(a.scales->mutable_data_ptr());
+  auto * word = static_cast<float *>(a.g->mutable_data_ptr());
+  const void * xp = a.x->const_data_ptr(), * rp = residual != nullptr ? residual->const_data_ptr() : nullptr;
+  const int ldr = residual != nullptr ? static_cast<int>(residual->stride(0)) : 0, ldc = static_cast<int>(out->stride(0));
+  void * cp = out->mutable_data_ptr();
   const int st = without_gil([&] {
-    if (const int q = a.quantize(stream)) return q;
-    return gemm_call(w, *a.codes, *a.scales, *a.g, a.m, residual, *out, stream);
+    return q35b_project_prefill(w, xp, a.bf16 ? 0 : 1, a.m, a.scale, codes, scales, word, a.workspace, rp, ldr, cp, ldc, nullptr, stream);
   });
   if (st != 0) return raise_status(st);
   return returned(args[2], made);

@@ -177,3 +177,50 @@ def test_a_run_that_gives_up_leaves_a_list_that_works(engine, m, hidden, inter):
         batch.run()
         torch.cuda.synchronize()
         assert batch.status() == 0 and torch.equal(y, good)
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "f32"])
+@pytest.mark.parametrize("m,n,k", [(1, 64, 64), (3, 129, 5184), (4, 2100, 1344), (9, 471, 2432), (14, 1500, 320), (28, 300, 256), (2, 12500, 2816)])
+def test_prefill_in_one_launch(engine, m, n, k, dtype):
+    """Quantisation and projection of a small activation: outputs, codes, scales and scale word of the two launches, bit for
+    bit; K ending anywhere in a K step, residuals on unaligned rows, zeros, infinities and NaNs among the activations."""
+    import torch
+
+    gen = torch.Generator(device="cuda").manual_seed(m + n)
+    (codes, scales), _ = _weight(engine, torch, gen, n, k)
+    w = engine.Nvfp4Weight.from_device(codes, scales, 2.0 ** -12)
+    for kind in range(4):
+        x = torch.randn((m, k), device="cuda", generator=gen)
+        if kind == 1:
+            x[:, ::100] *= 50.0
+        if kind == 2:
+            x *= 0.0
+        if kind == 3:
+            x[0, 3], x[-1, k - 1] = float("nan"), float("inf")
+        x = x.to(torch.bfloat16 if dtype == "bf16" else torch.float32)
+        res = torch.randn((m, n + 3), device="cuda", generator=gen).to(torch.bfloat16)[:, :n] if kind == 1 else None
+        one, two = engine.act_scratch(m, k, x.device), engine.act_scratch(m, k, x.device)
+        for t in one:
+            t.fill_(3)
+        a = engine.quantize_activations(x, scratch=two)
+        before = engine.launch_count()
+        got = engine.project_prefill(w, x, scratch=one, residual=res)
+        assert engine.launch_count() - before == 1
+        want = engine.gemm_w4a4(w, *a, m, residual=res)
+        assert torch.equal(got.view(torch.int16), want.view(torch.int16)) or (kind == 3 and torch.equal(got.nan_to_num(7.0), want.nan_to_num(7.0)))
+        assert all(torch.equal(p.view(torch.uint8), q.view(torch.uint8)) for p, q in zip(one, two))
+    assert engine.gemm_default_status() == 0
+
+
+def test_prefill_of_a_gate_up_weight_in_one_launch(engine):
+    import torch
+
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    parts = [_weight(engine, torch, gen, 200, 576)[0] for _ in range(2)]
+    host = [t.cpu().numpy() for p in parts for t in p]
+    w = engine.Nvfp4Weight.gate_up_from_host(host[0], host[1], 2.0 ** -12, host[2], host[3], 2.0 ** -13)
+    x = torch.randn((7, 576), device="cuda", generator=gen).to(torch.bfloat16)
+    want = engine.gemm_w4a4(w, *engine.quantize_activations(x), 7)
+    before = engine.launch_count()
+    got = engine.project_prefill(w, x)
+    assert engine.launch_count() - before == 1 and torch.equal(got, want)
