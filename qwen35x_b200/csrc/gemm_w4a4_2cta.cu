@@ -109,6 +109,11 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
     "l"(map), "r"(leader_bar), "r"(x), "r"(y)
     : "memory");
 }
+__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap * map, uint32_t bar, int x, int y) {
+  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst), "l"(map),
+               "r"(bar), "r"(x), "r"(y)
+               : "memory");
+}
 __device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap * map, int x, int y) {
   asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
 }
@@ -179,13 +184,6 @@ __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// The first `count` (below eight) of eight BF16 values, as a register each two: the ragged end of a residual's row.
-__device__ __noinline__ uint4 load_bf16_tail(const __nv_bfloat16 * p, int count) {
-  uint64_t w[2] = {0u, 0u};
-  for (int i = 0; i < count; ++i) w[i >> 2] |= static_cast<uint64_t>(__ldca(reinterpret_cast<const unsigned short *>(p) + i)) << (16 * (i & 3));
-  return make_uint4(static_cast<uint32_t>(w[0]), static_cast<uint32_t>(w[0] >> 32), static_cast<uint32_t>(w[1]), static_cast<uint32_t>(w[1] >> 32));
-}
-
 // The first `count` (up to eight) of eight BF16 values into 16-byte aligned memory.
 __device__ __noinline__ void store_bf16_tail(__nv_bfloat16 * p, uint4 v, int count) {
   if (count >= 8) {
@@ -200,7 +198,7 @@ template <int kEpilogueWarps>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((2 + kEpilogueWarps) * 32, 1)
 gemm_w4a4_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                       const __grid_constant__ CUtensorMap tmap_sfa, const __grid_constant__ CUtensorMap tmap_sfb,
-                      const __grid_constant__ CUtensorMap tmap_c,  // of the output, for the plain epilogue
+                      const __grid_constant__ CUtensorMap tmap_c, const __grid_constant__ CUtensorMap tmap_res,  // output and residual of the plain epilogue
                       const float * __restrict__ g_dev, const GemmEpilogue ep, int m, int n, int k_bytes, int m_tiles, int num_tiles,
                       __nv_bfloat16 * __restrict__ c, int ldc, unsigned int * status) {
   constexpr int kColWarps = kEpilogueWarps / 4, kTurns = kChunks / kColWarps;  // chunks of a tile that one epilogue warp takes
@@ -216,7 +214,8 @@ gemm_w4a4_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
   uint64_t * empty = bars + kStages;            // in each CTA: its own stages are free
   uint64_t * tmem_full = bars + 2 * kStages;    // in each CTA: the tile's accumulator is complete
   uint64_t * drained = tmem_full + 1;           // used in the leader: both CTAs' epilogue warps have read the columns that the next tile's accumulator shares
-  uint32_t * tmem_slot = reinterpret_cast<uint32_t *>(drained + 1);
+  uint64_t * res_full = drained + 1;            // [2 per epilogue warp of the plain epilogue]: the residual's box has landed
+  uint32_t * tmem_slot = reinterpret_cast<uint32_t *>(res_full + 2 * kEpiWarpsPlain);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -234,6 +233,7 @@ gemm_w4a4_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     }
     mbar_init(smem_u32(tmem_full), 1);
     mbar_init(smem_u32(drained), 2 * kEpilogueWarps);
+    for (int i = 0; i < 2 * kEpiWarpsPlain; ++i) mbar_init(smem_u32(res_full + i), 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -380,6 +380,7 @@ gemm_w4a4_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     }
     uint32_t li = 0;
     bool ok = !aborted;
+    int res_loads = 0;  // lane 0: residual boxes asked for
     for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, ++li) {
       const int tm = tile % m_tiles;
       const int tn = tile / m_tiles;
@@ -389,20 +390,28 @@ gemm_w4a4_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       const int chunk0 = (li & 1) != 0u ? col_warp : col_warp + kChunks - 2;
       if constexpr (kEpilogueWarps == kEpiWarpsPlain) {
         const uint32_t box0 = smem_u32(smem + kBoxOffset) + (warp - 2) * 2 * kBoxBytes;
-        const __nv_bfloat16 * res = ep.residual != nullptr && row0 + lane < m ? ep.residual + static_cast<size_t>(row0 + lane) * ep.ldr : nullptr;
 #pragma unroll 1
         for (int turn = 0; turn < kTurns; ++turn) {
           const int chunk = (chunk0 + turn * kColWarps) & (kChunks - 1);
           const int col0 = tn * kTileN + chunk * kChunkCols;
-          uint4 rr[4] = {};
-          if (res != nullptr) {  // asked for before the sums are there
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              if (col0 + 8 * i + 8 <= n) {
-                rr[i] = __ldca(reinterpret_cast<const uint4 *>(res + col0 + 8 * i));
-              } else if (col0 + 8 * i < n) {
-                rr[i] = load_bf16_tail(res + col0 + 8 * i, n - col0 - 8 * i);
-              }
+          // The residual's boxes come by TMA into the boxes that the sums leave from, each while the one before is worked on;
+          // the first one of a tile under the tile before.
+          auto load_residual = [&](int at_tile, int at_turn, uint32_t at_li) {
+            const int at_chunk = (col_warp + ((at_li & 1) != 0u ? 0 : kChunks - 2) + at_turn * kColWarps) & (kChunks - 1);
+            const uint32_t at_box = box0 + (at_turn & 1) * kBoxBytes, bar = smem_u32(res_full + 2 * (warp - 2) + (at_turn & 1));
+            ++res_loads;
+            mbar_expect_tx(bar, kBoxBytes);
+            tma_load_2d(at_box, &tmap_res, bar, at_tile / m_tiles * kTileN + at_chunk * kChunkCols,
+                        at_tile % m_tiles * kTileM + static_cast<int>(rank) * kCtaRows + quarter * 32);
+          };
+          if (ep.residual != nullptr && lane == 0) {
+            if (li == 0 && turn == 0) load_residual(tile, 0, 0);
+            // the box after this one: its last store has been read
+            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+            if (turn + 1 < kTurns) {
+              load_residual(tile, turn + 1, li);
+            } else if (tile + num_pairs < num_tiles) {
+              load_residual(tile + num_pairs, 0, li + 1);
             }
           }
           if (turn == 0) {
@@ -418,15 +427,27 @@ gemm_w4a4_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             __syncwarp();
             if (lane == 0) mbar_arrive_leader(smem_u32(drained));
           }
-          // the box before last has been read
-          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-          __syncwarp();
           const uint32_t box = box0 + (turn & 1) * kBoxBytes;
+          if (ep.residual != nullptr) {
+            ok = mbar_wait(smem_u32(res_full + 2 * (warp - 2) + (turn & 1)), (li * (kTurns / 2) + turn / 2) & 1);
+            if (!__all_sync(0xffffffffu, ok)) {
+              ok = false;
+              break;
+            }
+          } else {
+            // the box before last has been read
+            if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+            __syncwarp();
+          }
           const bool whole = col0 + kChunkCols <= n;  // a box that is cut off in the middle of 16 bytes writes them all
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            const uint32_t rw[4] = {rr[i].x, rr[i].y, rr[i].z, rr[i].w};
-            uint32_t p[4];
+            // 64-byte swizzle: eight lanes' pieces lie in eight different sixteenths of the 128-byte span of the banks
+            const uint32_t piece = box + lane * 64 + ((i ^ (lane >> 1 & 3)) << 4);
+            uint32_t rw[4] = {0u, 0u, 0u, 0u}, p[4];
+            if (ep.residual != nullptr) {
+              asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(rw[0]), "=r"(rw[1]), "=r"(rw[2]), "=r"(rw[3]) : "r"(piece) : "memory");
+            }
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
               p[e] = pack_bf16(fmaf(__uint_as_float(r[8 * i + 2 * e]), alpha, __uint_as_float(rw[e] << 16)),
@@ -436,8 +457,7 @@ gemm_w4a4_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
               if (row0 + lane < m && col0 + 8 * i < n) store_bf16_tail(c + static_cast<size_t>(row0 + lane) * ldc + col0 + 8 * i, make_uint4(p[0], p[1], p[2], p[3]), n - col0 - 8 * i);
               continue;
             }
-            // 64-byte swizzle: eight lanes' pieces lie in eight different sixteenths of the 128-byte span of the banks
-            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(box + lane * 64 + ((i ^ (lane >> 1 & 3)) << 4)), "r"(p[0]), "r"(p[1]), "r"(p[2]), "r"(p[3]) : "memory");
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(piece), "r"(p[0]), "r"(p[1]), "r"(p[2]), "r"(p[3]) : "memory");
           }
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           __syncwarp();
@@ -474,7 +494,10 @@ gemm_w4a4_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       }
     }
     if (!ok && !aborted && lane == 0) atomicExch(status, kEpilogueWait);
-    // the boxes stay until they have been stored
+    // the boxes stay until they have been stored, and until what was asked for has landed
+    if (!ok) {
+      for (int i = max(res_loads - 2, 0); i < res_loads; ++i) mbar_wait(smem_u32(res_full + 2 * (warp - 2) + (i & 1)), i >> 1 & 1);
+    }
     if (kEpilogueWarps == kEpiWarpsPlain && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
 
@@ -518,7 +541,7 @@ int encode_map(CUtensorMap * map, CUtensorMapDataType type, const void * base, c
   return Q35B_OK;
 }
 
-// 2-D map over the BF16 output [m, n] with rows ldc apart: boxes of 32 x 32 values.
+// 2-D map over the BF16 output or residual [m, n] with rows ldc apart: boxes of 32 x 32 values.
 int make_output_map(CUtensorMap * map, const void * c, int m, int n, int ldc) {
   return encode_map(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, c, static_cast<cuuint64_t>(n), static_cast<cuuint64_t>(m), static_cast<cuuint64_t>(ldc) * 2,
                     kChunkCols, 32, CU_TENSOR_MAP_SWIZZLE_64B, "output");
@@ -563,14 +586,17 @@ int launch_gemm_w4a4_2cta(const q35b_weight * w, const uint8_t * a_codes, const 
   // plain and residual epilogues without peers whose rows a TMA box can be stored to
   const bool plain = !ep.gate_up && ep.q_codes == nullptr && ep.n_peers == 0 && (ldc % 8) == 0 && (reinterpret_cast<uintptr_t>(c_bf16) & 15u) == 0 &&
                      (ep.residual == nullptr || ((ep.ldr % 8) == 0 && (reinterpret_cast<uintptr_t>(ep.residual) & 15u) == 0));
-  CUtensorMap tmap_c = tmap_a;
+  CUtensorMap tmap_c = tmap_a, tmap_res = tmap_a;
   if (plain) {
     if (const int st = make_output_map(&tmap_c, c_bf16, m, w->rows, ldc)) return st;
+    if (ep.residual != nullptr) {
+      if (const int st = make_output_map(&tmap_res, ep.residual, m, w->rows, ep.ldr)) return st;
+    }
   }
   const int epi_warps = plain ? kEpiWarpsPlain : kEpiWarpsWide;
   const auto kernel = plain ? gemm_w4a4_2cta_kernel<kEpiWarpsPlain> : gemm_w4a4_2cta_kernel<kEpiWarpsWide>;
   const cudaError_t le = launch_pdl(kernel, dim3(2 * pairs), dim3((2 + epi_warps) * 32), plain ? kSmemBytesPlain : kSmemBytes, s, tmap_a, w->tmap2_codes,
-                                    tmap_sfa, w->tmap2_sf, tmap_c, g_dev, ep, m, w->rows, w->k / 2, m_tiles, num_tiles,
+                                    tmap_sfa, w->tmap2_sf, tmap_c, tmap_res, g_dev, ep, m, w->rows, w->k / 2, m_tiles, num_tiles,
                                     static_cast<__nv_bfloat16 *>(c_bf16), ldc, status_dev);
   count_launch();
   Q35B_CUDA_TRY(le, "gemm_w4a4_2cta_kernel launch");
