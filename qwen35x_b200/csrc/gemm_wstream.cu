@@ -588,18 +588,24 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
 
 // ---- decode: BF16 activations -> octal digits in NVFP4 ----------------------------------------------------------
 
+// What a CTA per token expands: columns 8 * begin .. 8 * end (whole K steps) of one item's activations.
 struct ExpandItem {
   const __nv_bfloat16 * x;   // [tokens, k], k a multiple of 256
   uint8_t * ops;             // see WItem::x_ops; operand row = token * digits + digit, and likewise of the deep digits
   uint32_t * deep;           // see WItem::x_deep
   float * g;                 // [tokens]: scale of each token's expansion
   int k;
+  int begin, end;
   int step_bytes;            // of a K step of ops
   int scales_at;             // its scale tiles
   int deep_row, deep_at, deep_scales_at;  // the deep digits' first operand row, their codes and scale tiles
 };
 
 constexpr int kSplitThreads = 256;
+// Of eight columns that a CTA expands, a multiple of 32.  A CTA per token of [.., 9216] was still at work 15 us after the first ones
+// had started, and every CTA of the projection kernel waits for the last.  0.8B-class step one token 42.1 -> 41.2 us, eight 51.7 ->
+// 50.9, 4B-class one 290.0 -> 289.8, four 311.7 -> 308.4; 512 chunks 42.1, 52.2, 292.0 and 306.3, 128 42.5, 52.1, 290.1 and 310.3.
+constexpr int kSplitChunks = 256;
 constexpr int kDeepWords = 64;   // of 32 K steps each: 524288 columns, more than a list on either path can have
 
 // One CTA per (projection, token); digits.cuh has what they are.
@@ -648,10 +654,10 @@ __global__ void __launch_bounds__(kSplitThreads) split_digits_kernel(const Expan
 #pragma unroll
   for (int i = 0; i < kSplitThreads / 32; ++i) best = max(best, red[i]);
   const int top = max(static_cast<int>(best >> 7), 1);  // exponent field of the token's largest value
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == 0 && it.begin == 0) {
     it.g[token] = best > 0x7f80u ? __uint_as_float(0x7fffffffu) : (best == 0x7f80u ? __uint_as_float(0x7f800000u) : digits_scale(top));
   }
-  for (int c = threadIdx.x; c < chunks; c += kSplitThreads) {  // whole warps: chunks is a multiple of 32
+  for (int c = it.begin + threadIdx.x; c < it.end; c += kSplitThreads) {  // whole warps: both are multiples of 32
     const uint4 q = best < 0x7f80u ? load(c) : make_uint4(0u, 0u, 0u, 0u);  // the epilogue has no use for the digits then
     uint32_t b = bf16x8_abs_max(q);
     b = max(b, __shfl_xor_sync(0xffffffffu, b, 1));
@@ -693,7 +699,14 @@ __global__ void __launch_bounds__(kSplitThreads) split_digits_kernel(const Expan
   }
   if (it.deep != nullptr) {
     __syncthreads();
-    if (static_cast<int>(threadIdx.x) < words && deep_now[threadIdx.x] != before) it.deep[8 * threadIdx.x + token] = deep_now[threadIdx.x];
+    if (static_cast<int>(threadIdx.x) < words) {
+      // this CTA's steps of the word: the others' bits are others' to change
+      const int lo = max(it.begin / 32 - 32 * static_cast<int>(threadIdx.x), 0), hi = min(it.end / 32 - 32 * static_cast<int>(threadIdx.x), 32);
+      const uint32_t own = hi > lo ? (hi == 32 ? ~0u : (1u << hi) - 1u) & ~((1u << lo) - 1u) : 0u;
+      const uint32_t now = deep_now[threadIdx.x], gone = before & own & ~now, come = now & ~before;
+      if (gone != 0u) atomicAnd(it.deep + 8 * threadIdx.x + token, ~gone);
+      if (come != 0u) atomicOr(it.deep + 8 * threadIdx.x + token, come);
+    }
   }
 }
 
@@ -720,7 +733,7 @@ int ensure_attr() {
 // ---- decode work list on the tensor path ------------------------------------------------------------------------
 
 struct WBatch {
-  int count = 0, m = 0, digits = 0, grid = 0, stages = 0, b_slot = 0, deep_bytes = 0, smem = 0;
+  int count = 0, m = 0, digits = 0, expand_count = 0, grid = 0, stages = 0, b_slot = 0, deep_bytes = 0, smem = 0;
   void * dev_base = nullptr;
   WItem * items = nullptr;
   WTile * tiles = nullptr;
@@ -838,10 +851,12 @@ int wbatch_build(const q35b_gemv_item * items, int count, int m, int digits, boo
   }
   h_begin.push_back(static_cast<int>(h_tiles.size()));
   auto up = [](size_t v, size_t a) { return (v + a - 1) / a * a; };
+  size_t expand_count = 0;
+  for (int i = 0; i < count; ++i) expand_count += (items[i].weight->k / 8 + kSplitChunks - 1) / kSplitChunks;
   const size_t o_tiles = up(sizeof(WItem) * count, 256);
   const size_t o_begin = up(o_tiles + sizeof(WTile) * all.size(), 256);
   const size_t o_expand = up(o_begin + sizeof(int) * (grid + 1), 256);
-  const size_t o_status = up(o_expand + sizeof(ExpandItem) * count, 256);
+  const size_t o_status = up(o_expand + sizeof(ExpandItem) * expand_count, 256);
   size_t o_data = o_status + 256;
   std::vector<size_t> o_ops(count), o_g(count), o_deep(count);
   for (int i = 0; i < count; ++i) {
@@ -864,7 +879,7 @@ int wbatch_build(const q35b_gemv_item * items, int count, int m, int digits, boo
   b->expand = reinterpret_cast<ExpandItem *>(base + o_expand);
   b->status = reinterpret_cast<unsigned int *>(base + o_status);
   std::vector<WItem> h_items(count);
-  std::vector<ExpandItem> h_expand(count);
+  std::vector<ExpandItem> h_expand;
   for (int i = 0; i < count; ++i) {
     const q35b_weight * w = items[i].weight;
     WItem & it = h_items[i];
@@ -890,17 +905,20 @@ int wbatch_build(const q35b_gemv_item * items, int count, int m, int digits, boo
     it.s2 = w->s2;
     it.s2_up = w->s2_up;
     it.epilogue = w->gate_up ? kEpiGateUp : kEpiPlain;
-    h_expand[i] = ExpandItem{static_cast<const __nv_bfloat16 *>(items[i].x_bf16), base + o_ops[i],
-                             exact ? reinterpret_cast<uint32_t *>(base + o_deep[i]) : nullptr,
-                             reinterpret_cast<float *>(base + o_g[i]), w->k, b->b_slot, n_cols * kStepBytes, inside ? op_rows : 0,
-                             inside ? 0 : n_cols * kStepBytes + kSfBytes,
-                             inside ? n_cols * kStepBytes : (n_cols + deep_cols) * kStepBytes + kSfBytes};
+    for (int begin = 0; begin < w->k / 8; begin += kSplitChunks) {
+      h_expand.push_back(ExpandItem{static_cast<const __nv_bfloat16 *>(items[i].x_bf16), base + o_ops[i],
+                                    exact ? reinterpret_cast<uint32_t *>(base + o_deep[i]) : nullptr, reinterpret_cast<float *>(base + o_g[i]), w->k, begin,
+                                    std::min(begin + kSplitChunks, w->k / 8), b->b_slot, n_cols * kStepBytes, inside ? op_rows : 0,
+                                    inside ? 0 : n_cols * kStepBytes + kSfBytes,
+                                    inside ? n_cols * kStepBytes : (n_cols + deep_cols) * kStepBytes + kSfBytes});
+    }
   }
+  b->expand_count = static_cast<int>(h_expand.size());
   e = cudaMemset(b->dev_base, 0, o_data);
   if (e == cudaSuccess) e = cudaMemcpy(b->items, h_items.data(), sizeof(WItem) * count, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(b->tiles, h_tiles.data(), sizeof(WTile) * h_tiles.size(), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(b->cta_begin, h_begin.data(), sizeof(int) * (grid + 1), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(b->expand, h_expand.data(), sizeof(ExpandItem) * count, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(b->expand, h_expand.data(), sizeof(ExpandItem) * h_expand.size(), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
     cudaFree(b->dev_base);
     delete b;
@@ -913,7 +931,7 @@ int wbatch_build(const q35b_gemv_item * items, int count, int m, int digits, boo
 int wbatch_launch(const WBatch * b, cudaStream_t s) {
   // 1. the digits of every item's activations (one CTA per item and token); 2. the streaming kernel, whose weight
   // producer starts at once while its activation producer waits for the expansion
-  cudaError_t le = launch_pdl(split_digits_kernel, dim3(b->count, b->m), dim3(kSplitThreads), 0, s,
+  cudaError_t le = launch_pdl(split_digits_kernel, dim3(b->expand_count, b->m), dim3(kSplitThreads), 0, s,
                               static_cast<const ExpandItem *>(b->expand), b->digits, b->exact ? 1 : 0);
   count_launch();
   Q35B_CUDA_TRY(le, "split_digits_kernel launch");
