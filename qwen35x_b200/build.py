@@ -92,7 +92,7 @@ def build_binding(force: bool = False) -> Path:
         cmd = ["g++", "-std=c++17", "-O2", "-fPIC", "-shared", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
                f"-I{root / 'include'}", f"-I{root / 'include' / 'torch' / 'csrc' / 'api' / 'include'}", f"-I{cuda / 'include'}",
                f"-I{sysconfig.get_paths()['include']}", str(src), "-o", str(BINDING), f"-L{LIB_DIR}", "-lq35b", f"-L{root / 'lib'}",
-               "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python", "-Wl,-rpath,$ORIGIN"]
+               "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-Wl,-rpath,$ORIGIN"]
         subprocess.run(cmd, check=True)
         BINDING_STAMP.write_text(stamp)
     return BINDING

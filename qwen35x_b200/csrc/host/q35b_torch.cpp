@@ -7,8 +7,10 @@
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <ATen/cuda/EmptyTensor.h>
 #include <ATen/ops/empty.h>
 #include <c10/cuda/CUDAFunctions.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAStream.h>
 
 #include "../../../include/q35b_nvfp4.h"
@@ -71,10 +73,17 @@ int without_gil(F && f) {
   return status;
 }
 
+// A new tensor.  Without the dispatcher, unless someone listens to it: 0.9 us instead of 1.4, of 4.2 for the smallest projection.
+at::Tensor empty(at::IntArrayRef size, at::ScalarType type, c10::DeviceIndex device) {
+  const c10::Device where(at::kCUDA, device);
+  if (c10::impl::TorchDispatchModeTLS::any_modes_set()) return at::empty(size, at::TensorOptions().dtype(type).device(where));
+  return at::detail::empty_cuda(size, type, where, std::nullopt);
+}
+
 // The caller's output [m, cols] BF16 with unit column stride, or a new one in `made`; NULL: not the plain form.
 const at::Tensor * output(PyObject * o, int64_t m, int64_t cols, c10::DeviceIndex device, at::Tensor & made) {
   if (o == Py_None) {
-    made = at::empty({m, cols}, at::TensorOptions().dtype(at::kBFloat16).device(at::kCUDA, device));
+    made = empty({m, cols}, at::kBFloat16, device);
     return &made;
   }
   const at::Tensor * t = nullptr;
@@ -121,7 +130,7 @@ PyObject * gemv_f32(PyObject *, PyObject * const * args, Py_ssize_t n) {
   float scale = 0.0f;
   int kernel = 0;
   if (!float_arg(args[2], &scale) || !int_arg(args[3], &kernel)) return not_plain();
-  at::Tensor y = at::empty({q35b_weight_rows(w)}, x->options());
+  at::Tensor y = empty({q35b_weight_rows(w)}, at::kFloat, device);
   const float * xp = x->const_data_ptr<float>();
   float * yp = y.mutable_data_ptr<float>();
   void * stream = stream_of(device);
