@@ -1005,26 +1005,62 @@ Assignment assign_tiles(const std::vector<GemvTile> & all, const std::vector<int
 // Whether a list runs on the tensor cores (gemm_wstream.cu): independent items, block scales the tensor cores read as this
 // kernel does, enough weights, and whole tiles that come out even.  That path puts one more launch in front of every run (5 us
 // for one token, 9 for eight, under which the next weights fill the rings), issues a fifth of the instructions and, in runs
-// long enough to meet the power cap, keeps its clock; and it never splits a tile.  us, this kernel / tensor cores, one, four and
-// eight tokens.  In runs of 0.2 s and more: 223 MiB of 1024-column projections 49 / 45, -, 61 / 55; 1.8 GiB 358 / 308, 405 / 339.
-// In runs of 80 ms, by the longest CTA's share of the K steps over an even share:
-//   1.0 to 1.4: 231 MiB 53 / 48, 51 / 50, 61 / 52; 202 MiB 55 / 49, 53 / 51, 55 / 53; 180 MiB 35.4 / 34.5, 37.0 / 36.3, 41.9 / 37.8;
-//               142 MiB (1.3) 31 / 35, 36 / 37, 39 / 38; 111 MiB 26.0 / 26.5, 28.0 / 29.8, 32.1 / 32.7; 90 MiB 19.3 / 20.7, 20.2 / 21.9,
-//               25.2 / 23.4; 72 MiB 17.4 / 16.4, 18.1 / 18.1, 20.2 / 22.4; 56 MiB 16.3 / 17.3, 17.7 / 18.7, 21.7 / 22.6
-//   1.55: 115 MiB 30 / 33, 35 / 34, 35 / 36; 58 MiB 17 / 20, 19 / 22, 22 / 24
-//   1.85: 101 MiB 24 / 34, 38 / 36, 31 / 37; 51 MiB 16 / 20, 18 / 21, 21 / 23; 2.3: 72 MiB 21 / 30, 23 / 31
+// long enough to meet the power cap, keeps its clock; it deals its tiles out longest first, where this kernel's contiguous runs
+// (a change of projection costs it a conversion) leave some CTA with up to twice an even share; and it never splits a tile.
+// From 128 MiB on it takes whatever it can deal out to 1.45 of an even share: us, this kernel / tensor cores in runs of 0.2 s,
+// 223 MiB of 1024-column projections one token 49 / 42, eight 61 / 55, 1.8 GiB one token 358 / 292, four 405 / 317; a list with a longest share of 1.55
+// to 2.3 of an even one took 1.1 to 1.4 times as long there.  Below, lists of tiles of four and more K steps on average,
+// with 250 and more rows per token (the digits are made once per column, whatever the rows), that it deals out better than this
+// kernel by as much as the constants say.  One, four and eight tokens, by the ratio of the shares:
+//   1.42 to 2: 26 MiB 12.7 / 8.5, 13.5 / 9.4, 14.3 / 10.4; 28 MiB 12.8 / 9.1, 13.6 / 10.3, 14.2 / 12.1; 37 MiB 13.2 / 12.0, 14.1 / 12.7,
+//              15.7 / 16.3; 47 MiB 15.5 / 14.2, 17.2 / 15.4, 18.5 / 16.2; 71 MiB 20.9 / 17.7, 22.7 / 19.1, 23.8 / 19.9; 74 MiB 21.1 / 17.5, 22.0 / 20.2,
+//              25.0 / 24.0
+//   1.32 to 1.42: 51 MiB 14.5 / 14.6, 15.2 / 15.7, 19.3 / 18.5; 93 MiB 23.5 / 20.7, 24.9 / 23.9, 29.0 / 26.7; 115 MiB 29.7 / 24.7, 34.9 / 26.2, 34.7 / 29.6
+//   1.2 to 1.3: 84 MiB four tokens 21.6 / 22.6; 102 MiB 22.2 / 22.0, 23.6 / 24.8, 28.1 / 27.0
+//   tiles of 2.3 steps on average: 25 MiB 9.7 / 9.7, 10.3 / 12.8, 11.4 / 16.5; 160 rows per token: 47 MiB seven tokens 16.8 / 20.0
 constexpr int kTensorDigits = 8;  // three bits each, and more of them where a value needs them (gemm_wstream.cu)
-constexpr size_t kTensorBytes = 128u << 20;
-constexpr double kTensorLongest = 1.45;
+constexpr size_t kTensorBytes = 128u << 20, kTensorBytesEven = 64u << 20, kTensorBytesLeast = 24u << 20;
+constexpr double kTensorLongest = 1.45, kTensorBetterEven = 1.32, kTensorBetterLeast = 1.42;
+constexpr int kTensorSteps = 4, kTensorRows = 250;
 
-bool tensor_list(const q35b_gemv_item * items, int count) {
+// The longest CTA's share of a list's K steps over an even one, two CTAs per SM and whole tiles in contiguous runs.
+double contiguous_share(const q35b_gemv_item * items, int count) {
+  long total = 0, tiles = 0, done = 0, share = 0, longest = 0;
+  for (int i = 0; i < count; ++i) tiles += (items[i].weight->rows + kTileRows - 1) / kTileRows;
+  for (int i = 0; i < count; ++i) total += static_cast<long>((items[i].weight->rows + kTileRows - 1) / kTileRows) * (items[i].weight->k / 256 + 1);
+  const long grid = std::min<long>(2 * sm_count(), tiles);
+  long c = 0;
+  for (int i = 0; i < count; ++i) {
+    const long cost = items[i].weight->k / 256 + 1;
+    for (int t = 0; t < (items[i].weight->rows + kTileRows - 1) / kTileRows; ++t) {
+      while (c + 1 < grid && (done + cost / 2) * grid >= (c + 1) * total) {
+        ++c;
+        share = 0;
+      }
+      longest = std::max(longest, share += cost);
+      done += cost;
+    }
+  }
+  return total > 0 ? static_cast<double>(longest) * grid / total : 1.0;
+}
+
+bool tensor_list(const q35b_gemv_item * items, int count, int m) {
   size_t bytes = 0;
+  long steps = 0, tiles = 0, columns = 0;
+  double weights = 0.0;
   for (int i = 0; i < count; ++i) {
     const q35b_weight * w = items[i].weight;
     if (items[i].after != 0 || w->rows <= 0 || !w->has_maps || w->nan_scales || items[i].x_bf16 == nullptr || items[i].y_bf16 == nullptr) return false;
     bytes += w->codes_bytes + w->scales_bytes;
+    tiles += (w->rows + kTileRows - 1) / kTileRows;
+    steps += static_cast<long>((w->rows + kTileRows - 1) / kTileRows) * (w->k / 256);
+    columns += w->k;
+    weights += static_cast<double>(w->rows) * w->k;
   }
-  return bytes >= kTensorBytes && wbatch_longest_share(items, count) <= kTensorLongest;
+  if (bytes < kTensorBytesLeast) return false;
+  const double longest = wbatch_longest_share(items, count);
+  if (bytes >= kTensorBytes) return longest <= kTensorLongest;
+  return steps >= kTensorSteps * tiles && weights >= static_cast<double>(kTensorRows) * m * columns && contiguous_share(items, count) >= longest * (bytes >= kTensorBytesEven ? kTensorBetterEven : kTensorBetterLeast);
 }
 
 // Whether a list runs as one launch per item in which the operand is made in shared memory (gemm_resident.cu): a chain, so
@@ -1066,7 +1102,7 @@ int gemv_batch_build(const q35b_gemv_item * items, int count, int m, bool share_
     max_k = std::max(max_k, w->k);
   }
   // only what the plan below takes too: a list whose activations do not fit it is refused whatever its size
-  if (Plan fits_plan; share_tiles && tensor_list(items, count) && make_plan(m, max_k, &fits_plan)) {
+  if (Plan fits_plan; share_tiles && tensor_list(items, count, m) && make_plan(m, max_k, &fits_plan)) {
     WBatch * t = nullptr;
     if (const int st = wbatch_build(items, count, m, kTensorDigits, true, &t)) return st;
     auto * b = new q35b_gemv_batch();
