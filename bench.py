@@ -289,7 +289,7 @@ def run_engine(args, rank: int, world: int, local_rank: int) -> dict | None:
     step_bytes = sum(algorithmic_bytes(n, k, args.m) for n, k in shapes)
     stream = torch.cuda.Stream(device=device)
 
-    # The step's work list: all 96 projections in one persistent launch (they are independent in this workload).
+    # The step's work list: all 96 projections in one run (they are independent in this workload).
     batches = [q.GemvBatch(list(zip(models[s], xs, ys)), args.m, digits=args.digits) for s in range(sets)]
     launched = q.launch_count()
     batches[0].run()

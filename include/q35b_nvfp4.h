@@ -154,11 +154,12 @@ Q35B_API int q35b_gemv_w4a16_bf16(const q35b_weight * w, const void * x_bf16, in
 Q35B_API int q35b_gemv_w4a16_f32(const q35b_weight * w, const float * x_f32, float input_scale, float * y_f32,
                                  int kernel, q35b_stream stream);
 
-/* One persistent launch over several projections (the work list of a decode step, or of one phase of it).
+/* Several projections as one work list (of a decode step, or of one phase of it): one persistent launch, two on the tensor
+ * cores, or for a chain one per item; see q35b_gemv_batch_create.
  * Replaces the per-phase matvec loops of the reference's persistent decode kernel
  * (src/kernels/cuda/decode_kernel.cuh:58-84).  Every weight needs cols % 256 == 0 and unsigned block scales.
  * Items are independent unless one names an earlier item in `after`: then its x_bf16 may be that item's y_bf16 (the
- * down projection reading the gate/up output), and the kernel holds its activations back until every tile of the
+ * down projection reading the gate/up output), and its activations are held back until every tile of the
  * earlier item has been stored -- where the reference's decode kernel puts a grid-wide barrier between the two
  * phases (decode_kernel.cuh:76-84), with a bounded wait instead of an unbounded one. */
 typedef struct q35b_gemv_item {
@@ -177,10 +178,11 @@ Q35B_API size_t q35b_gemv_item_bytes(void);
 typedef struct q35b_gemv_batch q35b_gemv_batch;
 /* Builds the tile schedule and uploads the descriptors (allocates, synchronises).
  * How exact a list is does not depend on what is in it: sums are fp32, and of a BF16 activation nothing is lost above 2^-39
- * of its token's largest one.  Lists with dependent items, and small ones, convert every token to fp16 with one power of two;
+ * of its token's largest one.  Most lists with dependent items, and small ones, convert every token to fp16 with one power of two;
  * large lists of independent items run on the tensor cores (see below) with as many octal digits as that takes: eight in
  * every K step, and six more in the steps of 256 columns where a value has bits below 2^-16 of the largest of its sixteen
- * neighbours.  Infinities and NaNs reach the outputs as fp32 arithmetic has it, on either path.
+ * neighbours.  So do chains of up to six tokens, lists in which every item runs after the one before it (an MLP block): one
+ * launch per item, which makes the digits itself and owns no memory for them.  Infinities and NaNs reach the outputs as fp32 arithmetic has it, on either path.
  * Device memory a list owns: descriptors and counters, some hundred KB; on the tensor cores also the operand rows, per 256
  * columns of every item 4 KB for one token, 8 KB for two, 12 KB for four and 18 KB for eight (a 4B-class step 9 and 41 MB). */
 Q35B_API int q35b_gemv_batch_create(const q35b_gemv_item * items, int count, int m, q35b_gemv_batch ** out);
@@ -195,7 +197,7 @@ Q35B_API int q35b_gemv_batch_create(const q35b_gemv_item * items, int count, int
  * launches two kernels (the digits, then the projection, whose weight stream starts at once). */
 Q35B_API int q35b_gemv_batch_create_tensor(const q35b_gemv_item * items, int count, int m, int digits,
                                            q35b_gemv_batch ** out);
-/* One kernel launch on `stream`, or two (see above); no allocation, no synchronisation.  The launch uses programmatic stream
+/* One kernel launch on `stream`, or two, or for a chain one per item (see above); no allocation, no synchronisation.  The launch uses programmatic stream
  * serialisation: the kernel may begin streaming WEIGHTS while the previous kernel of the stream is still finishing
  * (activations, residuals and outputs are touched only after that kernel is complete).  Weights are therefore
  * treated as constant from q35b_weight_create* on; a host that rewrites weight memory must synchronise the stream
@@ -209,7 +211,7 @@ Q35B_API int q35b_gemv_batch_status(const q35b_gemv_batch * batch, unsigned int 
 /* Test hook for the bounded device-side waits of a work list built by q35b_gemv_batch_create: every wait of the
  * following runs (ring barriers, activation hand-over, dependency poll) gives up after `wait_limit_polls` polls
  * instead of 2^22, and (lists on the other path than the tensor cores) in every other CTA, the first included, a dependent item demands `extra_completions` more
- * completions of the item it runs after than that item can deliver.  With a small limit and one extra completion the dependency poll runs out within
+ * completions of the item it runs after than that item can deliver (a chain then runs as one launch again).  With a small limit and one extra completion the dependency poll runs out within
  * microseconds, 15 lands in the status word, the remaining roles run out on their own waits and the kernel returns:
  * what an item whose producer never finishes looks like, without a kernel that hangs.  (0 extra completions and
  * 1 << 22 polls restore normal operation.)  Also clears the list's status word; the counters of a run are at zero

@@ -349,8 +349,8 @@ class _GemvItem(C.Structure):
 
 
 class GemvBatch:
-    """A prepared work list of decode projections run by one persistent launch (q35b_gemv_batch_* in
-    include/q35b_nvfp4.h).  items: sequence of (Nvfp4Weight, x [m,K] bf16, y [m,out_rows] bf16),
+    """A prepared work list of decode projections run by one persistent launch, two on the tensor cores, or for a chain of
+    dependent items one per item (q35b_gemv_batch_* in include/q35b_nvfp4.h).  items: sequence of (Nvfp4Weight, x [m,K] bf16, y [m,out_rows] bf16),
     (weight, x, y, residual [m,rows] bf16) or (weight, x, y, residual-or-None, after): with a residual the projection
     is added to it before the BF16 rounding; a gate/up weight (Nvfp4Weight.gate_up_from_host) yields silu(gate)*up
     with out_rows = rows/2; `after` = index of an earlier item whose y this item's x is (the down projection after
