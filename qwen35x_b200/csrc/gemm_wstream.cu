@@ -12,7 +12,7 @@
 // a TMA-fed shared-memory ring (weights and activations have separate producer threads: weights are constant and
 // start streaming before the previous kernel of the stream has finished, activations wait for it), one MMA thread
 // issuing tcgen05.mma kind::mxf4nvf4.block_scale per 64 columns of K, two TMEM accumulators so that the epilogue of
-// a tile runs under the MMAs of the next, and four epilogue warps that turn accumulator lanes into BF16 outputs
+// a tile runs under the MMAs of the next, and epilogue warps that turn accumulator lanes into BF16 outputs
 // y[token, row].
 //
 // Decode (W4A16, 1..8 tokens): every token enters as `digits` operand rows, the octal digits of its BF16 activations
@@ -49,8 +49,15 @@ constexpr int kABytes = kRows * kStepBytes;          // 16 KB
 constexpr int kSfBytes = kMmaPerStage * kSfChunk;    // 2 KB (weights, and activations: at most 128 operand rows)
 constexpr int kMaxCols = 128;
 constexpr int kMaxStages = 8;
-constexpr int kEpilogueWarps = 8;        // two per quarter of the TMEM lanes, each taking every other token
-constexpr int kThreads = (3 + kEpilogueWarps) * 32;  // warp 0 weight producer, 1 MMA, 2 activation producer
+// Warp 0 weight producer, 1 MMA, 2 activation producer, the others epilogue: two per quarter of the TMEM lanes, which take turns
+// at the tokens; three from seven tokens on in lists of short tiles, which are over before two have the sums out.  us, two /
+// three, lists of 0.3 GB of [4096, K], eight tokens: K = 768 84.0 / 78.8, 1024 70.1 / 67.6, 1536 60.0 / 60.4, 2048 58.4 / 59.0, 2560 58.2 / 58.4
+// (seven the same); 0.8B-class step (5.1 K steps per tile) seven tokens 52.1 / 51.3, eight 54.8 / 53.4, six 48.9 / 49.1, one 41.6 / 44.2;
+// 4B-class eight 339.7 / 344.9.  Four per quarter: 0.8B-class eight tokens as with three, but no CTA of the digits' kernel fits beside them.
+constexpr int kEpilogueWarps = 8, kEpilogueWarpsWide = 12, kWideTokens = 7, kWideSteps = 6;
+constexpr int threads_for(int epilogue_warps) { return (3 + epilogue_warps) * 32; }
+// Registers: of 112 per thread the wide CTA leaves room for one of split_digits_kernel's.
+constexpr int kLaunchBound = 512;
 constexpr int kTmemCols = 512;           // two accumulator buffers ...
 constexpr int kAccBufCols = 224;         // partial accumulators of the operand rows, then those of the deep digits' rows
 constexpr int kSfaCol = 2 * kAccBufCols;   // ... and two sets of scale-factor columns (A 16 + B 16 each), used by stages in turn,
@@ -222,7 +229,7 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
 }
 
 // CTA b walks tiles[cta_begin[b] .. cta_begin[b + 1]).
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kLaunchBound, 1)
 gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__ tiles, const int * __restrict__ cta_begin,
                     int stages, int b_slot_bytes, int deep_bytes, unsigned int * status, uint32_t wait_limit) {
   extern __shared__ uint8_t smem_raw[];
@@ -274,7 +281,7 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
     d.s2_up = it->s2_up;
   };
   // tile descriptors are constant for the life of a work list (and of a launch): read them before anything else
-  for (int ti = threadIdx.x; ti < min(n_tiles, kMaxTilesInSmem); ti += kThreads) {
+  for (int ti = threadIdx.x; ti < min(n_tiles, kMaxTilesInSmem); ti += blockDim.x) {
     describe(ti, stile[ti]);
     if (ti == 0 || tiles[tile_begin + ti - 1].item != tiles[tile_begin + ti].item) {
       asm volatile("prefetch.tensormap [%0];" ::"l"(stile[ti].tmap_w) : "memory");
@@ -294,7 +301,7 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(tmem_full + i), 1);
-      mbar_init(smem_u32(tmem_empty + i), kEpilogueWarps);
+      mbar_init(smem_u32(tmem_empty + i), blockDim.x / 32 - 3);
     }
     mbar_init(smem_u32(mma_done), 1);
     gave_up = 0;
@@ -468,7 +475,7 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
   } else {
     // ------------------------------------------------------------ epilogue: lane = weight row, column = operand row
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int quarter = warp & 3, first_token = (warp - 3) >> 2;
+    const int quarter = warp & 3, first_token = (warp - 3) >> 2, turns = (static_cast<int>(blockDim.x) - 96) >> 7;
     const int row_in_tile = quarter * 32 + lane;
     STile spill;
     const float * scales_of = nullptr;
@@ -508,7 +515,7 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
       // One token at a time, in a compact loop: a small part of a tile's time as long as its code stays resident (with all
       // columns unrolled a 0.8B-class step of eight tokens took 99 us instead of 54).
 #pragma unroll 1
-      for (int token = first_token; token < tokens; token += 2) {
+      for (int token = first_token; token < tokens; token += turns) {
         uint32_t col = taddr + token * digits;
         int stride = n_cols, count = digits, sums = parts;
         float g = __shfl_sync(0xffffffffu, scales, token);
@@ -741,6 +748,7 @@ struct WBatch {
   ExpandItem * expand = nullptr;
   unsigned int * status = nullptr;
   size_t bytes_per_run = 0;
+  bool wide = false;        // more epilogue warps
   bool exact = false;       // all bits of the activations, their infinities and NaNs too, reach the outputs
   uint32_t wait_limit = kWaitLimit;
 };
@@ -841,6 +849,9 @@ int wbatch_build(const q35b_gemv_item * items, int count, int m, int digits, boo
     for (int rb = 0; rb < (w->rows + kRows - 1) / kRows; ++rb) all.push_back(WTile{i, rb});
     b->bytes_per_run += w->codes_bytes + w->scales_bytes;
   }
+  long steps = 0;
+  for (const WTile & t : all) steps += items[t.item].weight->k / 256;
+  b->wide = m >= kWideTokens && steps < static_cast<long>(kWideSteps) * static_cast<long>(all.size());
   const int grid = std::max(1, std::min<int>(sm_count(), static_cast<int>(all.size())));
   b->grid = grid;
   std::vector<WTile> h_tiles;
@@ -935,7 +946,7 @@ int wbatch_launch(const WBatch * b, cudaStream_t s) {
                               static_cast<const ExpandItem *>(b->expand), b->digits, b->exact ? 1 : 0);
   count_launch();
   Q35B_CUDA_TRY(le, "split_digits_kernel launch");
-  le = launch_pdl(gemm_wstream_kernel, dim3(b->grid), dim3(kThreads), static_cast<size_t>(b->smem), s,
+  le = launch_pdl(gemm_wstream_kernel, dim3(b->grid), dim3(threads_for(b->wide ? kEpilogueWarpsWide : kEpilogueWarps)), static_cast<size_t>(b->smem), s,
                   static_cast<const WItem *>(b->items), static_cast<const WTile *>(b->tiles), static_cast<const int *>(b->cta_begin),
                   b->stages, b->b_slot, b->deep_bytes, b->status, b->wait_limit);
   count_launch();

@@ -284,3 +284,36 @@ def test_lists_whose_whole_tiles_come_out_uneven_stay_on_the_other_kernel(engine
         items.append((w, torch.randn((m, k), device="cuda", generator=gen).to(torch.bfloat16),
                       torch.empty((m, n), dtype=torch.bfloat16, device="cuda")))
     _run(engine, torch, items, m, launches=launches)
+
+
+@pytest.mark.parametrize("m", [6, 7, 8])
+def test_lists_of_short_tiles(engine, m):
+    """Tiles of four K steps on average, from seven tokens on with another number of warps that take turns at the tokens: rows
+    around a tile, a residual, one to four K steps, an infinity and a NaN in the last tokens."""
+    import torch
+
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    n, k = 28672, 1024
+    w = engine.Nvfp4Weight.from_device(torch.randint(0, 256, (n, k // 2), dtype=torch.uint8, device="cuda", generator=gen),
+                                       torch.full((n, k // 16), 0x30, dtype=torch.uint8, device="cuda"), 1e-3)
+    items = [(w, torch.randn((m, k), device="cuda", generator=gen).to(torch.bfloat16), torch.empty((m, n), dtype=torch.bfloat16, device="cuda")) for _ in range(10)]
+    first = len(items)
+    want = []
+    for j, (n, k) in enumerate([(1, 256), (129, 1024), (300, 768), (640, 512), (256, 1024)]):
+        w, wd = _random_weight(engine, torch, gen, n, k)
+        x = torch.randn((m, k), device="cuda", generator=gen)
+        if j == 2:
+            x *= torch.exp2(torch.randint(-30, 30, (m, k), device="cuda", generator=gen).float())
+        if j == 4:
+            x[m - 1, 700], x[m - 2, 3] = float("inf"), float("nan")
+        x = x.to(torch.bfloat16)
+        res = torch.randn((m, n), device="cuda", generator=gen).to(torch.bfloat16) if j == 3 else None
+        y = torch.zeros((m, n), dtype=torch.bfloat16, device="cuda")
+        items.append((w, x, y, res))
+        want.append(x.double() @ wd.T + (res.double() if res is not None else 0.0))
+    _run(engine, torch, items, m)
+    for item, e in zip(items[first:], want):
+        rows = m - 2 if item is items[-1] else m
+        assert _rel(item[2][:rows], e[:rows]) <= 2e-4, item[0].rows
+    last, e = items[-1][2].double(), want[-1]
+    assert bool(torch.isnan(last[m - 2]).all()) and torch.equal(last[m - 1].nan_to_num(0.5), e[m - 1].nan_to_num(0.5))
