@@ -309,7 +309,8 @@ Q35B_API int q35b_gemm_w4a4_bf16_residual(const q35b_weight * w, const uint8_t *
 
 /* q35b_quantize_nvfp4_bf16 (x_is_f32: _f32) of x [m, cols] followed by q35b_gemm_w4a4_bf16 or, with a residual,
  * q35b_gemm_w4a4_bf16_residual: the same outputs, codes, scales and scale word, in one launch where the activation is
- * small enough for every CTA to quantise the columns that it multiplies.  `workspace` as for the quantisation. */
+ * small enough for every CTA to quantise the columns that it multiplies.  `workspace` as for the quantisation.  The output
+ * may lie over x, as with the two calls (it takes two launches then). */
 Q35B_API int q35b_project_prefill(const q35b_weight * w, const void * x, int x_is_f32, int m, float global_scale, uint8_t * codes,
                                   uint8_t * scales_tiled, float * input_scale_dev, void * workspace, const void * residual_bf16,
                                   int ldr, void * c_bf16, int ldc, unsigned int * status_dev, q35b_stream stream);

@@ -833,14 +833,21 @@ int launch_gemm_w4a4(const q35b_weight * w, const uint8_t * a_codes, const uint8
 int launch_project_prefill(const q35b_weight * w, const void * x, bool f32, int m, float global_scale, uint8_t * codes, uint8_t * scales_tiled, float * g_dev,
                            void * workspace, const void * residual_bf16, int ldr, void * c_bf16, int ldc, unsigned int * status_dev, cudaStream_t s) {
   // One launch where the operand is made in shared memory (gemm_resident.cu); whatever is not in order goes the general way,
-  // which says so.
+  // which says so.  So does a call whose output or scratch lies over the activations: in one launch some CTAs store while others
+  // still read x, of two the first has read all of it.
+  auto apart = [&](const void * written, size_t bytes) {
+    const auto a = reinterpret_cast<uintptr_t>(x), b = reinterpret_cast<uintptr_t>(written);
+    return a + static_cast<size_t>(m) * w->k * (f32 ? 4 : 2) <= b || b + bytes <= a;
+  };
   auto aligned = [](const void * p) { return p != nullptr && (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
   if (w != nullptr && m >= 1 && m <= kSplitTokens && w->rows > 0 && w->has_maps && (w->k % 64) == 0 && aligned(x) && aligned(codes) && aligned(scales_tiled) && g_dev != nullptr &&
       (global_scale > 0.0f || workspace != nullptr) && c_bf16 != nullptr && ldc >= (w->gate_up ? w->rows / 2 : w->rows) &&
       (residual_bf16 == nullptr || (!w->gate_up && ldr >= w->rows))) {
     const GemmPlan plan = plan_gemm(m, w->rows, w->n_total, w->k, sm_count(), false, true);
     int stages = 0, smem = 0;
-    if (!plan.pairs && plan.tile_cols >= m && prefill_resident_shape(w, m, global_scale, plan.split, &stages, &smem)) {
+    if (!plan.pairs && plan.tile_cols >= m && prefill_resident_shape(w, m, global_scale, plan.split, &stages, &smem) &&
+        apart(c_bf16, (static_cast<size_t>(m - 1) * ldc + (w->gate_up ? w->rows / 2 : w->rows)) * 2) &&
+        apart(codes, q35b_act_codes_bytes(m, w->k)) && apart(scales_tiled, q35b_act_scales_bytes(m, w->k))) {
       if (const int st = check_weight_device(w)) return st;
       if (status_dev == nullptr) {
         if (const int st = default_status_word(&status_dev)) return st;

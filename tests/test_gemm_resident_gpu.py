@@ -224,3 +224,30 @@ def test_prefill_of_a_gate_up_weight_in_one_launch(engine):
     before = engine.launch_count()
     got = engine.project_prefill(w, x)
     assert engine.launch_count() - before == 1 and torch.equal(got, want)
+
+
+@pytest.mark.parametrize("m,n,k,at", [(4, 1344, 1344, 0), (9, 2432, 2432, 0), (3, 129, 5184, 3 * 5184 - 8), (7, 640, 576, -3 * 640)])
+def test_prefill_whose_output_lies_over_its_activations(engine, m, n, k, at):
+    """All of x is read before anything is stored over it, so two launches; in place, over the last eight values, over the first
+    rows."""
+    import torch
+
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    (codes, scales), _ = _weight(engine, torch, gen, n, k)
+    w = engine.Nvfp4Weight.from_device(codes, scales, 2.0 ** -12)
+    scratch = engine.act_scratch(m, k, "cuda")
+    memory = torch.zeros(3 * m * (n + k), dtype=torch.bfloat16, device="cuda")
+    begin = (m * n + 7) // 8 * 8
+    x, out = memory[begin: begin + m * k].view(m, k), memory[begin + at: begin + at + m * n].view(m, n)
+    for _ in range(5):
+        value = torch.randn((m, k), device="cuda", generator=gen).to(torch.bfloat16)
+        engine.project_prefill(w, value, scratch=scratch)  # the stream's workspace
+        before = engine.launch_count()
+        want = engine.project_prefill(w, value, scratch=scratch)
+        assert engine.launch_count() - before == 1
+        x.copy_(value)
+        before = engine.launch_count()
+        got = engine.project_prefill(w, x, out=out, scratch=scratch)
+        assert engine.launch_count() - before == 2
+        assert torch.equal(got, want)
+    assert engine.gemm_default_status() == 0
