@@ -160,7 +160,7 @@ Q35B_API int q35b_gemv_w4a16_f32(const q35b_weight * w, const float * x_f32, flo
  * (src/kernels/cuda/decode_kernel.cuh:58-84).  Every weight needs cols % 256 == 0 and unsigned block scales.
  * Items are independent unless one names an earlier item in `after`: then its x_bf16 may be that item's y_bf16 (the
  * down projection reading the gate/up output), and its activations are held back until every tile of the
- * earlier item has been stored -- where the reference's decode kernel puts a grid-wide barrier between the two
+ * earlier item has been stored (never, and nothing is stored, in a run in which that one gave up) -- where the reference's decode kernel puts a grid-wide barrier between the two
  * phases (decode_kernel.cuh:76-84), with a bounded wait instead of an unbounded one. */
 typedef struct q35b_gemv_item {
   const q35b_weight * weight;
@@ -218,6 +218,10 @@ Q35B_API int q35b_gemv_batch_status(const q35b_gemv_batch * batch, unsigned int 
  * after it, also after one that gave up. */
 Q35B_API int q35b_debug_gemv_batch_wait(q35b_gemv_batch * batch, unsigned int wait_limit_polls,
                                         unsigned int extra_completions);
+/* Test hook for a chain (one launch per item): in the following runs every other block of 128 rows of item `item`, the first
+ * included, gives up after the limit set above because its activations are never ready, so that these rows stay as they were, its
+ * code (53) lands in the status word and no later item of the run stores anything.  -1: none. */
+Q35B_API int q35b_debug_gemv_batch_absent(q35b_gemv_batch * batch, int item);
 /* The shared-memory plan a work list of `m` tokens over weights of at most `max_k` columns would get (host
  * arithmetic only, no device needed): ctas_per_sm is 2 for the shape with eight consumer warps and half an SM's
  * shared memory, 1 for the shape with sixteen consumer warps and all of it; ring_stages are 18 KB each;

@@ -317,7 +317,7 @@ int q35b_gemv_w4a16_bf16(const q35b_weight * w, const void * x_bf16, int m, void
     if (const int st = check_weight_device(w)) return st;
     unsigned int * status = nullptr;
     if (const int st = default_status_word(&status)) return st;
-    return launch_decode_resident(w, x_bf16, m, y_bf16, nullptr, false, nullptr, status, 1u << 20, static_cast<cudaStream_t>(stream));
+    return launch_decode_resident(w, x_bf16, m, y_bf16, nullptr, nullptr, status, 1u << 20, static_cast<cudaStream_t>(stream));
   }
   if (kernel == Q35B_GEMV_AUTO && w != nullptr && m >= 1 && m <= 8 && !w->gate_up &&
       w->codes_bytes + w->scales_bytes >= kAutoStreamBytes && x_bf16 != nullptr &&
@@ -386,6 +386,8 @@ int q35b_debug_gemv_plan(int m, int max_k, int * ctas_per_sm, int * ring_stages,
 int q35b_debug_gemv_batch_wait(q35b_gemv_batch * batch, unsigned int wait_limit_polls, unsigned int extra_completions) {
   return gemv_batch_debug_wait(batch, wait_limit_polls, extra_completions);
 }
+
+int q35b_debug_gemv_batch_absent(q35b_gemv_batch * batch, int item) { return gemv_batch_debug_absent(batch, item); }
 
 size_t q35b_gemv_batch_stream_bytes(const q35b_gemv_batch * batch) { return gemv_batch_bytes(batch); }
 

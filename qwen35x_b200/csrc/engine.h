@@ -123,6 +123,7 @@ int gemv_batch_read_status(const struct q35b_gemv_batch * b, unsigned int * out)
 size_t gemv_batch_bytes(const struct q35b_gemv_batch * b);
 int gemv_plan_debug(int m, int max_k, int * ctas_per_sm, int * ring_stages, int * activation_buffers, int * smem_bytes);
 int gemv_batch_debug_wait(struct q35b_gemv_batch * b, unsigned int wait_limit, unsigned int extra_completions);
+int gemv_batch_debug_absent(struct q35b_gemv_batch * b, int item);
 
 // gemm_w4a4_tcgen05.cu
 int gemm_plan_debug(int m, int rows, int n_total, int k, int sms, bool gather, bool rows_aligned, int * pairs, int * tile_cols,
@@ -173,10 +174,16 @@ int wbatch_debug_wait(WBatch * b, unsigned int wait_limit);
 
 // gemm_resident.cu: few tokens, the operand made in shared memory
 bool decode_resident_chain(const q35b_weight * w, int m);  // fits as one launch of several
+// What a launch of a chain has to know of its neighbours.
+struct ResidentChain {
+  const q35b_weight * next;      // the weight that the launch after it streams (brought into L2 under it), or NULL
+  unsigned int * gave, * before;  // two words of this launch, and those of the launch before it, or NULL
+  bool absent;                   // test hook: see q35b_debug_gemv_batch_absent
+};
 double decode_resident_ns(const q35b_weight * w, int m);  // estimate for one projection; 0: it does not fit
-// next: the weight that the launch after this one streams (brought into L2 under this one), or NULL
-int launch_decode_resident(const q35b_weight * w, const void * x_bf16, int m, void * y_bf16, const void * residual_bf16, bool chain,
-                           const q35b_weight * next, unsigned int * status, unsigned int wait_limit, cudaStream_t s);
+// chain: NULL for a projection by itself
+int launch_decode_resident(const q35b_weight * w, const void * x_bf16, int m, void * y_bf16, const void * residual_bf16, const ResidentChain * chain,
+                           unsigned int * status, unsigned int wait_limit, cudaStream_t s);
 bool prefill_resident_shape(const q35b_weight * w, int m, float scale, int split, int * stages, int * smem);
 int launch_prefill_resident(const q35b_weight * w, const void * x, bool f32, int m, float scale, uint8_t * codes, uint8_t * scales, float * g_dev, int split, int stages,
                             int smem, const void * residual, int ldr, void * c, int ldc, unsigned int * status, cudaStream_t s);

@@ -82,6 +82,12 @@ struct ResidentArgs {
   const uint8_t * next_codes, * next_scales;
   unsigned long long next_codes_bytes, next_scales_bytes;
   uint32_t next_codes_share, next_scales_share;  // of a CTA
+  // Of a chain: two words of this launch and of the one before it (or NULL).  The first is set where a CTA gives up; then the
+  // launch after it stores nothing, since what it would read may be an earlier run's, and sets its own.  Its CTAs count themselves
+  // in the second, and the last one clears both for the next run.  Otherwise a launch reads a word that nobody writes (a word per
+  // CTA, written in every run, cost half a microsecond of 10 to 18).
+  unsigned int * gave, * before;
+  int absent;                      // test hook: 1: in every other row block, the first included, the operand is never complete
   // W4A4: given per-tensor scale (or 0: from the tensor), and the caller's scratch
   float scale;
   uint8_t * codes, * scales;
@@ -277,7 +283,7 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
       mbar_init(smem_u32(empty + i), 1);
     }
     mbar_init(smem_u32(acc_full), 1);
-    mbar_init(smem_u32(op_ready), kMakers);
+    mbar_init(smem_u32(op_ready), kMakers + (OP == kDigits ? a.absent & ~rb : 0));
     mbar_init(smem_u32(amax_bar), 1);
     mbar_init(smem_u32(mma_done), 1);
     mbar_init(smem_u32(sums), 1);
@@ -587,6 +593,8 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     return o;
   };
   Out out = output(threadIdx.x);
+  uint32_t held_back = 0;
+  if (OP == kDigits && threadIdx.x == 0 && a.before != nullptr) held_back = __ldcg(a.before);
   if (split > 1 && (OP == kDigits || warp < 2)) cluster_wait();  // the makers of NVFP4 codes have
 
   // ---------------- TMEM -> the CTA that stores ----------------
@@ -685,6 +693,7 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
         atomicOr(&gave_up, 2u);
       }
     }
+    if (OP == kDigits && held_back != 0u) atomicOr(&gave_up, 2u);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 1) {
@@ -738,7 +747,12 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     }
   };
   send_and_wait();
-  if (gave_up == 0u) finish();
+  if (gave_up == 0u) {
+    finish();
+  } else if (OP == kDigits && threadIdx.x == 0) {
+    if (a.gave != nullptr) atomicExch(a.gave, 1u);
+    if (held_back != 0u && atomicAdd(a.before + 1, 1u) == gridDim.x * gridDim.z - 1) a.before[0] = a.before[1] = 0u;
+  }
   if ((gave_up & 1u) != 0u && split > 1) {
     __syncthreads();  // with warp 1, which has waited for the other CTAs' sums
     cluster_arrive();
@@ -848,10 +862,10 @@ double decode_resident_ns(const q35b_weight * w, int m) {
   return ns > 0.0 ? 4500.0 + ns : 0.0;
 }
 
-int launch_decode_resident(const q35b_weight * w, const void * x_bf16, int m, void * y_bf16, const void * residual_bf16, bool chain,
-                           const q35b_weight * next, unsigned int * status, unsigned int wait_limit, cudaStream_t s) {
+int launch_decode_resident(const q35b_weight * w, const void * x_bf16, int m, void * y_bf16, const void * residual_bf16,
+                           const ResidentChain * chain, unsigned int * status, unsigned int wait_limit, cudaStream_t s) {
   Shape shape;
-  if (decode_shape(w, m, chain, &shape) == 0.0) return fail(Q35B_ERR_SHAPE, "NVFP4 projection does not fit the resident kernel.");
+  if (decode_shape(w, m, chain != nullptr, &shape) == 0.0) return fail(Q35B_ERR_SHAPE, "NVFP4 projection does not fit the resident kernel.");
   ResidentArgs a = {};
   a.x = x_bf16;
   a.y = static_cast<__nv_bfloat16 *>(y_bf16);
@@ -859,7 +873,12 @@ int launch_decode_resident(const q35b_weight * w, const void * x_bf16, int m, vo
   a.ldy = w->gate_up ? w->rows / 2 : w->rows;
   a.ldr = w->rows;
   a.m = m;
-  if (next != nullptr) {
+  if (chain != nullptr) {
+    a.gave = chain->gave;
+    a.before = chain->before;
+    a.absent = chain->absent ? 1 : 0;
+  }
+  if (const q35b_weight * next = chain != nullptr ? chain->next : nullptr) {
     a.next_codes = next->codes;
     a.next_codes_bytes = next->codes_bytes & ~size_t(15);
     a.next_scales = next->scales_tiled;

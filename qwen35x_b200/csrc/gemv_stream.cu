@@ -865,7 +865,7 @@ struct q35b_gemv_batch {
   unsigned long long * item_done = nullptr;  // per item: storing warps that finished a tile in the current run
   unsigned int * arrivals = nullptr;         // per shared tile and row group: parts that have left their sums
   float * partials = nullptr;                // the parts' sums
-  size_t counter_bytes = 0;                  // status, item_done and arrivals, contiguous and zero between runs
+  size_t counter_bytes = 0;                  // status, item_done, arrivals and chain_gave, contiguous and zero between runs
   bool has_dependencies = false;
   bool shared = false;                       // some tiles are shared by several CTAs
   size_t bytes_per_run = 0;
@@ -873,6 +873,8 @@ struct q35b_gemv_batch {
   unsigned int wait_extra = 0;        // test hook: completions that every other CTA demands on top of what a dependency delivers
   q35b::WBatch * tensor = nullptr;   // set: the list runs on the tensor path (gemm_wstream.cu), nothing above is used
   std::vector<q35b_gemv_item> chain;  // set: it runs as one launch per item, in this order (gemm_resident.cu)
+  unsigned int * chain_gave = nullptr;  // of a chain, two words per item: whether its launch gave up (gemm_resident.cu)
+  int chain_absent = -1;              // test hook: item whose operand is never complete in every other row block
 };
 
 namespace q35b {
@@ -1228,7 +1230,8 @@ int gemv_batch_build(const q35b_gemv_item * items, int count, int m, bool share_
   const size_t o_status = (o_begin + sizeof(int) * (grid + 1) + 15) / 16 * 16;
   const size_t o_done = o_status + 16;
   const size_t o_arrivals = o_done + sizeof(unsigned long long) * (count + 1);  // + the finished-CTA count
-  const size_t o_partials = (o_arrivals + sizeof(unsigned int) * kRowGroups * todo.splits + 127) / 128 * 128;
+  const size_t o_gave = o_arrivals + sizeof(unsigned int) * kRowGroups * todo.splits;
+  const size_t o_partials = (o_gave + sizeof(unsigned int) * 2 * count + 127) / 128 * 128;
   const size_t part_bytes = sizeof(float) * kRowGroups * 32 * 4;  // four sums per lane, in either MMA mapping
   const size_t total = o_partials + part_bytes * todo.slots;
   cudaError_t e = cudaMalloc(&b->dev_base, total);
@@ -1243,6 +1246,7 @@ int gemv_batch_build(const q35b_gemv_item * items, int count, int m, bool share_
   b->status = reinterpret_cast<unsigned int *>(base + o_status);
   b->item_done = reinterpret_cast<unsigned long long *>(base + o_done);
   b->arrivals = reinterpret_cast<unsigned int *>(base + o_arrivals);
+  b->chain_gave = reinterpret_cast<unsigned int *>(base + o_gave);
   b->partials = reinterpret_cast<float *>(base + o_partials);
   b->counter_bytes = o_partials - o_status;
   e = cudaMemcpy(b->items, h_items.data(), sizeof(GemvItem) * count, cudaMemcpyHostToDevice);
@@ -1279,8 +1283,9 @@ int gemv_batch_launch(const q35b_gemv_batch * b, const void * x_override, void *
   if (!b->chain.empty() && b->wait_extra == 0) {
     for (size_t i = 0; i < b->chain.size(); ++i) {
       const q35b_gemv_item & it = b->chain[i];
-      const q35b_weight * next = i + 1 < b->chain.size() ? b->chain[i + 1].weight : nullptr;
-      if (const int st = launch_decode_resident(it.weight, it.x_bf16, b->m, it.y_bf16, it.residual_bf16, true, next, b->status, b->wait_limit, s)) return st;
+      const ResidentChain neighbours = {i + 1 < b->chain.size() ? b->chain[i + 1].weight : nullptr, b->chain_gave + 2 * i,
+                                        i > 0 ? b->chain_gave + 2 * (i - 1) : nullptr, static_cast<int>(i) == b->chain_absent};
+      if (const int st = launch_decode_resident(it.weight, it.x_bf16, b->m, it.y_bf16, it.residual_bf16, &neighbours, b->status, b->wait_limit, s)) return st;
     }
     return Q35B_OK;
   }
@@ -1333,6 +1338,13 @@ int gemv_batch_debug_wait(q35b_gemv_batch * b, unsigned int wait_limit, unsigned
   b->wait_extra = extra_completions;
   // only the recorded code: every run leaves its counters at zero, also one that gave up
   Q35B_CUDA_TRY(cudaMemset(b->status, 0, sizeof(unsigned int)), "cudaMemset(work list status)");
+  return Q35B_OK;
+}
+
+int gemv_batch_debug_absent(q35b_gemv_batch * b, int item) {
+  if (b == nullptr || item < -1 || item >= b->count) return fail(Q35B_ERR_ARGUMENT, "Invalid NVFP4 projection work list.");
+  if (b->chain.empty()) return fail(Q35B_ERR_SHAPE, "The NVFP4 projection work list is not a chain of launches.");
+  b->chain_absent = item;
   return Q35B_OK;
 }
 

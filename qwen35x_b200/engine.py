@@ -85,6 +85,8 @@ def lib() -> C.CDLL:
     L.q35b_debug_gemv_plan.argtypes = [i, i, C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_int)]
     L.q35b_debug_gemv_batch_wait.restype = i
     L.q35b_debug_gemv_batch_wait.argtypes = [vp, C.c_uint, C.c_uint]
+    L.q35b_debug_gemv_batch_absent.restype = i
+    L.q35b_debug_gemv_batch_absent.argtypes = [vp, i]
     L.q35b_gemv_batch_stream_bytes.restype = sz
     L.q35b_gemv_batch_stream_bytes.argtypes = [vp]
     L.q35b_act_codes_bytes.restype = sz
@@ -399,6 +401,10 @@ class GemvBatch:
     def debug_wait(self, wait_limit_polls: int, extra_completions: int) -> None:
         """Test hook (q35b_debug_gemv_batch_wait): short wait limit and extra completions demanded of dependencies."""
         _check(lib().q35b_debug_gemv_batch_wait(self._h, wait_limit_polls, extra_completions))
+
+    def debug_absent(self, item: int) -> None:
+        """Test hook (q35b_debug_gemv_batch_absent): an item of a chain whose activations are never ready in every other row block."""
+        _check(lib().q35b_debug_gemv_batch_absent(self._h, item))
 
     def close(self) -> None:
         if self._h is not None and self._h.value:

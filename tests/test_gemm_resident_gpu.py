@@ -179,6 +179,41 @@ def test_a_run_that_gives_up_leaves_a_list_that_works(engine, m, hidden, inter):
         assert batch.status() == 0 and torch.equal(y, good)
 
 
+@pytest.mark.parametrize("m,sizes", [(1, (300, 512, 700)), (2, (2560, 9216, 2560)), (4, (1024, 300 * 8, 512, 256))])
+def test_what_runs_after_an_item_that_gave_up_stores_nothing(engine, m, sizes):
+    """Every other row block of one item of a chain gives up: its other rows are stored, none of the later items' are (what they
+    read would be an earlier run's), and the next run is right with nothing reset but the hook."""
+    import torch
+
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    sizes = [-(-n // 256) * 256 for n in sizes[:-1]] + [sizes[-1]]
+    xs = [torch.randn((m, sizes[0]), device="cuda", generator=gen).to(torch.bfloat16)]
+    items = []
+    for i, (k, n) in enumerate(zip(sizes, sizes[1:])):
+        (codes, scales), _ = _weight(engine, torch, gen, n, k)
+        xs.append(torch.zeros((m, n), dtype=torch.bfloat16, device="cuda"))
+        items.append((engine.Nvfp4Weight.from_device(codes, scales, 2.0 ** -18), xs[i], xs[i + 1], None) + ((i - 1,) if i else ()))
+    batch = _run(engine, torch, items, m, len(items))
+    good = [x.clone() for x in xs[1:]]
+    for item in range(len(items)):
+        batch.debug_wait(4096, 0)
+        batch.debug_absent(item)
+        for x in xs[1:]:
+            x.fill_(7.0)
+        for _ in range(2):
+            batch.run()
+        torch.cuda.synchronize()
+        assert batch.status() == 53
+        for i, (x, want) in enumerate(zip(xs[1:], good)):
+            gave = (torch.arange(x.shape[1], device="cuda") // 128 % 2 == 0) if i == item else torch.full((x.shape[1],), i > item, device="cuda")
+            assert bool((x[:, gave] == 7.0).all()) and torch.equal(x[:, ~gave], want[:, ~gave]), (item, i)
+        batch.debug_wait(1 << 22, 0)
+        batch.debug_absent(-1)
+        batch.run()
+        torch.cuda.synchronize()
+        assert batch.status() == 0 and all(torch.equal(x, want) for x, want in zip(xs[1:], good))
+
+
 @pytest.mark.parametrize("dtype", ["bf16", "f32"])
 @pytest.mark.parametrize("m,n,k", [(1, 64, 64), (3, 129, 5184), (4, 2100, 1344), (9, 471, 2432), (14, 1500, 320), (28, 300, 256), (2, 12500, 2816)])
 def test_prefill_in_one_launch(engine, m, n, k, dtype):
