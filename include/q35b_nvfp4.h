@@ -68,8 +68,9 @@ typedef void * q35b_stream;
  * --nvfp4-projection-kernel accepts map onto these (reference:
  * src/runtime/runtime.cpp:378-390, values 0..3 are the reference's). */
 typedef enum q35b_gemv_kernel {
-  Q35B_GEMV_AUTO = -1,  /* STREAM for a weight of 24 MiB or more that it can take (unless that would allocate on a
-                         * capturing stream), else SIMT */
+  Q35B_GEMV_AUTO = -1,  /* for long K or several tokens a tensor-core kernel that makes its operand in shared memory, where that
+                         * is the fastest; else STREAM for a weight of 24 MiB or more that it can take (unless that would
+                         * allocate on a capturing stream), else SIMT */
   Q35B_GEMV_SIMT = 10,  /* contiguous loads, in-register dequant, packed fp32 FMA, warp-shuffle reduction */
   Q35B_GEMV_STREAM = 11 /* persistent, TMA-fed shared-memory ring; first use per (weight, m) allocates its work list */
 } q35b_gemv_kernel;
@@ -145,7 +146,9 @@ Q35B_API int q35b_shard_range(int n, int shard_index, int shard_count, int * row
  * src/runtime/qwen35x_cuda_backend.cpp:2320).  Replaces matvec_nvfp4_bf16 /
  * nvfp4_row_dot (src/kernels/cuda/decode_layers.cuh:200-284) and the scalar
  * projection kernels (src/runtime/cuda_bench.cu:283-429).
- * x: [m, K] bf16 device, y: [m, rows] bf16 device (rows = this shard's). */
+ * x: [m, K] bf16 device, y: [m, rows] bf16 device (rows = this shard's).
+ * SIMT and what AUTO takes below 24 MiB use every bit of an activation; STREAM converts each token to fp16 with one power of
+ * two, in which nothing is lost above 2^-39 of the token's largest activation. */
 Q35B_API int q35b_gemv_w4a16_bf16(const q35b_weight * w, const void * x_bf16, int m, void * y_bf16, int kernel,
                                   q35b_stream stream);
 
@@ -182,7 +185,7 @@ typedef struct q35b_gemv_batch q35b_gemv_batch;
  * large lists of independent items run on the tensor cores (see below) with as many octal digits as that takes: eight in
  * every K step, and six more in the steps of 256 columns where a value has bits below 2^-16 of the largest of its sixteen
  * neighbours.  So do chains of up to six tokens, lists in which every item runs after the one before it (an MLP block): one
- * launch per item, which makes the digits itself and owns no memory for them.  Infinities and NaNs reach the outputs as fp32 arithmetic has it, on either path.
+ * launch per item, which makes the digits itself, adds in fp32 what fourteen of them leave, and owns no memory for them.  Infinities and NaNs reach the outputs as fp32 arithmetic has it, on either path.
  * Device memory a list owns: descriptors and counters, some hundred KB; on the tensor cores also the operand rows, per 256
  * columns of every item 4 KB for one token, 8 KB for two, 12 KB for four and 18 KB for eight (a 4B-class step 9 and 41 MB). */
 Q35B_API int q35b_gemv_batch_create(const q35b_gemv_item * items, int count, int m, q35b_gemv_batch ** out);

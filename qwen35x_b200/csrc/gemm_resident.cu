@@ -10,7 +10,8 @@
 //           scales and scale word also go to the caller's scratch, K steps dealt out over the clusters.
 //   W4A16   octal digits (digits.cuh), eight rows per token and six of deep digits, which are multiplied only where the CTA's
 //           columns have some.  A token is counted against the largest exponent in the CTA's columns, whose power of two the
-//           sums are multiplied with before they are sent.
+//           sums are multiplied with before they are sent.  What fourteen digits leave of a value (which has to be some 2^-33 of
+//           its block's largest, or less) the epilogue adds in fp32: nothing of an activation is lost.
 //
 // The partial sums are pushed into the shared memory of the CTA that stores them (it owns some of the tile's 16-row groups),
 // so that behind the cluster barrier there are only local reads.
@@ -236,6 +237,61 @@ __device__ __forceinline__ Unit next_unit(Unit u, int steps) {
   return u;
 }
 
+// Above this exponent field of the largest value the smallest BF16 values vanish in units of it, before there are digits.
+constexpr int kTopUnderflows = 144;
+
+// What the digits of a token's columns k0 .. k1 (k0 a multiple of 256) leave, times the weights of `row` of `rows` (one per lane),
+// without the tensor's scale: 256 columns at a time a warp looks for values far enough below their block's largest one, makes
+// their digits again and takes the products of the remainders.  It is for the few values that outliers leave behind.  [4096, 2560], four
+// tokens, us: none 6.6, one value 7.1, one column in a hundred 19.3, all but an outlier per block 62; the rows kernel, which unpacks
+// all weights, 9.1.
+__device__ __noinline__ float left_dot(const uint8_t * w_codes, const uint8_t * w_scales, const __nv_bfloat16 * x_row, int rows, int k, int k0, int k1, int row,
+                                       int top, int lane) {
+  constexpr int kDigits14 = 8 + kDeepDigits;
+  const bool live = row < rows;
+  const uint8_t * codes = w_codes + static_cast<size_t>(live ? row : 0) * (k >> 1);
+  const uint4 * x = reinterpret_cast<const uint4 *>(x_row);
+  float sum = 0.0f;
+#pragma unroll 1
+  for (int base = k0 >> 3; base < k1 >> 3; base += 32) {
+    const uint4 q = base + lane < k1 >> 3 ? __ldcg(x + base + lane) : make_uint4(0u, 0u, 0u, 0u);
+    uint32_t b = bf16x8_abs_max(q);
+    b = max(b, __shfl_xor_sync(0xffffffffu, b, 1));
+    const int e = digits_exponent(b, top);
+    const uint32_t r[4] = {q.x, q.y, q.z, q.w};
+    uint32_t low = 0;  // bit i: value i has bits below the last digit's unit, or may have
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int magnitude = r[i >> 1] >> (16 * (i & 1)) & 0x7fffu;
+      if (magnitude != 0 && max(magnitude >> 7, 1) + 3 * kDigits14 - 9 < e) low |= 1u << i;
+    }
+    uint32_t lanes = __ballot_sync(0xffffffffu, low != 0u);
+    if (lanes == 0u) continue;
+    float v[8];
+    digits_begin(q, e, v);
+#pragma unroll 1
+    for (int i = 0; i < kDigits14; ++i) digits_next(v);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      // v: 8^14 times what is left, in units of 2^(e - 128).  Far below its block a value has no digits, and may have vanished
+      // in these units.
+      const float whole = __uint_as_float((i & 1) != 0 ? r[i >> 1] & 0xffff0000u : r[i >> 1] << 16);
+      const int field = static_cast<int>(__float_as_uint(whole) >> 23 & 255u);
+      v[i] = field + 60 < e ? whole : ldexpf(v[i], e - 128 - 3 * kDigits14);
+    }
+    for (; lanes != 0u; lanes &= lanes - 1) {
+      const int src = __ffs(lanes) - 1, c = base + src;  // eight columns of one block
+      const uint32_t word = *reinterpret_cast<const uint32_t *>(codes + c * 4);
+      const float scale = live ? decode_e4m3(w_scales[tiled_scale_offset(row, c >> 1, round_up_int(k >> 4, 4))]) : 0.0f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        sum = fmaf(decode_e2m1(static_cast<uint8_t>(word >> (4 * i) & 15u)) * __shfl_sync(0xffffffffu, v[i], src), scale, sum);
+      }
+    }
+  }
+  return sum;
+}
+
 // grid (row blocks, 1, split), cluster (1, 1, split).
 template <int OP>
 __global__ void __launch_bounds__(kThreads, 2)
@@ -273,7 +329,7 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
   __shared__ uint32_t gave_up, issued;             // 1: some role of this CTA gave up, 2: an earlier error is on record; K steps whose weights were asked for
   __shared__ float red[kMakers];
   __shared__ uint32_t s_amax[kMaxSplit], s_good[kMaxSplit];  // every CTA's maximum, and whether its sums count
-  __shared__ uint32_t s_top[8], s_deep;            // W4A16: largest magnitude of every token here; some value has deep digits
+  __shared__ uint32_t s_top[8], s_deep;            // W4A16: largest magnitude of every token here; 1: some value has deep digits, 256 << token: which leave something
   __shared__ float s_scale;                        // W4A4: the tensor's scale
   __shared__ float table[128];
 
@@ -430,7 +486,7 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
         }
       }
       makers_sync();
-      bool deep = false;
+      uint32_t deep = 0;
       uint4 q = first;
 #pragma unroll 1
       for (Unit u = start; u.token < a.m;) {
@@ -466,11 +522,14 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
         if (has) {
 #pragma unroll 1
           for (int i = 0; i < kDeepDigits; ++i) write(deep_row + i, digits_next(v));
-          deep = true;
+          rest = 0;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) rest |= __float_as_uint(v[i]);
+          deep |= (rest & 0x7fffffffu) != 0u ? 256u << token | 1u : 1u;
         }
         q = next;
       }
-      if (deep && lane == 0) s_deep = 1u;
+      if (deep != 0u) atomicOr(&s_deep, deep);
     } else {
       using T = std::conditional_t<OP == kNvfp4Bf16, __nv_bfloat16, float>;
       constexpr int kVecs = sizeof(T);  // 16-byte loads per block
@@ -648,16 +707,22 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
             col = taddr + a.m * 8 + token * kDeepDigits;  // the same code once more
             count = kDeepDigits;
           }
-          if (best >= 0x7f80u && ran) {
-            // a token with NaNs has nothing else to give: a NaN times anything is one
-            sum = best > 0x7f80u ? __uint_as_float(0x7fffffffu)
-                                 : infinite_dot(a.w_codes, a.w_scales, static_cast<const __nv_bfloat16 *>(a.x) + static_cast<size_t>(token) * a.k, a.n, a.k,
-                                                ks0 * 256, min((ks0 + steps) * 256, a.k), rb * kRows + tile_row, lane);
-          }
           // The token's scale is a power of two, possibly a subnormal one: it comes last, so that nothing underflows before the
           // output does.
           const float s2 = a.gate_up != 0 && (tile_row & 8) != 0 ? a.s2_up : a.s2;
-          push(token, !ran ? 0.0f : best < 0x7f80u ? sum * s2 * digits_scale(max(static_cast<int>(best >> 7), 1)) : sum * s2);
+          const int top = max(static_cast<int>(best >> 7), 1);
+          float v = sum * s2 * digits_scale(top);
+          if ((top > kTopUnderflows || (s_deep >> token & 256u) != 0u) && ran) {
+            const __nv_bfloat16 * x = static_cast<const __nv_bfloat16 *>(a.x) + static_cast<size_t>(token) * a.k;
+            const int k0 = ks0 * 256, k1 = min((ks0 + steps) * 256, a.k), row = rb * kRows + tile_row;
+            if (best < 0x7f80u) {
+              v = fmaf(left_dot(a.w_codes, a.w_scales, x, a.n, a.k, k0, k1, row, top, lane), s2, v);
+            } else {
+              // a token with NaNs has nothing else to give: a NaN times anything is one
+              v = best > 0x7f80u ? __uint_as_float(0x7fffffffu) : infinite_dot(a.w_codes, a.w_scales, x, a.n, a.k, k0, k1, row, lane) * s2;
+            }
+          }
+          push(token, ran ? v : 0.0f);
         }
       } else {
         const int c0 = group * 8;  // up to 32 columns

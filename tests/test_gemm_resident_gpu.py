@@ -134,6 +134,37 @@ def test_small_values_beside_large_ones(engine, m, depth):
     assert _rel(y, x.double() @ wd.T) <= max(4e-3, 2.0 ** (depth - 39))
 
 
+@pytest.mark.parametrize("large,small", [(0, -33), (0, -41), (3, -60), (100, -100), (127, -133), (17, -133)])
+@pytest.mark.parametrize("m,n,k", [(1, 2500, 4160), (2, 2560, 9216), (4, 9000, 2624), (5, 1300, 7232), (8, 2500, 4160)])
+def test_nothing_of_an_activation_is_lost(engine, m, n, k, large, small):
+    """Values far below what fourteen digits beside the largest of their block hold, down to the smallest there is, in rows whose
+    weights are zero at the large ones: the outputs are the sums of the small ones alone.  Also some small values in one token
+    only, and one block of nothing else."""
+    import torch
+
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    (codes, scales), wd = _weight(engine, torch, gen, n, k)
+    codes[:, ::8] &= 0xf0  # the first element of every block
+    wd[:, ::16] = 0.0
+    s2 = 2.0 ** min(-small, 30)
+    w = engine.Nvfp4Weight.from_device(codes, scales, s2)
+    for kind in range(3):
+        x = torch.randn((m, k), device="cuda", generator=gen, dtype=torch.float64) * 2.0 ** small
+        if kind == 1:
+            x[: m - 1] *= 2.0 ** (min(large, 30) - small - 4)  # one token only
+        if kind == 2:
+            x[:, torch.rand(k, device="cuda", generator=gen) < 0.99] = 0.0
+        x[:, ::16] = 2.0 ** large
+        x[:, 32:48] = 2.0 ** small
+        x = x.to(torch.bfloat16)
+        want = x.double() @ (wd * 2.0 ** 12 * s2).T
+        assert _rel(engine.gemv_w4a16(w, x), want) <= 1e-3, kind
+        if k % 256 == 0 and m <= 6:
+            y = torch.zeros((m, n), dtype=torch.bfloat16, device="cuda")
+            _run(engine, torch, [(w, x, y)], m, 1)
+            assert _rel(y, want) <= 1e-3, kind
+
+
 @pytest.mark.parametrize("m", [1, 4])
 def test_infinities_and_nans(engine, m):
     import torch
