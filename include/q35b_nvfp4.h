@@ -148,9 +148,15 @@ Q35B_API int q35b_shard_range(int n, int shard_index, int shard_count, int * row
  * projection kernels (src/runtime/cuda_bench.cu:283-429).
  * x: [m, K] bf16 device, y: [m, rows] bf16 device (rows = this shard's).
  * SIMT and what AUTO takes below 24 MiB use every bit of an activation; STREAM converts each token to fp16 with one power of
- * two, in which nothing is lost above 2^-39 of the token's largest activation. */
+ * two, in which nothing is lost above 2^-39 of the token's largest activation.
+ * The tensor-core kernel's waits are bounded: where one expires, rows of y stay as they were and a code (51 to 56) stays until
+ * q35b_gemm_default_status reads it.  It keeps no other call from running. */
 Q35B_API int q35b_gemv_w4a16_bf16(const q35b_weight * w, const void * x_bf16, int m, void * y_bf16, int kernel,
                                   q35b_stream stream);
+/* Test hook: the tensor-core kernel of Q35B_GEMV_AUTO for any projection that fits it (Q35B_ERR_SHAPE: it does not), its waits
+ * giving up after `wait_limit_polls` polls instead of 2^20. */
+Q35B_API int q35b_debug_gemv_resident(const q35b_weight * w, const void * x_bf16, int m, void * y_bf16, unsigned int wait_limit_polls,
+                                      q35b_stream stream);
 
 /* The reference benchmark's contract (src/runtime/cuda_bench.cu:2042-2188):
  * fp32 input of one token, activations multiplied by input_scale, fp32 output. */
@@ -302,7 +308,8 @@ Q35B_API int q35b_gemm_w4a4_bf16(const q35b_weight * w, const uint8_t * a_codes,
 Q35B_API int q35b_debug_gemm_plan(int m, int rows, int n_total, int k, int sms, int gather, int rows_aligned, int * pairs,
                                   int * tile_cols, int * split, int * accumulators);
 
-/* Copies the library's status word of the current device to the host (synchronises the device) and clears it. */
+/* Copies the library's status word of the current device to the host (synchronises the device) and clears it.  Without a code
+ * in it, the one that a single decode projection left (a word of its own, which stops no GEMM). */
 Q35B_API int q35b_gemm_default_status(unsigned int * status_out);
 
 /* Same GEMM with the residual add fused into the epilogue: c = bf16(projection + residual), residual [m, rows] BF16

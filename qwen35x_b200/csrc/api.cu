@@ -132,6 +132,13 @@ static bool resident_projection(const q35b_weight * w, int m) {
   return ns > 0.0 && ns + 700.0 < other;
 }
 
+static int run_resident(const q35b_weight * w, const void * x_bf16, int m, void * y_bf16, unsigned int wait_limit, cudaStream_t s) {
+  if (const int st = check_weight_device(w)) return st;
+  unsigned int * status = nullptr;
+  if (const int st = default_status_word(&status, kDecodeStatus)) return st;
+  return launch_decode_resident(w, x_bf16, m, y_bf16, nullptr, nullptr, status, wait_limit, s);
+}
+
 extern "C" {
 
 const char * q35b_last_error(void) { return t_error.c_str(); }
@@ -314,10 +321,7 @@ int q35b_gemv_w4a16_bf16(const q35b_weight * w, const void * x_bf16, int m, void
                          q35b_stream stream) {
   if (kernel == Q35B_GEMV_AUTO && w != nullptr && x_bf16 != nullptr && y_bf16 != nullptr && m >= 1 && m <= 8 && w->rows > 0 && !w->gate_up &&
       (reinterpret_cast<uintptr_t>(x_bf16) & 15u) == 0 && resident_projection(w, m)) {
-    if (const int st = check_weight_device(w)) return st;
-    unsigned int * status = nullptr;
-    if (const int st = default_status_word(&status)) return st;
-    return launch_decode_resident(w, x_bf16, m, y_bf16, nullptr, nullptr, status, 1u << 20, static_cast<cudaStream_t>(stream));
+    return run_resident(w, x_bf16, m, y_bf16, 1u << 20, static_cast<cudaStream_t>(stream));
   }
   if (kernel == Q35B_GEMV_AUTO && w != nullptr && m >= 1 && m <= 8 && !w->gate_up &&
       w->codes_bytes + w->scales_bytes >= kAutoStreamBytes && x_bf16 != nullptr &&
@@ -357,6 +361,12 @@ int q35b_gemv_w4a16_bf16(const q35b_weight * w, const void * x_bf16, int m, void
     return gemv_batch_launch(batch, x_bf16, y_bf16, static_cast<cudaStream_t>(stream));
   }
   return launch_gemv_bf16(w, x_bf16, m, y_bf16, kernel, static_cast<cudaStream_t>(stream));
+}
+
+int q35b_debug_gemv_resident(const q35b_weight * w, const void * x_bf16, int m, void * y_bf16, unsigned int wait_limit_polls, q35b_stream stream) {
+  if (w == nullptr || x_bf16 == nullptr || y_bf16 == nullptr || wait_limit_polls == 0) return fail(Q35B_ERR_ARGUMENT, "NVFP4 projection received a null buffer.");
+  if ((reinterpret_cast<uintptr_t>(x_bf16) & 15u) != 0 || w->gate_up) return fail(Q35B_ERR_ARGUMENT, "NVFP4 projection does not fit the resident kernel.");
+  return run_resident(w, x_bf16, m, y_bf16, wait_limit_polls, static_cast<cudaStream_t>(stream));
 }
 
 size_t q35b_gemv_item_bytes(void) { return sizeof(q35b_gemv_item); }

@@ -152,7 +152,8 @@ int build_weight_maps(q35b_weight * w);
 // The library's own status word of the current device (a file-scope device variable): what the GEMM entry points
 // use when the caller passes no status word.  Resolved once per device; q35b_weight_create* calls it so that the
 // first projection does not have to.
-int default_status_word(unsigned int ** out);
+enum DefaultStatus : int { kGemmStatus = 0, kDecodeStatus = 1 };
+int default_status_word(unsigned int ** out, DefaultStatus which = kGemmStatus);
 int launch_gemm_w4a4(const q35b_weight * w, const uint8_t * a_codes, const uint8_t * a_scales_tiled, const float * g_dev,
                      int m, void * c_bf16, int ldc, const void * residual_bf16, int ldr, unsigned int * status_dev,
                      cudaStream_t s, const GemmQuantOut * qout = nullptr, const GemmGather * gather = nullptr);

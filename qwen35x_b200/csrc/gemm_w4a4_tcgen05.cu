@@ -705,9 +705,10 @@ int launch_gemm_ksplit(const q35b_weight * w, const uint8_t * a_codes, const uin
   return Q35B_OK;
 }
 
-// What the GEMM entry points use as *status when the caller passes none: one word per device inside the library
-// (no allocation anywhere on that path).
-__device__ unsigned int g_default_status;
+// What the entry points use as *status when the caller passes none: two words per device inside the library (no allocation
+// anywhere on that path), the prefill GEMMs', which a GEMM that finds a code in it stores nothing after, and that of single decode
+// projections, which keeps nothing else from running.
+__device__ unsigned int g_default_status[2];
 
 }  // namespace
 
@@ -725,7 +726,7 @@ int gemm_plan_debug(int m, int rows, int n_total, int k, int sms, bool gather, b
   return Q35B_OK;
 }
 
-int default_status_word(unsigned int ** out) {
+int default_status_word(unsigned int ** out, DefaultStatus which) {
   static std::mutex mutex;
   static unsigned int * word[64] = {nullptr};
   int dev = 0;
@@ -738,7 +739,7 @@ int default_status_word(unsigned int ** out) {
     Q35B_CUDA_TRY(cudaGetSymbolAddress(&p, g_default_status), "cudaGetSymbolAddress(default status word)");
     word[dev] = static_cast<unsigned int *>(p);
   }
-  *out = word[dev];
+  *out = word[dev] + which;
   return Q35B_OK;
 }
 
@@ -749,8 +750,10 @@ extern "C" int q35b_gemm_default_status(unsigned int * status_out) {
   if (status_out == nullptr) return fail(Q35B_ERR_ARGUMENT, "Null status pointer.");
   unsigned int * word = nullptr;
   if (const int st = default_status_word(&word)) return st;
-  Q35B_CUDA_TRY(cudaMemcpy(status_out, word, sizeof(unsigned int), cudaMemcpyDeviceToHost), "cudaMemcpy(default status word)");
-  if (*status_out != 0u) Q35B_CUDA_TRY(cudaMemset(word, 0, sizeof(unsigned int)), "cudaMemset(default status word)");
+  unsigned int codes[2];
+  Q35B_CUDA_TRY(cudaMemcpy(codes, word, sizeof codes, cudaMemcpyDeviceToHost), "cudaMemcpy(default status words)");
+  *status_out = codes[0] != 0u ? codes[0] : codes[1];
+  if (*status_out != 0u) Q35B_CUDA_TRY(cudaMemset(word, 0, sizeof codes), "cudaMemset(default status words)");
   return Q35B_OK;
 }
 

@@ -85,6 +85,8 @@ def lib() -> C.CDLL:
     L.q35b_debug_gemv_plan.argtypes = [i, i, C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_int)]
     L.q35b_debug_gemv_batch_wait.restype = i
     L.q35b_debug_gemv_batch_wait.argtypes = [vp, C.c_uint, C.c_uint]
+    L.q35b_debug_gemv_resident.restype = i
+    L.q35b_debug_gemv_resident.argtypes = [vp, vp, i, vp, C.c_uint, vp]
     L.q35b_debug_gemv_batch_absent.restype = i
     L.q35b_debug_gemv_batch_absent.argtypes = [vp, i]
     L.q35b_gemv_batch_stream_bytes.restype = sz
@@ -483,7 +485,7 @@ def gemm_plan(m: int, rows: int, k: int, n_total: int | None = None, sms: int = 
 
 
 def gemm_default_status() -> int:
-    """The library's own GEMM status word of the current device (used when a call passes no status word)."""
+    """The library's own status word of the current device: of GEMM calls that pass none, else of single decode projections."""
     out = C.c_uint(0)
     _check(lib().q35b_gemm_default_status(C.byref(out)))
     return int(out.value)

@@ -245,6 +245,33 @@ def test_what_runs_after_an_item_that_gave_up_stores_nothing(engine, m, sizes):
         assert batch.status() == 0 and all(torch.equal(x, want) for x, want in zip(xs[1:], good))
 
 
+def _resident(engine, torch, w, x, y, limit=1 << 20):
+    stream = torch.cuda.current_stream().cuda_stream
+    assert engine.lib().q35b_debug_gemv_resident(w.handle, x.data_ptr(), x.shape[0], y.data_ptr(), limit, stream) == 0
+
+
+def test_a_single_projection_that_gave_up_is_reported_and_stops_no_other_call(engine):
+    import torch
+
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    m, n, k = 2, 700, 4160
+    (codes, scales), wd = _weight(engine, torch, gen, n, k)
+    w = engine.Nvfp4Weight.from_device(codes, scales, 2.0 ** -12)
+    x = torch.randn((m, k), device="cuda", generator=gen).to(torch.bfloat16)
+    many = torch.randn((16, k), device="cuda", generator=gen).to(torch.bfloat16)
+    good, prefill = engine.gemv_w4a16(w, x), [engine.project_prefill(w, v).clone() for v in (x, many)]
+    y = torch.full((m, n), 7.0, dtype=torch.bfloat16, device="cuda")
+    assert engine.gemm_default_status() == 0
+    _resident(engine, torch, w, x, y, 1)
+    torch.cuda.synchronize()
+    assert bool((y == 7.0).all())
+    # the code is not read yet
+    assert all(torch.equal(engine.project_prefill(w, v), p) for v, p in zip((x, many), prefill))
+    _resident(engine, torch, w, x, y)
+    assert _rel(y, x.double() @ wd.T) <= 2e-4 and _rel(y, good.double()) <= 2e-4
+    assert 51 <= engine.gemm_default_status() <= 56 and engine.gemm_default_status() == 0
+
+
 @pytest.mark.parametrize("dtype", ["bf16", "f32"])
 @pytest.mark.parametrize("m,n,k", [(1, 64, 64), (3, 129, 5184), (4, 2100, 1344), (9, 471, 2432), (14, 1500, 320), (28, 300, 256), (2, 12500, 2816)])
 def test_prefill_in_one_launch(engine, m, n, k, dtype):
