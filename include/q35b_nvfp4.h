@@ -190,7 +190,7 @@ typedef struct q35b_gemv_batch q35b_gemv_batch;
  * of its token's largest one.  Most lists with dependent items, and small ones, convert every token to fp16 with one power of two;
  * large lists of independent items run on the tensor cores (see below) with as many octal digits as that takes: eight in
  * every K step, and six more in the steps of 256 columns where a value has bits below 2^-16 of the largest of its sixteen
- * neighbours.  So do chains of up to six tokens, lists in which every item runs after the one before it (an MLP block): one
+ * neighbours.  So do chains of up to six tokens where they are the faster ones, lists in which every item runs after the one before it (an MLP block): one
  * launch per item, which makes the digits itself, adds in fp32 what fourteen of them leave, and owns no memory for them.  Infinities and NaNs reach the outputs as fp32 arithmetic has it, on either path.
  * Device memory a list owns: descriptors and counters, some hundred KB; on the tensor cores also the operand rows, per 256
  * columns of every item 4 KB for one token, 8 KB for two, 12 KB for four and 18 KB for eight (a 4B-class step 9 and 41 MB). */
@@ -231,6 +231,8 @@ Q35B_API int q35b_debug_gemv_batch_wait(q35b_gemv_batch * batch, unsigned int wa
  * included, gives up after the limit set above because its activations are never ready, so that these rows stay as they were, its
  * code (53) lands in the status word and no later item of the run stores anything.  -1: none. */
 Q35B_API int q35b_debug_gemv_batch_absent(q35b_gemv_batch * batch, int item);
+/* Test hook: a list that can runs as a chain from now on, also where one launch is the faster one.  Q35B_ERR_SHAPE: it cannot. */
+Q35B_API int q35b_debug_gemv_batch_chain(q35b_gemv_batch * batch);
 /* The shared-memory plan a work list of `m` tokens over weights of at most `max_k` columns would get (host
  * arithmetic only, no device needed): ctas_per_sm is 2 for the shape with eight consumer warps and half an SM's
  * shared memory, 1 for the shape with sixteen consumer warps and all of it; ring_stages are 18 KB each;

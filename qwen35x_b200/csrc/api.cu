@@ -399,6 +399,8 @@ int q35b_debug_gemv_batch_wait(q35b_gemv_batch * batch, unsigned int wait_limit_
 
 int q35b_debug_gemv_batch_absent(q35b_gemv_batch * batch, int item) { return gemv_batch_debug_absent(batch, item); }
 
+int q35b_debug_gemv_batch_chain(q35b_gemv_batch * batch) { return gemv_batch_debug_chain(batch); }
+
 size_t q35b_gemv_batch_stream_bytes(const q35b_gemv_batch * batch) { return gemv_batch_bytes(batch); }
 
 int q35b_gemv_w4a16_f32(const q35b_weight * w, const float * x_f32, float input_scale, float * y_f32, int kernel,

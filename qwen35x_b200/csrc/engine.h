@@ -124,6 +124,7 @@ size_t gemv_batch_bytes(const struct q35b_gemv_batch * b);
 int gemv_plan_debug(int m, int max_k, int * ctas_per_sm, int * ring_stages, int * activation_buffers, int * smem_bytes);
 int gemv_batch_debug_wait(struct q35b_gemv_batch * b, unsigned int wait_limit, unsigned int extra_completions);
 int gemv_batch_debug_absent(struct q35b_gemv_batch * b, int item);
+int gemv_batch_debug_chain(struct q35b_gemv_batch * b);
 
 // gemm_w4a4_tcgen05.cu
 int gemm_plan_debug(int m, int rows, int n_total, int k, int sms, bool gather, bool rows_aligned, int * pairs, int * tile_cols,
@@ -174,7 +175,8 @@ size_t wbatch_bytes(const WBatch * b);
 int wbatch_debug_wait(WBatch * b, unsigned int wait_limit);
 
 // gemm_resident.cu: few tokens, the operand made in shared memory
-bool decode_resident_chain(const q35b_weight * w, int m);  // fits as one launch of several
+// Estimate for one launch of several (0: it does not fit), and whether the GPU holds all of its clusters at once.
+double decode_resident_chain_ns(const q35b_weight * w, int m, bool * at_once);
 // What a launch of a chain has to know of its neighbours.
 struct ResidentChain {
   const q35b_weight * next;      // the weight that the launch after it streams (brought into L2 under it), or NULL

@@ -914,11 +914,49 @@ double decode_shape(const q35b_weight * w, int m, bool chain, Shape * out) {
   return best;
 }
 
+// Clusters of a shape's split that the GPU holds at once, at half an SM or all of it per CTA: 148 SMs hold 296 CTAs of half an SM, but
+// 56 clusters of five, 45 of six, 37 of seven and 33 of eight; of all of it 148, 74, 45, 33, 26, 22, 15 and 15.  Asked of a kernel of the
+// same size that is never launched: the runtime counts on one CTA per SM of any kernel with tcgen05.alloc, which is so only until
+// it gives up its right to allocate (clusters of two, 296 CTAs of 30 us each with 256 columns: 36 us).
+__global__ void __launch_bounds__(kThreads, 2) resident_size_kernel(float * p) {
+  extern __shared__ float words[];
+  p[threadIdx.x] = words[threadIdx.x];
+}
+int clusters_at_once(const Shape & shape) {
+  static std::atomic<int> known[64][2][kMaxSplit + 1];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  const bool full = shape.smem > kSmemHalf;
+  std::atomic<int> & held = known[dev][full ? 1 : 0][shape.split];
+  int n = held.load(std::memory_order_relaxed);
+  if (n != 0) return n;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(1, 1, static_cast<unsigned>(shape.split));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = static_cast<size_t>(full ? kSmemFull : kSmemHalf);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = static_cast<unsigned>(shape.split);
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cudaFuncSetAttribute(resident_size_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemFull) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, resident_size_kernel, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  held.store(n, std::memory_order_relaxed);
+  return n;
+}
+
 }  // namespace
 
-bool decode_resident_chain(const q35b_weight * w, int m) {
+double decode_resident_chain_ns(const q35b_weight * w, int m, bool * at_once) {
   Shape shape;
-  return decode_shape(w, m, true, &shape) > 0.0;
+  const double ns = decode_shape(w, m, true, &shape);
+  if (ns > 0.0) *at_once = (w->rows + kRows - 1) / kRows <= clusters_at_once(shape);
+  return ns;
 }
 
 double decode_resident_ns(const q35b_weight * w, int m) {

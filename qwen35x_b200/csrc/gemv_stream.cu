@@ -872,7 +872,8 @@ struct q35b_gemv_batch {
   uint32_t wait_limit = kWaitLimit;   // polls every device-side wait of a run may take
   unsigned int wait_extra = 0;        // test hook: completions that every other CTA demands on top of what a dependency delivers
   q35b::WBatch * tensor = nullptr;   // set: the list runs on the tensor path (gemm_wstream.cu), nothing above is used
-  std::vector<q35b_gemv_item> chain;  // set: it runs as one launch per item, in this order (gemm_resident.cu)
+  std::vector<q35b_gemv_item> chain;  // set: it can run as one launch per item, in this order (gemm_resident.cu)
+  bool chained = false;               // it does
   unsigned int * chain_gave = nullptr;  // of a chain, two words per item: whether its launch gave up (gemm_resident.cu)
   int chain_absent = -1;              // test hook: item whose operand is never complete in every other row block
 };
@@ -1066,18 +1067,47 @@ bool tensor_list(const q35b_gemv_item * items, int count, int m) {
 }
 
 // Whether a list runs as one launch per item in which the operand is made in shared memory (gemm_resident.cu): a chain, so
-// that the launches follow one another as the items would.
-// Up to six tokens: every row block makes the operand anew, and from seven on that costs more than the dependent items'
-// conversions in one launch do.  us, one launch / one per item, MLP blocks [2560, 9216], [1024, 3584], [512, 1280], one token 25.3 /
-// 15.9, 14.9 / 9.9, 9.8 / 8.9; two 26.2 / 17.1, 15.5 / 10.5, 10.4 / 9.5; four 26.8 / 22.5, 15.7 / 11.9, 10.7 / 9.9; six 28.5 / 28.7, 16.5 /
-// 14.0, 11.3 / 11.6; eight 28.9 / 29.2, 16.8 / 17.6, 11.5 / 11.7.
-constexpr int kResidentTokens = 6;
-bool resident_chain(const q35b_gemv_item * items, const std::vector<int> & level, int m) {
+// that the launches follow one another as the items would.  us, one launch / one per item, MLP blocks [hidden, inter], weights from HBM.
+//   Up to four tokens, unless all items are shorter than four K steps: the meeting inside one launch costs more than two launches do.
+//     [2560, 9216] one token 25.8 / 16.7, four 27.3 / 22.9; [1024, 3584] 15.3 / 10.3, 16.0 / 12.1; [512, 1024] 9.9 / 9.5, 10.5 / 10.2; [1024, 768] 10.2 /
+//     9.9, 11.1 / 10.5; not [512, 768] 9.2 / 9.7, 10.1 / 10.0, [256, 512] -, 8.9 / 9.9
+//   Five and six: every row block makes the operand anew, so only short shares of it, and not beside short items alone.  [1024, 3584] 16.7 /
+//     13.7, 16.9 / 14.5; [4096, 2048] 21.2 / 15.3, 21.6 / 16.0; not [768, 512] 10.5 / 11.5, 10.4 / 11.7, [512, 6400] 15.3 / 16.5, -, [2048, 6144] 22.5 / 20.0,
+//     22.6 / 26.4.  From seven on the one launch is ahead: [2560, 9216] 28.9 / 29.2, [512, 1280] 11.5 / 11.7.
+// A list of one item has nothing to wait for; what the one launch costs it is that CTAs share a tile of more than eight K steps
+// and meet, or walk 1792 columns and more one after the other.  us, weights from HBM, [rows, K]:
+//   one and two tokens: [300, 4096] 6.9 / 4.6, 7.1 / 4.6; [2560, 9216] 9.9 / 6.9, 10.1 / 7.4; [18432, 2560] 12.3 / 8.7, 12.4 / 9.3; not [9328, 8448] 15.9 / 17.9, -,
+//     whose clusters do not fit the GPU at once
+//   three and four: [2560, 4096] 8.2 / 6.1, 8.2 / 6.3; [2168, 5888] 8.9 / 6.7, -; not [3488, 6400] -, 9.6 / 10.6, [9432, 2816] -, 8.8 / 12.6
+//   five and six: [1024, 3584] 7.6 / 6.6, 7.7 / 6.2; [2560, 2560] 7.3 / 7.3, 7.3 / 7.1; not [2224, 5120] 8.6 / 8.9, 8.6 / 9.2
+//   up to eight K steps: [2048, 2048] one token 6.1 / 5.1, four 6.5 / 5.7; [4096, 2048] 6.0 / 5.0, 6.5 / 6.2; not [9000, 1792] two 6.1 / 6.4, [6144, 2048] four 6.6 /
+//     7.2; never below 1792 columns: [3584, 1024] 4.3 / 4.8, 4.6 / 5.5, [7200, 1536] 5.3 / 5.5, 5.6 / 6.3
+constexpr int kResidentTokens = 6, kResidentFewTokens = 4;
+constexpr int kChainColumns = 1024, kChainColumnsMany = 2048;
+constexpr double kChainMany = 2000.0;  // estimate (ns) up to which an item of a chain may make its operand for five and six tokens
+constexpr int kSingleColumns = 1792, kSingleOutputs = 8192;
+constexpr double kSingleFew = 1700.0, kSingleMany = 1300.0;
+
+// can: it could, whatever is faster.
+bool resident_chain(const q35b_gemv_item * items, const std::vector<int> & level, int m, bool * can) {
+  *can = false;
   if (m > kResidentTokens) return false;
+  int longest = 0;
+  double most = 0.0;
+  bool at_once = true;
   for (size_t i = 0; i < level.size(); ++i) {
-    if (level[i] != static_cast<int>(i) || items[i].x_bf16 == nullptr || items[i].y_bf16 == nullptr || !decode_resident_chain(items[i].weight, m)) return false;
+    const q35b_weight * w = items[i].weight;
+    bool held = false;
+    const double ns = level[i] == static_cast<int>(i) && items[i].x_bf16 != nullptr && items[i].y_bf16 != nullptr ? decode_resident_chain_ns(w, m, &held) : 0.0;
+    if (ns == 0.0) return false;
+    longest = std::max(longest, w->k);
+    most = std::max(most, ns);
+    at_once = at_once && held;
   }
-  return true;
+  *can = true;
+  if (level.size() > 1) return m <= kResidentFewTokens ? longest >= kChainColumns : longest >= kChainColumnsMany && most <= kChainMany;
+  if (longest <= kWholeSteps * 256) return longest >= kSingleColumns && static_cast<long>(items[0].weight->rows) * m <= kSingleOutputs;
+  return m <= 2 ? at_once : most <= (m <= kResidentFewTokens ? kSingleFew : kSingleMany);
 }
 
 }  // namespace
@@ -1258,7 +1288,9 @@ int gemv_batch_build(const q35b_gemv_item * items, int count, int m, bool share_
     delete b;
     return fail_cuda(e, "uploading the projection work list");
   }
-  if (callers_list && resident_chain(items, level, m)) b->chain.assign(items, items + count);
+  bool can = false;
+  b->chained = callers_list && resident_chain(items, level, m, &can);
+  if (can) b->chain.assign(items, items + count);
   *out = b;
   return Q35B_OK;
 }
@@ -1280,7 +1312,7 @@ int gemv_batch_build_tensor(const q35b_gemv_item * items, int count, int m, int 
 int gemv_batch_launch(const q35b_gemv_batch * b, const void * x_override, void * y_override, cudaStream_t s) {
   if (b == nullptr) return fail(Q35B_ERR_ARGUMENT, "Null NVFP4 projection work list.");
   if (b->tensor != nullptr) return wbatch_launch(b->tensor, s);
-  if (!b->chain.empty() && b->wait_extra == 0) {
+  if (b->chained && b->wait_extra == 0) {
     for (size_t i = 0; i < b->chain.size(); ++i) {
       const q35b_gemv_item & it = b->chain[i];
       const ResidentChain neighbours = {i + 1 < b->chain.size() ? b->chain[i + 1].weight : nullptr, b->chain_gave + 2 * i,
@@ -1343,8 +1375,14 @@ int gemv_batch_debug_wait(q35b_gemv_batch * b, unsigned int wait_limit, unsigned
 
 int gemv_batch_debug_absent(q35b_gemv_batch * b, int item) {
   if (b == nullptr || item < -1 || item >= b->count) return fail(Q35B_ERR_ARGUMENT, "Invalid NVFP4 projection work list.");
-  if (b->chain.empty()) return fail(Q35B_ERR_SHAPE, "The NVFP4 projection work list is not a chain of launches.");
+  if (!b->chained) return fail(Q35B_ERR_SHAPE, "The NVFP4 projection work list is not a chain of launches.");
   b->chain_absent = item;
+  return Q35B_OK;
+}
+
+int gemv_batch_debug_chain(q35b_gemv_batch * b) {
+  if (b == nullptr || b->chain.empty()) return fail(Q35B_ERR_SHAPE, "The NVFP4 projection work list does not fit a chain of launches.");
+  b->chained = true;
   return Q35B_OK;
 }
 

@@ -87,6 +87,8 @@ def lib() -> C.CDLL:
     L.q35b_debug_gemv_batch_wait.argtypes = [vp, C.c_uint, C.c_uint]
     L.q35b_debug_gemv_resident.restype = i
     L.q35b_debug_gemv_resident.argtypes = [vp, vp, i, vp, C.c_uint, vp]
+    L.q35b_debug_gemv_batch_chain.restype = i
+    L.q35b_debug_gemv_batch_chain.argtypes = [vp]
     L.q35b_debug_gemv_batch_absent.restype = i
     L.q35b_debug_gemv_batch_absent.argtypes = [vp, i]
     L.q35b_gemv_batch_stream_bytes.restype = sz
@@ -407,6 +409,10 @@ class GemvBatch:
     def debug_absent(self, item: int) -> None:
         """Test hook (q35b_debug_gemv_batch_absent): an item of a chain whose activations are never ready in every other row block."""
         _check(lib().q35b_debug_gemv_batch_absent(self._h, item))
+
+    def debug_chain(self) -> None:
+        """Test hook (q35b_debug_gemv_batch_chain): one launch per item, also where one for all is faster."""
+        _check(lib().q35b_debug_gemv_batch_chain(self._h))
 
     def close(self) -> None:
         if self._h is not None and self._h.value:

@@ -32,6 +32,7 @@ def _limit(count):
 
 def _run(engine, torch, items, m, launches):
     batch = engine.GemvBatch(items, m)
+    engine.lib().q35b_debug_gemv_batch_chain(batch._h)  # sizes at which one launch of the other kernel is the faster one, too
     before = engine.launch_count()
     batch.run()
     assert engine.launch_count() - before == launches
@@ -270,6 +271,46 @@ def test_a_single_projection_that_gave_up_is_reported_and_stops_no_other_call(en
     _resident(engine, torch, w, x, y)
     assert _rel(y, x.double() @ wd.T) <= 2e-4 and _rel(y, good.double()) <= 2e-4
     assert 51 <= engine.gemm_default_status() <= 56 and engine.gemm_default_status() == 0
+
+
+@pytest.mark.parametrize("m,sizes,launches", [(2, (2560, 9216, 2560), 2), (4, (1024, 3584, 1024), 2), (6, (1024, 3584, 1024), 2), (4, (512, 1024, 512), 2),
+                                             (4, (512, 768, 512), 1), (5, (1024, 1024, 1024), 1), (6, (2048, 12288, 2048), 1), (7, (1024, 3584, 1024), 1)])
+def test_where_a_chain_is_one_launch_per_item(engine, m, sizes, launches):
+    """Both sides of each line of the rule, with the same results."""
+    import torch
+
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    xs, items = [torch.randn((m, sizes[0]), device="cuda", generator=gen).to(torch.bfloat16)], []
+    want = xs[0]
+    for i, (k, n) in enumerate(zip(sizes, sizes[1:])):
+        (codes, scales), wd = _weight(engine, torch, gen, n, k)
+        xs.append(torch.zeros((m, n), dtype=torch.bfloat16, device="cuda"))
+        items.append((engine.Nvfp4Weight.from_device(codes, scales, 2.0 ** -18), xs[i], xs[i + 1], None) + ((i - 1,) if i else ()))
+        want = (want.double() @ wd.T * 2.0 ** -6).to(torch.bfloat16)
+    batch = engine.GemvBatch(items, m)
+    before = engine.launch_count()
+    batch.run()
+    assert engine.launch_count() - before == launches
+    torch.cuda.synchronize()
+    # an input of the second item that was rounded the other way, a few in 10^4, moves its outputs by 2^-9 of its share
+    assert batch.status() == 0 and _rel(xs[-1], want.double()) <= 1e-3
+
+
+@pytest.mark.parametrize("m,n,k,chain", [(1, 300, 4096, True), (2, 2560, 9216, True), (1, 9328, 8448, False), (4, 2560, 4096, True), (4, 9432, 2816, False), (6, 1024, 3584, True),
+                                         (6, 9432, 2816, False), (4, 2048, 2048, True), (4, 2049, 2048, False), (1, 3584, 1024, False), (1, 1024, 1536, False)])
+def test_which_kernel_a_list_of_one_item_takes(engine, m, n, k, chain):
+    """Both sides of each line of the rule: only a chain takes the hook of one."""
+    import torch
+
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    (codes, scales), wd = _weight(engine, torch, gen, n, k)
+    x = torch.randn((m, k), device="cuda", generator=gen).to(torch.bfloat16)
+    y = torch.zeros((m, n), dtype=torch.bfloat16, device="cuda")
+    batch = engine.GemvBatch([(engine.Nvfp4Weight.from_device(codes, scales, 2.0 ** -12), x, y)], m)
+    batch.run()
+    torch.cuda.synchronize()
+    assert batch.status() == 0 and _rel(y, x.double() @ wd.T) <= _limit(m * n)
+    assert (engine.lib().q35b_debug_gemv_batch_absent(batch._h, -1) == 0) == chain
 
 
 @pytest.mark.parametrize("dtype", ["bf16", "f32"])
