@@ -1070,7 +1070,8 @@ bool tensor_list(const q35b_gemv_item * items, int count, int m) {
 // that the launches follow one another as the items would.  us, one launch / one per item, MLP blocks [hidden, inter], weights from HBM.
 //   Up to four tokens, unless all items are shorter than four K steps: the meeting inside one launch costs more than two launches do.
 //     [2560, 9216] one token 25.8 / 16.7, four 27.3 / 22.9; [1024, 3584] 15.3 / 10.3, 16.0 / 12.1; [512, 1024] 9.9 / 9.5, 10.5 / 10.2; [1024, 768] 10.2 /
-//     9.9, 11.1 / 10.5; not [512, 768] 9.2 / 9.7, 10.1 / 10.0, [256, 512] -, 8.9 / 9.9
+//     9.9, 11.1 / 10.5; not [512, 768] 9.2 / 9.7, 10.1 / 10.0, [256, 512] -, 8.9 / 9.9; and with three and four not what does not fit the GPU at once:
+//     [5120, 5120] twice one 21.9 / 14.3, four 22.6 / 26.5; [5136, 8704] and [1024, 5120] two 23.4 / 19.6, four 25.1 / 24.9
 //   Five and six: every row block makes the operand anew, so only short shares of it, and not beside short items alone.  [1024, 3584] 16.7 /
 //     13.7, 16.9 / 14.5; [4096, 2048] 21.2 / 15.3, 21.6 / 16.0; not [768, 512] 10.5 / 11.5, 10.4 / 11.7, [512, 6400] 15.3 / 16.5, -, [2048, 6144] 22.5 / 20.0,
 //     22.6 / 26.4.  From seven on the one launch is ahead: [2560, 9216] 28.9 / 29.2, [512, 1280] 11.5 / 11.7.
@@ -1105,7 +1106,10 @@ bool resident_chain(const q35b_gemv_item * items, const std::vector<int> & level
     at_once = at_once && held;
   }
   *can = true;
-  if (level.size() > 1) return m <= kResidentFewTokens ? longest >= kChainColumns : longest >= kChainColumnsMany && most <= kChainMany;
+  if (level.size() > 1) {
+    if (m <= kResidentFewTokens) return longest >= kChainColumns && (at_once || m <= 2);
+    return longest >= kChainColumnsMany && most <= kChainMany;
+  }
   if (longest <= kWholeSteps * 256) return longest >= kSingleColumns && static_cast<long>(items[0].weight->rows) * m <= kSingleOutputs;
   return m <= 2 ? at_once : most <= (m <= kResidentFewTokens ? kSingleFew : kSingleMany);
 }

@@ -274,7 +274,7 @@ def test_a_single_projection_that_gave_up_is_reported_and_stops_no_other_call(en
 
 
 @pytest.mark.parametrize("m,sizes,launches", [(2, (2560, 9216, 2560), 2), (4, (1024, 3584, 1024), 2), (6, (1024, 3584, 1024), 2), (4, (512, 1024, 512), 2),
-                                             (4, (512, 768, 512), 1), (5, (1024, 1024, 1024), 1), (6, (2048, 12288, 2048), 1), (7, (1024, 3584, 1024), 1)])
+                                             (4, (512, 768, 512), 1), (2, (5120, 5120, 5120), 2), (4, (5120, 5120, 5120), 1), (5, (1024, 1024, 1024), 1), (6, (2048, 12288, 2048), 1), (7, (1024, 3584, 1024), 1)])
 def test_where_a_chain_is_one_launch_per_item(engine, m, sizes, launches):
     """Both sides of each line of the rule, with the same results."""
     import torch
