@@ -153,6 +153,8 @@ Q35B_API int q35b_shard_range(int n, int shard_index, int shard_count, int * row
  * q35b_gemm_default_status reads it.  It keeps no other call from running. */
 Q35B_API int q35b_gemv_w4a16_bf16(const q35b_weight * w, const void * x_bf16, int m, void * y_bf16, int kernel,
                                   q35b_stream stream);
+/* Whether Q35B_GEMV_AUTO takes its tensor-core kernel for m tokens of 16-byte aligned activations. */
+Q35B_API int q35b_debug_gemv_auto(const q35b_weight * w, int m, int * resident);
 /* Test hook: the tensor-core kernel of Q35B_GEMV_AUTO for any projection that fits it (Q35B_ERR_SHAPE: it does not), its waits
  * giving up after `wait_limit_polls` polls instead of 2^20. */
 Q35B_API int q35b_debug_gemv_resident(const q35b_weight * w, const void * x_bf16, int m, void * y_bf16, unsigned int wait_limit_polls,

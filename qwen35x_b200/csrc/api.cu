@@ -113,23 +113,32 @@ using namespace q35b;
 // short K or several tokens the streaming kernel would be ahead from 4 to 12 MiB on.
 static constexpr size_t kAutoStreamBytes = 24u << 20;
 
-// Q35B_GEMV_AUTO sends one to the resident tensor-core kernel (gemm_resident.cu) where the estimates, fitted to graph replays,
-// are more than 0.7 us apart: long K or several tokens, for which the rows kernel's warps unpack one piece after the other.
+// Q35B_GEMV_AUTO sends one to the resident tensor-core kernel (gemm_resident.cu) where the estimates say so with room to spare, as much as
+// they were found wrong by, which is more with more tokens.  That is for long K or several tokens, for which the rows kernel's warps
+// unpack one piece after the other.
 // us, rows or streaming kernel / resident kernel, one, two and four tokens: [2560, 9216] 17.1 / 6.6, 18.3 / 7.5, 26.9 / 10.2;
-// [2560, 2560] 5.6 / 4.9, 5.8 / 5.2, 8.6 / 6.3; [32768, 1024] 8.2 / 6.1, 11.3 / 7.0, 16.7 / 9.6; [16000, 4096] 14.7 / 9.7, 15.1 / 12.8, -;
-// left where they were [3584, 1024] 2.6 / 4.6, 2.8 / 5.0, 4.3 / 5.4 and [300, 4096] 2.0 / 4.5, 2.3 / 4.5, 2.9 / 5.0.
+// [2560, 2560] 5.6 / 4.9, 5.8 / 5.2, 8.6 / 6.3; [32768, 1024] 8.2 / 6.1, 11.3 / 7.0, 16.7 / 9.6; [16000, 4096] 14.7 / 9.7, 15.1 / 12.8, -; eight
+// [2464, 5376] 19.7 / 10.7, [2040, 8256] 39.3 / 20.1;
+// left where they were [3584, 1024] 2.6 / 4.6, 2.8 / 5.0, 4.3 / 5.4; [27760, 2816] one 12.9 / 14.0; [7048, 1280] five 6.3 / 7.2;
+// [3952, 1536] seven 6.4 / 6.8; [4720, 4096] eight 15.5 / 19.0.
+// Of 2550 drawn calls (100 to 40000 rows, 512 to 10240 columns, one to eight tokens) some 650 come here, from 0.95 to 2.6 times as fast; of some 30
+// left out that would gain more than 3 %, most do less than 1.15.
 static bool resident_projection(const q35b_weight * w, int m) {
   double other;
-  if (w->codes_bytes + w->scales_bytes >= kAutoStreamBytes && gemv_stream_eligible(w, m)) {
-    // whole tiles, one or two to an SM at a time, and so much per K step
+  const bool streams = w->codes_bytes + w->scales_bytes >= kAutoStreamBytes && gemv_stream_eligible(w, m);
+  if (streams) {
+    // whole tiles, one or two to an SM at a time, and so much per K step: [9440, 5632] 74 tiles 13.2 us, [12792, 6144] 100 tiles 17.6, [19888, 4096] 156
+    // tiles 16.0
     const int tiles = (w->rows + 127) / 128, sms = sm_count();
-    other = 2000.0 + w->k / 256 * (tiles <= sms ? 780.0 : 960.0) * ((tiles + 2 * sms - 1) / (2 * sms));
+    const double per_step = tiles <= 90 ? 500.0 + 20 * m : tiles <= sms ? 640.0 + 20 * m : 960.0;
+    other = 2000.0 + w->k / 256 * per_step * ((tiles + 2 * sms - 1) / (2 * sms));
   } else {
     other = gemv_rows_ns(w, m);
   }
   if (other < 5500.0) return false;
-  const double ns = decode_resident_ns(w, m);
-  return ns > 0.0 && ns + 700.0 < other;
+  static constexpr double room[9] = {0.0, 1.0, 1.0, 1.15, 1.18, 1.25, 1.18, 1.25, 1.25}, least[9] = {0.0, 700.0, 700.0, 700.0, 700.0, 1600.0, 1000.0, 1600.0, 1600.0};
+  const double ns = decode_resident_ns(w, m, streams);
+  return ns > 0.0 && std::max(ns * room[m], ns + least[m]) < other;
 }
 
 static int run_resident(const q35b_weight * w, const void * x_bf16, int m, void * y_bf16, unsigned int wait_limit, cudaStream_t s) {
@@ -367,6 +376,12 @@ int q35b_debug_gemv_resident(const q35b_weight * w, const void * x_bf16, int m, 
   if (w == nullptr || x_bf16 == nullptr || y_bf16 == nullptr || wait_limit_polls == 0) return fail(Q35B_ERR_ARGUMENT, "NVFP4 projection received a null buffer.");
   if ((reinterpret_cast<uintptr_t>(x_bf16) & 15u) != 0 || w->gate_up) return fail(Q35B_ERR_ARGUMENT, "NVFP4 projection does not fit the resident kernel.");
   return run_resident(w, x_bf16, m, y_bf16, wait_limit_polls, static_cast<cudaStream_t>(stream));
+}
+
+int q35b_debug_gemv_auto(const q35b_weight * w, int m, int * resident) {
+  if (w == nullptr || resident == nullptr || m < 1 || m > 8) return fail(Q35B_ERR_ARGUMENT, "Invalid arguments for the kernel of an NVFP4 projection.");
+  *resident = w->rows > 0 && !w->gate_up && resident_projection(w, m) ? 1 : 0;
+  return Q35B_OK;
 }
 
 size_t q35b_gemv_item_bytes(void) { return sizeof(q35b_gemv_item); }

@@ -93,7 +93,7 @@ namespace q35b {
 // gemv_w4a16.cu
 int launch_dequant_bf16(const q35b_weight * w, void * w_bf16, cudaStream_t s);
 int launch_gemv_bf16(const q35b_weight * w, const void * x_bf16, int m, void * y_bf16, int kernel, cudaStream_t s);
-double gemv_rows_ns(const q35b_weight * w, int m);  // estimate for the kernel of any shape
+double gemv_rows_ns(const q35b_weight * w, int m);  // estimate for the kernel of any shape; 0: not worth comparing
 int launch_gemv_f32(const q35b_weight * w, const float * x, float input_scale, float * y, int kernel, cudaStream_t s);
 
 // act_quant.cu
@@ -183,7 +183,7 @@ struct ResidentChain {
   unsigned int * gave, * before;  // two words of this launch, and those of the launch before it, or NULL
   bool absent;                   // test hook: see q35b_debug_gemv_batch_absent
 };
-double decode_resident_ns(const q35b_weight * w, int m);  // estimate for one projection; 0: it does not fit
+double decode_resident_ns(const q35b_weight * w, int m, bool large);  // estimate for one projection; 0: it does not fit, or is too long a way
 // chain: NULL for a projection by itself
 int launch_decode_resident(const q35b_weight * w, const void * x_bf16, int m, void * y_bf16, const void * residual_bf16, const ResidentChain * chain,
                            unsigned int * status, unsigned int wait_limit, cudaStream_t s);

@@ -959,10 +959,28 @@ double decode_resident_chain_ns(const q35b_weight * w, int m, bool * at_once) {
   return ns;
 }
 
-double decode_resident_ns(const q35b_weight * w, int m) {
+// Where not all clusters fit the GPU at once the rest, waiting for whole clusters' room, takes as long again, with all of an SM's shared
+// memory per CTA several times as long: [6072, 4352] two tokens (48 clusters of six, 45 fit) 11.6 us, [4720, 4096] eight (37 of four, 33
+// fit) 19.0, [4648, 9280] eight 35.1, where the plain estimate says 7.0, 7.1 and 11.6.  large: a weight that the streaming kernel would take; whole
+// tiles then go in rounds, with all of an SM's shared memory per CTA nothing of the next call overlaps ([9088, 5632] four tokens 14.0, estimate 10.6;
+// [11648, 4096] 18.8, 13.7), and more than twenty K steps per CTA are too long a way ([15992, 6400] two tokens 25.8, estimate 17.6, streaming 20.0; where only
+// the rows kernel could have it, [14840, 5184] two 15.9 against 26.0).
+double decode_resident_ns(const q35b_weight * w, int m, bool large) {
   Shape shape;
-  const double ns = decode_shape(w, m, false, &shape);
-  return ns > 0.0 ? 4500.0 + ns : 0.0;
+  double ns = decode_shape(w, m, false, &shape);
+  if (ns == 0.0) return 0.0;
+  const int row_blocks = (w->rows + kRows - 1) / kRows, steps = ((w->k + 255) / 256 + shape.split - 1) / shape.split, sms = sm_count();
+  const bool full = shape.smem > kSmemHalf;
+  if (large && steps > 20 && m > 1) return 0.0;
+  if (large && shape.split == 1 && row_blocks > sms) {
+    ns = (steps * 230 + (m * steps + kMakers - 1) / kMakers * 450) * ((row_blocks + sms - 1) / sms) + std::max(0, steps - shape.stages) * 250;
+  }
+  if (row_blocks > clusters_at_once(shape)) {
+    ns *= full ? 4.5 : 2.5;
+  } else if (full && large) {
+    ns *= m <= 3 ? 1.2 : 1.5;
+  }
+  return 4500.0 + ns;
 }
 
 int launch_decode_resident(const q35b_weight * w, const void * x_bf16, int m, void * y_bf16, const void * residual_bf16,

@@ -362,13 +362,25 @@ int launch_gemv_bf16(const q35b_weight * w, const void * x_bf16, int m, void * y
                     kernel, s);
 }
 
-// The rows kernel, from a fit to graph replays: so much per 256 columns and turn of the warps that the SMs hold.
+// The rows kernel, from fits to graph replays: so much per 256 columns for every turn of the warps that the SMs hold, and from five tokens
+// on no less than so much for every block that an SM has to run (either is at most a quarter off for nine calls in ten; [6072, 4352] eight
+// tokens, whose blocks go round twice, 28.0 us, 17.3 by the first, 26.0 by the second; with few tokens the second is too much for blocks that just
+// overflow: [6208, 2560] two 6.1, 6.6 and 7.1).  Where four warps
+// share a row, which is rarely slower than what it is compared with, 0: [112, 8192] seven tokens 5.3 us, [1064, 6912] four 5.4, [888, 5056] six
+// 6.3, where the resident kernel takes 8.2, 8.4 and 7.5; except with many tokens, rows and columns: [408, 10112] five to eight 10.0 to 11.4 / 7.8 to 10.0,
+// [744, 9600] 10.1 to 11.9 / 7.9 to 9.8, [488, 8448] five to seven 8.7 / 8.1, 8.9 / 9.4, 9.8 / 9.3.
 double gemv_rows_ns(const q35b_weight * w, int m) {
-  static constexpr int per_piece[9] = {0, 480, 480, 620, 720, 950, 1100, 1000, 840};
+  static constexpr int per_turn[9] = {0, 480, 480, 620, 720, 950, 1100, 1000, 840};
+  static constexpr int per_block[9] = {0, 0, 0, 0, 0, 340, 445, 461, 471}, fixed[9] = {0, 0, 0, 0, 0, 1990, 1750, 1710, 2020};
   const int sms = sm_count(), pieces = (w->k + kPiece - 1) / kPiece;
-  const bool four = w->rows < kWarpsPerBlock * sms && w->k > pieces_ahead(m) * kPiece;  // as launch_simt deals them out
-  const double warps = four ? 4.0 * w->rows : (w->rows < 2 * kWarpsPerBlock * sms ? w->rows : 0.5 * w->rows);
-  return 1000.0 + per_piece[m] * std::max(1.0, pieces / (four ? 4.0 : 1.0)) * std::max(1.0, warps / (sms * (m == 1 ? 32.0 : 18.0)));
+  if (w->rows < kWarpsPerBlock * sms && w->k > pieces_ahead(m) * kPiece) {  // as launch_simt deals them out
+    if (m < 5 || w->rows < 400 || w->k < 8400) return 0.0;
+    return 1000.0 + per_turn[m] * (pieces / 4.0) * std::max(1.0, 4.0 * w->rows / (sms * 18.0));
+  }
+  const int warps = w->rows < 2 * kWarpsPerBlock * sms ? w->rows : (w->rows + 1) / 2;
+  const int blocks = ((warps + kWarpsPerBlock - 1) / kWarpsPerBlock + sms - 1) / sms;
+  return std::max(1000.0 + per_turn[m] * pieces * std::max(1.0, warps / (sms * (m == 1 ? 32.0 : 18.0))),
+                  fixed[m] + static_cast<double>(per_block[m]) * pieces * blocks);  // 0 up to four tokens
 }
 
 int launch_gemv_f32(const q35b_weight * w, const float * x, float input_scale, float * y, int kernel, cudaStream_t s) {

@@ -85,6 +85,8 @@ def lib() -> C.CDLL:
     L.q35b_debug_gemv_plan.argtypes = [i, i, C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_int)]
     L.q35b_debug_gemv_batch_wait.restype = i
     L.q35b_debug_gemv_batch_wait.argtypes = [vp, C.c_uint, C.c_uint]
+    L.q35b_debug_gemv_auto.restype = i
+    L.q35b_debug_gemv_auto.argtypes = [vp, i, C.POINTER(C.c_int)]
     L.q35b_debug_gemv_resident.restype = i
     L.q35b_debug_gemv_resident.argtypes = [vp, vp, i, vp, C.c_uint, vp]
     L.q35b_debug_gemv_batch_chain.restype = i

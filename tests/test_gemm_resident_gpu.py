@@ -251,6 +251,59 @@ def _resident(engine, torch, w, x, y, limit=1 << 20):
     assert engine.lib().q35b_debug_gemv_resident(w.handle, x.data_ptr(), x.shape[0], y.data_ptr(), limit, stream) == 0
 
 
+@pytest.mark.parametrize("m,n,k,resident", [(1, 2500, 4160, True), (4, 1300, 7232, True), (8, 9000, 2624, True), (2, 2560, 9216, True), (8, 2560, 9216, True), (1, 3584, 1024, False),
+                                            (8, 300, 8192, False), (4, 1183, 6912, False), (4, 1300, 6912, True), (8, 4720, 4096, False), (2, 6072, 4352, False),
+                                            (2, 15992, 6400, False), (1, 27760, 2816, False), (1, 16000, 4096, True), (5, 7048, 1280, False), (7, 7048, 1280, True)])
+def test_which_kernel_a_single_projection_takes(engine, m, n, k, resident):
+    """Both sides of each line of the rule, and the same sums."""
+    import ctypes
+
+    import torch
+
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    (codes, scales), wd = _weight(engine, torch, gen, n, k)
+    w = engine.Nvfp4Weight.from_device(codes, scales, 2.0 ** -12)
+    taken = ctypes.c_int(-1)
+    assert engine.lib().q35b_debug_gemv_auto(w.handle, m, ctypes.byref(taken)) == 0 and taken.value == resident
+    x = torch.randn((m, k), device="cuda", generator=gen).to(torch.bfloat16)
+    assert _rel(engine.gemv_w4a16(w, x), x.double() @ wd.T) <= 2e-4
+
+
+@pytest.mark.parametrize("m", [1, 7, 8])
+@pytest.mark.parametrize("n,k", [(130, 192), (300, 4160), (1300, 7232), (257, 2624)])
+def test_single_projections_over_the_range_of_activations(engine, m, n, k):
+    """The resident kernel whatever AUTO says, at its most operand rows and with K ending inside a K step: tokens of wide range and of
+    zeros; infinities and NaNs, among them in the last columns, as fp32 arithmetic has them; residues that differ from CTA to CTA."""
+    import torch
+
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    (codes, scales), wd = _weight(engine, torch, gen, n, k)
+    codes[: n // 2, k // 2 - 1] &= 0x0f  # zero weights in the last column
+    wd[: n // 2, k - 1] = 0.0
+    w = engine.Nvfp4Weight.from_device(codes, scales, 2.0 ** -12)
+    y = torch.zeros((m, n), dtype=torch.bfloat16, device="cuda")
+    for kind in range(3):
+        x = torch.randn((m, k), device="cuda", generator=gen)
+        if kind == 1:
+            x *= torch.exp2(torch.randint(-60, 60, (m, k), device="cuda", generator=gen).float())
+        if kind == 2:
+            x[:, k // 2:] *= 2.0 ** -90
+            x[0] *= 0.0 if m > 1 else 1.0
+        x = x.to(torch.bfloat16)
+        _resident(engine, torch, w, x, y)
+        assert _rel(y, x.double() @ wd.T) <= _limit(m * n), kind
+    for places in ([(k - 1, float("inf"))], [(k - 70 if k > 70 else 3, float("-inf")), (k - 1, float("inf"))], [(k - 1, float("nan"))], [(5, float("inf")), (k - 3, 2.0 ** 100)]):
+        x = torch.randn((m, k), device="cuda", generator=gen).to(torch.bfloat16)
+        for at, v in places:
+            x[m - 1, at] = v
+        _resident(engine, torch, w, x, y)
+        want = engine.gemv_w4a16(w, x, kernel=engine.GEMV_SIMT)
+        assert torch.equal(y.isnan(), want.isnan()) and torch.equal(y[want.isinf()], want[want.isinf()])
+        finite = want.isfinite()
+        assert not bool(finite.any()) or _rel(y[finite], want[finite].double()) <= 4e-3
+    assert engine.gemm_default_status() == 0
+
+
 def test_a_single_projection_that_gave_up_is_reported_and_stops_no_other_call(engine):
     import torch
 
