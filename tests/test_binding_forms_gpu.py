@@ -89,3 +89,39 @@ def test_kernel_numbers_and_scales_of_other_types_stay_refused(engine, weight, b
             engine.quantize_activations(x, bad, scratch)
     else:
         assert torch.equal(engine.gemv_w4a16_f32(weight, x[0].float(), bad), engine.gemv_w4a16_f32(weight, x[0].float(), float(bad)))
+
+
+def _events(torch, call):
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]) as prof:
+        call()
+    return {e.key for e in prof.key_averages()}
+
+
+def _nodes(torch, call, tmp_path):
+    """Kernels of a captured call."""
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    graph.enable_debug_mode()
+    with torch.cuda.graph(graph):
+        call()
+    path = tmp_path / f"{len(list(tmp_path.iterdir()))}.dot"
+    graph.debug_dump(str(path))
+    return path.read_text()
+
+
+def test_new_outputs_are_seen_by_a_profiler_and_filled_where_that_is_asked_for(engine, weight, tmp_path):
+    """Outputs are made without the dispatcher, but not where someone would miss it."""
+    import torch
+
+    x = to_torch_bf16(make_activations(2, 512, seed=4))
+    calls = [lambda: engine.gemv_w4a16(weight, x), lambda: engine.gemv_w4a16_f32(weight, x[0].float()), lambda: engine.project_prefill(weight, x)]
+    for call in calls:
+        call()
+        assert "aten::empty" in _events(torch, call)
+    plain = _nodes(torch, calls[0], tmp_path)
+    assert torch.utils.deterministic.fill_uninitialized_memory
+    torch.use_deterministic_algorithms(True)
+    try:
+        filled = _nodes(torch, calls[0], tmp_path)
+    finally:
+        torch.use_deterministic_algorithms(False)
+    assert "FillFunctor" not in plain and "FillFunctor" in filled
