@@ -20,19 +20,6 @@ namespace q35b {
 
 constexpr int kDeepDigits = 6;
 
-// Eight fp32 values -> one word of eight E2M1 codes, nearest; element 2j in the low nibble of byte j.
-__device__ __forceinline__ uint32_t to_e2m1x8(const float (&q)[8]) {
-  uint32_t w;
-  asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\t"
-      "cvt.rn.satfinite.e2m1x2.f32 b0, %2, %1;\n\t"
-      "cvt.rn.satfinite.e2m1x2.f32 b1, %4, %3;\n\t"
-      "cvt.rn.satfinite.e2m1x2.f32 b2, %6, %5;\n\t"
-      "cvt.rn.satfinite.e2m1x2.f32 b3, %8, %7;\n\t"
-      "mov.b32 %0, {b0, b1, b2, b3};\n\t}"
-      : "=r"(w)
-      : "f"(q[0]), "f"(q[1]), "f"(q[2]), "f"(q[3]), "f"(q[4]), "f"(q[5]), "f"(q[6]), "f"(q[7]));
-  return w;
-}
 // The two E2M1 codes of a byte (low nibble first) -> fp32.
 __device__ __forceinline__ void from_e2m1x2(uint32_t byte, float & lo, float & hi) {
   asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\t.reg .b32 h;\n\t.reg .b16 l, u;\n\t"

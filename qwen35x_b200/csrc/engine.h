@@ -188,8 +188,8 @@ double decode_resident_ns(const q35b_weight * w, int m, bool large);  // estimat
 int launch_decode_resident(const q35b_weight * w, const void * x_bf16, int m, void * y_bf16, const void * residual_bf16, const ResidentChain * chain,
                            unsigned int * status, unsigned int wait_limit, cudaStream_t s);
 bool prefill_resident_shape(const q35b_weight * w, int m, float scale, int split, int * stages, int * smem);
-int launch_prefill_resident(const q35b_weight * w, const void * x, bool f32, int m, float scale, uint8_t * codes, uint8_t * scales, float * g_dev, int split, int stages,
-                            int smem, const void * residual, int ldr, void * c, int ldc, unsigned int * status, cudaStream_t s);
+int launch_prefill_resident(const q35b_weight * w, const void * x, bool f32, int m, uint8_t * codes, uint8_t * scales, float * g_dev, int split, int stages, int smem,
+                            const void * residual, int ldr, void * c, int ldc, unsigned int * status, cudaStream_t s);
 
 // gemm_w4a4_2cta.cu
 bool gemm_2cta_eligible(int rows, int m, int k);

@@ -51,7 +51,6 @@ constexpr int kMakerThreads = kMakers * 32;
 constexpr int kThreads = 64 + kMakerThreads;
 constexpr int kGroupRows = 16;           // rows of a tile that one CTA of the cluster stores together (8 gate / 8 up)
 constexpr int kGroups = kRows / kGroupRows;
-constexpr int kMaxTokens = 32;           // W4A4
 constexpr int kAccCols = 192;            // accumulators, up to four partial ones side by side ...
 constexpr int kSfSetCols = 32;           // ... and two sets of scale-factor columns, used by stages in turn
 constexpr int kTmemCols = 256;
@@ -89,8 +88,7 @@ struct ResidentArgs {
   // CTA, written in every run, cost half a microsecond of 10 to 18).
   unsigned int * gave, * before;
   int absent;                      // test hook: 1: in every other row block, the first included, the operand is never complete
-  // W4A4: given per-tensor scale (or 0: from the tensor), and the caller's scratch
-  float scale;
+  // W4A4: the caller's scratch
   uint8_t * codes, * scales;
   float * g_out;
   unsigned int * status;
@@ -533,86 +531,60 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     } else {
       using T = std::conditional_t<OP == kNvfp4Bf16, __nv_bfloat16, float>;
       constexpr int kVecs = sizeof(T);  // 16-byte loads per block
-      const int per_row = a.k >> 4, first = ks0 * 16, last = min(first + steps * 16, per_row);  // this CTA's blocks of every token
-      const int width = last - first, total = a.m * width;
-      const uint4 * x = static_cast<const uint4 *>(a.x);
-      const float per_width = __fdividef(1.0f, static_cast<float>(width));
-      auto token_of = [&](int i) { return static_cast<int>((static_cast<float>(i) + 0.5f) * per_width); };  // i / width, up to 18432 / 576
-      uint64_t mine = 0;  // this CTA's K steps that its cluster writes to the scratch
+      // one block of sixteen per thread at most: block b of this CTA's columns of a token
+      const int per_row = a.k >> 4, first = ks0 * 16, width = min(first + steps * 16, per_row) - first;
+      const int token = static_cast<int>((static_cast<float>(mt) + 0.5f) * __fdividef(1.0f, static_cast<float>(width)));  // mt / width, up to 448 / 448
+      const int b = mt - token * width;
+      const bool has = token < a.m;
+      uint32_t mine = 0;  // this CTA's K steps (28 at most) that its cluster writes to the scratch
       {
         int it = rb - ks0;
         while (it < 0) it += gridDim.x;
-        for (; it < steps; it += gridDim.x) mine |= 1ull << it;
+        for (; it < steps; it += gridDim.x) mine |= 1u << it;
       }
-      auto load = [&](int i, uint4 (&r)[kVecs]) {
-        const int token = token_of(i), b = first + i - token * width;
-        const uint4 * src = x + (static_cast<size_t>(token) * per_row + b) * kVecs;
-#pragma unroll
-        for (int v = 0; v < kVecs; ++v) r[v] = __ldca(src + v);
-      };
-      const bool dynamic = !(a.scale > 0.0f);
-      float g = a.scale;
-      // the multipliers of quantize_block_bf16, per scale byte
-      auto fill_table = [&] {
-        if (OP == kNvfp4Bf16) {
-          if (mt < 127) table[mt] = bf16_block_multiplier(mt, g);
-          makers_sync();
-        }
-      };
-      if (!dynamic) fill_table();
       asm volatile("griddepcontrol.wait;" ::: "memory");  // the activations may come from the kernel before, which may also read the scratch
       if (split > 1) cluster_wait();
-      uint4 held[kVecs] = {};
-      if (mt < total) load(mt, held);
-      if (dynamic) {
-        float best = 0.0f;
+      uint4 r[kVecs] = {};
+      if (has) {
+        const uint4 * src = static_cast<const uint4 *>(a.x) + (static_cast<size_t>(token) * per_row + first + b) * kVecs;
 #pragma unroll
-        for (int v = 0; v < kVecs; ++v) best = abs_max<T>(held[v], best);
-#pragma unroll 2
-        for (int i = mt + kMakerThreads; i < total; i += kMakerThreads) {
-          uint4 r[kVecs];
-          load(i, r);
+        for (int v = 0; v < kVecs; ++v) r[v] = __ldca(src + v);
+      }
+      float best = 0.0f;
 #pragma unroll
-          for (int v = 0; v < kVecs; ++v) best = abs_max<T>(r[v], best);
+      for (int v = 0; v < kVecs; ++v) best = abs_max<T>(r[v], best);
+      // magnitudes: their bit patterns are ordered as they are
+      const uint32_t warp_best = __reduce_max_sync(0xffffffffu, __float_as_uint(best));
+      if (lane == 0) red[mw] = __uint_as_float(warp_best);
+      makers_sync();
+      float amax = red[0];
+#pragma unroll
+      for (int i = 1; i < kMakers; ++i) amax = fmaxf(amax, red[i]);
+      if (split > 1) {
+        if (mt < split) st_async(map_to_rank(smem_u32(&s_amax[rank]), mt), __float_as_uint(amax), map_to_rank(smem_u32(amax_bar), mt));
+        if (!mbar_wait(smem_u32(amax_bar), 0, a.wait_limit)) {
+          if (lane == 0) give_up(kAmaxWait);
+        } else {
+          for (int i = 0; i < split; ++i) amax = fmaxf(amax, __uint_as_float(*reinterpret_cast<volatile uint32_t *>(&s_amax[i])));
         }
-        // magnitudes: their bit patterns are ordered as they are
-        const uint32_t warp_best = __reduce_max_sync(0xffffffffu, __float_as_uint(best));
-        if (lane == 0) red[mw] = __uint_as_float(warp_best);
+      }
+      const float g = amax > 0.0f ? __fdiv_rn(amax, 6.0f * 448.0f) : 1.0f;
+      if (OP == kNvfp4Bf16) {
+        if (mt < 127) table[mt] = bf16_block_multiplier(mt, g);  // the multipliers of quantize_block_bf16, per scale byte
         makers_sync();
-        float amax = red[0];
-#pragma unroll
-        for (int i = 1; i < kMakers; ++i) amax = fmaxf(amax, red[i]);
-        if (split > 1) {
-          if (mt < split) st_async(map_to_rank(smem_u32(&s_amax[rank]), mt), __float_as_uint(amax), map_to_rank(smem_u32(amax_bar), mt));
-          if (!mbar_wait(smem_u32(amax_bar), 0, a.wait_limit)) {
-            if (lane == 0) give_up(kAmaxWait);
-          } else {
-            for (int i = 0; i < split; ++i) amax = fmaxf(amax, __uint_as_float(*reinterpret_cast<volatile uint32_t *>(&s_amax[i])));
-          }
-        }
-        g = amax > 0.0f ? __fdiv_rn(amax, 6.0f * 448.0f) : 1.0f;
-        fill_table();
       }
       if (mt == 0) s_scale = g;
       const float rg = __frcp_rn(g);
       if (a.g_out != nullptr && rb == 0 && rank == 0 && mt == 0) *a.g_out = g;
-#pragma unroll 1
-      for (int i = mt; i < total; i += kMakerThreads) {
-        uint4 r[kVecs];
-        if (i == mt) {
-#pragma unroll
-          for (int v = 0; v < kVecs; ++v) r[v] = held[v];
-        } else {
-          load(i, r);
-        }
+      if (has) {
         uint2 packed;
         const uint32_t sb = quantize_raw<T, OP == kNvfp4Bf16>(r, g, rg, table, packed);
-        const int token = token_of(i), b = i - token * width, it = b >> 4, in = b & 15;
+        const int it = b >> 4, in = b & 15;
         *reinterpret_cast<uint2 *>(smem_op + it * op_bytes + token * kStepBytes + (((in >> 1) ^ (token & 7)) << 4) + (in & 1) * 8) = packed;
         smem_sfo[it * kSfBytes + scale_word(token, in >> 2) + (in & 3)] = static_cast<uint8_t>(sb);
         if ((mine >> it & 1u) != 0u) {
           *reinterpret_cast<uint2 *>(a.codes + (static_cast<size_t>(token) * per_row + first + b) * 8) = packed;
-          a.scales[static_cast<size_t>(ks0 + it) * kSfBytes + (in >> 2) * kSfChunk + token * 16 + (in & 3)] = static_cast<uint8_t>(sb);  // up to 32 tokens
+          a.scales[static_cast<size_t>(ks0 + it) * kSfBytes + (in >> 2) * kSfChunk + token * 16 + (in & 3)] = static_cast<uint8_t>(sb);  // fewer than 32 tokens
         }
       }
       // the scratch's scale bytes of rows m .. 127 are zero
@@ -1026,7 +998,7 @@ int launch_decode_resident(const q35b_weight * w, const void * x_bf16, int m, vo
 // [22014, 3008] 12.5 / 13.3.
 bool prefill_resident_shape(const q35b_weight * w, int m, float scale, int split, int * stages, int * smem) {
   const int k_steps = (w->k + 255) / 256, steps = (k_steps + split - 1) / split;
-  if (scale > 0.0f || m > kMaxTokens || m * steps * 16 > kMakerThreads) return false;
+  if (scale > 0.0f || m * steps * 16 > kMakerThreads) return false;  // so fewer than 32 tokens
   Shape shape;
   if (!shape_for((w->rows + kRows - 1) / kRows, w->k, m, round_up_int(m, 16), split, sm_count(), steps, &shape)) return false;
   *stages = shape.stages;
@@ -1034,8 +1006,8 @@ bool prefill_resident_shape(const q35b_weight * w, int m, float scale, int split
   return true;
 }
 
-int launch_prefill_resident(const q35b_weight * w, const void * x, bool f32, int m, float scale, uint8_t * codes, uint8_t * scales, float * g_dev, int split, int stages,
-                            int smem, const void * residual, int ldr, void * c, int ldc, unsigned int * status, cudaStream_t s) {
+int launch_prefill_resident(const q35b_weight * w, const void * x, bool f32, int m, uint8_t * codes, uint8_t * scales, float * g_dev, int split, int stages, int smem,
+                            const void * residual, int ldr, void * c, int ldc, unsigned int * status, cudaStream_t s) {
   ResidentArgs a = {};
   a.x = x;
   a.y = static_cast<__nv_bfloat16 *>(c);
@@ -1044,7 +1016,6 @@ int launch_prefill_resident(const q35b_weight * w, const void * x, bool f32, int
   a.ldr = ldr;
   a.m = m;
   a.cols_plain = a.cols_deep = round_up_int(m, 16);
-  a.scale = scale > 0.0f ? scale : 0.0f;
   a.codes = codes;
   a.scales = scales;
   a.g_out = g_dev;

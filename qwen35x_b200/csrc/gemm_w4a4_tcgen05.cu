@@ -855,7 +855,7 @@ int launch_project_prefill(const q35b_weight * w, const void * x, bool f32, int 
       if (status_dev == nullptr) {
         if (const int st = default_status_word(&status_dev)) return st;
       }
-      return launch_prefill_resident(w, x, f32, m, global_scale, codes, scales_tiled, g_dev, plan.split, stages, smem, residual_bf16, ldr, c_bf16, ldc, status_dev, s);
+      return launch_prefill_resident(w, x, f32, m, codes, scales_tiled, g_dev, plan.split, stages, smem, residual_bf16, ldr, c_bf16, ldc, status_dev, s);
     }
   }
   const int k = w != nullptr ? w->k : 0;

@@ -740,7 +740,7 @@ int ensure_attr() {
 // ---- decode work list on the tensor path ------------------------------------------------------------------------
 
 struct WBatch {
-  int count = 0, m = 0, digits = 0, expand_count = 0, grid = 0, stages = 0, b_slot = 0, deep_bytes = 0, smem = 0;
+  int m = 0, digits = 0, expand_count = 0, grid = 0, stages = 0, b_slot = 0, deep_bytes = 0, smem = 0;
   void * dev_base = nullptr;
   WItem * items = nullptr;
   WTile * tiles = nullptr;
@@ -828,7 +828,6 @@ int wbatch_build(const q35b_gemv_item * items, int count, int m, int digits, boo
   }
   if (const int st = ensure_attr()) return st;
   auto * b = new WBatch();
-  b->count = count;
   b->m = m;
   b->digits = digits;
   b->exact = exact;

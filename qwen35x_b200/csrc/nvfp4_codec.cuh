@@ -158,4 +158,21 @@ Q35B_HD int64_t tiled_scale_offset(int row, int col, int padded_cols) {
 
 Q35B_HD int round_up_int(int v, int m) { return ((v + m - 1) / m) * m; }
 
+#if defined(__CUDACC__)
+// Eight fp32 values -> one word of eight E2M1 codes with the hardware converter (nearest on the E2M1 grid, saturating
+// at 6, sign kept): byte j holds element 2j in its low nibble and 2j + 1 in its high nibble.
+__device__ __forceinline__ uint32_t to_e2m1x8(const float (&q)[8]) {
+  uint32_t w;
+  asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\t"
+      "cvt.rn.satfinite.e2m1x2.f32 b0, %2, %1;\n\t"
+      "cvt.rn.satfinite.e2m1x2.f32 b1, %4, %3;\n\t"
+      "cvt.rn.satfinite.e2m1x2.f32 b2, %6, %5;\n\t"
+      "cvt.rn.satfinite.e2m1x2.f32 b3, %8, %7;\n\t"
+      "mov.b32 %0, {b0, b1, b2, b3};\n\t}"
+      : "=r"(w)
+      : "f"(q[0]), "f"(q[1]), "f"(q[2]), "f"(q[3]), "f"(q[4]), "f"(q[5]), "f"(q[6]), "f"(q[7]));
+  return w;
+}
+#endif
+
 }  // namespace q35b

@@ -41,21 +41,6 @@ __device__ __forceinline__ uint32_t e2m1_code_bounded(float q) {
   return ((a >= 1.0f) ? high : low) | ((q < 0.0f) ? 8u : 0u);
 }
 
-// Eight quotients -> one word of eight E2M1 codes with the hardware converter (nearest on the E2M1 grid, saturating
-// at 6, sign kept): byte j holds element 2j in its low nibble and 2j + 1 in its high nibble.
-__device__ __forceinline__ uint32_t cvt_e2m1x8(const float (&q)[8]) {
-  uint32_t w;
-  asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\t"
-      "cvt.rn.satfinite.e2m1x2.f32 b0, %2, %1;\n\t"
-      "cvt.rn.satfinite.e2m1x2.f32 b1, %4, %3;\n\t"
-      "cvt.rn.satfinite.e2m1x2.f32 b2, %6, %5;\n\t"
-      "cvt.rn.satfinite.e2m1x2.f32 b3, %8, %7;\n\t"
-      "mov.b32 %0, {b0, b1, b2, b3};\n\t}"
-      : "=r"(w)
-      : "f"(q[0]), "f"(q[1]), "f"(q[2]), "f"(q[3]), "f"(q[4]), "f"(q[5]), "f"(q[6]), "f"(q[7]));
-  return w;
-}
-
 // Quantise one 16-block; returns the scale byte, writes 8 code bytes.
 template <int RECIPE>
 __device__ __forceinline__ uint32_t quantize_block(const float (&v)[16], float g, bool swap, uint2 & out) {
@@ -106,7 +91,7 @@ __device__ __forceinline__ uint32_t quantize_block(const float (&v)[16], float g
         lo[i] = __fmaf_rn(v[8 * h + i], r_lo, 0.0f);
         hi[i] = __fmaf_rn(v[8 * h + i], r_hi, 0.0f);
       }
-      const uint32_t w_lo = cvt_e2m1x8(lo), w_hi = cvt_e2m1x8(hi);
+      const uint32_t w_lo = to_e2m1x8(lo), w_hi = to_e2m1x8(hi);
       uint32_t w = w_lo;
       const uint32_t diff = w_lo ^ w_hi;
       if (diff != 0u) {
@@ -236,12 +221,12 @@ __device__ __forceinline__ uint32_t quantize_block_bf16(const uint4 a, const uin
   bf16x2_scaled(a.y, m, q[2], q[3]);
   bf16x2_scaled(a.z, m, q[4], q[5]);
   bf16x2_scaled(a.w, m, q[6], q[7]);
-  out.x = cvt_e2m1x8(q);
+  out.x = to_e2m1x8(q);
   bf16x2_scaled(b.x, m, q[0], q[1]);
   bf16x2_scaled(b.y, m, q[2], q[3]);
   bf16x2_scaled(b.z, m, q[4], q[5]);
   bf16x2_scaled(b.w, m, q[6], q[7]);
-  out.y = cvt_e2m1x8(q);
+  out.y = to_e2m1x8(q);
   return sb;
 }
 
