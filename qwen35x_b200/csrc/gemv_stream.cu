@@ -874,6 +874,7 @@ struct q35b_gemv_batch {
   q35b::WBatch * tensor = nullptr;   // set: the list runs on the tensor path (gemm_wstream.cu), nothing above is used
   std::vector<q35b_gemv_item> chain;  // set: it can run as one launch per item, in this order (gemm_resident.cu)
   bool chained = false;               // it does
+  q35b_gemv_batch * one_launch = nullptr;  // test hook: the same list without a chain, for dependencies that cannot be met
   unsigned int * chain_gave = nullptr;  // of a chain, two words per item: whether its launch gave up (gemm_resident.cu)
   int chain_absent = -1;              // test hook: item whose operand is never complete in every other row block
 };
@@ -1116,7 +1117,32 @@ bool resident_chain(const q35b_gemv_item * items, const std::vector<int> & level
 
 }  // namespace
 
-int gemv_batch_build(const q35b_gemv_item * items, int count, int m, bool share_tiles, q35b_gemv_batch ** out) {
+namespace {
+
+// A list that runs as one launch per item owns a status word and the items' words.
+int build_chain(const q35b_gemv_item * items, int count, int m, q35b_gemv_batch ** out) {
+  auto * b = new q35b_gemv_batch();
+  b->count = count;
+  b->m = m;
+  b->chain.assign(items, items + count);
+  b->chained = true;
+  for (int i = 0; i < count; ++i) b->bytes_per_run += items[i].weight->codes_bytes + items[i].weight->scales_bytes;
+  b->counter_bytes = sizeof(unsigned int) * (4 + 2 * static_cast<size_t>(count));
+  cudaError_t e = cudaMalloc(&b->dev_base, b->counter_bytes);
+  if (e == cudaSuccess) e = cudaMemset(b->dev_base, 0, b->counter_bytes);
+  if (e != cudaSuccess) {
+    cudaFree(b->dev_base);
+    delete b;
+    return fail_cuda(e, "cudaMalloc(projection work list)");
+  }
+  b->status = static_cast<unsigned int *>(b->dev_base);
+  b->chain_gave = b->status + 4;
+  *out = b;
+  return Q35B_OK;
+}
+
+// share_tiles: a caller's list, tiles of which several CTAs may share; chains: which may run as one launch per item.
+int build_list(const q35b_gemv_item * items, int count, int m, bool share_tiles, bool chains, q35b_gemv_batch ** out) {
   if (items == nullptr || out == nullptr || count <= 0) return fail(Q35B_ERR_ARGUMENT, "Invalid NVFP4 projection work list.");
   if (m < 1 || m > 8) return fail(Q35B_ERR_SHAPE, "NVFP4 decode projection supports 1..8 tokens.");
   *out = nullptr;
@@ -1149,6 +1175,12 @@ int gemv_batch_build(const q35b_gemv_item * items, int count, int m, bool share_
     *out = b;
     return Q35B_OK;
   }
+  std::vector<int> level(count, 0);
+  for (int i = 0; i < count; ++i) {
+    if (items[i].after > 0) level[i] = level[items[i].after - 1] + 1;
+  }
+  bool can = false;
+  if (Plan fits_plan; share_tiles && resident_chain(items, level, m, &can) && chains && make_plan(m, max_k, &fits_plan)) return build_chain(items, count, m, out);
   auto * b = new q35b_gemv_batch();
   b->count = count;
   b->m = m;
@@ -1212,13 +1244,7 @@ int gemv_batch_build(const q35b_gemv_item * items, int count, int m, bool share_
     }
     b->bytes_per_run += w->codes_bytes + w->scales_bytes;
   }
-  std::vector<int> level(count, 0);
-  int max_level = 0;
-  for (int i = 0; i < count; ++i) {
-    if (items[i].after > 0) level[i] = level[items[i].after - 1] + 1;
-    max_level = std::max(max_level, level[i]);
-  }
-  const bool callers_list = share_tiles;
+  const int max_level = *std::max_element(level.begin(), level.end());
   const int most = share_tiles ? static_cast<int>(std::min<long>(total_steps, 1 << 20)) : static_cast<int>(all.size());
   auto grid_for = [&](int ksplit) { return std::max(1, std::min(sm_count() * ctas_per_sm(ksplit), most)); };
   int grid = grid_for(b->plan.ksplit);
@@ -1292,11 +1318,15 @@ int gemv_batch_build(const q35b_gemv_item * items, int count, int m, bool share_
     delete b;
     return fail_cuda(e, "uploading the projection work list");
   }
-  bool can = false;
-  b->chained = callers_list && resident_chain(items, level, m, &can);
   if (can) b->chain.assign(items, items + count);
   *out = b;
   return Q35B_OK;
+}
+
+}  // namespace
+
+int gemv_batch_build(const q35b_gemv_item * items, int count, int m, bool share_tiles, q35b_gemv_batch ** out) {
+  return build_list(items, count, m, share_tiles, true, out);
 }
 
 int gemv_batch_build_tensor(const q35b_gemv_item * items, int count, int m, int digits, q35b_gemv_batch ** out) {
@@ -1316,7 +1346,8 @@ int gemv_batch_build_tensor(const q35b_gemv_item * items, int count, int m, int 
 int gemv_batch_launch(const q35b_gemv_batch * b, const void * x_override, void * y_override, cudaStream_t s) {
   if (b == nullptr) return fail(Q35B_ERR_ARGUMENT, "Null NVFP4 projection work list.");
   if (b->tensor != nullptr) return wbatch_launch(b->tensor, s);
-  if (b->chained && b->wait_extra == 0) {
+  if (b->one_launch != nullptr && b->wait_extra != 0) return gemv_batch_launch(b->one_launch, x_override, y_override, s);
+  if (b->chained) {
     for (size_t i = 0; i < b->chain.size(); ++i) {
       const q35b_gemv_item & it = b->chain[i];
       const ResidentChain neighbours = {i + 1 < b->chain.size() ? b->chain[i + 1].weight : nullptr, b->chain_gave + 2 * i,
@@ -1354,6 +1385,7 @@ int gemv_batch_launch(const q35b_gemv_batch * b, const void * x_override, void *
 void gemv_batch_free(q35b_gemv_batch * b) {
   if (b == nullptr) return;
   wbatch_free(b->tensor);
+  gemv_batch_free(b->one_launch);
   if (b->dev_base != nullptr) cudaFree(b->dev_base);
   delete b;
 }
@@ -1362,6 +1394,7 @@ int gemv_batch_read_status(const q35b_gemv_batch * b, unsigned int * out) {
   if (b == nullptr || out == nullptr) return fail(Q35B_ERR_ARGUMENT, "Null NVFP4 projection work list.");
   if (b->tensor != nullptr) return wbatch_status(b->tensor, out);
   Q35B_CUDA_TRY(cudaMemcpy(out, b->status, sizeof(unsigned int), cudaMemcpyDeviceToHost), "cudaMemcpy(work list status)");
+  if (*out == 0u && b->one_launch != nullptr) return gemv_batch_read_status(b->one_launch, out);
   return Q35B_OK;
 }
 
@@ -1370,6 +1403,12 @@ size_t gemv_batch_bytes(const q35b_gemv_batch * b) { return b ? b->bytes_per_run
 int gemv_batch_debug_wait(q35b_gemv_batch * b, unsigned int wait_limit, unsigned int extra_completions) {
   if (b == nullptr || wait_limit == 0) return fail(Q35B_ERR_ARGUMENT, "Invalid NVFP4 projection work list.");
   if (b->tensor != nullptr) return wbatch_debug_wait(b->tensor, wait_limit);
+  if (b->chained && extra_completions != 0 && b->one_launch == nullptr) {
+    if (const int st = build_list(b->chain.data(), b->count, b->m, true, false, &b->one_launch)) return st;
+  }
+  if (b->one_launch != nullptr) {
+    if (const int st = gemv_batch_debug_wait(b->one_launch, wait_limit, extra_completions)) return st;
+  }
   b->wait_limit = wait_limit;
   b->wait_extra = extra_completions;
   // only the recorded code: every run leaves its counters at zero, also one that gave up
