@@ -75,3 +75,22 @@ def test_gate_up(engine, oracle, m, inter, k):
     _, u = oracle.gemm_w4a4(halves[3][rows], halves[4][rows], halves[5], *e, threads=8)
     want = oracle.bf16_to_f32(oracle.bf16_round((g / (1 + np.exp(-g)) * u).astype(np.float32)))
     assert oracle.rel_l2(oracle.bf16_to_f32(got)[:, rows], want) <= REL_L2_TOL
+
+
+@pytest.mark.parametrize("m,n,k", [(1100, 9216, 512), (1111, 9203, 320), (4096, 2560, 1024)])
+def test_residual_in_place(engine, m, n, k):
+    """The output over its residual, several tiles per CTA pair and a ragged last chunk: every box is read before it is written."""
+    import torch
+
+    codes, scales, s2 = _weight(engine, n, k, seed=n)
+    w = engine.Nvfp4Weight.from_device(codes, scales, s2)
+    assert engine.gemm_plan(m, n, k)["pairs"]
+    a = engine.quantize_activations(to_torch_bf16(make_activations(m, k, seed=m)))
+    res = torch.randn((m, (n + 15) // 8 * 8), device="cuda", generator=torch.Generator(device="cuda").manual_seed(m)).to(torch.bfloat16)
+    want = torch.empty_like(res)
+    engine.gemm_w4a4(w, *a, m, out=want[:, :n], residual=res[:, :n])
+    for _ in range(5):
+        both = res.clone()
+        engine.gemm_w4a4(w, *a, m, out=both[:, :n], residual=both[:, :n])
+        assert torch.equal(both[:, :n], want[:, :n]) and torch.equal(both[:, n:], res[:, n:])
+    assert engine.gemm_default_status() == 0

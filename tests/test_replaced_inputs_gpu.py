@@ -127,3 +127,52 @@ def test_prefill_reading_what_the_call_before_wrote(engine, m):
             engine.project_prefill(w1, x, out=between, scratch=s1)
             got.append(engine.project_prefill(w2, between, scratch=s2))
         assert all(_same(torch, a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("m,hidden,inter", [(1, 1024, 3584), (2, 2560, 9216), (4, 512, 4096)])
+def test_decode_chain(engine, m, hidden, inter):
+    """One launch per item, each started under the one before it: what the second one reads has the same address in every run, and
+    none of it may be left from the run before."""
+    import torch
+
+    up, down = _weight(engine, torch, inter, hidden, 1), _weight(engine, torch, hidden, inter, 2)
+    x, h, y = (torch.empty((m, n), dtype=torch.bfloat16, device="cuda") for n in (hidden, inter, hidden))
+    res = torch.zeros((m, hidden), dtype=torch.bfloat16, device="cuda")
+    batch = engine.GemvBatch([(up, x, h), (down, h, y, res, 0)], m)
+    before = engine.launch_count()
+    batch.run()
+    assert engine.launch_count() - before == 2
+    versions, residuals = _versions(torch, m, hidden, m), _versions(torch, m, hidden, m + 10)
+    want = []
+    for v, r in zip(versions, residuals):
+        x.copy_(v)
+        res.copy_(r)
+        torch.cuda.synchronize()
+        batch.run()
+        torch.cuda.synchronize()
+        want.append((h.clone(), y.clone()))
+        plain = engine.gemv_w4a16(up, v, kernel=engine.GEMV_SIMT)
+        assert _same(torch, want[-1][0].isfinite(), plain.isfinite())
+        kept, ref = want[-1][0].nan_to_num(0.0, 0.0, 0.0).double(), plain.nan_to_num(0.0, 0.0, 0.0).double()
+        assert float((kept - ref).norm()) <= 1e-3 * float(ref.norm())  # both fp32 sums: flipped roundings, a few in 10^4
+    for _ in range(10):
+        got = []
+        torch.cuda.synchronize()
+        for v, r in zip(versions, residuals):
+            x.copy_(v)
+            res.copy_(r)
+            batch.run()
+            got.append((h.clone(), y.clone()))
+        assert all(_same(torch, a, b) for g, w in zip(got, want) for a, b in zip(g, w))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):  # run behind run, with nothing but the copies between
+        got = []
+        for v, r in zip(versions, residuals):
+            x.copy_(v)
+            res.copy_(r)
+            batch.run()
+            got.append((h.clone(), y.clone()))
+    for _ in range(3):
+        graph.replay()
+    torch.cuda.synchronize()
+    assert all(_same(torch, a, b) for g, w in zip(got, want) for a, b in zip(g, w)) and batch.status() == 0
