@@ -650,7 +650,8 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
         }
       };
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
-      const int n_cols = OP == kDigits && s_deep == 0u ? a.cols_plain : a.cols_deep;
+      const uint32_t deep = OP == kDigits ? s_deep : 1u;
+      const int n_cols = deep == 0u ? a.cols_plain : a.cols_deep;
       const int mmas = min(steps * kMmaPerStage, sf_col_blocks - ks0 * kMmaPerStage);
       const int parts = min(partial_accumulators(n_cols), mmas);  // accumulators that were written
       if constexpr (OP == kDigits) {
@@ -661,7 +662,7 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
           int count = 8;
           const uint32_t best = s_top[token];
 #pragma unroll 1
-          for (bool again = s_deep != 0u;; again = false) {
+          for (bool again = deep != 0u;; again = false) {
             uint32_t r[4][8] = {};
             tmem_ld8(col, r[0]);  // what lies behind the deep digits is not used
             if (parts > 1) tmem_ld8(col + n_cols, r[1]);
@@ -684,7 +685,7 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
           const float s2 = a.gate_up != 0 && (tile_row & 8) != 0 ? a.s2_up : a.s2;
           const int top = max(static_cast<int>(best >> 7), 1);
           float v = sum * s2 * digits_scale(top);
-          if ((top > kTopUnderflows || (s_deep >> token & 256u) != 0u) && ran) {
+          if ((top > kTopUnderflows || (deep >> token & 256u) != 0u) && ran) {
             const __nv_bfloat16 * x = static_cast<const __nv_bfloat16 *>(a.x) + static_cast<size_t>(token) * a.k;
             const int k0 = ks0 * 256, k1 = min((ks0 + steps) * 256, a.k), row = rb * kRows + tile_row;
             if (best < 0x7f80u) {
