@@ -438,3 +438,35 @@ def test_prefill_whose_output_lies_over_its_activations(engine, m, n, k, at):
         assert engine.launch_count() - before == 2
         assert torch.equal(got, want)
     assert engine.gemm_default_status() == 0
+
+
+CAPTURED = """
+import torch
+import qwen35x_b200 as q
+torch.manual_seed(0)
+w = q.Nvfp4Weight.from_device(*q.quantize_weight(torch.randn((2560, 4160), device="cuda")))
+xs = [torch.randn((m, 4160), device="cuda").to(torch.bfloat16) for m in (1, 4, 8)]
+outs = [torch.empty((x.shape[0], 2560), dtype=torch.bfloat16, device="cuda") for x in xs]
+torch.cuda.synchronize()
+stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+with torch.cuda.stream(stream):
+    with torch.cuda.graph(graph, stream=stream):
+        for x, out in zip(xs, outs):
+            q.gemv_w4a16(w, x, out=out)
+    graph.replay()
+    stream.synchronize()
+    for x, out in zip(xs, outs):
+        assert torch.equal(out, q.gemv_w4a16(w, x))
+        assert float((out.double() - q.gemv_w4a16(w, x, kernel=q.GEMV_SIMT).double()).norm()) <= 1e-3 * float(out.double().norm())
+assert q.gemm_default_status() == 0
+"""
+
+
+def test_the_first_single_projection_of_a_process_inside_a_capture():
+    """The rule asks the runtime how many clusters fit, once per shape: also under capture."""
+    import subprocess
+    import sys
+    from pathlib import Path
+
+    r = subprocess.run([sys.executable, "-c", CAPTURED], cwd=Path(__file__).resolve().parent.parent, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
