@@ -415,7 +415,7 @@ gemm_w4a4_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             }
           }
           if (turn == 0) {
-            ok = mbar_wait(smem_u32(tmem_full), li & 1);
+            ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(tmem_full), li & 1));  // the whole warp goes on, or none of it
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           }
@@ -473,7 +473,7 @@ gemm_w4a4_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         // plain BF16 output of a gathering launch: store locally, then forward whole rows, whose chunks are neighbours then;
         // the fused epilogues (and a launch without peers) store per lane
         const bool forward = ep.n_peers > 0 && !ep.gate_up && ep.forward_rows != 0;
-        ok = mbar_wait(smem_u32(tmem_full), li & 1);
+        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(tmem_full), li & 1));
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1

@@ -419,7 +419,7 @@ gemm_w4a4_ksplit_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
 
   // ---------------- epilogue: TMEM -> shared memory -> sum over the cluster -> global ----------------
   bool ran = !aborted;
-  if (ran && !mbar_wait(smem_u32(acc_full), 0)) {
+  if (ran && !__all_sync(0xffffffffu, mbar_wait(smem_u32(acc_full), 0))) {  // the whole warp goes on, or none of it
     if (lane == 0) {
       atomicExch(status, kStatusEpilogueWait);
       s_stop = 1u;

@@ -495,7 +495,7 @@ gemm_wstream_kernel(const WItem * __restrict__ items, const WTile * __restrict__
         }
         deep_tokens = __ballot_sync(0xffffffffu, any != 0u);
       }
-      if (!mbar_wait(smem_u32(tmem_full + ab), (ti >> 1) & 1, wait_limit)) {
+      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(tmem_full + ab), (ti >> 1) & 1, wait_limit))) {  // the whole warp goes on, or none of it
         if (lane == 0) {
           atomicExch(status, kEpilogueWait);
           gave_up = 1;
